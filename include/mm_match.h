@@ -175,8 +175,8 @@ mm_status mm_match_drawn(mm_graph *g, int type, uint32_t barrier, uint32_t (*dra
  *                          is at most 1/value of round 0's; default 12 (24 for
  *                          mm_match_policy, whose retirement shrinks the active
  *                          set sooner), at least 2, -1 never
- *   MM_TUNE_BLOCKS_PER_SM  blocks of 512 threads per multiprocessor for the round
- *                          and finish kernels; default all that fit (2)
+ *   MM_TUNE_BLOCKS_PER_SM  blocks of 512 threads per multiprocessor, at most;
+ *                          default all that fit (2)
  */
 enum { MM_TUNE_FINISH_DIV = 1, MM_TUNE_BLOCKS_PER_SM = 2 };
 mm_status mm_graph_tune(mm_graph *g, int key, int value);
@@ -195,20 +195,17 @@ mm_status mm_match_stats(mm_graph *g, int type, uint32_t barrier, const uint32_t
                          int stats_rounds, int path, void *stream);
 
 /*
- * Measurement entry: the same launches as mm_match_device, with timestamps
- * taken by the kernels as their grid barriers complete (the device's global
+ * Measurement entry: the same launch as mm_match_device, with timestamps
+ * taken by the kernel as its grid barriers complete (the device's global
  * timer, nanoseconds).
  * ms_per_kernel[r * MM_PROFILE_KERNELS + k] receives, for each round r <
  * cap_rounds that the kernel executed, k = 0 the window scan (blue vertices'
  * preference windows and proposals), k = 1 the fallback scan of lists longer
  * than their window (0 in rounds without one), k = 2 the commit phase
  * (commit, recolour, worklist compaction), k = 3 their sum; rows of rounds
- * not executed are zero; the finish kernel's work is reported in the row of
+ * not executed are zero; the finish phase's work is reported in the row of
  * the round it took over at, its scan pass as k = 0 and the rest as k = 1.
- * *launches receives the number of kernels launched: 3 on the symmetric path
- * (contiguous sorted lists, every entry with a reverse entry of the same
- * weight): the round kernel, the finish kernel and the round kernel again,
- * each returning at once when nothing is left for it; else 1.  Same matching
+ * *launches receives the number of kernels launched (1).  Same matching
  * result.
  */
 #define MM_PROFILE_KERNELS 4
@@ -333,10 +330,9 @@ mm_status mm_probe_gather_rate(int device, long long table_bytes, double *gather
  * Testing hook, no counterpart in the reference: lets tests drive the library's
  * failure handling without any GPU fault.  Process-wide; not for production
  * use.  *out (may be NULL) receives the previous value, or the queried one.
- *   MM_DEBUG_SPIN_LIMIT    polls a grid-barrier wait of the round and finish
- *                          kernels makes before giving up (0: the default,
- *                          2^22); a wait that gives up makes the call return
- *                          MM_ERR_DEVICE
+ *   MM_DEBUG_SPIN_LIMIT    polls a grid-barrier wait of the round kernel makes
+ *                          before giving up (0: the default, 2^22); a wait
+ *                          that gives up makes the call return MM_ERR_DEVICE
  *   MM_DEBUG_SKIP_BARRIER  mark of a grid barrier at which block 0 does not
  *                          arrive, so every wait on it runs out (-1: none);
  *                          marks: 0 after set-up, 3r + 1 after round r's

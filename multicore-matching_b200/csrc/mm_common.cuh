@@ -103,7 +103,7 @@ struct mm_graph {
     unsigned long long *d_revkey[2] = {nullptr, nullptr};  // [0] random, [1] weighted
     long long *d_slot_off = nullptr;  // non-contiguous CSR: slot index of vertex v's first entry
     int2 *d_pwin = nullptr;           // weighted types: preference windows {neighbour, position | flag}
-    long long *d_pwin_off = nullptr;  // weighted types: first window slot of each vertex; [n] = total
+    int *d_pwin_off = nullptr;        // weighted types, [n + 1]: first window slot (even), bit 0: list longer than 32
     bool pwin_weights = false;        // d_pwin's second words hold weights (symmetric weighted path)
     int2 *win_build = nullptr;        // windows while being built (d_pwin once complete)
     int *win_big = nullptr;           // while being built: queued lists longer than a window chunk

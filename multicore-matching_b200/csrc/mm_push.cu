@@ -25,9 +25,11 @@
 //     unmatched neighbour; readers of that colour byte see "unmatched, not red"
 //     either way, so their outcome is unchanged.
 //
-// Work layout.  Vertices that can still be matched sit in worklists; an item
-// carries the vertex, its neighbour range and its window offset, so the scans
-// never read neighbourRanges again.
+// Work layout.  Every vertex belongs to one block for the whole matching: the
+// vertices are dealt to the blocks in chunks of 64, and a block keeps the ones
+// that can still be matched in lists of its own (4 bytes an item: the vertex).
+// So no counter, list or request is shared between blocks: all that crosses
+// them are the colour bytes, the proposals' atomic maxima and the barriers.
 //   windows        a blue vertex's choice is the first red candidate among its
 //                  best min(deg, 32) entries in order of preference (weight,
 //                  then position; list order for random types), stored at
@@ -35,24 +37,28 @@
 //                  window entries a step, refilled from a prefetched item as
 //                  soon as its vertex is decided (scan_window).
 //   fallback       a list longer than its window with no red candidate in it
-//                  is appended to the round's fallback list; that entry space
-//                  is cut into 256-entry segments and a warp walks one segment
-//                  in coalesced rows of 32 (scan_long).  A list cut by segment
-//                  edges is combined by atomics and its last piece proposes.
+//                  is scanned whole, by a warp or by the block that owns it;
+//                  the longest lists (hubs) go to a list of the round that all
+//                  blocks share, cut into 256-entry segments (scan_long).
 //   finish phase   once the active set is small its components are tiny, and
-//                  a second cooperative kernel plays the remaining rounds of
-//                  each component on its own (k_finish), with no grid barrier.
+//                  the remaining rounds of each component are played on their
+//                  own, with two more grid barriers in all (finish_scan,
+//                  finish_roots).
 // A list's best entry is kept as a 64-bit key (weight order << 32 | ~position),
 // which orders ties by position exactly as the reference's strict ">" scan in
 // list order does.
 //
-// Loop.  k_rounds is launched cooperatively (all blocks resident) and runs
-// set-up, then per round the window scan (A1), the fallback scan (A2, only in
-// rounds that have fallback lists) and the commit phase (B: commit + recolour
-// + worklist compaction), with bounded grid barriers in between, until it
-// hands over to the finish kernel.  Nothing returns to the host until the
+// Loop.  k_match is launched cooperatively (all blocks resident) and runs
+// set-up, then per round the window scan (A1, with the owner's fallback
+// scans), the shared fallback scan (A2, only in rounds that have such lists)
+// and the commit phase (B: commit + recolour + worklist compaction), with
+// bounded grid barriers in between.  A barrier carries a sum (the vertices
+// still active, the blocks with shared fallback lists), so nothing else has to
+// be read to decide what comes next.  A graph that fits one block runs
+// without grid barriers at all.  Nothing returns to the host until the
 // matching is maximal (the reference copies a flag back every round,
-// matchgpu.cu:607-614), and no round pays for kernel launches.
+// matchgpu.cu:607-614): the call is one launch, its arguments (seeds among
+// them) travel as launch parameters and its result is written to host memory.
 #include <cuda_runtime.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
@@ -71,65 +77,72 @@ constexpr int kThreads = 512;            // threads per block of the round kerne
 constexpr int kWarps = kThreads / 32;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWin = 32;                 // preference window: the first min(deg, 32) choices
-constexpr int kReqFallback = -3;         // reqi: the item's list went to the fallback scan
+constexpr int kChunk = 64;               // vertices dealt to the blocks at a time
 constexpr int kSegEntries = 256;         // entries per fallback segment: 8 rows of 32; at most 9
                                          // pieces of lists > 32 entries overlap one segment
 
-// Worklists: blue and red vertices by round parity; the staged list holds the round's
-// fallback lists (blue lists longer than the window with no red choice in
-// it) with their offsets in the concatenated fallback entry space.
-enum : int { kBlue = 0, kRed = 1, kParityLists = 2 };
+// Request codes of a blue item (a target vertex otherwise).
+enum : int { kReqDead = -1, kReqNone = -2, kReqShared = -3 };
 
+// Control block of one call, zero at launch.  A graph has two, used by
+// alternate calls: each call clears the other one, so no call pays for a
+// memory operation ahead of its launch.
+constexpr int kRing = 4;        // barrier words in use by turns
+constexpr int kRingStride = 16; // words of 8 bytes per barrier line (128 bytes)
 struct Ctl {
-    int *match;            // output array of this call
-    uint32_t barrier;
-    int cap;               // 20 or 255
-    int maximal;
-    int nseeds;
-    int rounds;            // rounds the reference executes (set at loop exit)
-    int status;            // 0 ok, 1 seeds exhausted, 2 a bounded grid-barrier wait gave up
-    int cnt[2][kParityLists];      // worklist lengths by round parity
-    unsigned long long staged_pack;  // fallback list of the round: (items << 32) | entries
-    int retired[2];        // vertices of the round that were unmatchable as soon as coloured
+    unsigned long long ring[kRing * kRingStride];  // (sum << 32) | blocks arrived
+    unsigned long long staged_pack;  // shared fallback list of the round: (items << 32) | entries
     int fin_abort;         // finish phase: t + 1 if the attempt in round t was called off
     int fin_last;          // finish phase: last round in which any of its vertices was active
-    int fin_round;         // finish phase: the round it starts at (set by k_rounds)
-    int fin_state;         // finish phase: kFinState*
-    long long active0;     // vertices active at round 0 (for a resumed round kernel)
     int iso_last;          // 1 + the last round in which a vertex without neighbours was active (0: none)
+    int pad;
 };
 
-// Finish-phase hand-over between the launches of one matching.
-enum : int { kFinStateNone = 0, kFinStatePending = 1, kFinStateDone = 2, kFinStateResume = 3 };
+// What a call returns, in page-locked host memory that the kernel writes.
+struct Result {
+    int rounds;            // rounds the reference executes (-1: the kernel did not end its loop)
+    int status;            // 0 ok, 1 seeds exhausted, 2 a bounded grid-barrier wait gave up
+};
 
 struct Params {
     int n;
     int contiguous;
     int sym;                        // proposal keys computed from the proposer's entry (no reverse index)
+    int region;                     // list slots of a block
     const int2 *ranges;
     const int *nbrs;
     const float *w;
     const unsigned long long *revkey;
     const long long *slot_off;
-    const int2 *pwin;               // weighted: preference windows {neighbour, position | flag or weight}
-    int wwin;                       // pwin's second words are weights (symmetric weighted path)
-    const long long *pwin_off;      // weighted: first window slot of each vertex (< 2^31)
+    // weighted: preference windows, {neighbour, weight} on the symmetric path,
+    // else {neighbour, position | flag}; an odd window ends with a filler
+    // {-1, flag}
+    const int2 *pwin;
+    const int *pwin_off;            // weighted, [n + 1]: first window slot (even), bit 0: list longer than the window
     uint8_t *col;
-    int2 *req;                      // per vertex: proposal of a fallback list (and the finish phase's item map)
-    int2 *reqi;                     // per blue item of the round: {target, key low half}, -1 unmatchable,
-                                    // -2 no proposal, kReqFallback: look in req
+    int2 *req;                      // per vertex: proposal of a shared fallback list {target or code, key low half};
+                                    // finish phase: a vertex's record
+    int *lists[2];                  // items (vertices) by round parity: block b's region starts at b * region,
+                                    // blue items from its front, red items from its back
+    int *prop;                      // per blue item: target or code
+    uint32_t *prop_key;             // per blue item, off the symmetric path: the proposal key's low half
     unsigned long long *best;       // per red vertex: max proposal key this round
     unsigned long long *part_key;   // per cut fallback list: max over finished pieces
     int *part_cnt;                  // per cut fallback list: finished pieces
-    int4 *lists[2][kParityLists];   // items {v, begin, end, window offset} by parity and colour
-    int4 *staged;                   // fallback items {v, begin, end, entry offset}
+    int4 *staged;                   // shared fallback items {v, begin, end, entry offset}
     int *seg_first;                 // per fallback segment: item holding its first entry
-    const uint32_t *seeds;
+    int4 *rec;                      // finish phase: records (3 int4 an item), rec_region of them for a block
+    int rec_region;
+    int *match;                     // output array of this call
+    uint32_t barrier;
+    int cap;                        // 20 or 255
+    int maximal;
+    int nseeds;
     Ctl *ctl;
+    Ctl *ctl_next;                  // the next call's control block, cleared by this call
+    Result *result;                 // host memory
     unsigned long long *stats;      // [kMaxRounds][MM_STATS_COLS] or null
     unsigned long long *tstamp;     // [3 * kMaxRounds + 1] barrier times (ns) or null
-    unsigned *bar;                  // [kBarWords] grid barrier words, zero at launch
-    int resume;                     // round kernel: continue from ctl->fin_round (finish called off)
     int zero_parts;                 // set-up clears part_key and part_cnt (not known to be zero)
     int fin_div;                    // finish phase from the round whose active set is <= 1/fin_div of round 0's (0: never)
     // testing hooks (mm_debug): polls before a barrier wait gives up, and the
@@ -140,10 +153,11 @@ struct Params {
     // vertex's graph starts at vbase[v], and the graph's own numbering (v -
     // vbase[v]) drives the colouring and the match values, so every graph gets
     // the matching a call on it alone would give.  last[v] is the last round
-    // at whose colouring v was still unmatched.  Both null for one graph.
+    // at whose colouring v was still unmatched, written once, when v leaves.
+    // Both null for one graph.
     const int *vbase;
     uint8_t *last;
-    // Learned colouring (k_rounds<..., kPolicy>): blue iff hash < p_v * 2^32 with
+    // Learned colouring (k_match<..., kPolicy>): blue iff hash < p_v * 2^32 with
     // p_v from a per-vertex MLP over local features.  wfeat[v]: (max, mean)
     // incident weight; trace: per round and vertex, the features, colour and
     // outcome (for training), or null.
@@ -151,10 +165,6 @@ struct Params {
     const float2 *wfeat;
     float *trace;
     int trace_rounds;
-    // The policy's weights travel by value in the launch parameters: every
-    // thread reads the same one, so the unrolled MLP takes them straight from
-    // the constant bank as operands, with no load instruction per weight.
-    float mlp[MM_POLICY_FLOATS];
     // A policy whose output weights are all zero ignores the features: its
     // threshold, computed once on the host, is policy_bar (policy_const = 1).
     int policy_const;
@@ -162,26 +172,19 @@ struct Params {
     // Learned colouring with a constant policy: the finish phase plays the
     // remaining rounds under the policy's threshold and its retirement rule.
     int fin_retire;
+    // The policy's weights and the colouring seeds travel by value in the
+    // launch parameters: every thread reads the same one, so they come straight
+    // from the constant bank, and no copy precedes the launch.
+    float mlp[MM_POLICY_FLOATS];
+    uint32_t seeds[256];
 };
 static_assert(sizeof(Params) <= 4096, "launch parameters stay within the classic 4 KB limit");
 
-template <class P>
-__device__ __forceinline__ int base_of(const P &p, int v) { return p.vbase ? __ldg(p.vbase + v) : 0; }
+__device__ __forceinline__ int base_of(const Params &p, int v) { return p.vbase ? __ldg(p.vbase + v) : 0; }
 
 __device__ __forceinline__ int degree_of(int2 r) { return r.y > r.x ? r.y - r.x : 0; }
 __device__ __forceinline__ int degree_of(int4 it) { return it.z > it.y ? it.z - it.y : 0; }
 __device__ __forceinline__ int win_len(int deg) { return deg < kWin ? deg : kWin; }
-
-__device__ __forceinline__ int warp_incl_scan(int v)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(kFull, v, o);
-        if (lane >= o) v += y;
-    }
-    return v;
-}
 
 template <class P>
 __device__ __forceinline__ void stat_add(const P &p, int round, int col, unsigned long long v)
@@ -191,34 +194,18 @@ __device__ __forceinline__ void stat_add(const P &p, int round, int col, unsigne
     if ((threadIdx.x & 31) == 0 && v) atomicAdd(&p.stats[(size_t)round * MM_STATS_COLS + col], v);
 }
 
-// ---- grid barrier ----
-//
-// The round kernel is launched cooperatively, so all its blocks are resident
-// at once and a barrier over them cannot deadlock on scheduling.  Blocks
-// arrive in groups of kBarGroup on their group's word, and the last of each
-// group arrives on the top word, which every block polls; each word sits in
-// its own 128-byte line, so no word sees more than kBarGroup (or group-count)
-// atomics per barrier.  Every word uses the same counting: the first member
-// adds 2^31 - (members - 1), every other member adds 1, so the top bit flips
-// exactly when the last member arrives and the low bits return to where they
-// were.  Each wait is still bounded: after kSpinLimitDefault polls (a testing
-// hook, mm_debug, can set fewer) the block records
-// status 2 and the kernel returns; the other blocks then give up at their next
-// barrier.  Thread 0's fences (release before arriving, acquire after the
-// wait), with the block barriers around them, make every block's writes of
-// the phase visible to every thread of every block afterwards.
-constexpr int kBarGroup = 16;
-constexpr int kBarStride = 32;   // words per barrier line (128 bytes)
-constexpr int kBarMaxGroups = 64;
-constexpr int kBarWords = (kBarMaxGroups + 1) * kBarStride;  // group words, then the top word
-
-__device__ __forceinline__ unsigned ld_acquire(const unsigned *p)
+// The vertex at slot k of this block's share, or -1: chunk q of block b is
+// chunk q * gridDim.x + (b + 61 q) % gridDim.x of the vertex range.  The turn
+// by 61 keeps a block off one residue: ids cluster by degree (R-MAT hubs have
+// ids with low bits zero), and a plain stride of a multiple of 8 blocks would
+// give every eighth block the hubs.
+__device__ __forceinline__ int own_vertex(const Params &p, int k)
 {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
+    const unsigned nb = gridDim.x, q = (unsigned)k / kChunk;
+    const unsigned c = q * nb + (blockIdx.x + 61u * q) % nb;
+    const unsigned v = c * kChunk + (unsigned)k % kChunk;
+    return v < (unsigned)p.n ? (int)v : -1;
 }
-__device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 
 __device__ __forceinline__ unsigned long long global_ns()
 {
@@ -226,47 +213,6 @@ __device__ __forceinline__ unsigned long long global_ns()
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-
-__device__ __noinline__ bool grid_sync(unsigned *bar, Ctl *ctl, unsigned long long *tstamp, int mark,
-                                       long long spin_limit, int skip_mark)
-{
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const unsigned nb = gridDim.x, b = blockIdx.x;
-        const unsigned g = b / kBarGroup, ngroups = (nb + kBarGroup - 1) / kBarGroup;
-        const unsigned gsize = min((unsigned)kBarGroup, nb - g * kBarGroup);
-        unsigned *gword = bar + g * kBarStride;
-        unsigned *top = bar + kBarMaxGroups * kBarStride;
-        const unsigned top_before = ld_acquire(top);  // cannot flip before this block arrives
-        fence_acq_rel();
-        // testing hook: block 0 leaves this barrier out, so every wait on it runs out
-        if (!(b == 0 && mark >= 0 && mark == skip_mark)) {
-            const unsigned ginc = b % kBarGroup == 0 ? 0x80000000u - (gsize - 1u) : 1u;
-            const unsigned gold = atomicAdd(gword, ginc);
-            if (((gold + ginc) ^ gold) & 0x80000000u) {  // last of the group
-                const unsigned tinc = g == 0 ? 0x80000000u - (ngroups - 1u) : 1u;
-                atomicAdd(top, tinc);
-            }
-        }
-        int ok = 1;
-        long long it = 0;
-        while (((top_before ^ ld_acquire(top)) & 0x80000000u) == 0u) {
-            if (++it > spin_limit) {
-                ok = 0;
-                break;
-            }
-            if (it > 64) __nanosleep(32);
-        }
-        fence_acq_rel();
-        if (!ok) atomicExch(&ctl->status, 2);
-        s_ok = ok;
-        if (tstamp && b == 0 && mark >= 0) tstamp[mark] = global_ns();
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
 
 // L2 residency: the colour bytes, which every scan reads at random, are loaded
 // with an evict-last policy, the streamed worklists and requests with
@@ -306,14 +252,6 @@ __device__ __forceinline__ unsigned long long cand_key(int j, float w)
     return (unsigned long long)(uint32_t)~j;
 }
 
-// Scan result of one adjacency entry with neighbour colour c.
-template <bool kW>
-__device__ __forceinline__ unsigned long long entry_key(uint8_t c, int j, float w)
-{
-    if (c == kRed) return cand_key<kW>(j, w);
-    return c == kMatched ? 0ull : 1ull;
-}
-
 // Key of a scan's best entry: weight order and position of its best red
 // neighbour (the reference's rule: strict > from -1 in list order), else 1 if
 // an unmatched neighbour was seen, else 0.
@@ -341,10 +279,27 @@ __device__ __forceinline__ void fold_entry(uint8_t c, float w, int j, float &bw,
     }
 }
 
+// Where a blue vertex's request goes: the item's slot, or (shared fallback
+// lists) the vertex's own word.
+struct ItemReq {
+    const Params &p;
+    long long slot;
+    __device__ __forceinline__ void put(int target, uint32_t low) const
+    {
+        __stcs(p.prop + slot, target);
+        if (!p.sym) __stcs(p.prop_key + slot, low);
+    }
+};
+struct VertexReq {
+    const Params &p;
+    int v;
+    __device__ __forceinline__ void put(int target, uint32_t low) const { __stcs(p.req + v, make_int2(target, (int)low)); }
+};
+
 // Blue vertex v proposes to `target`, the neighbour at position j of its list
 // (begin = first position): the reverse key of that slot goes to best[target].
-template <bool kW>
-__device__ __forceinline__ void propose_to(const Params &p, int2 *rq, int v, int begin, int j, int target)
+template <bool kW, class Req>
+__device__ __forceinline__ void propose_to(const Params &p, Req rq, int v, int begin, int j, int target)
 {
     unsigned long long rk;
     if (p.sym) {
@@ -361,42 +316,33 @@ __device__ __forceinline__ void propose_to(const Params &p, int2 *rq, int v, int
         rk = __ldg(p.revkey + slot);
     }
     if (rk) atomicMax(&p.best[target], rk);
-    __stcs(rq, make_int2(target, (int)(uint32_t)rk));
+    rq.put(target, (uint32_t)rk);
 }
 
-// Symmetric weighted path, windows carrying weights: blue v proposes to
-// `target` through an entry of weight w (w > -1); the target's entry for v has
-// the same weight, and v's id breaks ties (smaller first).
-__device__ __forceinline__ void propose_weight(const Params &p, int2 *rq, int v, float w, int target)
+// Symmetric weighted path: blue v proposes to `target` through an entry of
+// weight w (w > -1); the target's entry for v has the same weight, and v's id
+// breaks ties (smaller first).
+template <class Req>
+__device__ __forceinline__ void propose_weight(const Params &p, Req rq, int v, float w, int target)
 {
     const unsigned long long rk = ((unsigned long long)weight_order(w) << 32) | (uint32_t)~v;
     atomicMax(&p.best[target], rk);
-    __stcs(rq, make_int2(target, (int)(uint32_t)rk));
+    rq.put(target, (uint32_t)rk);
 }
 
 // Blue vertex v without a red choice: unmatchable if no neighbour is
 // unmatched (requests == n + 1), else no proposal this round.
-__device__ __forceinline__ void no_proposal(const Params &p, int2 *rq, int v, bool alive)
+template <class Req>
+__device__ __forceinline__ void no_proposal(const Params &p, Req rq, int v, bool alive, int t)
 {
     if (!alive) {
         p.col[v] = kDead;
-        p.ctl->match[v] = 2;
-        __stcs(rq, make_int2(-1, 0));
+        p.match[v] = 2;
+        if (p.last) p.last[v] = (uint8_t)t;
+        rq.put(kReqDead, 0u);
     } else {
-        __stcs(rq, make_int2(-2, 0));
+        rq.put(kReqNone, 0u);
     }
-}
-
-// Finish blue vertex v after a full scan whose result is `key`.
-template <bool kW>
-__device__ __forceinline__ void propose(const Params &p, int v, int begin, unsigned long long key)
-{
-    if (key < 2) {
-        no_proposal(p, p.req + v, v, key == 1);
-        return;
-    }
-    const int j = (int)~(uint32_t)key;
-    propose_to<kW>(p, p.req + v, v, begin, j, __ldg(p.nbrs + j));
 }
 
 // Adjacency entries the reference's request loop inspects for this vertex
@@ -408,43 +354,151 @@ __device__ __forceinline__ unsigned long long request_seen(int begin, int deg, i
     return (unsigned long long)(j - begin + 1);
 }
 
-template <bool kW, bool kStats>
-__device__ __forceinline__ void propose_counted(const Params &p, int4 it, unsigned long long key, int t)
+// Finish blue vertex v (entries from `begin`, deg of them) after a full scan whose result is `key`.
+template <bool kW, bool kStats, class Req>
+__device__ __forceinline__ void propose_key(const Params &p, Req rq, int v, int begin, int deg, unsigned long long key,
+                                            int t)
 {
     if (kStats) {
         const int j = key >= 2 ? (int)~(uint32_t)key : -1;
-        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_REQ_ENTRIES], request_seen<kW>(it.y, degree_of(it), j));
-        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_BLUE_DEG], (unsigned long long)degree_of(it));
+        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_REQ_ENTRIES], request_seen<kW>(begin, deg, j));
+        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_BLUE_DEG], (unsigned long long)deg);
     }
-    propose<kW>(p, it.x, it.y, key);
+    if (key < 2) {
+        no_proposal(p, rq, v, key == 1, t);
+        return;
+    }
+    const int j = (int)~(uint32_t)key;
+    propose_to<kW>(p, rq, v, begin, j, __ldg(p.nbrs + j));
 }
 
-constexpr int kRows = 4;    // fallback scan: rows of 32 entries per iteration
-constexpr int kStages = 3;  // fallback scan: iterations staged in shared memory (2 loading, 1 in use)
+constexpr int kRows = 4;    // fallback scans: rows of 32 entries per iteration
+constexpr int kStages = 3;  // shared fallback scan: iterations staged in shared memory (2 loading, 1 in use)
 
-// Fallback-scan staging of one warp: neighbour ids and weights of kStages
+// Shared-fallback staging of one warp: neighbour ids and weights of kStages
 // iterations, written by cp.async.
 struct LongStage {
     int nb[kStages][kRows * 32];
     float w[kStages][kRows * 32];
 };
 
-// Shared memory of the round kernel (dynamic).
-struct Smem {
-    int delta[kWarps][33];                // fallback scan: global position of segment entry e = e + delta[k]
-    int pend[kWarps][33];                 // fallback scan: segment-relative end of each piece
+// Window scan: the block's lists that go to a fallback scan.
+constexpr int kStageCap = 4096;
+struct FallbackStage {
+    int2 item[kStageCap];          // {vertex, list slot}
+    unsigned short big[kStageCap]; // the ones the whole block scans
+};
+
+// Set-up: queue of vertices without neighbours (two halves).
+constexpr int kIsoHalf = 6144;
+struct IsoQueue {
+    int half[2][kIsoHalf];
+};
+
+struct LongScan {
+    int delta[kWarps][33];                // global position of segment entry e = e + delta[k]
+    int pend[kWarps][33];                 // segment-relative end of each piece
     LongStage stage[kWarps];
-    int tile_warp[kWarps][2];             // compaction: per-warp counts, then offsets
-    int tile_base[2];                     // compaction: tile bases
-    uint32_t seeds[256];                  // the call's colouring seeds (finish phase)
-    int wnext;                            // window scan: next item of the block's share
+};
+
+// ---- finish phase: a warp's component ----
+constexpr int kFinMembers = 32;    // members of a component played by one warp (one per lane)
+constexpr int kFinEntries = 128;   // entries between members of one component
+
+// One warp's component: members' first entry, list start and degree, the
+// entries between members (preference key and the target's member slot), the
+// members' colours of the round being played and the best proposal each
+// received.
+struct FinWarp {
+    unsigned long long pref[kFinEntries];
+    unsigned long long best[kFinMembers];
+    int mem[kFinMembers];
+    int eoff[kFinMembers + 1];
+    int mbeg[kFinMembers];
+    int mdeg[kFinMembers];
+    uint8_t tgt[kFinEntries];
+    uint8_t st[kFinMembers];
+};
+
+// Shared memory of the round kernel (dynamic); the phases' working areas share it.
+struct Smem {
+    union {
+        IsoQueue iso;
+        FallbackStage fb;
+        LongScan ls;
+        FinWarp fin[kWarps];
+    };
+    unsigned tile_cnt[2][kWarps];         // compaction: per-warp counts, (red << 16) | blue, by tile parity
+    unsigned long long red_key[kWarps];   // block-wide list scan: the warps' best keys
+    unsigned sync_sum;                    // grid barrier: the sum it carried
+    int sync_ok;
+    int wnext;                            // window scan: next item of the block
     int iso_n;                            // set-up: queued vertices without neighbours
     int iso_cnt[3];                       // set-up: survivors of a round of the queue (rotating)
     int stage_n;                          // window scan: fallback lists collected by the block
+    int big_n;                            // window scan: of those, lists for the whole block
+    int big_next;
+    int shared_n;                         // window scan: lists appended to the shared list
 };
+static_assert(sizeof(Smem) <= 56 * 1024, "two blocks per multiprocessor, with room for L1");
 
-// window scan: fallback lists a block collects in its (then unused) staging area
-constexpr int kStageCap = (int)(sizeof(LongStage) * kWarps / sizeof(int4));
+// ---- grid barrier ----
+//
+// The kernel is launched cooperatively, so all its blocks are resident at once
+// and a barrier over them cannot deadlock on scheduling.  Each block adds
+// (its summand << 32) | 1 to the barrier's word and polls until all blocks
+// have: one release-add and one round trip after the last arrival (2500
+// cycles over 148 blocks, where a two-level tree of counters took 3800), and
+// the sum of the summands comes with it.  The words are used by turns; block 0
+// clears the word after next, which every block has left behind since the
+// barrier before.  A single block needs no word.  Each wait is bounded: after
+// spin_limit polls (a testing hook, mm_debug, can set fewer) the block records
+// status 2 and the kernel returns; the other blocks then give up at their next
+// barrier.  Thread 0's release and acquire, with the block barriers around
+// them, make every block's writes of the phase visible to every thread of
+// every block afterwards.
+__device__ __noinline__ bool grid_sync(Smem &sm, Ctl *ctl, unsigned &turn, unsigned add, unsigned *sum, Result *result,
+                                       unsigned long long *tstamp, int mark, long long spin_limit, int skip_mark)
+{
+    const unsigned nb = gridDim.x, w = turn & (kRing - 1);
+    turn += 1;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int ok = 1;
+        unsigned total = add;
+        // testing hook: block 0 leaves this barrier out, so every wait on it runs out
+        const bool skip = blockIdx.x == 0 && mark >= 0 && mark == skip_mark;
+        if (nb > 1) {
+            unsigned long long *word = ctl->ring + w * kRingStride;
+            if (blockIdx.x == 0) ctl->ring[((w + 2) & (kRing - 1)) * kRingStride] = 0ull;
+            if (!skip)
+                asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word),
+                             "l"(((unsigned long long)add << 32) | 1ull)
+                             : "memory");
+            unsigned long long got;
+            long long it = 0;
+            for (;;) {
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(got) : "l"(word) : "memory");
+                if ((unsigned)got == nb) break;
+                if (++it > spin_limit) {
+                    ok = 0;
+                    break;
+                }
+                if (it > 4096) __nanosleep(100);
+            }
+            total = (unsigned)(got >> 32);
+        } else if (skip) {
+            ok = 0;
+        }
+        if (!ok) *(volatile int *)&result->status = 2;
+        sm.sync_ok = ok;
+        sm.sync_sum = total;
+        if (tstamp && blockIdx.x == 0 && mark >= 0) tstamp[mark] = global_ns();
+    }
+    __syncthreads();
+    *sum = sm.sync_sum;
+    return sm.sync_ok != 0;
+}
 
 // ---- learned colouring ----
 //
@@ -499,7 +553,6 @@ __device__ __forceinline__ uint32_t policy_barrier(const Params &p, const float 
     return (uint32_t)(prob * 4294967296.0f);
 }
 
-// Colour of vertex v for round t: the select barrier, or the policy's.
 // Whether colouring round t needs the features: a policy that ignores them
 // needs them only for the trace.
 __device__ __forceinline__ bool policy_needs_features(const Params &p, int t)
@@ -507,16 +560,17 @@ __device__ __forceinline__ bool policy_needs_features(const Params &p, int t)
     return !p.policy_const || (p.trace && t < p.trace_rounds);
 }
 
+// Colour of vertex v for round t: the select barrier, or the policy's.
 template <bool kPolicy>
-__device__ __forceinline__ bool colour_blue(const Params &p, int v, int deg, float role, float2 wf, int t,
-                                            uint32_t seed, uint32_t barrier)
+__device__ __forceinline__ bool colour_blue(const Params &p, int v, int base, float role, int t, uint32_t seed)
 {
-    uint32_t bar = barrier;
+    uint32_t bar = p.barrier;
     if (kPolicy) {
         float x[kFeat];
-        if (policy_needs_features(p, t)) policy_features(p, wf, deg, role, t, x);
+        if (policy_needs_features(p, t))
+            policy_features(p, __ldg(p.wfeat + v), degree_of(__ldg(p.ranges + v)), role, t, x);
         bar = p.policy_const ? p.policy_bar : policy_barrier(p, x);
-        const bool blue = colour_of((uint32_t)(v - base_of(p, v)), seed, bar) == kBlue;
+        const bool blue = colour_of((uint32_t)(v - base), seed, bar) == kBlue;
         if (p.trace && t < p.trace_rounds) {
             float *row = p.trace + ((size_t)t * p.n + v) * kTraceCols;
 #pragma unroll
@@ -526,58 +580,55 @@ __device__ __forceinline__ bool colour_blue(const Params &p, int v, int deg, flo
         }
         return blue;
     }
-    return colour_of((uint32_t)(v - base_of(p, v)), seed, bar) == kBlue;
+    return colour_of((uint32_t)(v - base), seed, bar) == kBlue;
 }
 
 // ---- worklist compaction for the set-up and commit passes ----
 //
-// A block handles tiles of kTileItems vertices, kPer per thread.  Each thread
-// decides the next list of its vertices; the block counts them per list with
-// warp scans, takes one atomic per list and tile, and writes its items.
-
+// A block handles tiles of up to kTileItems items, a warp up to 128 consecutive
+// ones of them (lane l items l, l + 32, l + 64, l + 96), so that a list keeps
+// its vertices in increasing order.  The warps' counts meet in shared memory (one
+// block barrier a tile: the two parities' words are used by turns) and each
+// warp adds up those before it.  The block's running counts (cb blue, cr red)
+// are the same in every thread.
 constexpr int kPer = 4;
 constexpr int kTileItems = kThreads * kPer;
+enum : int { kDrop = -1, kToBlue = 0, kToRed = 1 };
 
-// dest[k]: -1 (drop), kBlue or kRed.
-__device__ __forceinline__ void compact_tile(const Params &p, Smem &sm, int parity, const int (&dest)[kPer],
-                                             const int4 (&item)[kPer])
+// Items a lane handles in a tile (fewer when the block has few, so that all
+// warps share them), and its first one.
+__device__ __forceinline__ int tile_per(int total) { return min(kPer, max(1, (total + kThreads - 1) / kThreads)); }
+__device__ __forceinline__ int tile_first(int per) { return (int)(threadIdx.x >> 5) * 32 * per + (int)(threadIdx.x & 31); }
+
+__device__ __forceinline__ void compact_tile(Smem &sm, int *list, int region, unsigned tile, const int (&dest)[kPer],
+                                             const int (&item)[kPer], int &cb, int &cr)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int c[2] = {0, 0};
+    const unsigned below = (1u << lane) - 1u;
+    unsigned mb[kPer], mr[kPer], cnt = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        c[0] += dest[k] == kBlue;
-        c[1] += dest[k] == kRed;
+        mb[k] = __ballot_sync(kFull, dest[k] == kToBlue);
+        mr[k] = __ballot_sync(kFull, dest[k] == kToRed);
+        cnt += (unsigned)__popc(mb[k]) | ((unsigned)__popc(mr[k]) << 16);
     }
-    int ex[2];
-#pragma unroll
-    for (int l = 0; l < 2; ++l) {
-        const int incl = warp_incl_scan(c[l]);
-        ex[l] = incl - c[l];
-        if (lane == 31) sm.tile_warp[warp][l] = incl;
-    }
+    unsigned *words = sm.tile_cnt[tile & 1];
+    if (lane == 0) words[warp] = cnt;
     __syncthreads();
-    if (threadIdx.x < 2) {
-        const int l = threadIdx.x;
-        int run = 0;
-        for (int w = 0; w < kWarps; ++w) {
-            const int x = sm.tile_warp[w][l];
-            sm.tile_warp[w][l] = run;
-            run += x;
-        }
-        sm.tile_base[l] = run ? atomicAdd(&p.ctl->cnt[parity][l], run) : 0;
-    }
-    __syncthreads();
-    int rc[2] = {0, 0};
+    // (two 16-bit counts a word: a tile holds 2048 items)
+    unsigned x = lane < kWarps ? words[lane] : 0u;
+    const unsigned all = __reduce_add_sync(kFull, x);
+    unsigned before = __reduce_add_sync(kFull, lane < warp ? x : 0u);
+    int ob = cb + (int)(before & 0xffffu), orr = cr + (int)(before >> 16);
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        const int l = dest[k];
-        if (l < 0) continue;
-        const int idx = l == kBlue ? sm.tile_base[0] + sm.tile_warp[warp][0] + ex[0] + rc[0]++
-                                   : sm.tile_base[1] + sm.tile_warp[warp][1] + ex[1] + rc[1]++;
-        __stcs(&p.lists[parity][l][idx], item[k]);
+        if (dest[k] == kToBlue) __stcs(list + ob + __popc(mb[k] & below), item[k]);
+        if (dest[k] == kToRed) __stcs(list + (region - 1 - orr - __popc(mr[k] & below)), item[k]);
+        ob += __popc(mb[k]);
+        orr += __popc(mr[k]);
     }
-    __syncthreads();  // tile_warp / tile_base are reused by the next tile
+    cb += (int)(all & 0xffffu);
+    cr += (int)(all >> 16);
 }
 
 // Vertices without neighbours on the symmetric path: no list names them, so
@@ -586,24 +637,20 @@ __device__ __forceinline__ void compact_tile(const Params &p, Smem &sm, int pari
 // to the cap (match value 1).  The set-up queues the ones red in round 0 in
 // shared memory and resolves the queue round by round, a hash per queued
 // vertex and round (a walk per thread would cost every lane its warp's longest
-// walk); a vertex that finds the queue full stays in the rounds, which give it
-// the same fate.  iso_last: the last round in which any of them is active (the cap's
+// walk).  iso_last: the last round in which any of them is active (the cap's
 // last round if one stays red to it, nseeds if the seeds run out first: the
 // reference would draw more, and the round count then exceeds nseeds).
-constexpr int kIsoHalf = (int)(sizeof(LongStage) * kWarps / sizeof(int) / 2);  // queue capacity (two halves)
-
-// Called by the whole block once, after the set-up's last tile (whose
-// compaction ends with a barrier, after the last append).
+//
+// Called by the whole block, after a tile's compaction and a block barrier.
 // Round r reads the queue half qa and appends its survivors to the other,
 // counting them in iso_cnt[r % 3]: that counter is cleared by thread 0 in
 // round r - 1, after every thread read it (in round r - 3's closing step) and
 // before any thread appends to it, so one barrier a round suffices.
-__device__ void resolve_isolated(const Params &p, Smem &sm, int &iso_last)
+__device__ __noinline__ void resolve_isolated(const Params &p, Smem &sm, int &iso_last)
 {
-    const Ctl *ctl = p.ctl;
-    int *qa = reinterpret_cast<int *>(&sm.stage[0]), *qb = qa + kIsoHalf;
-    const int cap = ctl->cap, lim = min(cap, ctl->nseeds);
-    const uint32_t barrier = ctl->barrier;
+    int *qa = sm.iso.half[0], *qb = sm.iso.half[1];
+    const int cap = p.cap, lim = min(cap, p.nseeds);
+    const uint32_t barrier = p.barrier;
     int nq = min(sm.iso_n, kIsoHalf);
     if (threadIdx.x == 0) sm.iso_cnt[1] = 0;
     __syncthreads();
@@ -614,11 +661,11 @@ __device__ void resolve_isolated(const Params &p, Smem &sm, int &iso_last)
             const int v = qa[i];
             if (r >= lim) {
                 // red in every round up to the limit
-                p.ctl->match[v] = 1;
+                p.match[v] = 1;
                 if (p.last) p.last[v] = (uint8_t)(cap - 1);
                 iso_last = max(iso_last, lim == cap ? cap - 1 : lim);
             } else if (colour_of((uint32_t)(v - base_of(p, v)), p.seeds[r], barrier) == kBlue) {
-                p.ctl->match[v] = 2;
+                p.match[v] = 2;
                 if (p.last) p.last[v] = (uint8_t)r;
                 iso_last = max(iso_last, r);
             } else {
@@ -641,76 +688,76 @@ __device__ void resolve_isolated(const Params &p, Smem &sm, int &iso_last)
 // vertex that receives a proposal is matched in the same round.  On the
 // symmetric path the vertices without neighbours are resolved here, whatever
 // their colour (resolve_isolated); the instrumented kernel keeps them in the
-// rounds, whose per-round counters count them as the reference does.
+// rounds, whose per-round counters count them as the reference does.  A list
+// is known to be empty, or longer than its window, from its window's offsets
+// (weighted types) or from its range.
 template <bool kW, bool kStats, bool kPolicy>
-__device__ void init_phase(const Params &p, Smem &sm)
+__device__ __forceinline__ void init_phase(const Params &p, Smem &sm, int *list, int &cb, int &cr)
 {
-    const Ctl *ctl = p.ctl;
-    const uint32_t seed = p.seeds[0], barrier = ctl->barrier;
-    const int n = p.n;
+    const uint32_t seed = p.seeds[0];
     int iso_last = -1;
+    cb = cr = 0;
     if (threadIdx.x == 0) sm.iso_n = 0;
     __syncthreads();
-    const int ntiles = (n + kTileItems - 1) / kTileItems;
-    // each tile's ranges and window offsets are loaded while the tile before
-    // it is coloured and compacted
+    const int per = tile_per(p.region);
+    const int first = tile_first(per), ntiles = (p.region + per * kThreads - 1) / (per * kThreads);
+    // each tile's ranges are loaded while the tile before it is coloured and compacted
+    int vv[kPer];
     int2 rr[kPer];
-    long long wo[kPer];
     auto fetch = [&](int tile) {
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const int v = tile * kTileItems + k * kThreads + threadIdx.x;
+            const int s = tile * per * kThreads + first + k * 32;
+            vv[k] = k < per && s < p.region ? own_vertex(p, s) : -1;
             rr[k] = make_int2(0, 0);
-            wo[k] = 0;
-            if (tile < ntiles && v < n) {
-                rr[k] = __ldg(p.ranges + v);
-                if (kW) wo[k] = __ldg(p.pwin_off + v);
+            if (vv[k] >= 0) {
+                if (kW) rr[k] = make_int2(__ldg(p.pwin_off + vv[k]), __ldg(p.pwin_off + vv[k] + 1));
+                else rr[k] = __ldg(p.ranges + vv[k]);
             }
         }
     };
-    fetch(blockIdx.x);
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        int dest[kPer];
-        int4 item[kPer];
+    fetch(0);
+    for (int tile = 0; tile < ntiles; ++tile) {
+        int dest[kPer], item[kPer];
+        bool none[kPer], longer[kPer];
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) item[k] = make_int4(tile * kTileItems + k * kThreads + threadIdx.x, rr[k].x, rr[k].y, (int)wo[k]);
-        fetch(tile + gridDim.x);
+        for (int k = 0; k < kPer; ++k) {
+            item[k] = vv[k];
+            none[k] = kW ? (rr[k].y & ~1) == (rr[k].x & ~1) : degree_of(rr[k]) == 0;
+            longer[k] = kW ? (rr[k].x & 1) != 0 : degree_of(rr[k]) > kWin;
+        }
+        if (tile + 1 < ntiles) fetch(tile + 1);
         unsigned long long act = 0, blue_n = 0;
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const int v = item[k].x;
-            dest[k] = -1;
-            if (v < n) {
-                int slot;
-                const int deg = degree_of(item[k]);
-                const float2 wf = kPolicy && policy_needs_features(p, 0) ? __ldg(p.wfeat + v) : make_float2(0.0f, 0.0f);
-                const bool blue = colour_blue<kPolicy>(p, v, deg, 0.0f, wf, 0, seed, barrier);
-                if (p.last) p.last[v] = 0;
-                p.best[v] = 0ull;
+            const int v = item[k];
+            dest[k] = kDrop;
+            if (v >= 0) {
+                const bool blue = colour_blue<kPolicy>(p, v, base_of(p, v), 0.0f, 0, seed);
                 // (every completed round leaves them zero: a cut list's last piece clears them)
-                if (deg > kWin && p.zero_parts) {
+                if (longer[k] && p.zero_parts) {
                     p.part_key[v] = 0ull;
                     p.part_cnt[v] = 0;
                 }
                 ++act;
                 blue_n += blue;
-                // no neighbours: unmatchable as soon as it is blue (learned
-                // colouring on the symmetric path: at once, whatever its colour;
-                // elsewhere another list may still name it, and a blue vertex
-                // there must keep seeing it red)
-                if ((blue || (kPolicy && p.sym)) && deg == 0) {
+                int slot;
+                if (!kStats && p.sym && none[k] && (kPolicy || blue)) {
+                    // no neighbours: unmatchable as soon as it is blue (learned
+                    // colouring: at once, whatever its colour)
                     p.col[v] = kDead;
-                    p.ctl->match[v] = 2;
+                    p.match[v] = 2;
+                    if (p.last) p.last[v] = 0;
+                    if (!kPolicy) iso_last = max(iso_last, 0);
                     trace_left<kPolicy>(p, 0, v);
-                } else if (!kPolicy && !kStats && p.sym && deg == 0 &&
-                           (slot = atomicAdd(&sm.iso_n, 1)) < kIsoHalf) {
-                    // red in round 0: queued, resolved with the block's others (a
-                    // vertex that finds the queue full stays in the rounds)
+                } else if (!kStats && !kPolicy && p.sym && none[k] && (slot = atomicAdd(&sm.iso_n, 1)) < kIsoHalf) {
+                    // red in round 0: queued, resolved with the block's others
                     p.col[v] = kDead;
-                    reinterpret_cast<int *>(&sm.stage[0])[slot] = v;
+                    sm.iso.half[0][slot] = v;
                 } else {
+                    p.best[v] = 0ull;
                     p.col[v] = blue ? kBlue : kRed;
-                    dest[k] = blue ? kBlue : kRed;
+                    dest[k] = blue ? kToBlue : kToRed;
                 }
             }
         }
@@ -719,13 +766,22 @@ __device__ void init_phase(const Params &p, Smem &sm)
             stat_add(p, 0, MM_ST_BLUE, blue_n);
             stat_add(p, 0, MM_ST_RED, act - blue_n);
         }
-        compact_tile(p, sm, 0, dest, item);
+        compact_tile(sm, list, p.region, (unsigned)tile, dest, item, cb, cr);
+        if (!kPolicy && !kStats && p.sym) {
+            __syncthreads();  // the tile's appends are complete
+            // (every thread reads the same count: appends resume after the next barrier)
+            const bool flush = sm.iso_n > kIsoHalf - kTileItems || (tile + 1 == ntiles && sm.iso_n > 0);
+            __syncthreads();
+            if (flush) resolve_isolated(p, sm, iso_last);
+        }
     }
     if (!kPolicy && !kStats) {
-        if (sm.iso_n > 0) resolve_isolated(p, sm, iso_last);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) iso_last = max(iso_last, __shfl_xor_sync(kFull, iso_last, o));
+        iso_last = __reduce_max_sync(kFull, iso_last);
         if ((threadIdx.x & 31) == 0 && iso_last >= 0) atomicMax(&p.ctl->iso_last, iso_last + 1);
+    }
+    if (threadIdx.x == 0) {  // for the first window scan (read after the barrier)
+        sm.wnext = 3 * kThreads;
+        sm.stage_n = sm.big_n = sm.big_next = sm.shared_n = 0;
     }
 }
 
@@ -742,8 +798,7 @@ __device__ void init_phase(const Params &p, Smem &sm)
 // window is the reference's choice, and the scan stops there.  A list that
 // fits in its window and has no red candidate is decided too (unmatchable iff
 // no entry is unmatched).  A longer list with no red candidate in its window
-// falls back to a full scan in phase A2: it is appended to the round's
-// fallback list.
+// falls back to a full scan.
 
 // Learned colouring, graphs with symmetric structure: a red vertex of at most
 // kRetireMaxDeg entries whose neighbours are all matched leaves in phase A of
@@ -761,97 +816,61 @@ __device__ void init_phase(const Params &p, Smem &sm)
 // time.  A retired vertex's worklist item is marked with its id complemented,
 // so the commit phase sees the retirement in the item it loads anyway.
 template <bool kPolicy>
-__device__ __forceinline__ void retire_red(const Params &p, int t, int par, int n_red)
+__device__ __forceinline__ void retire_red(const Params &p, int t, int *list, int cr)
 {
-    int4 *list = p.lists[par][kRed];
-    const long long stride = (long long)gridDim.x * kThreads;
-    const long long tid = stride - 1 - ((long long)blockIdx.x * kThreads + threadIdx.x);
-    for (long long i = tid; i < n_red; i += stride) {
-        const int4 it = __ldcg(list + i);
-        if (degree_of(it) > kRetireMaxDeg) continue;
+    for (int i = kThreads - 1 - (int)threadIdx.x; i < cr; i += kThreads) {
+        int *slot = list + (p.region - 1 - i);
+        const int v = *slot;
+        const int2 r = __ldg(p.ranges + v);
+        if (degree_of(r) > kRetireMaxDeg) continue;
         bool gone = true;
-        {
+        for (int j0 = r.x; gone && j0 < r.y; j0 += 16) {
             int nb[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) nb[u] = it.y + u < it.z ? __ldg(p.nbrs + it.y + u) : -1;
-#pragma unroll
-            for (int u = 0; u < 16; ++u)
-                if (nb[u] >= 0 && p.col[nb[u]] != kMatched) gone = false;
-        }
-        for (int j0 = it.y + 16; gone && j0 < it.z; j0 += 16) {
-            int nb[16];
-#pragma unroll
-            for (int u = 0; u < 16; ++u) nb[u] = j0 + u < it.z ? __ldg(p.nbrs + j0 + u) : -1;
+            for (int u = 0; u < 16; ++u) nb[u] = j0 + u < r.y ? __ldg(p.nbrs + j0 + u) : -1;
 #pragma unroll
             for (int u = 0; u < 16; ++u)
                 if (nb[u] >= 0 && p.col[nb[u]] != kMatched) gone = false;
         }
         if (gone) {
-            p.col[it.x] = kDead;
-            p.ctl->match[it.x] = 2;
-            list[i].x = ~it.x;
-            trace_left<kPolicy>(p, t, it.x);
+            p.col[v] = kDead;
+            p.match[v] = 2;
+            if (p.last) p.last[v] = (uint8_t)t;
+            *slot = ~v;
+            trace_left<kPolicy>(p, t, v);
         }
     }
 }
 
-// The end of a blue vertex's window scan: propose to the red candidate found,
-// or decide "no proposal" / "unmatchable" for a list that fits its window, or
-// stage a longer list with no red candidate in its window for the fallback scan.
-template <bool kW, bool kStats>
-__device__ __forceinline__ void window_done(const Params &p, Smem &sm, int t, long long i, int4 it, bool found, int cj,
-                                            int ct, bool alive, int seen)
+// Append blue vertex v (list r) to the round's shared fallback list: one
+// 64-bit atomic hands out the item and its offset in the concatenated entries.
+__device__ __forceinline__ void stage_shared(const Params &p, Smem &sm, int v, long long slot, int2 r)
 {
-    Ctl *ctl = p.ctl;
-    const int v = it.x, deg = degree_of(it);
-    if (kStats) atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_WINDOW_ENTRIES], (unsigned long long)seen);
-    if (found || deg <= kWin) {
-        if (kStats) {
-            atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_REQ_ENTRIES],
-                      request_seen<kW>(it.y, deg, found ? cj : -1));
-            atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_BLUE_DEG], (unsigned long long)deg);
-        }
-        if (found) {
-            if (kW && p.wwin) propose_weight(p, p.reqi + i, v, __int_as_float(cj), ct);
-            else propose_to<kW>(p, p.reqi + i, v, it.y, cj & 0x7fffffff, ct);
-        } else {
-            no_proposal(p, p.reqi + i, v, alive);
-        }
-    } else {
-        // the fallback scan proposes through req[v]
-        p.reqi[i] = make_int2(kReqFallback, 0);
-        // fallback: the whole list is scanned in phase A2.  The block collects
-        // its fallback lists in shared memory and appends them to the round's
-        // list at the end of the phase, with one global atomic; only a list
-        // that finds the block's buffer full is appended at once.
-        const int slot = atomicAdd(&sm.stage_n, 1);
-        if (slot < kStageCap) {
-            reinterpret_cast<int4 *>(&sm.stage[0])[slot] = make_int4(v, it.y, it.z, 0);
-            return;
-        }
-        const unsigned long long old = atomicAdd(&ctl->staged_pack, (1ull << 32) | (unsigned long long)(unsigned)deg);
-        const int idx = (int)(old >> 32), off = (int)(old & 0xffffffffull);
-        p.staged[idx] = make_int4(v, it.y, it.z, off);
-        for (int s = (off + kSegEntries - 1) / kSegEntries; s * kSegEntries < off + deg; ++s) p.seg_first[s] = idx;
-    }
+    const int deg = degree_of(r);
+    const unsigned long long old = atomicAdd(&p.ctl->staged_pack, (1ull << 32) | (unsigned long long)(unsigned)deg);
+    const int idx = (int)(old >> 32), off = (int)(old & 0xffffffffull);
+    p.staged[idx] = make_int4(v, r.x, r.y, off);
+    for (int s = (off + kSegEntries - 1) / kSegEntries; s * kSegEntries < off + deg; ++s) p.seg_first[s] = idx;
+    p.prop[slot] = kReqShared;  // it proposes through req[v]
+    atomicAdd(&sm.shared_n, 1);
 }
 
-// Window entries q and q + 1 of a blue vertex (item it, window length wl):
+// Window entries q and q + 1 of a blue vertex (window from `off`, length wl):
 // neighbours and second words (weight, position | flag, or position).
 template <bool kW>
-__device__ __forceinline__ void window_pair(const Params &p, int4 it, int wl, int q, int &n0, int &j0, int &n1, int &j1)
+__device__ __forceinline__ void window_pair(const Params &p, int off, int wl, int q, int &n0, int &j0, int &n1, int &j1)
 {
-    n0 = n1 = 0;
+    n0 = n1 = -1;
     j0 = j1 = 0;
     if (q >= wl) return;
     if (kW) {
-        const int4 x = __ldg(reinterpret_cast<const int4 *>(p.pwin + it.w + q));
+        const int4 x = __ldg(reinterpret_cast<const int4 *>(p.pwin + off + q));
         n0 = x.x;
         j0 = x.y;
         n1 = x.z;
         j1 = x.w;
     } else {
-        j0 = it.y + q;
+        j0 = off + q;
         j1 = j0 + 1;
         n0 = __ldg(p.nbrs + j0);
         if (q + 1 < wl) n1 = __ldg(p.nbrs + j1);
@@ -865,65 +884,166 @@ __device__ __forceinline__ void window_pair(const Params &p, int4 it, int wl, in
 template <bool kW>
 __device__ __forceinline__ bool window_choice(const Params &p, uint8_t c, int j)
 {
-    return c == kRed && (!kW || (p.wwin ? __int_as_float(j) > -1.0f : j >= 0));
+    return c == kRed && (!kW || (p.sym ? __int_as_float(j) > -1.0f : j >= 0));
 }
 
-// Phase A1.  Each block takes an equal share of the round's blue items, in
-// chunks of kScanChunk interleaved with the other blocks' (ids, and with them
-// degrees, cluster in the worklists: on R-MAT graphs the hubs have small ids),
-// and hands them to its warps 32 at a time from a counter in shared memory.  A lane
-// holds one vertex at a time and reads its window eight entries a step (four
-// 16-byte loads, then the eight colours); as soon as a lane's vertex is decided it
-// swaps in the item it prefetched and prefetches the next, so every lane keeps
-// an independent chain of loads in flight and no lane waits for the slowest
-// vertex of its warp or block.  Block barriers come only before the scan (the
-// counter) and after it (the block's fallback lists are appended at once).
-constexpr int kScanChunk = 64;
-
-template <bool kW, bool kStats, bool kPolicy>
-__device__ void scan_window(const Params &p, Smem &sm, int t, int par)
+// A window's place: first slot, length (even for the weighted types, whose odd
+// windows end with a filler) and whether the list is longer.  raw is the pair
+// of window offsets (weighted) or the range.
+template <bool kW>
+__device__ __forceinline__ int2 window_raw(const Params &p, int v)
 {
-    Ctl *ctl = p.ctl;
-    const int n_blue = __ldcg(&ctl->cnt[par][kBlue]);
-    const int n_red = kPolicy ? __ldcg(&ctl->cnt[par][kRed]) : 0;  // read with n_blue: one round trip
-    const int4 *list = p.lists[par][kBlue];
+    return kW ? make_int2(__ldg(p.pwin_off + v), __ldg(p.pwin_off + v + 1)) : __ldg(p.ranges + v);
+}
+template <bool kW>
+__device__ __forceinline__ void window_place(int2 raw, int &off, int &wl, bool &longer)
+{
+    if (kW) {
+        off = raw.x & ~1;
+        wl = (raw.y & ~1) - off;
+        longer = (raw.x & 1) != 0;
+    } else {
+        const int deg = degree_of(raw);
+        off = raw.x;
+        wl = win_len(deg);
+        longer = deg > kWin;
+    }
+}
+
+// Full scan of a list by the lanes of one or more warps: entries b + first,
+// b + first + step, ... in rows of 32 * kRows per warp; the lanes' best keys.
+// Random types stop at the first row with a red entry.
+template <bool kW>
+__device__ __forceinline__ unsigned long long scan_rows(const Params &p, int b, int e, int first, int step)
+{
     const int lane = threadIdx.x & 31;
-    const unsigned below = (1u << lane) - 1u;
-    // this block's items: chunk c of its share is chunk c * gridDim.x + blockIdx.x of the list
-    const long long span = (long long)gridDim.x * kScanChunk;
-    const long long full = n_blue / span, rest = n_blue - full * span;
-    const int bhi = (int)(full * kScanChunk + min((long long)kScanChunk, max(0ll, rest - (long long)blockIdx.x * kScanChunk)));
-    if (threadIdx.x == 0) {
-        sm.wnext = 0;
-        sm.stage_n = 0;
+    float bw = -1.0f;
+    int bj = 0;
+    bool alive = false;
+    for (int j0 = b + first; j0 < e; j0 += step) {
+        int nb[kRows];
+        float wv[kRows];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            const int j = j0 + r * 32 + lane;
+            nb[r] = j < e ? __ldg(p.nbrs + j) : -1;
+            wv[r] = kW && j < e ? __ldg(p.w + j) : 0.0f;
+        }
+        uint8_t c[kRows];
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) c[r] = nb[r] >= 0 ? ld_col(p.col + nb[r]) : (uint8_t)kMatched;
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) fold_entry<kW>(c[r], wv[r], j0 + r * 32 + lane, bw, bj, alive);
+        if (!kW && __any_sync(kFull, bw > -1.0f)) break;
+    }
+    return strip_key<kW>(bw, bj, alive);
+}
+
+__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long k)
+{
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long y = __shfl_xor_sync(kFull, k, o);
+        k = y > k ? y : k;
+    }
+    return k;
+}
+
+template <bool kStats>
+__device__ __forceinline__ void count_fallback(const Params &p, int t, int deg)
+{
+    if (kStats) {
+        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_STAGED_DEG], (unsigned long long)deg);
+        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_STAGED_ITEMS], 1ull);
+    }
+}
+
+// The block's fallback lists, collected by its window scan: a warp scans a
+// list of up to kWarpList entries, the whole block one of up to kBlockList
+// (a round trip of its 16 warps covers 2048 entries); a longer one (a hub,
+// which would keep one block busy while the others wait) goes to the shared
+// list, at the price of one more grid barrier in that round.
+constexpr int kWarpList = 512;
+constexpr int kBlockList = 32768;
+
+template <bool kW, bool kStats>
+__device__ __noinline__ void scan_fallback(const Params &p, Smem &sm, int t, long long rbase)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ns = min(sm.stage_n, kStageCap);
+    for (int i = warp; i < ns; i += kWarps) {
+        const int2 it = sm.fb.item[i];
+        const int2 r = __ldg(p.ranges + it.x);
+        const int deg = degree_of(r);
+        if (deg > kBlockList) {
+            if (lane == 0) stage_shared(p, sm, it.x, rbase + it.y, r);
+        } else if (deg > kWarpList) {
+            if (lane == 0) sm.fb.big[atomicAdd(&sm.big_n, 1)] = (unsigned short)i;
+        } else {
+            const unsigned long long key = warp_max_u64(scan_rows<kW>(p, r.x, r.y, 0, 32 * kRows));
+            if (lane == 0) {
+                count_fallback<kStats>(p, t, deg);
+                propose_key<kW, kStats>(p, ItemReq{p, rbase + it.y}, it.x, r.x, deg, key, t);
+            }
+        }
     }
     __syncthreads();
-    bool dry = bhi == 0;  // warp-uniform: the block's share is handed out
+    const int nbig = sm.big_n;
+    for (int i = 0; i < nbig; ++i) {
+        const int2 it = sm.fb.item[sm.fb.big[i]];
+        const int2 r = __ldg(p.ranges + it.x);
+        const int deg = degree_of(r);
+        const unsigned long long mine = warp_max_u64(scan_rows<kW>(p, r.x, r.y, warp * 32 * kRows, kThreads * kRows));
+        if (lane == 0) sm.red_key[warp] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long key = 0ull;
+            for (int w = 0; w < kWarps; ++w) key = sm.red_key[w] > key ? sm.red_key[w] : key;
+            count_fallback<kStats>(p, t, deg);
+            propose_key<kW, kStats>(p, ItemReq{p, rbase + it.y}, it.x, r.x, deg, key, t);
+        }
+        __syncthreads();  // the keys are reused
+    }
+}
+
+// Phase A1 over the block's cb blue items.  The first items go to the threads
+// in order, the rest to the warps from a counter in shared memory.  A lane
+// holds one vertex at a time and reads its window eight entries a step (four
+// 16-byte loads, then the eight colours); as soon as a lane's vertex is
+// decided it takes the next one, whose window offsets it has prefetched, loads
+// the offsets of the one after that, whose id it has prefetched, and prefetches
+// another id.  So every lane keeps an independent chain of loads in flight and
+// no lane waits for the slowest vertex of its warp or block.
+template <bool kW, bool kStats, bool kPolicy>
+__device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, int *list, long long rbase, int cb, int cr)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    bool dry = 3 * kThreads >= cb;  // warp-uniform: the block's items are handed out
     // Items for the lanes in `mask`: one shared atomic per warp.  Returns this
-    // lane's item index in the list, or -1.
-    auto grab = [&](unsigned mask) -> long long {
+    // lane's item, or -1.
+    auto grab = [&](unsigned mask) -> int {
         const int leader = __ffs(mask) - 1;
         int base = 0;
         if (lane == leader) base = atomicAdd(&sm.wnext, __popc(mask));
         base = __shfl_sync(kFull, base, leader);
-        dry = base + __popc(mask) >= bhi;
+        dry = base + __popc(mask) >= cb;
         const int k = base + __popc(mask & below);
-        if (!((mask >> lane) & 1u) || k >= bhi) return -1;
-        return (long long)(k / kScanChunk) * span + (long long)blockIdx.x * kScanChunk + k % kScanChunk;
+        return ((mask >> lane) & 1u) && k < cb ? k : -1;
     };
-    // the lane's vertex and its prefetched next, with their item indices
-    int4 cur = make_int4(-1, 0, 0, 0), nxt = make_int4(-1, 0, 0, 0);
-    int ci = -1, ni = -1;  // item indices (a list holds at most n < 2^31 items)
-    if (!dry) {
-        ci = (int)grab(kFull);
-        if (ci >= 0) cur = __ldcs(list + ci);
-    }
-    if (!dry) {
-        ni = (int)grab(kFull);
-        if (ni >= 0) nxt = __ldcs(list + ni);
-    }
-    bool has = cur.x >= 0, alive = false;
-    int q = 0, wl = has ? win_len(degree_of(cur)) : 0;
+    // the lane's vertex, its next (window offsets loaded) and the one after (id loaded)
+    int ci = threadIdx.x, ni = threadIdx.x + kThreads, mi = threadIdx.x + 2 * kThreads;
+    ci = ci < cb ? ci : -1;
+    ni = ni < cb ? ni : -1;
+    mi = mi < cb ? mi : -1;
+    int cv = ci >= 0 ? __ldcs(list + ci) : -1, nv = ni >= 0 ? __ldcs(list + ni) : -1, mv = mi >= 0 ? __ldcs(list + mi) : -1;
+    int2 nraw = make_int2(0, 0);
+    int off = 0, wl = 0;
+    bool longer = false;
+    if (cv >= 0) window_place<kW>(window_raw<kW>(p, cv), off, wl, longer);
+    if (nv >= 0) nraw = window_raw<kW>(p, nv);
+    bool has = cv >= 0, alive = false;
+    int q = 0;
     while (__any_sync(kFull, has)) {
         if (has) {
             // eight entries a step (one dependent round trip for each 8: the scan
@@ -934,17 +1054,18 @@ __device__ void scan_window(const Params &p, Smem &sm, int t, int par)
             int nb[8], jv[8];
 #pragma unroll
             for (int h = 0; h < 4; ++h) {
-                nb[2 * h] = nb[2 * h + 1] = jv[2 * h] = jv[2 * h + 1] = 0;
-                if (2 * h < width) window_pair<kW>(p, cur, wl, q + 2 * h, nb[2 * h], jv[2 * h], nb[2 * h + 1], jv[2 * h + 1]);
+                nb[2 * h] = nb[2 * h + 1] = -1;
+                jv[2 * h] = jv[2 * h + 1] = 0;
+                if (2 * h < width) window_pair<kW>(p, off, wl, q + 2 * h, nb[2 * h], jv[2 * h], nb[2 * h + 1], jv[2 * h + 1]);
             }
             uint8_t c[8];
 #pragma unroll
-            for (int x = 0; x < 8; ++x) c[x] = x < width && q + x < wl ? ld_col(p.col + nb[x]) : (uint8_t)kMatched;
+            for (int x = 0; x < 8; ++x) c[x] = nb[x] >= 0 ? ld_col(p.col + nb[x]) : (uint8_t)kMatched;
             bool found = false;
             int cj = -1, ct = 0, seen = q;
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
-                if (x >= width || q + x >= wl || found) continue;
+                if (nb[x] < 0 || found) continue;
                 seen = q + x + 1;
                 if (window_choice<kW>(p, c[x], jv[x])) {
                     found = true;
@@ -956,69 +1077,59 @@ __device__ void scan_window(const Params &p, Smem &sm, int t, int par)
             }
             q += width;
             if (found || q >= wl) {
-                window_done<kW, kStats>(p, sm, t, ci, cur, found, cj, ct, alive, seen);
+                const ItemReq rq{p, rbase + ci};
+                if (kStats) {
+                    atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_WINDOW_ENTRIES], (unsigned long long)seen);
+                    if (found || !longer) {
+                        const int2 r = __ldg(p.ranges + cv);
+                        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_REQ_ENTRIES],
+                                  request_seen<kW>(r.x, degree_of(r), found ? cj : -1));
+                        atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_BLUE_DEG], (unsigned long long)degree_of(r));
+                    }
+                }
+                if (found) {
+                    if (kW && p.sym) propose_weight(p, rq, cv, __int_as_float(cj), ct);
+                    else propose_to<kW>(p, rq, cv, kW && !p.contiguous ? __ldg(p.ranges + cv).x : off, cj & 0x7fffffff, ct);
+                } else if (!longer) {
+                    no_proposal(p, rq, cv, alive, t);
+                } else {
+                    // the whole list is scanned after the windows; only a list that
+                    // finds the block's buffer full goes to the shared list at once
+                    const int slot = atomicAdd(&sm.stage_n, 1);
+                    if (slot < kStageCap) sm.fb.item[slot] = make_int2(cv, ci);
+                    else stage_shared(p, sm, cv, rbase + ci, __ldg(p.ranges + cv));
+                }
                 has = false;
             }
         }
-        // lanes whose vertex is decided take their prefetched item and prefetch the next
-        const unsigned need = __ballot_sync(kFull, !has && nxt.x >= 0);
+        // lanes whose vertex is decided take their prefetched one
+        const unsigned need = __ballot_sync(kFull, !has && nv >= 0);
         if (need) {
-            if (!has && nxt.x >= 0) {
-                cur = nxt;
+            const bool take = !has && nv >= 0;
+            if (take) {
+                cv = nv;
                 ci = ni;
-                nxt.x = -1;
+                window_place<kW>(nraw, off, wl, longer);
                 has = true;
                 alive = false;
                 q = 0;
-                wl = win_len(degree_of(cur));
+                nv = mv;
+                ni = mi;
+                mv = mi = -1;
+                if (nv >= 0) nraw = window_raw<kW>(p, nv);
             }
             if (!dry) {
-                const int i = (int)grab(need);
+                const int i = grab(need);
                 if (i >= 0) {
-                    nxt = __ldcs(list + i);
-                    ni = i;
+                    mi = i;
+                    mv = __ldcs(list + i);
                 }
             }
         }
     }
-    // append the block's fallback lists: one atomic for the block, item
-    // offsets by a block-wide prefix sum of their lengths
+    if (kPolicy && p.sym && t >= kRetireFrom) retire_red<kPolicy>(p, t, list, cr);
     __syncthreads();
-    const int ns = min(sm.stage_n, kStageCap);
-    if (ns > 0) {
-        const int4 *buf = reinterpret_cast<const int4 *>(&sm.stage[0]);
-        const int warp = threadIdx.x >> 5;
-        const int per = (ns + kThreads - 1) / kThreads;
-        const int lo = min(ns, (int)threadIdx.x * per), hi = min(ns, lo + per);
-        int s = 0;
-        for (int i = lo; i < hi; ++i) s += degree_of(buf[i]);
-        const int incl = warp_incl_scan(s);
-        if (lane == 31) sm.tile_warp[warp][0] = incl;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int run = 0;
-            for (int w = 0; w < kWarps; ++w) {
-                const int x = sm.tile_warp[w][0];
-                sm.tile_warp[w][0] = run;
-                run += x;
-            }
-            const unsigned long long old =
-                atomicAdd(&ctl->staged_pack, ((unsigned long long)ns << 32) | (unsigned long long)(unsigned)run);
-            sm.tile_base[0] = (int)(old >> 32);
-            sm.tile_base[1] = (int)(old & 0xffffffffull);
-        }
-        __syncthreads();
-        int off = sm.tile_base[1] + sm.tile_warp[warp][0] + incl - s;
-        for (int i = lo; i < hi; ++i) {
-            const int4 it = buf[i];
-            const int idx = sm.tile_base[0] + i, deg = degree_of(it);
-            p.staged[idx] = make_int4(it.x, it.y, it.z, off);
-            for (int sg = (off + kSegEntries - 1) / kSegEntries; sg * kSegEntries < off + deg; ++sg) p.seg_first[sg] = idx;
-            off += deg;
-        }
-        __syncthreads();  // the buffer and the tile words are reused
-    }
-    if (kPolicy && p.sym && t >= kRetireFrom) retire_red<kPolicy>(p, t, par, n_red);
+    if (sm.stage_n > 0) scan_fallback<kW, kStats>(p, sm, t, rbase);
 }
 
 // ---- phase A2: fallback lists, entry-balanced segments ----
@@ -1045,7 +1156,7 @@ template <bool kW, bool kStats>
 __device__ __forceinline__ void finish_piece(const Params &p, int4 it, int pieces, unsigned long long key, int t)
 {
     if (pieces == 1) {
-        propose_counted<kW, kStats>(p, it, key, t);
+        propose_key<kW, kStats>(p, VertexReq{p, it.x}, it.x, it.y, degree_of(it), key, t);
         return;
     }
     const int v = it.x;
@@ -1057,7 +1168,7 @@ __device__ __forceinline__ void finish_piece(const Params &p, int4 it, int piece
     if (done == pieces - 1) {
         const unsigned long long all = atomicExch(&p.part_key[v], 0ull);
         atomicExch(&p.part_cnt[v], 0);
-        propose_counted<kW, kStats>(p, it, all, t);
+        propose_key<kW, kStats>(p, VertexReq{p, v}, v, it.y, degree_of(it), all, t);
     }
 }
 
@@ -1066,16 +1177,6 @@ __device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_g
 __device__ __forceinline__ void cp_async4_s(unsigned saddr, const void *gmem)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr), "l"(gmem) : "memory");
-}
-
-__device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long k)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const unsigned long long y = __shfl_xor_sync(kFull, k, o);
-        k = y > k ? y : k;
-    }
-    return k;
 }
 
 // Finish piece k of the segment table: lane k holds its item.
@@ -1100,9 +1201,9 @@ __device__ void scan_long(const Params &p, Smem &sm, int t, int gwarp, int nwarp
     const int nentries = (int)(pack & 0xffffffffull);
     const int nseg = (nentries + kSegEntries - 1) / kSegEntries;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int *pend = sm.pend[warp];
-    int *delta = sm.delta[warp];
-    LongStage &stg = sm.stage[warp];
+    int *pend = sm.ls.pend[warp];
+    int *delta = sm.ls.delta[warp];
+    LongStage &stg = sm.ls.stage[warp];
     // shared addresses of this lane's slots in stage 0 (stage k: + k * kStageBytes)
     constexpr unsigned kStageBytes = kRows * 32 * 4;
     const unsigned nb_slot = (unsigned)__cvta_generic_to_shared(&stg.nb[0][lane]);
@@ -1235,138 +1336,122 @@ __device__ void scan_long(const Params &p, Smem &sm, int t, int gwarp, int nwarp
 }
 
 // Phase B: commit proposals, recolour survivors with the next seed, compact
-// the worklists of round t+1.
+// the block's lists of round t+1 (ncb blue, ncr red).  A colour byte is
+// written only when it changes.
 template <bool kW, bool kStats, bool kPolicy>
-__device__ void commit_phase(const Params &p, Smem &sm, int t, bool has_next)
+__device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, bool has_next, const int *list, int *next,
+                                             long long rbase, int cb, int cr, int &ncb, int &ncr)
 {
-    Ctl *ctl = p.ctl;
-    const int par = t & 1;
     const uint32_t next_seed = has_next ? p.seeds[t + 1] : 0u;
-    const uint32_t barrier = ctl->barrier;
-    const int c0 = __ldcg(&ctl->cnt[par][kBlue]), c1 = __ldcg(&ctl->cnt[par][kRed]);
-    const long long total = (long long)c0 + c1;
-    // tiles of at most kTileItems items, as many for every block (the last tile may be short)
-    const long long per_block = (total + (long long)gridDim.x * kTileItems - 1) / ((long long)gridDim.x * kTileItems);
-    const long long tsize = per_block > 0 ? (total + (long long)gridDim.x * per_block - 1) / ((long long)gridDim.x * per_block) : 1;
-    const long long ntiles = (total + tsize - 1) / tsize;
-    int *match = ctl->match;
-    int retired = 0;
-    for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const long long base = tile * tsize, tend = min(total, base + tsize);
+    const int total = cb + cr;
+    const int per = tile_per(total), first = tile_first(per), tsize = per * kThreads;
+    ncb = ncr = 0;
+    for (int base = 0, tile = 0; base < total; base += tsize, ++tile) {
         // items, and with a blue item its request, loaded together
-        int4 it[kPer];
-        int2 q[kPer];
-        bool in[kPer], blue[kPer], gone[kPer];
+        int vv[kPer], tg[kPer];
+        uint32_t low[kPer];
+        bool blue[kPer], gone[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const long long i = base + k * kThreads + threadIdx.x;
-            in[k] = i < tend;
-            blue[k] = i < c0;
-            it[k] = make_int4(0, 0, 0, 0);
-            q[k] = make_int2(-1, 0);
-            if (in[k]) {
-                if (blue[k]) {
-                    it[k] = __ldcs(p.lists[par][kBlue] + i);
-                } else {
-                    it[k] = __ldcs(p.lists[par][kRed] + (i - c0));
+            const int i = base + first + k * 32;
+            const bool in = k < per && i < total;
+            blue[k] = in && i < cb;
+            gone[k] = false;
+            vv[k] = -1;
+            tg[k] = kReqNone;
+            low[k] = 0u;
+            if (blue[k]) {
+                vv[k] = __ldcs(list + i);
+                tg[k] = __ldcs(p.prop + rbase + i);
+                if (!p.sym) low[k] = __ldcs(p.prop_key + rbase + i);
+            } else if (in) {
+                vv[k] = __ldcs(list + (p.region - 1 - (i - cb)));
+                // learned colouring: a red item retired in phase A carries its id complemented
+                if (kPolicy && vv[k] < 0) {
+                    gone[k] = true;
+                    vv[k] = ~vv[k];
                 }
             }
-            // learned colouring: a red item retired in phase A carries its id complemented
-            gone[k] = kPolicy && in[k] && !blue[k] && it[k].x < 0;
-            if (gone[k]) it[k].x = ~it[k].x;
         }
-        // proposal state: blue -> its request (a fallback list's is in req), red -> the
+        // proposal state: blue -> its request (a shared fallback list's is in req), red -> the
         // best proposal it received
         unsigned long long key[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             key[k] = 0ull;
-            if (in[k]) {
-                if (blue[k]) {
-                    q[k] = __ldcs(p.reqi + (base + k * kThreads + threadIdx.x));
-                    if (q[k].x == kReqFallback) q[k] = __ldcg(p.req + it[k].x);
-                } else {
-                    key[k] = __ldcg(p.best + it[k].x);
-                }
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < kPer; ++k)
-            if (in[k] && blue[k] && q[k].y != 0) key[k] = __ldcg(p.best + q[k].x);
-        int partner[kPer];
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            partner[k] = -1;
-            if (!in[k]) continue;
             if (blue[k]) {
-                if (q[k].y != 0 && (uint32_t)key[k] == (uint32_t)q[k].y) partner[k] = q[k].x;
-            } else if (key[k]) {
-                // the low half of the key names the proposer: its id on the
-                // symmetric path, else the position of the red's entry for it
-                partner[k] = p.sym ? (int)~(uint32_t)key[k] : __ldg(p.nbrs + (int)~(uint32_t)key[k]);
+                if (tg[k] == kReqShared) {
+                    const int2 q = __ldcg(p.req + vv[k]);
+                    tg[k] = q.x;
+                    low[k] = (uint32_t)q.y;
+                } else if (p.sym) {
+                    low[k] = ~(uint32_t)vv[k];
+                }
+                if (tg[k] >= 0 && low[k] != 0u) key[k] = __ldcg(p.best + tg[k]);
+            } else if (vv[k] >= 0) {
+                key[k] = __ldcg(p.best + vv[k]);
             }
         }
         int dest[kPer];
         unsigned long long matched = 0, seen = 0, rdeg = 0, act = 0, nblue = 0;
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            dest[k] = -1;
-            if (!in[k]) continue;
-            const int v = it[k].x;
-            const int deg = degree_of(it[k]);
+            dest[k] = kDrop;
+            const int v = vv[k];
+            if (v < 0) continue;
+            int partner = -1;
+            if (blue[k]) {
+                if (tg[k] >= 0 && low[k] != 0u && (uint32_t)key[k] == low[k]) partner = tg[k];
+            } else if (key[k]) {
+                // the low half of the key names the proposer: its id on the
+                // symmetric path, else the position of the red's entry for it
+                partner = p.sym ? (int)~(uint32_t)key[k] : __ldg(p.nbrs + (int)~(uint32_t)key[k]);
+            }
             if (kStats && !blue[k]) {
+                const int2 r = __ldg(p.ranges + v);
+                const int deg = degree_of(r);
                 rdeg += deg;
                 // random mode: grRespond stops at its first proposer, whose position
                 // is the key's low half (symmetric path: found in the sorted list)
-                int first = -1;
+                int at = -1;
                 if (!kW && key[k]) {
-                    first = (int)~(uint32_t)key[k];
+                    at = (int)~(uint32_t)key[k];
                     if (p.sym) {
-                        int lo = it[k].y, hi = it[k].z;
+                        int lo = r.x, hi = r.y;
                         while (lo < hi) {
                             const int mid = (int)(((long long)lo + hi) >> 1);
-                            if (__ldg(p.nbrs + mid) < first) lo = mid + 1;
+                            if (__ldg(p.nbrs + mid) < at) lo = mid + 1;
                             else hi = mid;
                         }
-                        first = lo;
+                        at = lo;
                     }
                 }
-                seen += first >= 0 ? (unsigned long long)(first - it[k].y + 1) : (unsigned long long)deg;
+                seen += at >= 0 ? (unsigned long long)(at - r.x + 1) : (unsigned long long)deg;
             }
-            if (partner[k] >= 0) {
+            if (partner >= 0) {
                 trace_left<kPolicy>(p, t, v);
-                match[v] = 4 + min(v, partner[k]) - base_of(p, v);
+                p.match[v] = 4 + min(v, partner) - base_of(p, v);
                 p.col[v] = kMatched;
+                if (p.last) p.last[v] = (uint8_t)t;
                 ++matched;
                 continue;
             }
             // unmatchable (marked in phase A; learned colouring: red ones too)
-            if ((blue[k] && q[k].x == -1) || gone[k]) {
+            if ((blue[k] && tg[k] == kReqDead) || gone[k]) {
                 trace_left<kPolicy>(p, t, v);
                 continue;
             }
             // survivor
             if (!has_next) {
-                dest[k] = blue[k] ? kBlue : kRed;
+                dest[k] = blue[k] ? kToBlue : kToRed;
                 continue;
             }
-            const float role = blue[k] ? (q[k].y != 0 ? 1.0f : 0.5f) : 0.0f;
-            const float2 wf =
-                kPolicy && policy_needs_features(p, t + 1) ? __ldg(p.wfeat + v) : make_float2(0.0f, 0.0f);
-            const bool nb = colour_blue<kPolicy>(p, v, deg, role, wf, t + 1, next_seed, barrier);
-            if (p.last) p.last[v] = (uint8_t)(t + 1);
+            const float role = blue[k] ? (tg[k] >= 0 && low[k] != 0u ? 1.0f : 0.5f) : 0.0f;
+            const bool nb = colour_blue<kPolicy>(p, v, base_of(p, v), role, t + 1, next_seed);
             ++act;
             nblue += nb;
-            // no neighbours: unmatchable as soon as it is blue
-            if (nb && deg == 0) {
-                p.col[v] = kDead;
-                match[v] = 2;
-                ++retired;
-                trace_left<kPolicy>(p, t + 1, v);
-            } else {
-                p.col[v] = nb ? kBlue : kRed;
-                dest[k] = nb ? kBlue : kRed;
-            }
+            if (nb != blue[k]) p.col[v] = nb ? kBlue : kRed;
+            dest[k] = nb ? kToBlue : kToRed;
         }
         if (kStats) {
             stat_add(p, t, MM_ST_MATCHED, matched);
@@ -1378,11 +1463,12 @@ __device__ void commit_phase(const Params &p, Smem &sm, int t, bool has_next)
                 stat_add(p, t + 1, MM_ST_RED, act - nblue);
             }
         }
-        compact_tile(p, sm, par ^ 1, dest, it);
+        compact_tile(sm, next, p.region, (unsigned)tile, dest, vv, ncb, ncr);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) retired += __shfl_xor_sync(kFull, retired, o);
-    if ((threadIdx.x & 31) == 0 && retired) atomicAdd(&ctl->retired[par ^ 1], retired);
+    if (threadIdx.x == 0) {  // for the next window scan (read after the barrier)
+        sm.wnext = 3 * kThreads;
+        sm.stage_n = sm.big_n = sm.big_next = sm.shared_n = 0;
+    }
 }
 
 // ---- finish phase ----
@@ -1421,35 +1507,26 @@ __device__ void commit_phase(const Params &p, Smem &sm, int t, bool has_next)
 // Every vertex's match value is then final, and the matching executed
 // max(last active round) + 2 rounds, the reference's closing round included
 // (at most the cap).
-constexpr int kFinMembers = 32;    // members of a component played by one warp (one per lane)
-constexpr int kFinEntries = 128;   // entries between members of one component
 constexpr int kFinShort = 32;      // lists a thread scans on its own; longer ones its warp scans
 constexpr int kFinMaxDeg = 2048;   // longest list the finish phase accepts
 constexpr int kFinDiv = 12;        // default: first attempt once the active set is at most 1/kFinDiv of round 0's
 enum : int { kFinSingle = 1, kFinMember = 2, kFinRootCand = 3 };
 enum : int { kFinNotRoot = 0, kFinRoot = 1, kFinTooBig = 2 };
 
-// One warp's component: members' first entry, list start and degree, the
-// entries between members (preference key and the target's member slot), the
-// members' colours of the round being played and the best proposal each
-// received.
-struct FinWarp {
-    unsigned long long pref[kFinEntries];
-    unsigned long long best[kFinMembers];
-    int mem[kFinMembers];
-    int eoff[kFinMembers + 1];
-    int mbeg[kFinMembers];
-    int mdeg[kFinMembers];
-    uint8_t tgt[kFinEntries];
-    uint8_t st[kFinMembers];
-};
-static_assert(sizeof(FinWarp) * kWarps <= offsetof(Smem, tile_warp),
-              "the finish phase reuses the fallback scan's shared memory");
-
-// Item i of round parity `par` (blue list first, then red).
-__device__ __forceinline__ int4 item_at(const Params &p, int par, int c0, long long i)
+// Item i of the block's lists (cb blue, then the red ones).
+__device__ __forceinline__ int item_at(const Params &p, const int *list, int cb, int i)
 {
-    return i < c0 ? __ldcg(p.lists[par][kBlue] + i) : __ldcg(p.lists[par][kRed] + (i - c0));
+    return __ldcs(list + (i < cb ? i : p.region - 1 - (i - cb)));
+}
+
+// Preference key of an entry naming u with weight w, as the finish phase
+// compares them: on the symmetric path a list is strictly increasing, so the
+// smaller id is the earlier position.  1: a neighbour that is never chosen.
+template <bool kW>
+__device__ __forceinline__ unsigned long long fin_key(int u, float w)
+{
+    if (kW) return w > -1.0f ? (((unsigned long long)weight_order(w) << 32) | (uint32_t)~u) : 1ull;
+    return (unsigned long long)(uint32_t)~u;
 }
 
 // Own-list scan of vertex v, entries [b, e): active neighbours (blue or red),
@@ -1567,7 +1644,7 @@ __device__ __forceinline__ int fin_search(const Params &p, FinWarp &fw, int v, i
             if (__any_sync(kFull, in && u < v)) return kFinNotRoot;
             unsigned m = __ballot_sync(kFull, in);
             unsigned long long pref = 0;
-            if (in) pref = kW ? cand_key<true>(j, wj) : (unsigned long long)(uint32_t)~j;
+            if (in) pref = fin_key<kW>(u, wj);
             while (m) {
                 const int s = __ffs(m) - 1;
                 m &= m - 1;
@@ -1622,15 +1699,14 @@ __device__ __forceinline__ unsigned long long respond_seen(const Params &p, int 
 // writes every member's match value (and batch round marks).  Returns, in
 // every lane, the last round in which a member was active.
 template <bool kW, bool kStats>
-__device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, const uint32_t *seeds, int t0, int cap, int mem,
-                                       int k)
+__device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, int t0, int mem, int k)
 {
     const int lane = threadIdx.x & 31;
     const bool own = lane < k;
     const int g = own ? mem : 0;
     const int base = own ? base_of(p, g) : 0;
     const uint32_t hid = (uint32_t)(g - base);
-    const uint32_t bar = p.fin_retire ? p.policy_bar : p.ctl->barrier;
+    const uint32_t bar = p.fin_retire ? p.policy_bar : p.barrier;
     int eb = 0, ee = 0, deg = 0, beg = 0;
     if (own) {
         eb = fw.eoff[lane];
@@ -1644,9 +1720,9 @@ __device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, const uint
     bool act = own, blue = false;
     int val = 0, lastr = -1;
     __syncwarp();
-    for (int t = t0; t < cap && __any_sync(kFull, act); ++t) {
+    for (int t = t0; t < p.cap && __any_sync(kFull, act); ++t) {
         if (act) {
-            blue = colour_of(hid, seeds[t], bar) == kBlue;
+            blue = colour_of(hid, p.seeds[t], bar) == kBlue;
             lastr = t;
         }
         if (own) fw.st[lane] = act ? (blue ? kBlue : kRed) : (val == 2 ? kDead : kMatched);
@@ -1716,7 +1792,7 @@ __device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, const uint
             stat_add(p, t, MM_ST_BLUE_DEG, b ? (unsigned long long)deg : 0ull);
             stat_add(p, t, MM_ST_RED_DEG, r ? (unsigned long long)deg : 0ull);
             stat_add(p, t, MM_ST_REQ_ENTRIES,
-                     b ? request_seen<kW>(beg, deg, best >= 2 ? (int)~(uint32_t)best : -1) : 0ull);
+                     b ? (kW || best < 2 ? (unsigned long long)deg : respond_seen<kW>(p, beg, deg, best)) : 0ull);
             stat_add(p, t, MM_ST_RESP_ENTRIES, r ? respond_seen<kW>(p, beg, deg, kb) : 0ull);
             stat_add(p, t, MM_ST_MATCHED, matched ? 1ull : 0ull);
         }
@@ -1726,7 +1802,7 @@ __device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, const uint
     }
     if (own) {
         // members still unmatched at the cap keep their last colour
-        p.ctl->match[g] = act ? (blue ? 0 : 1) : val;
+        p.match[g] = act ? (blue ? 0 : 1) : val;
         if (p.last) p.last[g] = (uint8_t)lastr;
     }
 #pragma unroll
@@ -1754,29 +1830,31 @@ struct FinComp {
     int k;
 };
 
-// The finish phase's record of item i: four int4 slots, rec[4i .. 4i + 3], in
-// the worklist memory of the other parity (2n slots, which the round has not
-// written yet; an attempt has at most n / 2 items): {meta, v, 0, 0},
-// then the ids, preference-key low halves and high halves of its first
-// kFinRec entries that point at an active vertex.  meta = class | count << 8,
-// count = its active neighbours, kFinRec + 1 if more than a record holds.
+// The finish phase's record of an item: three int4, rec[3i .. 3i + 2] with i
+// counted from the block's own part of the record array: {meta, v, id 0, id 1},
+// {id 2, id 3, weight 0, weight 1}, {weight 2, weight 3, 0, 0}, the ids and
+// weight orders (0: never chosen) of its first kFinRec entries that point at
+// an active vertex.  meta = class | count << 8, count = its active neighbours,
+// kFinRec + 1 if more than a record holds.  A singleton needs the first int4
+// only, a vertex of two active neighbours of a random type too.
 __device__ __forceinline__ int fin_meta_class(int meta) { return meta & 0xff; }
 __device__ __forceinline__ int fin_meta_count(int meta) { return (meta >> 8) & 0xff; }
 
-// As fin_search, by one thread for root candidate v (item i), following the
+// As fin_search, by one thread for root candidate v (record i), following the
 // records instead of the lists: each member costs two loads from L2 (its
-// item index, its record).  kFinOverflow when a member's record is incomplete
-// or the component does not fit FinComp.  The lists' bounds are read only
-// for the instrumented kernel's counters.
+// record's index, its record).  kFinOverflow when a member's record is
+// incomplete or the component does not fit FinComp.  The lists' bounds are
+// read only for the instrumented kernel's counters.
 template <bool kW, bool kStats>
-__device__ __forceinline__ int fin_search_thread(const Params &p, const int4 *rec, int v, long long i, FinComp &cp)
+__device__ __forceinline__ int fin_search_thread(const Params &p, int v, int i, FinComp &cp)
 {
-    long long ix[kFinTMembers];
+    int ix[kFinTMembers];
     int k = 1, ne = 0;
     cp.mem[0] = v;
     ix[0] = i;
     for (int f = 0; f < k; ++f) {
-        const int4 r0 = __ldcg(rec + 4 * ix[f]);
+        const int4 *rec = p.rec + 3ll * ix[f];
+        const int4 r0 = __ldcg(rec), r1 = __ldcg(rec + 1), r2 = __ldcg(rec + 2);
         const int cnt = fin_meta_count(r0.x);
         if (cnt > kFinRec) return kFinOverflow;
         cp.eoff[f] = (uint8_t)ne;
@@ -1785,11 +1863,8 @@ __device__ __forceinline__ int fin_search_thread(const Params &p, const int4 *re
             cp.mbeg[f] = r.x;
             cp.mdeg[f] = r.y > r.x ? r.y - r.x : 0;
         }
-        if (cnt == 0) continue;
-        const int4 ru = __ldcg(rec + 4 * ix[f] + 1), rl = __ldcg(rec + 4 * ix[f] + 2), rh = __ldcg(rec + 4 * ix[f] + 3);
-        const int uu[kFinRec] = {ru.x, ru.y, ru.z, ru.w};
-        const int lo[kFinRec] = {rl.x, rl.y, rl.z, rl.w};
-        const int hi[kFinRec] = {rh.x, rh.y, rh.z, rh.w};
+        const int uu[kFinRec] = {r0.z, r0.w, r1.x, r1.y};
+        const int ww[kFinRec] = {r1.z, r1.w, r2.x, r2.y};
 #pragma unroll
         for (int q = 0; q < kFinRec; ++q) {
             if (q >= cnt) break;
@@ -1802,11 +1877,12 @@ __device__ __forceinline__ int fin_search_thread(const Params &p, const int4 *re
                 if (k == kFinTMembers) return kFinOverflow;
                 slot = k;
                 cp.mem[k] = u;
-                ix[k] = __ldcg(p.req + u).x;  // its item (written by the scan pass)
+                ix[k] = __ldcg(p.req + u).x;  // its record (written by the scan pass)
                 ++k;
             }
             if (ne == kFinTEntries) return kFinOverflow;
-            cp.pref[ne] = ((unsigned long long)(uint32_t)hi[q] << 32) | (uint32_t)lo[q];
+            cp.pref[ne] = !kW ? (unsigned long long)(uint32_t)~u
+                              : (ww[q] ? (((unsigned long long)(uint32_t)ww[q] << 32) | (uint32_t)~u) : 1ull);
             cp.tgt[ne] = (uint8_t)slot;
             ++ne;
         }
@@ -1819,19 +1895,18 @@ __device__ __forceinline__ int fin_search_thread(const Params &p, const int4 *re
 // Singletons of a tile (mine): each leaves in the first round from t on in
 // which it is blue (blue0: its colour in round t), or keeps red to the cap.
 template <bool kStats>
-__device__ __forceinline__ void fin_singles(const Params &p, const uint32_t *seeds, int t, int cap, bool mine, int v,
-                                            int deg, bool blue0, int &last_all)
+__device__ __forceinline__ void fin_singles(const Params &p, int t, bool mine, int v, int deg, bool blue0, int &last_all)
 {
-    const uint32_t bar = p.fin_retire ? p.policy_bar : p.ctl->barrier;
+    const uint32_t bar = p.fin_retire ? p.policy_bar : p.barrier;
     const uint32_t hid = mine ? (uint32_t)(v - base_of(p, v)) : 0u;
     // learned colouring: a short list retires as soon as it is red from round
     // kRetireFrom (a singleton's neighbours are all matched)
     const bool may_retire = p.fin_retire && deg <= kRetireMaxDeg;
     bool act = mine, blue = blue0;
     int lastr = -1;
-    for (int r = t; r < cap && __any_sync(kFull, act); ++r) {
+    for (int r = t; r < p.cap && __any_sync(kFull, act); ++r) {
         if (act) {
-            if (r > t) blue = colour_of(hid, seeds[r], bar) == kBlue;
+            if (r > t) blue = colour_of(hid, p.seeds[r], bar) == kBlue;
             lastr = r;
         }
         if (kStats) {
@@ -1850,41 +1925,49 @@ __device__ __forceinline__ void fin_singles(const Params &p, const uint32_t *see
     }
     if (mine) {
         // still red at the cap: it keeps that colour
-        p.ctl->match[v] = act ? 1 : 2;
+        p.match[v] = act ? 1 : 2;
         if (p.last) p.last[v] = (uint8_t)lastr;
         last_all = max(last_all, lastr);
     }
 }
 
-// Finish pass 1 over round t's items: scan each item's own list (a thread
-// each, its warp for lists longer than kFinShort), classify it, record its
-// first two active neighbours (non-singletons also record their item index
-// in req[v].x), and, with kSingles, resolve the singletons at once.  Calls
-// the attempt off for a list longer than kFinMaxDeg or an unmatchable
-// neighbour.
-template <bool kW, bool kStats, bool kSingles>
-__device__ __forceinline__ void finish_scan(const Params &p, Smem &sm, int t, int par, int c0, int c1, int cap,
-                                            int4 *rec)
+// The part of the block's `cnt` items that this warp handles in the finish
+// passes: equal shares, so that a small set still spreads over all warps.
+__device__ __forceinline__ void fin_share(int cnt, int &lo, int &hi)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const long long A = (long long)c0 + c1;
-    const long long gw = (long long)blockIdx.x * kWarps + warp, nw = (long long)gridDim.x * kWarps;
+    const int warp = threadIdx.x >> 5, share = (cnt + kWarps - 1) / kWarps;
+    lo = min(cnt, warp * share);
+    hi = min(cnt, lo + share);
+}
+
+// Finish pass 1 over the block's items of round t: scan each item's own list
+// (a thread each, its warp for lists longer than kFinShort), classify it,
+// record its first active neighbours (and in req[v].x the record's index),
+// and, with kSingles, resolve the singletons at once.  Returns whether the
+// attempt has to be called off: a list longer than kFinMaxDeg, an unmatchable
+// neighbour, or more items than the block has records for.
+template <bool kW, bool kStats, bool kSingles>
+__device__ __forceinline__ bool finish_scan(const Params &p, int t, const int *list, int cb, int cr)
+{
+    const int lane = threadIdx.x & 31;
+    const int cnt_all = cb + cr;
+    if (cnt_all > p.rec_region) return true;
     bool abort = false;
-    int last_all = -1;
-    for (long long base = gw * 32; base < A; base += nw * 32) {
-        // another warp may have called the attempt off: its remaining work is wasted
-        if (__shfl_sync(kFull, lane == 0 ? __ldcg(&p.ctl->fin_abort) : 0, 0) == t + 1) break;
-        const long long i = base + lane;
-        const int4 it = i < A ? item_at(p, par, c0, i) : make_int4(-1, 0, 0, 0);
-        const int deg = it.x >= 0 ? degree_of(it) : 0;
+    int last_all = -1, lo_i, hi_i;
+    fin_share(cnt_all, lo_i, hi_i);
+    for (int base = lo_i; base < hi_i; base += 32) {
+        const int i = base + lane;
+        const int v = i < hi_i ? item_at(p, list, cb, i) : -1;
+        const int2 r = v >= 0 ? __ldg(p.ranges + v) : make_int2(0, 0);
+        const int deg = degree_of(r);
         int nint = 0, jr[kFinRec] = {0, 0, 0, 0}, ur[kFinRec] = {0, 0, 0, 0};
         bool lower = false, bad = false;
-        if (it.x >= 0 && deg <= kFinShort) fin_scan_thread(p, it.x, it.y, it.y + deg, nint, lower, bad, jr, ur);
-        unsigned longs = __ballot_sync(kFull, it.x >= 0 && deg > kFinShort);
+        if (v >= 0 && deg <= kFinShort) fin_scan_thread(p, v, r.x, r.x + deg, nint, lower, bad, jr, ur);
+        unsigned longs = __ballot_sync(kFull, v >= 0 && deg > kFinShort);
         while (longs) {
             const int s = __ffs(longs) - 1;
             longs &= longs - 1;
-            const int vs = __shfl_sync(kFull, it.x, s), bs = __shfl_sync(kFull, it.y, s);
+            const int vs = __shfl_sync(kFull, v, s), bs = __shfl_sync(kFull, r.x, s);
             const int ds = __shfl_sync(kFull, deg, s);
             if (ds > kFinMaxDeg) {
                 if (lane == s) bad = true;
@@ -1904,76 +1987,70 @@ __device__ __forceinline__ void finish_scan(const Params &p, Smem &sm, int t, in
                 }
             }
         }
-        const int c = it.x < 0 ? 0 : (nint == 0 ? kFinSingle : (lower ? kFinMember : kFinRootCand));
+        const int c = v < 0 ? 0 : (nint == 0 ? kFinSingle : (lower ? kFinMember : kFinRootCand));
         abort |= bad;
-        if (it.x >= 0) {
+        if (v >= 0) {
             const int cnt = min(nint, kFinRec + 1);
-            rec[4 * i] = make_int4(c | (cnt << 8), it.x, 0, 0);
+            const int at = blockIdx.x * p.rec_region + i;
+            int4 *rec = p.rec + 3ll * at;
+            rec[0] = make_int4(c | (cnt << 8), v, ur[0], ur[1]);
             if (nint > 0) {
-                p.req[it.x].x = (int)i;
+                p.req[v].x = at;
                 if (cnt <= kFinRec) {
-                    uint32_t lo[kFinRec], hi[kFinRec];
+                    int o[kFinRec];
 #pragma unroll
                     for (int q = 0; q < kFinRec; ++q) {
-                        unsigned long long key = 0ull;
-                        if (q < cnt) key = kW ? cand_key<true>(jr[q], __ldg(p.w + jr[q])) : (unsigned long long)(uint32_t)~jr[q];
-                        lo[q] = (uint32_t)key;
-                        hi[q] = (uint32_t)(key >> 32);
+                        o[q] = 0;
+                        if (kW && q < cnt) {
+                            const float x = __ldg(p.w + jr[q]);
+                            if (x > -1.0f) o[q] = (int)weight_order(x);
+                        }
                     }
-                    rec[4 * i + 1] = make_int4(ur[0], ur[1], ur[2], ur[3]);
-                    rec[4 * i + 2] = make_int4((int)lo[0], (int)lo[1], (int)lo[2], (int)lo[3]);
-                    rec[4 * i + 3] = make_int4((int)hi[0], (int)hi[1], (int)hi[2], (int)hi[3]);
+                    rec[1] = make_int4(ur[2], ur[3], o[0], o[1]);
+                    rec[2] = make_int4(o[2], o[3], 0, 0);
                 }
             }
         }
         if (kStats) {
-            stat_add(p, t, MM_ST_FINISH_ITEMS, it.x >= 0 ? 1ull : 0ull);
+            stat_add(p, t, MM_ST_FINISH_ITEMS, v >= 0 ? 1ull : 0ull);
             stat_add(p, t, MM_ST_FINISH_ENTRIES, (unsigned long long)deg);
         }
-        if (__any_sync(kFull, abort)) {  // the attempt is off: tell the other warps now
-            if (lane == 0) atomicExch(&p.ctl->fin_abort, t + 1);
-            break;
-        }
-        if (kSingles) fin_singles<kStats>(p, sm.seeds, t, cap, c == kFinSingle, it.x, deg, i < c0, last_all);
+        if (__any_sync(kFull, abort)) break;
+        if (kSingles) fin_singles<kStats>(p, t, c == kFinSingle, v, deg, i < cb, last_all);
     }
-    if (abort && lane == 0) atomicExch(&p.ctl->fin_abort, t + 1);
     if (kSingles) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) last_all = max(last_all, __shfl_xor_sync(kFull, last_all, o));
+        last_all = __reduce_max_sync(kFull, last_all);
         if (lane == 0 && last_all >= 0) atomicMax(&p.ctl->fin_last, last_all);
     }
+    return abort;
 }
 
-// Finish pass 2 over round t's items: each root candidate's lane searches its
+// Finish pass 2 over the block's items: each root candidate's lane searches its
 // component through the records and, with kPlay, plays it; a component that
 // a lane cannot hold goes to the warp (list scans, up to kFinMembers members),
 // and one larger than that calls the attempt off.  With kSingles (the
 // instrumented kernel's last pass) the singletons are resolved here too.
 template <bool kW, bool kStats, bool kPlay, bool kSingles>
-__device__ __forceinline__ void finish_roots(const Params &p, Smem &sm, int t, int par, int c0, int c1, int cap,
-                                             const int4 *rec)
+__device__ __forceinline__ bool finish_roots(const Params &p, Smem &sm, int t, int cb, int cr)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    FinWarp &fw = reinterpret_cast<FinWarp *>(&sm)[warp];
-    const long long A = (long long)c0 + c1;
-    const long long gw = (long long)blockIdx.x * kWarps + warp, nw = (long long)gridDim.x * kWarps;
+    FinWarp &fw = sm.fin[warp];
     bool abort = false;
-    int last_all = -1;
-    for (long long base = gw * 32; base < A; base += nw * 32) {
-        if (__shfl_sync(kFull, lane == 0 ? __ldcg(&p.ctl->fin_abort) : 0, 0) == t + 1) break;
-        const long long i = base + lane;
-        const int4 r0 = i < A ? __ldcg(rec + 4 * i) : make_int4(0, -1, 0, 0);
-        const int meta = r0.x;
-        const int c = fin_meta_class(meta);
+    int last_all = -1, lo_i, hi_i;
+    fin_share(cb + cr, lo_i, hi_i);
+    for (int base = lo_i; base < hi_i; base += 32) {
+        const int i = base + lane;
+        const int at = blockIdx.x * p.rec_region + i;
+        const int4 r0 = i < hi_i ? __ldcg(p.rec + 3ll * at) : make_int4(0, -1, 0, 0);
+        const int c = fin_meta_class(r0.x);
         if (kSingles) {
-            const int4 it = c == kFinSingle ? item_at(p, par, c0, i) : make_int4(-1, 0, 0, 0);
-            fin_singles<kStats>(p, sm.seeds, t, cap, c == kFinSingle, it.x, c == kFinSingle ? degree_of(it) : 0,
-                                i < c0, last_all);
+            const bool single = c == kFinSingle;
+            fin_singles<kStats>(p, t, single, r0.y, single ? degree_of(__ldg(p.ranges + r0.y)) : 0, i < cb, last_all);
         }
         const int v = c == kFinRootCand ? r0.y : -1;
         int rres = kFinNotRoot;
         FinComp cp;
-        if (c == kFinRootCand) rres = fin_search_thread<kW, kStats>(p, rec, v, i, cp);
+        if (c == kFinRootCand) rres = fin_search_thread<kW, kStats>(p, v, at, cp);
         // the lanes' components, packed into the warp and played together, a lane
         // per member (a lane playing its component alone would colour its
         // members one after another)
@@ -2010,7 +2087,7 @@ __device__ __forceinline__ void finish_roots(const Params &p, Smem &sm, int t, i
             if (lane == 0) fw.eoff[ktot] = etot;
             __syncwarp();
             const int ml = lane < ktot ? fw.mem[lane] : 0;
-            last_all = max(last_all, fin_play<kW, kStats>(p, fw, sm.seeds, t, cap, ml, ktot));
+            last_all = max(last_all, fin_play<kW, kStats>(p, fw, t, ml, ktot));
             __syncwarp();  // fw is refilled by the next batch
             pend &= ~batch;
         }
@@ -2026,191 +2103,125 @@ __device__ __forceinline__ void finish_roots(const Params &p, Smem &sm, int t, i
                 abort = true;
                 break;
             }
-            if (kPlay && r == kFinRoot) last_all = max(last_all, fin_play<kW, kStats>(p, fw, sm.seeds, t, cap, mem, k));
+            if (kPlay && r == kFinRoot) last_all = max(last_all, fin_play<kW, kStats>(p, fw, t, mem, k));
             __syncwarp();  // fw is reused by the next root
         }
-        if (__any_sync(kFull, abort)) {
-            if (lane == 0) atomicExch(&p.ctl->fin_abort, t + 1);
-            break;
-        }
+        if (__any_sync(kFull, abort)) break;
     }
-    if (abort && lane == 0) atomicExch(&p.ctl->fin_abort, t + 1);
     if (kPlay) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) last_all = max(last_all, __shfl_xor_sync(kFull, last_all, o));
+        last_all = __reduce_max_sync(kFull, last_all);
         if (lane == 0 && last_all >= 0) atomicMax(&p.ctl->fin_last, last_all);
     }
+    return abort;
+}
+
+// One barrier of k_match, with the block's summand and the sum over the blocks.
+__device__ __forceinline__ bool barrier_sum(const Params &p, Smem &sm, unsigned &turn, unsigned add, unsigned *sum, int mark)
+{
+    return grid_sync(sm, p.ctl, turn, add, sum, p.result, p.tstamp, mark, p.spin_limit, p.skip_mark);
+}
+
+// The finish phase of round t.  Returns -1 if a barrier wait gave up, else
+// whether the phase completed (0: called off, the round has to be played).
+// Profile: the first pass is reported as round t's window scan, the rest as
+// its fallback scan.
+template <bool kW, bool kStats>
+__device__ __forceinline__ int finish_phase(const Params &p, Smem &sm, unsigned &turn, int t, const int *list, int cb, int cr)
+{
+    unsigned off;
+    // counters must not count a called-off attempt: the instrumented kernel
+    // checks, then resolves; the plain one is speculative (a called-off attempt
+    // leaves only values that the rounds write again)
+    bool abort = finish_scan<kW, kStats, !kStats>(p, t, list, cb, cr);
+    if (!barrier_sum(p, sm, turn, (unsigned)__syncthreads_or(abort), &off, 3 * t + 1)) return -1;
+    if (kStats && !off) {
+        abort = finish_roots<kW, kStats, false, false>(p, sm, t, cb, cr);
+        if (!barrier_sum(p, sm, turn, (unsigned)__syncthreads_or(abort), &off, -1)) return -1;
+    }
+    if (!off) {
+        abort = finish_roots<kW, kStats, true, kStats>(p, sm, t, cb, cr);
+        if (!barrier_sum(p, sm, turn, (unsigned)__syncthreads_or(abort), &off, 3 * t + 2)) return -1;
+    }
+    if (off) return 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        const int last = max(__ldcg(&p.ctl->fin_last), __ldcg(&p.ctl->iso_last) - 1);
+        p.result->rounds = p.maximal ? min(last + 2, p.cap) : p.cap;
+        if (p.tstamp) p.tstamp[3 * t + 3] = p.tstamp[3 * t + 2];
+    }
+    return 1;
 }
 
 // The whole matching in one cooperative launch: set-up, then per round the
-// window scan (A1), the fallback scan (A2, only in rounds that have fallback
-// lists) and the commit phase (B), separated by grid barriers.  Every block
-// reads the same counters after a barrier, so all blocks take the same
-// branches and leave the loop at the same round.  Afterwards, vertices that
-// could still be matched keep their last colour as their match value (the
-// reference leaves match[v] = 0 / 1 for them).
+// window scan (A1), the shared fallback scan (A2, only in rounds that have
+// such lists) and the commit phase (B), separated by grid barriers, until the
+// finish phase plays the remaining rounds or no vertex is left.  Every block
+// gets the same sums from the barriers, so all blocks take the same branches
+// and leave the loop at the same round.  Vertices that could still be matched
+// at the end keep their last colour as their match value (the reference
+// leaves match[v] = 0 / 1 for them).
 template <bool kW, bool kStats, bool kPolicy>
-__global__ void __launch_bounds__(kThreads, 2) k_rounds(Params p)
+__global__ void __launch_bounds__(kThreads, 2) k_match(const __grid_constant__ Params p)
 {
     extern __shared__ __align__(16) unsigned char dsmem[];
     Smem &sm = *reinterpret_cast<Smem *>(dsmem);
-    Ctl *ctl = p.ctl;
-    const int cap = ctl->cap;
-    const int maximal = ctl->maximal;
-    const int nseeds = ctl->nseeds;
-    const int gwarp = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    const int nwarps = gridDim.x * kWarps;
-
-    long long active0, fin_next;
-    int t;
-    if (p.resume) {
-        // the finish kernel called its attempt off: carry on from its round,
-        // without another attempt
-        if (ctl->fin_state != kFinStateResume) {
-            release_lines(p.col, p.n);
-            return;
-        }
-        t = ctl->fin_round;
-        active0 = ctl->active0;
-        fin_next = -1;
-    } else {
-        init_phase<kW, kStats, kPolicy>(p, sm);
-        if (!grid_sync(p.bar, p.ctl, p.tstamp, 0, p.spin_limit, p.skip_mark)) return;
-        // active vertices at round 0; round 1 clears these counters only after
-        // two more grid barriers
-        active0 = (long long)__ldcg(&ctl->cnt[0][kBlue]) + __ldcg(&ctl->cnt[0][kRed]);
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->active0 = active0;
-        fin_next = active0;  // finish phase: attempt once the active set is this small
-        t = 0;
-    }
+    const long long rbase = (long long)blockIdx.x * p.region;
+    const bool first = blockIdx.x == 0 && threadIdx.x == 0;
+    // the next call's control block (no block of this call reads it)
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < (int)(sizeof(Ctl) / 8); i += kThreads)
+            reinterpret_cast<unsigned long long *>(p.ctl_next)[i] = 0ull;
+    unsigned turn = 0, act = 0, shared = 0;
+    int cb, cr, t = 0;
+    init_phase<kW, kStats, kPolicy>(p, sm, p.lists[0] + rbase, cb, cr);
+    if (!barrier_sum(p, sm, turn, (unsigned)(cb + cr), &act, 0)) return;
+    const unsigned active0 = act;  // active vertices at round 0
+    unsigned fin_next = active0;   // finish phase: attempt once the active set is this small
     for (;; ++t) {
-        const int par = t & 1;
-        // Hand the rest to the finish kernel (the symmetric path of the
-        // reference's colouring only).  Every block reads the same counters and
-        // leaves here; round t's worklists and colours are complete.
-        if ((!kPolicy || p.fin_retire) && p.sym && t > 0) {
-            const long long act = (long long)__ldcg(&ctl->cnt[par][kBlue]) + __ldcg(&ctl->cnt[par][kRed]);
-            if (p.fin_div > 0 && act > 0 && act * p.fin_div <= active0 && act <= fin_next) {
-                if (blockIdx.x == 0 && threadIdx.x == 0) {
-                    ctl->fin_round = t;
-                    ctl->fin_state = kFinStatePending;
-                }
-                return;
-            }
+        int *list = p.lists[t & 1] + rbase, *next = p.lists[(t & 1) ^ 1] + rbase;
+        // the finish phase (the symmetric path of a constant colouring only); in
+        // one block the rounds cost less than it does
+        if ((!kPolicy || p.fin_retire) && p.sym && t > 0 && gridDim.x > 1 && p.fin_div > 0 && act > 0 && act <= fin_next &&
+            (unsigned long long)act * (unsigned)p.fin_div <= active0) {
+            const int done = finish_phase<kW, kStats>(p, sm, turn, t, list, cb, cr);
+            if (done < 0) return;
+            if (done) break;
+            fin_next = act / 2;  // called off: again when the set has halved
+            __syncthreads();     // the working areas change hands
         }
-        // phase A1; the next round's counters were last read in round t - 1
-        if (blockIdx.x == 0 && threadIdx.x < kParityLists) {
-            ctl->cnt[par ^ 1][threadIdx.x] = 0;
-            if (threadIdx.x == 0) ctl->retired[par ^ 1] = 0;
+        scan_window<kW, kStats, kPolicy>(p, sm, t, list, rbase, cb, cr);
+        if (!barrier_sum(p, sm, turn, sm.shared_n > 0 ? 1u : 0u, &shared, 3 * t + 1)) return;
+        if (shared) {
+            scan_long<kW, kStats>(p, sm, t, (int)(blockIdx.x * kWarps + (threadIdx.x >> 5)), (int)(gridDim.x * kWarps));
+            if (!barrier_sum(p, sm, turn, 0u, &shared, -1)) return;
+            if (first) p.ctl->staged_pack = 0ull;  // empty again for the next round
         }
-        scan_window<kW, kStats, kPolicy>(p, sm, t, par);
-        if (!grid_sync(p.bar, p.ctl, p.tstamp, 3 * t + 1, p.spin_limit, p.skip_mark)) return;
-        // phase A2 (all blocks see the same fallback count)
-        if (__ldcg(&ctl->staged_pack) != 0ull) {
-            scan_long<kW, kStats>(p, sm, t, gwarp, nwarps);
-            if (!grid_sync(p.bar, p.ctl, p.tstamp, -1, p.spin_limit, p.skip_mark)) return;
-        }
-        if (p.tstamp && blockIdx.x == 0 && threadIdx.x == 0) p.tstamp[3 * t + 2] = global_ns();
-        // phase B; the fallback list is empty again for the next round
-        bool has_next = t + 1 < cap;
-        const bool seeds_short = has_next && t + 1 >= nseeds;
+        if (p.tstamp && first) p.tstamp[3 * t + 2] = global_ns();
+        bool has_next = t + 1 < p.cap;
+        const bool seeds_short = has_next && t + 1 >= p.nseeds;
         if (seeds_short) has_next = false;
-        commit_phase<kW, kStats, kPolicy>(p, sm, t, has_next);
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctl->staged_pack = 0ull;
-        if (!grid_sync(p.bar, p.ctl, p.tstamp, 3 * t + 3, p.spin_limit, p.skip_mark)) return;
-        // close the round (every block decides alike)
-        const long long next = (long long)__ldcg(&ctl->cnt[par ^ 1][kBlue]) + __ldcg(&ctl->cnt[par ^ 1][kRed]);
-        const bool more = has_next && next > 0;
-        if (!more) {
-            if (blockIdx.x == 0 && threadIdx.x == 0) {
-                if (seeds_short) ctl->status = 1;
-                // Vertices retired while being coloured for round t+1 are still
-                // active in that round for the reference, so it runs round t+1
-                // and only finds nothing left at round t+2.
-                const int retired_all = __ldcg(&ctl->retired[par ^ 1]);
-                if (!maximal || next > 0) ctl->rounds = cap;
-                else ctl->rounds = min(retired_all > 0 ? t + 3 : t + 2, cap);
-                // vertices without neighbours resolved at set-up
-                const int iso = __ldcg(&ctl->iso_last) - 1;
-                if (maximal && iso >= 0) ctl->rounds = max(ctl->rounds, min(iso + 2, cap));
-            }
-            break;
+        int ncb, ncr;
+        commit_phase<kW, kStats, kPolicy>(p, sm, t, has_next, list, next, rbase, cb, cr, ncb, ncr);
+        cb = ncb;
+        cr = ncr;
+        if (!barrier_sum(p, sm, turn, (unsigned)(cb + cr), &act, 3 * t + 3)) return;
+        if (has_next && act > 0) continue;
+        // the loop ends; survivors of the last round keep its colours
+        if (first) {
+            int rounds = p.maximal && act == 0 ? min(t + 2, p.cap) : p.cap;
+            // vertices without neighbours resolved at set-up
+            const int iso = __ldcg(&p.ctl->iso_last) - 1;
+            if (p.maximal && iso >= 0) rounds = max(rounds, min(iso + 2, p.cap));
+            p.result->rounds = rounds;
+            if (seeds_short) p.result->status = 1;
         }
+        for (int i = threadIdx.x; i < cb + cr; i += kThreads) {
+            const int v = item_at(p, next, cb, i);
+            p.match[v] = i < cb ? kBlue : kRed;
+            if (p.last) p.last[v] = (uint8_t)t;
+        }
+        break;
     }
-    // finish: survivors of the last round (lists of parity (t + 1) & 1)
-    const int par = (t + 1) & 1;
-    const int cb = __ldcg(&ctl->cnt[par][kBlue]), cr = __ldcg(&ctl->cnt[par][kRed]);
-    const long long total = (long long)cb + cr;
-    int *match = ctl->match;
-    for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < total; i += (long long)gridDim.x * kThreads) {
-        const int v = i < cb ? __ldcg(p.lists[par][kBlue] + i).x : __ldcg(p.lists[par][kRed] + (i - cb)).x;
-        match[v] = __ldcg(p.col + v);
-    }
-    // the last launch of the matching (a finish kernel and a resumed round
-    // kernel follow only a hand-over, which returns above)
     release_lines(p.col, p.n);
-}
-
-// The finish phase as its own cooperative launch, after k_rounds has stopped
-// at round ctl->fin_round (its code inside the round kernel cost that kernel's
-// scan and commit loops registers: its rounds 0-4 ran 7% slower on R-MAT 2^23).
-// It returns at once if the round kernel finished the matching itself.  If the
-// attempt is called off, the resumed round kernel carries on from that round.
-template <bool kW, bool kStats>
-__global__ void __launch_bounds__(kThreads, 2) k_finish(Params p)
-{
-    extern __shared__ __align__(16) unsigned char dsmem[];
-    Smem &sm = *reinterpret_cast<Smem *>(dsmem);
-    Ctl *ctl = p.ctl;
-    if (ctl->fin_state != kFinStatePending) return;
-    const int cap = ctl->cap, maximal = ctl->maximal;
-    const int t = ctl->fin_round, par = t & 1;
-    const int c0 = ctl->cnt[par][kBlue], c1 = ctl->cnt[par][kRed];
-    // the seed buffer holds 256 words (only the call's seeds are meaningful)
-    for (int i = threadIdx.x; i < 256; i += kThreads) sm.seeds[i] = p.seeds[i];
-    __syncthreads();
-    // records: the worklist memory of the other parity (2n items, written by
-    // round t's commit only, which runs after this kernel if at all)
-    int4 *rec = p.lists[par ^ 1][kBlue];
-    // profile: the first pass is reported as round t's window scan, the rest
-    // as its fallback scan
-    bool done;
-    if (kStats) {
-        // counters must not count a called-off attempt: check, then resolve
-        finish_scan<kW, kStats, false>(p, sm, t, par, c0, c1, cap, rec);
-        if (!grid_sync(p.bar, p.ctl, p.tstamp, 3 * t + 1, p.spin_limit, p.skip_mark)) return;
-        done = __ldcg(&ctl->fin_abort) != t + 1;
-        if (done) {
-            finish_roots<kW, kStats, false, false>(p, sm, t, par, c0, c1, cap, rec);
-            if (!grid_sync(p.bar, p.ctl, p.tstamp, -1, p.spin_limit, p.skip_mark)) return;
-            done = __ldcg(&ctl->fin_abort) != t + 1;
-        }
-        if (done) {
-            finish_roots<kW, kStats, true, true>(p, sm, t, par, c0, c1, cap, rec);
-            if (!grid_sync(p.bar, p.ctl, p.tstamp, 3 * t + 2, p.spin_limit, p.skip_mark)) return;
-        }
-    } else {
-        // speculative: a called-off attempt leaves only values that the
-        // resumed rounds write again
-        finish_scan<kW, kStats, true>(p, sm, t, par, c0, c1, cap, rec);
-        if (!grid_sync(p.bar, p.ctl, p.tstamp, 3 * t + 1, p.spin_limit, p.skip_mark)) return;
-        done = __ldcg(&ctl->fin_abort) != t + 1;
-        if (done) {
-            finish_roots<kW, kStats, true, false>(p, sm, t, par, c0, c1, cap, rec);
-            if (!grid_sync(p.bar, p.ctl, p.tstamp, 3 * t + 2, p.spin_limit, p.skip_mark)) return;
-            done = __ldcg(&ctl->fin_abort) != t + 1;
-        }
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (done) {
-            const int last = max(__ldcg(&ctl->fin_last), __ldcg(&ctl->iso_last) - 1);
-            ctl->rounds = maximal ? min(last + 2, cap) : cap;
-            ctl->fin_state = kFinStateDone;
-            if (p.tstamp) p.tstamp[3 * t + 3] = p.tstamp[3 * t + 2];
-        } else {
-            ctl->fin_state = kFinStateResume;
-        }
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -2365,6 +2376,14 @@ __device__ __forceinline__ void warp_sort_desc(unsigned long long &k, int &nb, i
         for (int stride = size >> 1; stride > 0; stride >>= 1) cas_step(k, nb, j, lane, stride, (lane & size) == 0);
 }
 
+// Window offsets as the kernels read them: the first slot (even), and in bit 0
+// whether the list is longer than its window.
+__global__ void k_win_offsets(const int2 *ranges, const long long *off, int n, int *pwin_off)
+{
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
+        pwin_off[v] = (int)off[v] | (v < n && degree_of(ranges[v]) > kWin ? 1 : 0);
+}
+
 __global__ void k_win_sizes(const int2 *ranges, int n, long long *slots)
 {
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
@@ -2428,14 +2447,16 @@ __device__ __forceinline__ void win_top32(const int *nbrs, const float *w, int f
 
 __device__ __forceinline__ void win_store(int2 *pwin, long long off, int deg, int lane, unsigned long long k, int nb, int j)
 {
-    if (lane < win_len(deg)) pwin[off + lane] = make_int2(nb, k >= (1ull << 32) ? j : (int)((unsigned)j | 0x80000000u));
+    const int wl = win_len(deg);
+    if (lane < wl) pwin[off + lane] = make_int2(nb, k >= (1ull << 32) ? j : (int)((unsigned)j | 0x80000000u));
+    if (lane == wl && (wl & 1)) pwin[off + lane] = make_int2(-1, (int)0x80000000u);  // an odd window's filler
 }
 
 // Windows of lists of at most kWinChunk entries, a warp per list (vertices
 // dealt round-robin, so long lists spread over the grid); longer lists are
 // queued for the chunked kernels.
 __global__ void __launch_bounds__(256) k_win_build(const int2 *ranges, const int *nbrs, const float *w, int va, int vb,
-                                                   const long long *pwin_off, int2 *pwin, int *big, int *nbig)
+                                                   const int *pwin_off, int2 *pwin, int *big, int *nbig)
 {
     const int lane = threadIdx.x & 31;
     const long long gwarp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2451,7 +2472,7 @@ __global__ void __launch_bounds__(256) k_win_build(const int2 *ranges, const int
         unsigned long long k;
         int nb, j;
         win_top32(nbrs, w, r.x, r.y, lane, k, nb, j);
-        win_store(pwin, pwin_off[v], deg, lane, k, nb, j);
+        win_store(pwin, pwin_off[v] & ~1, deg, lane, k, nb, j);
     }
 }
 
@@ -2497,7 +2518,7 @@ __global__ void k_win_chunk_counts(const int2 *ranges, const int *big, int nbig,
 // Chunked lists, step 2: a warp per list merges its chunks' sorted best 32s.
 __global__ void __launch_bounds__(256) k_win_chunk_merge(const int2 *ranges, const int *big, int nbig,
                                                          const long long *chunk_off, const WinCand *cand,
-                                                         const long long *pwin_off, int2 *pwin)
+                                                         const int *pwin_off, int2 *pwin)
 {
     const int lane = threadIdx.x & 31;
     const long long gwarp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2518,7 +2539,7 @@ __global__ void __launch_bounds__(256) k_win_chunk_merge(const int2 *ranges, con
             for (int stride = 16; stride > 0; stride >>= 1) cas_step(k, nb, j, lane, stride, true);
         }
         const int v = big[i];
-        win_store(pwin, pwin_off[v], degree_of(ranges[v]), lane, k, nb, j);
+        win_store(pwin, pwin_off[v] & ~1, degree_of(ranges[v]), lane, k, nb, j);
     }
 }
 
@@ -2700,34 +2721,36 @@ __global__ void k_batch_rounds(const uint8_t *last, const int *goff, int ngraphs
     }
 }
 
-// Control block rounded to 256 bytes so the seeds that follow it stay aligned.
-constexpr size_t kCtlBytes = (sizeof(Ctl) + 255) / 256 * 256;
 constexpr int kStampCount = 3 * kMaxRounds + 1;
+constexpr size_t kResultBytes = 256;
+// Graphs of at most this many vertices are matched by one block: its rounds
+// need no grid barrier, and its reads stay in its L1.
+constexpr int kSoloVertices = 4096;
 
 struct PushState {
     uint8_t *col = nullptr;
     int2 *req = nullptr;
-    int2 *reqi = nullptr;
     unsigned long long *best = nullptr;
     unsigned long long *part_key = nullptr;
     int *part_cnt = nullptr;
-    int4 *list_mem = nullptr;
-    int4 *lists[2][kParityLists] = {};
+    int *list_mem = nullptr;          // the two parities' lists, list_cap items each
+    size_t list_cap = 0;
+    int *prop = nullptr;              // list_cap requests
+    uint32_t *prop_key = nullptr;     // list_cap key halves, once a type off the symmetric path needs them
+    int4 *rec = nullptr;              // finish phase: records, 3 int4 each, once a type on the symmetric path needs them
+    size_t rec_cap = 0;               // records that rec holds
     int4 *staged = nullptr;
     int *seg_first = nullptr;
-    uint32_t *seeds = nullptr;        // device: right after ctl in one allocation
-    Ctl *ctl = nullptr;
-    unsigned char *host_stage = nullptr;  // pinned: control block + seeds, uploaded in one copy
-    unsigned char *host_back = nullptr;   // pinned: control block read back
+    Ctl *ctl = nullptr;               // two control blocks, used by alternate calls
+    int ctl_turn = 0;
+    Result *result = nullptr;         // pinned: written by the kernel
     unsigned long long *stats = nullptr;
     unsigned long long *tstamp = nullptr;
-    unsigned *bar = nullptr;
-    int grid[2][3] = {{0, 0, 0}, {0, 0, 0}};  // co-resident blocks of k_rounds by weighting and mode
-    int fgrid[2][2] = {{0, 0}, {0, 0}};       // co-resident blocks of k_finish by weighting and stats
+    int grid[2][3] = {{0, 0, 0}, {0, 0, 0}};  // co-resident blocks of k_match by weighting and mode
     int sms = 0;                              // multiprocessors of the device
     // The last call on this state ended with every grid barrier complete (the
-    // barrier words are back at rest) and every fallback list combined (part_key
-    // and part_cnt all zero); false after a call that gave up or failed.
+    // next call's control block is clear) and every fallback list combined
+    // (part_key and part_cnt all zero); false after a call that gave up or failed.
     bool at_rest = false;
     bool zero_next = true;  // the call being launched resets them (the last one did not end at rest)
     float2 *wfeat = nullptr;              // learned colouring: (max, mean) incident weight per vertex
@@ -2738,47 +2761,37 @@ void free_state(PushState *s)
     // callers have synchronised the device (graph destroy or a failed set-up)
     dev_free(s->col, 0);
     dev_free(s->req, 0);
-    dev_free(s->reqi, 0);
     dev_free(s->best, 0);
     dev_free(s->part_key, 0);
     dev_free(s->part_cnt, 0);
     dev_free(s->list_mem, 0);
+    dev_free(s->prop, 0);
+    dev_free(s->prop_key, 0);
+    dev_free(s->rec, 0);
     dev_free(s->staged, 0);
     dev_free(s->seg_first, 0);
     dev_free(s->ctl, 0);
-    pinned_put(s->host_stage, kCtlBytes + 256 * sizeof(uint32_t));
-    pinned_put(s->host_back, kCtlBytes);
+    pinned_put(s->result, kResultBytes);
     dev_free(s->stats, 0);
     dev_free(s->tstamp, 0);
-    dev_free(s->bar, 0);
     dev_free(s->wfeat, 0);
     delete s;
-}
-
-template <bool kW, bool kStats>
-int coresident_finish_blocks(int sms)
-{
-    int occ = 0;
-    if (cudaFuncSetAttribute(k_finish<kW, kStats>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)) !=
-        cudaSuccess)
-        return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_finish<kW, kStats>, kThreads, sizeof(Smem)) != cudaSuccess)
-        return 0;
-    return occ * sms;
 }
 
 template <bool kW, bool kStats, bool kPolicy>
 int coresident_blocks(int sms)
 {
     int occ = 0;
-    if (cudaFuncSetAttribute(k_rounds<kW, kStats, kPolicy>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(k_match<kW, kStats, kPolicy>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(Smem)) != cudaSuccess)
         return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rounds<kW, kStats, kPolicy>, kThreads, sizeof(Smem)) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_match<kW, kStats, kPolicy>, kThreads, sizeof(Smem)) !=
         cudaSuccess)
         return 0;
     return occ * sms;
 }
+
+constexpr int kMaxBlocks = 1024;
 
 mm_status alloc_state(mm_graph *g, PushState **out)
 {
@@ -2792,27 +2805,22 @@ mm_status alloc_state(mm_graph *g, PushState **out)
     // lists longer than the window can fall back
     const size_t nseg_cap = (size_t)(g->long_entries / kSegEntries) + 2;
     const size_t nstaged = (size_t)(g->long_count > 0 ? g->long_count : 1);
+    // whatever the grid, its blocks' regions fit: (n / kChunk / blocks + 1) chunks each
+    s->list_cap = n + (size_t)kChunk * (kMaxBlocks + 1);
     // pooled on the legacy stream, then synchronised so that any stream may use them
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = dev_alloc((void **)&s->col, n, 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->req, n * sizeof(int2), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->reqi, n * sizeof(int2), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->best, n * sizeof(unsigned long long), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->part_key, n * sizeof(unsigned long long), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->part_cnt, n * sizeof(int), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->list_mem, 4 * n * sizeof(int4), 0);
+    if (e == cudaSuccess) e = dev_alloc((void **)&s->list_mem, 2 * s->list_cap * sizeof(int), 0);
+    if (e == cudaSuccess) e = dev_alloc((void **)&s->prop, s->list_cap * sizeof(int), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->staged, nstaged * sizeof(int4), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->seg_first, nseg_cap * sizeof(int), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->ctl, kCtlBytes + 256 * sizeof(uint32_t), 0);
-    if (e == cudaSuccess) s->seeds = reinterpret_cast<uint32_t *>(reinterpret_cast<unsigned char *>(s->ctl) + kCtlBytes);
-    if (e == cudaSuccess) e = pinned_get((void **)&s->host_stage, kCtlBytes + 256 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = pinned_get((void **)&s->host_back, kCtlBytes);
-    if (e == cudaSuccess)
-        e = dev_alloc((void **)&s->stats, sizeof(unsigned long long) * kMaxRounds * MM_STATS_COLS, 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->tstamp, sizeof(unsigned long long) * kStampCount, 0);
-    // two sets of barrier words: the round kernel's and the finish kernel's
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->bar, sizeof(unsigned) * 2 * kBarWords, 0);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->bar, 0, sizeof(unsigned) * 2 * kBarWords, 0);
+    if (e == cudaSuccess) e = dev_alloc((void **)&s->ctl, 2 * sizeof(Ctl), 0);
+    if (e == cudaSuccess) e = pinned_get((void **)&s->result, kResultBytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->ctl, 0, 2 * sizeof(Ctl), 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->part_key, 0, n * sizeof(unsigned long long), 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->part_cnt, 0, n * sizeof(int), 0);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
@@ -2823,9 +2831,6 @@ mm_status alloc_state(mm_graph *g, PushState **out)
         set_error(std::string("push: device allocation failed: ") + cudaGetErrorString(e));
         return MM_ERR_NOMEM;
     }
-    // a parity's two lists are adjacent: the finish phase uses both as one array of 2n
-    for (int par = 0; par < 2; ++par)
-        for (int l = 0; l < kParityLists; ++l) s->lists[par][l] = s->list_mem + (2 * par + l) * n;
     int sms = 0, dev = 0, coop = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -2837,30 +2842,21 @@ mm_status alloc_state(mm_graph *g, PushState **out)
     s->grid[1][0] = coresident_blocks<true, false, false>(sms);
     s->grid[1][1] = coresident_blocks<true, true, false>(sms);
     s->grid[1][2] = coresident_blocks<true, false, true>(sms);
-    s->fgrid[0][0] = coresident_finish_blocks<false, false>(sms);
-    s->fgrid[0][1] = coresident_finish_blocks<false, true>(sms);
-    s->fgrid[1][0] = coresident_finish_blocks<true, false>(sms);
-    s->fgrid[1][1] = coresident_finish_blocks<true, true>(sms);
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) {
         free_state(s);
         return cuda_fail(le, "push: kernel attributes");
     }
-    const int most = kBarMaxGroups * kBarGroup;
     bool over = false, under = false;
     for (int a = 0; a < 2; ++a) {
         for (int b = 0; b < 3; ++b) {
-            over |= s->grid[a][b] > most;
+            over |= s->grid[a][b] > kMaxBlocks;
             under |= s->grid[a][b] < 1;
-        }
-        for (int b = 0; b < 2; ++b) {
-            over |= s->fgrid[a][b] > most;
-            under |= s->fgrid[a][b] < 1;
         }
     }
     if (over) {
         free_state(s);
-        set_error("push: more co-resident blocks than the grid barrier supports");
+        set_error("push: more co-resident blocks than the lists are sized for");
         return MM_ERR_UNSUPPORTED;
     }
     if (!coop || under) {
@@ -2873,54 +2869,6 @@ mm_status alloc_state(mm_graph *g, PushState **out)
     return MM_OK;
 }
 
-Params make_params(mm_graph *g, PushState *s, bool weighted, bool stats, bool timing)
-{
-    Params p;
-    p.n = g->n;
-    p.contiguous = g->contiguous ? 1 : 0;
-    p.sym = (weighted ? g->sym_weights : g->sym_struct) ? 1 : 0;
-    p.ranges = g->d_ranges;
-    p.nbrs = g->d_nbrs;
-    p.w = g->d_w;
-    p.revkey = g->d_revkey[weighted ? 1 : 0];
-    p.slot_off = g->d_slot_off;
-    p.pwin = g->d_pwin;
-    p.wwin = weighted && g->pwin_weights ? 1 : 0;
-    p.pwin_off = g->d_pwin_off;
-    p.col = s->col;
-    p.req = s->req;
-    p.reqi = s->reqi;
-    p.best = s->best;
-    p.part_key = s->part_key;
-    p.part_cnt = s->part_cnt;
-    for (int par = 0; par < 2; ++par)
-        for (int l = 0; l < kParityLists; ++l) p.lists[par][l] = s->lists[par][l];
-    p.staged = s->staged;
-    p.seg_first = s->seg_first;
-    p.vbase = g->ngraphs > 0 ? g->d_vbase : nullptr;
-    p.last = g->ngraphs > 0 ? g->d_last : nullptr;
-    std::memset(p.mlp, 0, sizeof(p.mlp));
-    p.policy_const = 0;
-    p.policy_bar = 0u;
-    p.fin_retire = 0;
-    p.level = 0.0f;
-    p.wfeat = s->wfeat;
-    p.trace = nullptr;
-    p.trace_rounds = 0;
-    p.seeds = s->seeds;
-    p.ctl = s->ctl;
-    p.stats = stats ? s->stats : nullptr;
-    p.tstamp = timing ? s->tstamp : nullptr;
-    p.bar = s->bar;
-    p.resume = 0;
-    p.zero_parts = s->zero_next ? 1 : 0;
-    // at least 2: the finish phase's records take 4 slots an item in 2n
-    p.fin_div = g->opt_fin_div < 0 ? 0 : (g->opt_fin_div == 0 ? kFinDiv : max(g->opt_fin_div, 2));
-    p.spin_limit = debug_spin_limit();
-    p.skip_mark = debug_skip_mark();
-    return p;
-}
-
 struct PolicyArgs {
     const float *mlp = nullptr;  // host, MM_POLICY_FLOATS
     bool constant = false;       // output weights all zero: the threshold is constant_bar
@@ -2930,61 +2878,119 @@ struct PolicyArgs {
     int trace_rounds = 0;
 };
 
+// One matching call, between begin_call and end_call.
+struct Call {
+    mm_graph *g = nullptr;
+    PushState *s = nullptr;
+    int type = 0;
+    uint32_t barrier = 0u;
+    const uint32_t *seeds = nullptr;
+    int nseeds = 0;
+    int *match = nullptr;
+    bool stats = false, timing = false;
+    const PolicyArgs *pol = nullptr;
+    cudaStream_t stream = 0;
+};
+
 template <bool kW, bool kStats, bool kPolicy>
-mm_status launch_rounds(mm_graph *g, PushState *s, bool timing, cudaStream_t stream, const PolicyArgs *pol = nullptr)
+mm_status launch_match(const Call &c)
 {
-    Params prm = make_params(g, s, kW, kStats, timing);
+    mm_graph *g = c.g;
+    PushState *s = c.s;
+    const PolicyArgs *pol = c.pol;
+    Params p;
+    std::memset(&p, 0, sizeof p);
+    p.n = g->n;
+    p.contiguous = g->contiguous ? 1 : 0;
+    p.sym = (kW ? g->sym_weights : g->sym_struct) ? 1 : 0;
+    p.ranges = g->d_ranges;
+    p.nbrs = g->d_nbrs;
+    p.w = g->d_w;
+    p.revkey = g->d_revkey[kW ? 1 : 0];
+    p.slot_off = g->d_slot_off;
+    p.pwin = g->d_pwin;
+    p.pwin_off = g->d_pwin_off;
+    p.col = s->col;
+    p.req = s->req;
+    p.best = s->best;
+    p.part_key = s->part_key;
+    p.part_cnt = s->part_cnt;
+    p.lists[0] = s->list_mem;
+    p.lists[1] = s->list_mem + s->list_cap;
+    p.prop = s->prop;
+    p.staged = s->staged;
+    p.seg_first = s->seg_first;
+    p.vbase = g->ngraphs > 0 ? g->d_vbase : nullptr;
+    p.last = g->ngraphs > 0 ? g->d_last : nullptr;
+    p.wfeat = s->wfeat;
+    p.match = c.match;
+    p.barrier = c.barrier;
+    p.cap = max_rounds_of(c.type);
+    p.maximal = is_maximal(c.type) ? 1 : 0;
+    p.nseeds = c.nseeds < 256 ? c.nseeds : 256;
+    std::memcpy(p.seeds, c.seeds, sizeof(uint32_t) * (size_t)p.nseeds);
+    p.ctl = s->ctl + s->ctl_turn;
+    p.ctl_next = s->ctl + (s->ctl_turn ^ 1);
+    p.result = s->result;
+    p.stats = kStats ? s->stats : nullptr;
+    p.tstamp = c.timing ? s->tstamp : nullptr;
+    p.zero_parts = s->zero_next ? 1 : 0;
+    p.fin_div = g->opt_fin_div < 0 ? 0 : (g->opt_fin_div == 0 ? kFinDiv : max(g->opt_fin_div, 2));
+    p.spin_limit = debug_spin_limit();
+    p.skip_mark = debug_skip_mark();
     if (kPolicy) {
-        std::memcpy(prm.mlp, pol->mlp, sizeof(prm.mlp));
-        prm.policy_const = pol->constant ? 1 : 0;
-        prm.policy_bar = pol->constant_bar;
-        prm.level = pol->level;
-        prm.trace = pol->trace;
-        prm.trace_rounds = pol->trace_rounds;
+        std::memcpy(p.mlp, pol->mlp, sizeof(p.mlp));
+        p.policy_const = pol->constant ? 1 : 0;
+        p.policy_bar = pol->constant_bar;
+        p.level = pol->level;
+        p.trace = pol->trace;
+        p.trace_rounds = pol->trace_rounds;
         // the finish phase knows the policy's threshold, not its features
-        prm.fin_retire = pol->constant && !pol->trace ? 1 : 0;
+        p.fin_retire = pol->constant && !pol->trace ? 1 : 0;
         // Retirement shrinks the active set from round kRetireFrom on, so the
         // default threshold comes a round or two earlier than on the plain
-        // path, while components are still too large for the finish phase (on
-        // the R-MAT 2^22 hierarchy every level but the first called its attempt
-        // off, and the round kernel then played all the remaining rounds): the
+        // path, while components are still too large for the finish phase: the
         // default divisor is doubled here.
-        if (g->opt_fin_div == 0) prm.fin_div = 2 * kFinDiv;
+        if (g->opt_fin_div == 0) p.fin_div = 2 * kFinDiv;
     }
-    void *args[] = {&prm};
+    // blocks: all that fit at once, or the tuned number per SM (never more), and
+    // no more than give every thread a vertex
     const int mode = kPolicy ? 2 : (kStats ? 1 : 0);
-    // blocks: all that fit at once, or the tuned number per SM (never more)
     const int bps = g->opt_blocks_per_sm;
-    const int grid = bps > 0 ? min(s->grid[kW][mode], bps * s->sms) : s->grid[kW][mode];
-    const int fgrid = bps > 0 ? min(s->fgrid[kW][kStats ? 1 : 0], bps * s->sms) : s->fgrid[kW][kStats ? 1 : 0];
-    MM_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_rounds<kW, kStats, kPolicy>, dim3(grid),
-                                            dim3(kThreads), args, sizeof(Smem), stream),
-                "round kernel launch");
-    if ((!kPolicy || prm.fin_retire) && prm.sym) {
-        // the finish kernel (its own barrier words), then the round kernel again
-        // for the case that the finish phase is called off; each returns at once
-        // when there is nothing left for it
-        Params fin = prm;
-        fin.bar = s->bar + kBarWords;
-        void *fargs[] = {&fin};
-        MM_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_finish<kW, kStats>, dim3(fgrid),
-                                                dim3(kThreads), fargs, sizeof(Smem), stream),
-                    "finish kernel launch");
-        Params res = prm;
-        res.resume = 1;
-        void *rargs[] = {&res};
-        MM_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_rounds<kW, kStats, kPolicy>, dim3(grid),
-                                                dim3(kThreads), rargs, sizeof(Smem), stream),
-                    "round kernel launch (resumed)");
+    int grid = bps > 0 ? min(s->grid[kW][mode], bps * s->sms) : s->grid[kW][mode];
+    grid = g->n <= kSoloVertices ? 1 : min(grid, (g->n + kThreads - 1) / kThreads);
+    const int chunks = (int)(((long long)g->n + kChunk - 1) / kChunk);
+    p.region = (chunks + grid - 1) / grid * kChunk;
+    if (!p.sym) {
+        if (!s->prop_key)
+            MM_CUDA_TRY(dev_alloc((void **)&s->prop_key, sizeof(uint32_t) * s->list_cap, c.stream), "request keys");
+        p.prop_key = s->prop_key;
+    } else if (p.fin_div > 0 && grid > 1) {
+        // records for twice a block's share of the largest set the finish phase
+        // accepts (a block that holds more calls the attempt off)
+        p.rec_region = min(p.region, 2 * (p.region / p.fin_div) + kChunk);
+        const size_t need = (size_t)p.rec_region * grid;
+        if (need > s->rec_cap) {
+            dev_free(s->rec, c.stream);
+            s->rec = nullptr;
+            s->rec_cap = 0;
+            MM_CUDA_TRY(dev_alloc((void **)&s->rec, 3 * sizeof(int4) * need, c.stream), "finish records");
+            s->rec_cap = need;
+        }
+        p.rec = s->rec;
     }
+    void *args[] = {&p};
+    MM_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_match<kW, kStats, kPolicy>, dim3(grid), dim3(kThreads), args,
+                                            sizeof(Smem), c.stream),
+                "round kernel launch");
     return MM_OK;
 }
 
 // Shared set-up of one matching call: preparation, state, control block.
-mm_status begin_call(mm_graph *g, int type, uint32_t barrier, const uint32_t *seeds, int nseeds, int *d_match,
-                     cudaStream_t stream, PushState **out)
+mm_status begin_call(Call &c)
 {
-    mm_status st = push_prepare(g, is_weighted(type) ? 1 : 0, stream);
+    mm_graph *g = c.g;
+    mm_status st = push_prepare(g, is_weighted(c.type) ? 1 : 0, c.stream);
     if (st != MM_OK) return st;
     PushState *s = (PushState *)g->push_exec;
     if (!s) {
@@ -2992,53 +2998,41 @@ mm_status begin_call(mm_graph *g, int type, uint32_t barrier, const uint32_t *se
         if (st != MM_OK) return st;
         g->push_exec = s;
     }
-    // One pinned upload of control block + seeds.  The previous call on this
-    // graph synchronised its stream before returning, so the staging buffer is free.
-    // the barrier words: reset only after a call that did not end at rest; until
-    // this call ends well, the state counts as not at rest
+    c.s = s;
+    // the control blocks are reset only after a call that did not end at rest;
+    // until this call ends well, the state counts as not at rest
     s->zero_next = !s->at_rest;
     s->at_rest = false;
-    if (s->zero_next)
-        MM_CUDA_TRY(cudaMemsetAsync(s->bar, 0, sizeof(unsigned) * 2 * kBarWords, stream), "barrier clear");
-    Ctl *ctl = reinterpret_cast<Ctl *>(s->host_stage);
-    std::memset(ctl, 0, kCtlBytes);
-    ctl->match = d_match;
-    ctl->barrier = barrier;
-    ctl->cap = max_rounds_of(type);
-    ctl->maximal = is_maximal(type) ? 1 : 0;
-    ctl->nseeds = nseeds < 256 ? nseeds : 256;
-    std::memcpy(s->host_stage + kCtlBytes, seeds, sizeof(uint32_t) * ctl->nseeds);
-    MM_CUDA_TRY(cudaMemcpyAsync(s->ctl, s->host_stage, kCtlBytes + sizeof(uint32_t) * ctl->nseeds,
-                                cudaMemcpyHostToDevice, stream),
-                "control block");
-    *out = s;
+    if (s->zero_next) MM_CUDA_TRY(cudaMemsetAsync(s->ctl, 0, 2 * sizeof(Ctl), c.stream), "control block");
+    // the previous call on this graph synchronised its stream before returning
+    s->result->rounds = -1;
+    s->result->status = 0;
     return MM_OK;
 }
 
-mm_status end_call(mm_graph *g, PushState *s, int nseeds, int *rounds_out, long long *stats, int stats_rounds,
-                   unsigned long long *stamps, cudaStream_t stream)
+mm_status end_call(Call &c, int *rounds_out, long long *stats, int stats_rounds, unsigned long long *stamps)
 {
-    MM_CUDA_TRY(cudaMemcpyAsync(s->host_back, s->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, stream), "control read");
+    PushState *s = c.s;
     if (stats && stats_rounds > 0)
         MM_CUDA_TRY(cudaMemcpyAsync(stats, s->stats,
                                     sizeof(long long) * MM_STATS_COLS *
                                         (size_t)(stats_rounds < kMaxRounds ? stats_rounds : kMaxRounds),
-                                    cudaMemcpyDeviceToHost, stream),
+                                    cudaMemcpyDeviceToHost, c.stream),
                     "stats read");
     if (stamps)
         MM_CUDA_TRY(cudaMemcpyAsync(stamps, s->tstamp, sizeof(unsigned long long) * kStampCount,
-                                    cudaMemcpyDeviceToHost, stream),
+                                    cudaMemcpyDeviceToHost, c.stream),
                     "timestamps read");
-    MM_CUDA_TRY(cudaStreamSynchronize(stream), "round loop");
-    Ctl out;
-    std::memcpy(&out, s->host_back, sizeof out);
+    MM_CUDA_TRY(cudaStreamSynchronize(c.stream), "round loop");
+    const Result out = *s->result;
     // every barrier completed unless one gave up (status 2)
-    s->at_rest = out.status != 2;
-    if (out.status == 2) {
+    s->at_rest = out.status != 2 && out.rounds >= 0;
+    s->ctl_turn ^= 1;  // cleared by this call
+    if (!s->at_rest) {
         set_error("mm_match: a bounded grid-barrier wait in the round kernel gave up");
         return MM_ERR_DEVICE;
     }
-    if (out.status == 1 || out.rounds > nseeds) {
+    if (out.status == 1 || out.rounds > c.nseeds) {
         set_error("mm_match: fewer seeds than rounds");
         return MM_ERR_SEEDS;
     }
@@ -3046,17 +3040,25 @@ mm_status end_call(mm_graph *g, PushState *s, int nseeds, int *rounds_out, long 
     return MM_OK;
 }
 
-mm_status run_rounds(mm_graph *g, PushState *s, int type, bool stats, bool timing, cudaStream_t stream)
+// The counters' and timestamps' device arrays, once a call asks for them.
+mm_status run_rounds(Call &c)
 {
-    const bool w = is_weighted(type);
-    if (stats)
-        MM_CUDA_TRY(cudaMemsetAsync(s->stats, 0, sizeof(unsigned long long) * kMaxRounds * MM_STATS_COLS, stream),
-                    "stats clear");
-    if (w)
-        return stats ? launch_rounds<true, true, false>(g, s, timing, stream)
-                     : launch_rounds<true, false, false>(g, s, timing, stream);
-    return stats ? launch_rounds<false, true, false>(g, s, timing, stream)
-                 : launch_rounds<false, false, false>(g, s, timing, stream);
+    PushState *s = c.s;
+    if (c.stats) {
+        const size_t bytes = sizeof(unsigned long long) * kMaxRounds * MM_STATS_COLS;
+        if (!s->stats) MM_CUDA_TRY(dev_alloc((void **)&s->stats, bytes, c.stream), "stats");
+        MM_CUDA_TRY(cudaMemsetAsync(s->stats, 0, bytes, c.stream), "stats clear");
+    }
+    if (c.timing) {
+        const size_t bytes = sizeof(unsigned long long) * kStampCount;
+        if (!s->tstamp) MM_CUDA_TRY(dev_alloc((void **)&s->tstamp, bytes, c.stream), "timestamps");
+        MM_CUDA_TRY(cudaMemsetAsync(s->tstamp, 0, bytes, c.stream), "timestamps clear");
+    }
+    if (is_weighted(c.type))
+        return c.pol ? launch_match<true, false, true>(c)
+                     : (c.stats ? launch_match<true, true, false>(c) : launch_match<true, false, false>(c));
+    return c.pol ? launch_match<false, false, true>(c)
+                 : (c.stats ? launch_match<false, true, false>(c) : launch_match<false, false, false>(c));
 }
 
 }  // namespace
@@ -3256,19 +3258,26 @@ mm_status windows_begin(mm_graph *g, cudaStream_t stream)
     }
     int2 *win = nullptr;
     int *big = nullptr;  // [n + 1]: queued long lists, then their count
-    e = dev_alloc((void **)&win, sizeof(int2) * (size_t)(total > 0 ? total : 1), stream);
+    int *packed = nullptr;
+    e = dev_alloc((void **)&packed, sizeof(int) * ((size_t)n + 1), stream);
+    if (e == cudaSuccess) {
+        k_win_offsets<<<grid_for(n + 1ll, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, off, n, packed);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = dev_alloc((void **)&win, sizeof(int2) * (size_t)(total > 0 ? total : 1), stream);
     if (e == cudaSuccess) e = dev_alloc((void **)&big, sizeof(int) * ((size_t)n + 1), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(big + n, 0, sizeof(int), stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    dev_free(off, stream);
     if (e != cudaSuccess) {
         dev_free(win, stream);
         dev_free(big, stream);
-        dev_free(off, stream);
+        dev_free(packed, stream);
         return cuda_fail(e, "window buffers");
     }
     g->win_build = win;
     g->win_big = big;
-    g->d_pwin_off = off;
+    g->d_pwin_off = packed;
     return MM_OK;
 }
 
@@ -3286,7 +3295,7 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream)
     const int n = g->n;
     int *big = g->win_big;
     int2 *win = g->win_build;
-    const long long *off = g->d_pwin_off;
+    const int *off = g->d_pwin_off;
     int nbig = 0;
     cudaError_t e = cudaMemcpyAsync(&nbig, big + n, sizeof(int), cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -3344,11 +3353,11 @@ namespace {
 // weight, so a proposal needs no dependent load of it (the proposal key is the
 // weight and the proposer's id).  An entry flagged as never chosen keeps a
 // weight that fails the same test (<= -1 or NaN).
-__global__ void k_win_weights(const int2 *ranges, const float *w, const long long *pwin_off, int2 *pwin, int n)
+__global__ void k_win_weights(const int2 *ranges, const float *w, const int *pwin_off, int2 *pwin, int n)
 {
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int wl = win_len(degree_of(ranges[v]));
-        const long long o = pwin_off[v];
+        const int o = pwin_off[v] & ~1;
         for (int e = 0; e < wl; ++e) {
             int2 x = pwin[o + e];
             x.y = __float_as_int(__ldg(w + (x.y & 0x7fffffff)));
@@ -3412,12 +3421,11 @@ mm_status push_match(mm_graph *g, int type, uint32_t barrier, const uint32_t *se
         }
         return MM_OK;
     }
-    PushState *s = nullptr;
-    mm_status st = begin_call(g, type, barrier, seeds, nseeds, d_match, stream, &s);
+    Call c{g, nullptr, type, barrier, seeds, nseeds, d_match, stats != nullptr, false, nullptr, stream};
+    mm_status st = begin_call(c);
+    if (st == MM_OK) st = run_rounds(c);
     if (st != MM_OK) return st;
-    st = run_rounds(g, s, type, stats != nullptr, false, stream);
-    if (st != MM_OK) return st;
-    return end_call(g, s, nseeds, rounds_out, stats, stats_rounds, nullptr, stream);
+    return end_call(c, rounds_out, stats, stats_rounds, nullptr);
 }
 
 // The round kernel with the learned colouring: each vertex's blue probability
@@ -3429,9 +3437,10 @@ mm_status push_match_policy(mm_graph *g, int type, uint32_t barrier, const uint3
                             int trace_rounds, cudaStream_t stream)
 {
     if (g->n == 0) return push_match(g, type, barrier, seeds, nseeds, d_match, rounds_out, nullptr, 0, stream);
-    PushState *s = nullptr;
-    mm_status st = begin_call(g, type, barrier, seeds, nseeds, d_match, stream, &s);
+    Call c{g, nullptr, type, barrier, seeds, nseeds, d_match, false, false, nullptr, stream};
+    mm_status st = begin_call(c);
     if (st != MM_OK) return st;
+    PushState *s = c.s;
     if (!s->wfeat) {
         cudaError_t e = dev_alloc((void **)&s->wfeat, sizeof(float2) * (size_t)g->n, stream);
         if (e == cudaSuccess) {
@@ -3459,10 +3468,10 @@ mm_status push_match_policy(mm_graph *g, int type, uint32_t barrier, const uint3
     pol.level = level;
     pol.trace = trace;
     pol.trace_rounds = trace ? trace_rounds : 0;
-    st = is_weighted(type) ? launch_rounds<true, false, true>(g, s, false, stream, &pol)
-                           : launch_rounds<false, false, true>(g, s, false, stream, &pol);
+    c.pol = &pol;
+    st = run_rounds(c);
     if (st != MM_OK) return st;
-    return end_call(g, s, nseeds, rounds_out, nullptr, 0, nullptr, stream);
+    return end_call(c, rounds_out, nullptr, 0, nullptr);
 }
 
 // Same launch as push_match with barrier timestamps on: block 0 reads the
@@ -3472,14 +3481,12 @@ mm_status push_profile(mm_graph *g, int type, uint32_t barrier, const uint32_t *
                        int *rounds_out, float *ms_phases, int cap_rounds, int *launched, cudaStream_t stream)
 {
     if (g->n == 0) return push_match(g, type, barrier, seeds, nseeds, d_match, rounds_out, nullptr, 0, stream);
-    PushState *s = nullptr;
-    mm_status st = begin_call(g, type, barrier, seeds, nseeds, d_match, stream, &s);
-    if (st != MM_OK) return st;
-    MM_CUDA_TRY(cudaMemsetAsync(s->tstamp, 0, sizeof(unsigned long long) * kStampCount, stream), "timestamps clear");
-    st = run_rounds(g, s, type, false, true, stream);
+    Call c{g, nullptr, type, barrier, seeds, nseeds, d_match, false, true, nullptr, stream};
+    mm_status st = begin_call(c);
+    if (st == MM_OK) st = run_rounds(c);
     if (st != MM_OK) return st;
     unsigned long long stamps[kStampCount];
-    st = end_call(g, s, nseeds, rounds_out, nullptr, 0, stamps, stream);
+    st = end_call(c, rounds_out, nullptr, 0, stamps);
     if (st != MM_OK) return st;
     if (ms_phases) {
         const int r_exec = *rounds_out;
@@ -3496,7 +3503,7 @@ mm_status push_profile(mm_graph *g, int type, uint32_t barrier, const uint32_t *
             ms_phases[(size_t)r * MM_PROFILE_KERNELS + 3] = a + b + c;
         }
     }
-    if (launched) *launched = (is_weighted(type) ? g->sym_weights : g->sym_struct) ? 3 : 1;
+    if (launched) *launched = 1;
     return MM_OK;
 }
 

@@ -15,16 +15,19 @@ namespace mm {
 constexpr int kFixedRounds = 20;
 constexpr int kMaxRounds = 255;
 
-// Per-vertex colour state used by the kernels ("col"): one byte per vertex.
-// It carries exactly what a neighbour's request/respond test needs from the
-// reference's match value (src/matchgpu.cu:303-316, 380-386, 346, 431):
-//   kBlue (match 0), kRed (match 1), kDead (match 2), kMatched (match >= 4).
+// Per-vertex colour state.  It carries what a neighbour's request/respond test
+// needs from the reference's match value (src/matchgpu.cu:303-316, 380-386,
+// 346, 431): kBlue (match 0), kRed (match 1), kDead (match 2), kMatched (match >= 4).
 enum : uint8_t { kBlue = 0, kRed = 1, kDead = 2, kMatched = 3 };
 
 // Colouring hash of src/matchgpu.cu:196-217: 16 MD5-style steps over
 // (vertex id, round seed) with the first 16 SHA-256 constants, the MD5
-// round-1 rotations and the MD5 initial words.  Returns h0 + h1 + h2 + h3,
-// accumulated as one running sum (the four words are only ever added).
+// round-1 rotations and the MD5 initial words.  The reference adds up
+// h0 + h1 + h2 + h3 before the first step and after each.  A step moves the
+// four words along (h0 <- h3 <- h2 <- h1) and makes one new one, so with B_k
+// the word that step k makes, the sum is a constant plus 4 (B_1 + .. + B_13)
+// + 3 B_14 + 2 B_15 + B_16: one addition a step in place of four.  Set-up and
+// commit passes over millions of vertices are bound by these instructions.
 __device__ __forceinline__ uint32_t colour_hash(uint32_t v, uint32_t seed)
 {
     constexpr uint32_t K[16] = {0x428a2f98u, 0x71374491u, 0xb5c0fbcfu, 0xe9b5dba5u,
@@ -32,19 +35,19 @@ __device__ __forceinline__ uint32_t colour_hash(uint32_t v, uint32_t seed)
                                 0xd807aa98u, 0x12835b01u, 0x243185beu, 0x550c7dc3u,
                                 0x72be5d74u, 0x80deb1feu, 0x9bdc06a7u, 0xc19bf174u};
     constexpr int R[4] = {7, 12, 17, 22};
-    uint32_t a = 0x67452301u, b = 0xefcdab89u, c = 0x98badcfeu, d = 0x10325476u;
-    uint32_t sum = a + b + c + d;
-    uint32_t g = v;
+    constexpr uint32_t A = 0x67452301u, B = 0xefcdab89u, C = 0x98badcfeu, D = 0x10325476u;
+    uint32_t a = A, b = B, c = C, d = D;
+    uint32_t g = v, run = 0u, sum = A + 2u * D + 3u * C + 4u * B;
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
         const uint32_t f = (b & c) | (~b & d);
-        const uint32_t x = a + f + K[k] + g;
-        const uint32_t t = d;
+        const uint32_t x = a + f + (K[k] + g);
+        a = d;
         d = c;
         c = b;
         b = b + __funnelshift_l(x, x, R[k & 3]);
-        a = t;
-        sum += a + b + c + d;
+        run += b;
+        if (k >= 12) sum += run;
         g *= seed;
     }
     return sum;
@@ -103,7 +106,7 @@ struct mm_graph {
     unsigned long long *d_revkey[2] = {nullptr, nullptr};  // [0] random, [1] weighted
     long long *d_slot_off = nullptr;  // non-contiguous CSR: slot index of vertex v's first entry
     int2 *d_pwin = nullptr;           // weighted types: preference windows {neighbour, position | flag}
-    int *d_pwin_off = nullptr;        // weighted types, [n + 1]: first window slot (even), bit 0: list longer than 32
+    int *d_pwin_off = nullptr;        // weighted types, [n + 1]: first group of 4 window entries, bit 31: list longer than 32
     bool pwin_weights = false;        // d_pwin's second words hold weights (symmetric weighted path)
     int2 *win_build = nullptr;        // windows while being built (d_pwin once complete)
     int *win_big = nullptr;           // while being built: queued lists longer than a window chunk

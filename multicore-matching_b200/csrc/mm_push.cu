@@ -29,7 +29,7 @@
 // vertices are dealt to the blocks in chunks of 64, and a block keeps the ones
 // that can still be matched in lists of its own (4 bytes an item: the vertex).
 // So no counter, list or request is shared between blocks: all that crosses
-// them are the colour bytes, the proposals' atomic maxima and the barriers.
+// them are the colours, the proposals' atomic maxima and the barriers.
 //   windows        a blue vertex's choice is the first red candidate among its
 //                  best min(deg, 32) entries in order of preference (weight,
 //                  then position; list order for random types), stored at
@@ -78,8 +78,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kWin = 32;                 // preference window: the first min(deg, 32) choices
 constexpr int kChunk = 64;               // vertices dealt to the blocks at a time
-constexpr int kSegEntries = 256;         // entries per fallback segment: 8 rows of 32; at most 9
-                                         // pieces of lists > 32 entries overlap one segment
+constexpr int kPiece = 2048;             // shared fallback lists: entries a warp scans
 
 // Request codes of a blue item (a target vertex otherwise).
 enum : int { kReqDead = -1, kReqNone = -2, kReqShared = -3 };
@@ -91,7 +90,7 @@ constexpr int kRing = 4;        // barrier words in use by turns
 constexpr int kRingStride = 16; // words of 8 bytes per barrier line (128 bytes)
 struct Ctl {
     unsigned long long ring[kRing * kRingStride];  // (sum << 32) | blocks arrived
-    unsigned long long staged_pack;  // shared fallback list of the round: (items << 32) | entries
+    unsigned long long staged_pack;  // shared fallback list of the round: (items << 32) | pieces
     int fin_abort;         // finish phase: t + 1 if the attempt in round t was called off
     int fin_last;          // finish phase: last round in which any of its vertices was active
     int iso_last;          // 1 + the last round in which a vertex without neighbours was active (0: none)
@@ -109,17 +108,18 @@ struct Params {
     int contiguous;
     int sym;                        // proposal keys computed from the proposer's entry (no reverse index)
     int region;                     // list slots of a block
+    uint32_t turn_magic;            // floor(2^32 / blocks) + 1
     const int2 *ranges;
     const int *nbrs;
     const float *w;
     const unsigned long long *revkey;
     const long long *slot_off;
-    // weighted: preference windows, {neighbour, weight} on the symmetric path,
-    // else {neighbour, position | flag}; an odd window ends with a filler
-    // {-1, flag}
+    // weighted: preference windows in groups of four entries (32 bytes, one
+    // load), {neighbour, weight} on the symmetric path, else {neighbour,
+    // position | flag}; the last group is filled up with {-1, flag}
     const int2 *pwin;
-    const int *pwin_off;            // weighted, [n + 1]: first window slot (even), bit 0: list longer than the window
-    uint8_t *col;
+    const int *pwin_off;            // weighted, [n + 1]: first group, bit 31: list longer than the window
+    uint32_t *col;                  // colours, two bits a vertex
     int2 *req;                      // per vertex: proposal of a shared fallback list {target or code, key low half};
                                     // finish phase: a vertex's record
     int *lists[2];                  // items (vertices) by round parity: block b's region starts at b * region,
@@ -129,8 +129,8 @@ struct Params {
     unsigned long long *best;       // per red vertex: max proposal key this round
     unsigned long long *part_key;   // per cut fallback list: max over finished pieces
     int *part_cnt;                  // per cut fallback list: finished pieces
-    int4 *staged;                   // shared fallback items {v, begin, end, entry offset}
-    int *seg_first;                 // per fallback segment: item holding its first entry
+    int4 *staged;                   // shared fallback items {v, begin, end, first piece}
+    int *piece_item;                // per piece of the shared fallback lists: its item
     int4 *rec;                      // finish phase: records (3 int4 an item), rec_region of them for a block
     int rec_region;
     int *match;                     // output array of this call
@@ -198,11 +198,13 @@ __device__ __forceinline__ void stat_add(const P &p, int round, int col, unsigne
 // chunk q * gridDim.x + (b + 61 q) % gridDim.x of the vertex range.  The turn
 // by 61 keeps a block off one residue: ids cluster by degree (R-MAT hubs have
 // ids with low bits zero), and a plain stride of a multiple of 8 blocks would
-// give every eighth block the hubs.
+// give every eighth block the hubs.  The remainder comes from a multiplication
+// (exact: b + 61 q < 61 n / (64 blocks) + blocks, times blocks, stays below 2^32).
 __device__ __forceinline__ int own_vertex(const Params &p, int k)
 {
     const unsigned nb = gridDim.x, q = (unsigned)k / kChunk;
-    const unsigned c = q * nb + (blockIdx.x + 61u * q) % nb;
+    const unsigned x = blockIdx.x + 61u * q;
+    const unsigned c = nb == 1u ? q : q * nb + (x - __umulhi(x, p.turn_magic) * nb);
     const unsigned v = c * kChunk + (unsigned)k % kChunk;
     return v < (unsigned)p.n ? (int)v : -1;
 }
@@ -214,31 +216,38 @@ __device__ __forceinline__ unsigned long long global_ns()
     return t;
 }
 
-// L2 residency: the colour bytes, which every scan reads at random, are loaded
-// with an evict-last policy, the streamed worklists and requests with
-// evict-first (.cs) loads and stores.
-__device__ __forceinline__ unsigned long long pol_keep()
+// Colours are packed two bits a vertex, 16 to a word: the scans' gathers are
+// bound by the sectors they request from L2, and a matching's colours then fit
+// L1 (up to half a million vertices) or mostly hit it.  A chunk's words belong
+// to one block, which changes them by atomic XOR.  What scans need to tell
+// apart is red, matched and neither: a vertex that becomes unmatchable keeps
+// its colour's bits (blue, or red where no unmatched vertex lists it).
+__device__ __forceinline__ unsigned colour_bits(uint32_t word, int u)
 {
-    unsigned long long p;
-    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-    return p;
+    return __funnelshift_r(word, word, 2u * (unsigned)u) & 3u;  // the shift is taken modulo 32
 }
-__device__ __forceinline__ uint8_t ld_col(const uint8_t *a)
-{
-    unsigned short r;
-    asm volatile("ld.global.L2::cache_hint.u8 %0, [%1], %2;" : "=h"(r) : "l"(a), "l"(pol_keep()));
-    return (uint8_t)r;
-}
-// At the end of a matching the colour bytes go back to the normal eviction
-// priority, so that they do not crowd the L2 of the work that follows.
-template <class T>
-__device__ __forceinline__ void release_lines(const T *a, long long count)
-{
-    const uintptr_t lo = (uintptr_t)a & ~(uintptr_t)127, hi = (uintptr_t)(a + count);
-    const long long lines = (long long)((hi - lo + 127) / 128);
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < lines; i += (long long)gridDim.x * blockDim.x)
-        asm volatile("applypriority.global.L2::evict_normal [%0], 128;" ::"l"(lo + (uintptr_t)i * 128) : "memory");
-}
+
+// A matching's working arrays: in global memory, or (kSolo, a graph that one
+// block matches) in that block's shared memory.
+template <bool kSolo>
+struct Mem {
+    uint32_t *col_;
+    unsigned long long *best_;
+    __device__ __forceinline__ unsigned col(int u) const { return colour_bits(col_[(unsigned)u >> 4], u); }
+    __device__ __forceinline__ void flip(int v, unsigned delta) const
+    {
+        atomicXor(col_ + ((unsigned)v >> 4), delta << (2u * ((unsigned)v & 15u)));
+    }
+    __device__ __forceinline__ unsigned long long best(int v) const { return kSolo ? best_[v] : __ldcg(best_ + v); }
+    __device__ __forceinline__ void propose(int v, unsigned long long key) const { atomicMax(best_ + v, key); }
+    // list items, streamed
+    static __device__ __forceinline__ int item(const int *a) { return kSolo ? *a : __ldcs(a); }
+    static __device__ __forceinline__ void put(int *a, int v)
+    {
+        if (kSolo) *a = v;
+        else __stcs(a, v);
+    }
+};
 
 // Key under which a blue vertex ranks a red neighbour at position j
 // (gwRequest: strict > from -1, earliest j on ties; grRequest: earliest j).
@@ -267,7 +276,7 @@ __device__ __forceinline__ unsigned long long strip_key(float bw, int bj, bool a
 // lane's running best: strict > from -1 over increasing positions, so ties
 // keep the earliest entry; in random mode the first red entry.
 template <bool kW>
-__device__ __forceinline__ void fold_entry(uint8_t c, float w, int j, float &bw, int &bj, bool &alive)
+__device__ __forceinline__ void fold_entry(unsigned c, float w, int j, float &bw, int &bj, bool &alive)
 {
     alive |= c != kMatched;
     if (c == kRed) {
@@ -279,15 +288,95 @@ __device__ __forceinline__ void fold_entry(uint8_t c, float w, int j, float &bw,
     }
 }
 
-// Where a blue vertex's request goes: the item's slot, or (shared fallback
-// lists) the vertex's own word.
+constexpr int kRows = 4;    // fallback scans: rows of 32 entries per iteration
+
+// Window scan: the block's lists that go to a fallback scan.
+constexpr int kStageCap = 1024;
+struct FallbackStage {
+    int2 item[kStageCap];          // {vertex, list slot}
+    unsigned short big[kStageCap]; // the ones the whole block scans
+};
+
+// Requests of the block's first kPropCap blue items, from the window scan to
+// the commit (the rest are in global memory): a request is a 4-byte store of
+// its own, which cost the scan of RGG 2^20's round 0 a fifth of its time.
+constexpr int kPropCap = 4800;
+struct Requests {
+    int target[kPropCap];
+};
+
+constexpr int kPer = 4;  // items a lane handles at a time in the set-up and commit passes
+
+// Set-up: a warp's stack of vertices without neighbours, {vertex, next round}.
+constexpr int kIsoCap = 31 + 32 * kPer;
+struct IsoStack {
+    int2 item[kWarps][kIsoCap];
+    uint32_t seeds[256];
+};
+
+// ---- finish phase: a warp's component ----
+constexpr int kFinMembers = 32;    // members of a component played by one warp (one per lane)
+constexpr int kFinEntries = 128;   // entries between members of one component
+
+// One warp's component: members' first entry, the entries between members
+// (preference key and the target's member slot), the members' colours of the
+// round being played and the best proposal each received.
+struct FinWarp {
+    unsigned long long pref[kFinEntries];
+    unsigned long long best[kFinMembers];
+    int mem[kFinMembers];
+    int eoff[kFinMembers + 1];
+    uint8_t tgt[kFinEntries];
+    uint8_t st[kFinMembers];
+};
+
+// Shared memory of the round kernel (dynamic); the phases' working areas share
+// it.  Two blocks fit the 64 KB configuration, which leaves the rest to L1.
+struct Smem {
+    union {
+        IsoStack iso;
+        struct {
+            FallbackStage fb;
+            Requests req;
+        };
+        FinWarp fin[kWarps];
+    };
+    unsigned long long red_key[kWarps];   // block-wide list scan: the warps' best keys
+    int count[2][2];                      // the block's items by round parity and colour
+    unsigned sync_sum;                    // grid barrier: the sum it carried
+    int sync_ok;
+    int wnext;                            // window scan: next item of the block
+    int stage_n;                          // window scan: fallback lists collected by the block
+    int big_n;                            // window scan: of those, lists for the whole block
+    int flag;                             // window scan: lists appended to the shared list; finish phase: called off
+    int zero;                             // 0
+};
+static_assert(sizeof(Smem) <= 31 * 1024, "two blocks a multiprocessor in the 64 KB configuration");
+constexpr size_t kSmemBytes = (sizeof(Smem) + 127) / 128 * 128;
+
+// Graphs of at most this many vertices are matched by one block: its rounds
+// need no grid barrier, and its working arrays follow in its shared memory.
+constexpr int kSoloVertices = 4096;
+struct SoloMem {
+    unsigned long long best[kSoloVertices];
+    int lists[2][kSoloVertices];
+    uint32_t col[kSoloVertices / 16];
+};
+static_assert(kSoloVertices <= kPropCap, "its requests stay in shared memory too");
+
+// Where a blue vertex's request goes: the item's slot (in shared memory, or
+// past its capacity in global memory), or for shared fallback lists the
+// vertex's own word.
 struct ItemReq {
     const Params &p;
-    long long slot;
+    Smem &sm;
+    long long rbase;
+    int i;
     __device__ __forceinline__ void put(int target, uint32_t low) const
     {
-        __stcs(p.prop + slot, target);
-        if (!p.sym) __stcs(p.prop_key + slot, low);
+        if (i < kPropCap) sm.req.target[i] = target;
+        else __stcs(p.prop + rbase + i, target);
+        if (!p.sym) __stcs(p.prop_key + rbase + i, low);
     }
 };
 struct VertexReq {
@@ -298,8 +387,8 @@ struct VertexReq {
 
 // Blue vertex v proposes to `target`, the neighbour at position j of its list
 // (begin = first position): the reverse key of that slot goes to best[target].
-template <bool kW, class Req>
-__device__ __forceinline__ void propose_to(const Params &p, Req rq, int v, int begin, int j, int target)
+template <bool kW, bool kSolo, class Req>
+__device__ __forceinline__ void propose_to(const Params &p, const Mem<kSolo> &m, Req rq, int v, int begin, int j, int target)
 {
     unsigned long long rk;
     if (p.sym) {
@@ -315,18 +404,18 @@ __device__ __forceinline__ void propose_to(const Params &p, Req rq, int v, int b
         const long long slot = p.contiguous ? (long long)j : __ldg(p.slot_off + v) + (j - begin);
         rk = __ldg(p.revkey + slot);
     }
-    if (rk) atomicMax(&p.best[target], rk);
+    if (rk) m.propose(target, rk);
     rq.put(target, (uint32_t)rk);
 }
 
 // Symmetric weighted path: blue v proposes to `target` through an entry of
 // weight w (w > -1); the target's entry for v has the same weight, and v's id
 // breaks ties (smaller first).
-template <class Req>
-__device__ __forceinline__ void propose_weight(const Params &p, Req rq, int v, float w, int target)
+template <bool kSolo, class Req>
+__device__ __forceinline__ void propose_weight(const Mem<kSolo> &m, Req rq, int v, float w, int target)
 {
     const unsigned long long rk = ((unsigned long long)weight_order(w) << 32) | (uint32_t)~v;
-    atomicMax(&p.best[target], rk);
+    m.propose(target, rk);
     rq.put(target, (uint32_t)rk);
 }
 
@@ -336,7 +425,6 @@ template <class Req>
 __device__ __forceinline__ void no_proposal(const Params &p, Req rq, int v, bool alive, int t)
 {
     if (!alive) {
-        p.col[v] = kDead;
         p.match[v] = 2;
         if (p.last) p.last[v] = (uint8_t)t;
         rq.put(kReqDead, 0u);
@@ -355,8 +443,8 @@ __device__ __forceinline__ unsigned long long request_seen(int begin, int deg, i
 }
 
 // Finish blue vertex v (entries from `begin`, deg of them) after a full scan whose result is `key`.
-template <bool kW, bool kStats, class Req>
-__device__ __forceinline__ void propose_key(const Params &p, Req rq, int v, int begin, int deg, unsigned long long key,
+template <bool kW, bool kStats, bool kSolo, class Req>
+__device__ __forceinline__ void propose_key(const Params &p, const Mem<kSolo> &m, Req rq, int v, int begin, int deg, unsigned long long key,
                                             int t)
 {
     if (kStats) {
@@ -369,84 +457,14 @@ __device__ __forceinline__ void propose_key(const Params &p, Req rq, int v, int 
         return;
     }
     const int j = (int)~(uint32_t)key;
-    propose_to<kW>(p, rq, v, begin, j, __ldg(p.nbrs + j));
+    propose_to<kW>(p, m, rq, v, begin, j, __ldg(p.nbrs + j));
 }
-
-constexpr int kRows = 4;    // fallback scans: rows of 32 entries per iteration
-constexpr int kStages = 3;  // shared fallback scan: iterations staged in shared memory (2 loading, 1 in use)
-
-// Shared-fallback staging of one warp: neighbour ids and weights of kStages
-// iterations, written by cp.async.
-struct LongStage {
-    int nb[kStages][kRows * 32];
-    float w[kStages][kRows * 32];
-};
-
-// Window scan: the block's lists that go to a fallback scan.
-constexpr int kStageCap = 4096;
-struct FallbackStage {
-    int2 item[kStageCap];          // {vertex, list slot}
-    unsigned short big[kStageCap]; // the ones the whole block scans
-};
-
-// Set-up: queue of vertices without neighbours (two halves).
-constexpr int kIsoHalf = 6144;
-struct IsoQueue {
-    int half[2][kIsoHalf];
-};
-
-struct LongScan {
-    int delta[kWarps][33];                // global position of segment entry e = e + delta[k]
-    int pend[kWarps][33];                 // segment-relative end of each piece
-    LongStage stage[kWarps];
-};
-
-// ---- finish phase: a warp's component ----
-constexpr int kFinMembers = 32;    // members of a component played by one warp (one per lane)
-constexpr int kFinEntries = 128;   // entries between members of one component
-
-// One warp's component: members' first entry, list start and degree, the
-// entries between members (preference key and the target's member slot), the
-// members' colours of the round being played and the best proposal each
-// received.
-struct FinWarp {
-    unsigned long long pref[kFinEntries];
-    unsigned long long best[kFinMembers];
-    int mem[kFinMembers];
-    int eoff[kFinMembers + 1];
-    int mbeg[kFinMembers];
-    int mdeg[kFinMembers];
-    uint8_t tgt[kFinEntries];
-    uint8_t st[kFinMembers];
-};
-
-// Shared memory of the round kernel (dynamic); the phases' working areas share it.
-struct Smem {
-    union {
-        IsoQueue iso;
-        FallbackStage fb;
-        LongScan ls;
-        FinWarp fin[kWarps];
-    };
-    unsigned tile_cnt[2][kWarps];         // compaction: per-warp counts, (red << 16) | blue, by tile parity
-    unsigned long long red_key[kWarps];   // block-wide list scan: the warps' best keys
-    unsigned sync_sum;                    // grid barrier: the sum it carried
-    int sync_ok;
-    int wnext;                            // window scan: next item of the block
-    int iso_n;                            // set-up: queued vertices without neighbours
-    int iso_cnt[3];                       // set-up: survivors of a round of the queue (rotating)
-    int stage_n;                          // window scan: fallback lists collected by the block
-    int big_n;                            // window scan: of those, lists for the whole block
-    int big_next;
-    int shared_n;                         // window scan: lists appended to the shared list
-};
-static_assert(sizeof(Smem) <= 56 * 1024, "two blocks per multiprocessor, with room for L1");
 
 // ---- grid barrier ----
 //
 // The kernel is launched cooperatively, so all its blocks are resident at once
 // and a barrier over them cannot deadlock on scheduling.  Each block adds
-// (its summand << 32) | 1 to the barrier's word and polls until all blocks
+// (its summand, part[0] + part[1] in shared memory, << 32) | 1 to the barrier's word and polls until all blocks
 // have: one release-add and one round trip after the last arrival (2500
 // cycles over 148 blocks, where a two-level tree of counters took 3800), and
 // the sum of the summands comes with it.  The words are used by turns; block 0
@@ -457,7 +475,7 @@ static_assert(sizeof(Smem) <= 56 * 1024, "two blocks per multiprocessor, with ro
 // barrier.  Thread 0's release and acquire, with the block barriers around
 // them, make every block's writes of the phase visible to every thread of
 // every block afterwards.
-__device__ __noinline__ bool grid_sync(Smem &sm, Ctl *ctl, unsigned &turn, unsigned add, unsigned *sum, Result *result,
+__device__ __noinline__ bool grid_sync(Smem &sm, Ctl *ctl, unsigned &turn, const int *part, unsigned *sum, Result *result,
                                        unsigned long long *tstamp, int mark, long long spin_limit, int skip_mark)
 {
     const unsigned nb = gridDim.x, w = turn & (kRing - 1);
@@ -465,6 +483,7 @@ __device__ __noinline__ bool grid_sync(Smem &sm, Ctl *ctl, unsigned &turn, unsig
     __syncthreads();
     if (threadIdx.x == 0) {
         int ok = 1;
+        const unsigned add = (unsigned)(part[0] + part[1]);
         unsigned total = add;
         // testing hook: block 0 leaves this barrier out, so every wait on it runs out
         const bool skip = blockIdx.x == 0 && mark >= 0 && mark == skip_mark;
@@ -585,102 +604,83 @@ __device__ __forceinline__ bool colour_blue(const Params &p, int v, int base, fl
 
 // ---- worklist compaction for the set-up and commit passes ----
 //
-// A block handles tiles of up to kTileItems items, a warp up to 128 consecutive
-// ones of them (lane l items l, l + 32, l + 64, l + 96), so that a list keeps
-// its vertices in increasing order.  The warps' counts meet in shared memory (one
-// block barrier a tile: the two parities' words are used by turns) and each
-// warp adds up those before it.  The block's running counts (cb blue, cr red)
-// are the same in every thread.
-constexpr int kPer = 4;
-constexpr int kTileItems = kThreads * kPer;
+// A warp handles tiles of up to 128 consecutive items (lane l items l, l + 32,
+// l + 64, l + 96) and takes its places in the block's lists with one shared
+// atomic a tile and colour, so no warp waits for another: with block-wide
+// prefix sums, three block barriers a tile left the set-up of R-MAT 2^22 at
+// half the instruction rate its pipes allow.
 enum : int { kDrop = -1, kToBlue = 0, kToRed = 1 };
 
-// Items a lane handles in a tile (fewer when the block has few, so that all
-// warps share them), and its first one.
+// Items a lane handles in a tile: fewer when the block has few, so that all
+// warps share them.
 __device__ __forceinline__ int tile_per(int total) { return min(kPer, max(1, (total + kThreads - 1) / kThreads)); }
-__device__ __forceinline__ int tile_first(int per) { return (int)(threadIdx.x >> 5) * 32 * per + (int)(threadIdx.x & 31); }
 
-__device__ __forceinline__ void compact_tile(Smem &sm, int *list, int region, unsigned tile, const int (&dest)[kPer],
-                                             const int (&item)[kPer], int &cb, int &cr)
+template <bool kSolo>
+__device__ __forceinline__ void compact_tile(int *count, int *list, int region, const int (&dest)[kPer],
+                                             const int (&item)[kPer])
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    unsigned mb[kPer], mr[kPer], cnt = 0;
+    unsigned mb[kPer], mr[kPer];
+    int nb = 0, nr = 0;
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
         mb[k] = __ballot_sync(kFull, dest[k] == kToBlue);
         mr[k] = __ballot_sync(kFull, dest[k] == kToRed);
-        cnt += (unsigned)__popc(mb[k]) | ((unsigned)__popc(mr[k]) << 16);
+        nb += __popc(mb[k]);
+        nr += __popc(mr[k]);
     }
-    unsigned *words = sm.tile_cnt[tile & 1];
-    if (lane == 0) words[warp] = cnt;
-    __syncthreads();
-    // (two 16-bit counts a word: a tile holds 2048 items)
-    unsigned x = lane < kWarps ? words[lane] : 0u;
-    const unsigned all = __reduce_add_sync(kFull, x);
-    unsigned before = __reduce_add_sync(kFull, lane < warp ? x : 0u);
-    int ob = cb + (int)(before & 0xffffu), orr = cr + (int)(before >> 16);
+    int at = 0;
+    if (lane < 2) at = atomicAdd(count + lane, lane == 0 ? nb : nr);
+    int *blue = list + __shfl_sync(kFull, at, 0), *red = list + (region - 1 - __shfl_sync(kFull, at, 1));
 #pragma unroll
     for (int k = 0; k < kPer; ++k) {
-        if (dest[k] == kToBlue) __stcs(list + ob + __popc(mb[k] & below), item[k]);
-        if (dest[k] == kToRed) __stcs(list + (region - 1 - orr - __popc(mr[k] & below)), item[k]);
-        ob += __popc(mb[k]);
-        orr += __popc(mr[k]);
+        if (dest[k] == kToBlue) Mem<kSolo>::put(blue + __popc(mb[k] & below), item[k]);
+        if (dest[k] == kToRed) Mem<kSolo>::put(red - __popc(mr[k] & below), item[k]);
+        blue += __popc(mb[k]);
+        red -= __popc(mr[k]);
     }
-    cb += (int)(all & 0xffffu);
-    cr += (int)(all >> 16);
 }
 
 // Vertices without neighbours on the symmetric path: no list names them, so
 // nothing depends on them but their own match value and the round count.  One
 // leaves (match value 2) in the first round in which it is blue, or stays red
-// to the cap (match value 1).  The set-up queues the ones red in round 0 in
-// shared memory and resolves the queue round by round, a hash per queued
-// vertex and round (a walk per thread would cost every lane its warp's longest
-// walk).  iso_last: the last round in which any of them is active (the cap's
-// last round if one stays red to it, nseeds if the seeds run out first: the
-// reference would draw more, and the round count then exceeds nseeds).
-//
-// Called by the whole block, after a tile's compaction and a block barrier.
-// Round r reads the queue half qa and appends its survivors to the other,
-// counting them in iso_cnt[r % 3]: that counter is cleared by thread 0 in
-// round r - 1, after every thread read it (in round r - 3's closing step) and
-// before any thread appends to it, so one barrier a round suffices.
-__device__ __noinline__ void resolve_isolated(const Params &p, Smem &sm, int &iso_last)
+// to the cap (match value 1).  The set-up keeps the ones red in round 0 on a
+// stack of their warp in shared memory and hashes the top 32 of them for
+// their next round each, as long as there are 32, so every lane works (a walk
+// per vertex would cost every lane its warp's longest one); the few that are
+// left stay in the rounds, as red items, with the same fate.  iso_last: the
+// last round in which one was active (the cap's last round if it stays red to
+// it, nseeds if the seeds run out first: the reference would draw more, and
+// the round count then exceeds nseeds).
+__device__ __forceinline__ void resolve_isolated(const Params &p, Smem &sm, int &n, int &iso_last)
 {
-    int *qa = sm.iso.half[0], *qb = sm.iso.half[1];
-    const int cap = p.cap, lim = min(cap, p.nseeds);
-    const uint32_t barrier = p.barrier;
-    int nq = min(sm.iso_n, kIsoHalf);
-    if (threadIdx.x == 0) sm.iso_cnt[1] = 0;
-    __syncthreads();
-    for (int r = 1; nq > 0; ++r) {
-        int *cnt = &sm.iso_cnt[r % 3];
-        if (threadIdx.x == 0) sm.iso_cnt[(r + 1) % 3] = 0;
-        for (int i = threadIdx.x; i < nq; i += kThreads) {
-            const int v = qa[i];
-            if (r >= lim) {
-                // red in every round up to the limit
-                p.match[v] = 1;
-                if (p.last) p.last[v] = (uint8_t)(cap - 1);
-                iso_last = max(iso_last, lim == cap ? cap - 1 : lim);
-            } else if (colour_of((uint32_t)(v - base_of(p, v)), p.seeds[r], barrier) == kBlue) {
-                p.match[v] = 2;
-                if (p.last) p.last[v] = (uint8_t)r;
-                iso_last = max(iso_last, r);
-            } else {
-                qb[atomicAdd(cnt, 1)] = v;
-            }
+    const int lane = threadIdx.x & 31;
+    int2 *stack = sm.iso.item[threadIdx.x >> 5];
+    const int lim = min(p.cap, p.nseeds);
+    while (n >= 32) {
+        n -= 32;
+        const int2 e = stack[n + lane];
+        __syncwarp();  // the places above n are free
+        const int v = e.x, r = e.y;
+        bool stays = false;
+        if (r >= lim) {
+            // red in every round up to the limit
+            p.match[v] = 1;
+            if (p.last) p.last[v] = (uint8_t)(p.cap - 1);
+            iso_last = max(iso_last, lim == p.cap ? p.cap - 1 : lim);
+        } else if (colour_of((uint32_t)(v - base_of(p, v)), sm.iso.seeds[r], p.barrier) == kBlue) {
+            p.match[v] = 2;
+            if (p.last) p.last[v] = (uint8_t)r;
+            iso_last = max(iso_last, r);
+        } else {
+            stays = true;
         }
-        __syncthreads();  // the survivors and their count are complete
-        nq = r >= lim ? 0 : *cnt;
-        int *x = qa;
-        qa = qb;
-        qb = x;
+        const unsigned m = __ballot_sync(kFull, stays);
+        if (stays) stack[n + __popc(m & ((1u << lane) - 1u))] = make_int2(v, r + 1);
+        n += __popc(m);
+        __syncwarp();
     }
-    __syncthreads();  // every thread has left the loop before the queue is emptied
-    if (threadIdx.x == 0) sm.iso_n = 0;
-    __syncthreads();
 }
 
 // Set-up: colour every vertex with seeds[0] and fill the first worklists.
@@ -691,23 +691,28 @@ __device__ __noinline__ void resolve_isolated(const Params &p, Smem &sm, int &is
 // rounds, whose per-round counters count them as the reference does.  A list
 // is known to be empty, or longer than its window, from its window's offsets
 // (weighted types) or from its range.
-template <bool kW, bool kStats, bool kPolicy>
-__device__ __forceinline__ void init_phase(const Params &p, Smem &sm, int *list, int &cb, int &cr)
+template <bool kW, bool kStats, bool kPolicy, bool kSolo>
+__device__ __forceinline__ void init_phase(const Params &p, const Mem<kSolo> &m, Smem &sm, int *list)
 {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t seed = p.seeds[0];
-    int iso_last = -1;
-    cb = cr = 0;
-    if (threadIdx.x == 0) sm.iso_n = 0;
+    if (threadIdx.x == 0) {
+        sm.count[0][0] = sm.count[0][1] = sm.count[1][0] = sm.count[1][1] = 0;
+        sm.wnext = 3 * kThreads;
+        sm.stage_n = sm.big_n = sm.flag = sm.zero = 0;
+    }
+    for (int i = threadIdx.x; i < 256; i += kThreads) sm.iso.seeds[i] = p.seeds[i];
     __syncthreads();
-    const int per = tile_per(p.region);
-    const int first = tile_first(per), ntiles = (p.region + per * kThreads - 1) / (per * kThreads);
+    int iso_n = 0, iso_last = -1;
+    const int per = tile_per(p.region), tsize = 32 * per;
+    const int ntiles = (p.region + tsize - 1) / tsize;
     // each tile's ranges are loaded while the tile before it is coloured and compacted
     int vv[kPer];
     int2 rr[kPer];
     auto fetch = [&](int tile) {
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const int s = tile * per * kThreads + first + k * 32;
+            const int s = tile * tsize + k * 32 + lane;
             vv[k] = k < per && s < p.region ? own_vertex(p, s) : -1;
             rr[k] = make_int2(0, 0);
             if (vv[k] >= 0) {
@@ -716,49 +721,57 @@ __device__ __forceinline__ void init_phase(const Params &p, Smem &sm, int *list,
             }
         }
     };
-    fetch(0);
-    for (int tile = 0; tile < ntiles; ++tile) {
+    fetch(warp);
+    for (int tile = warp; tile < ntiles; tile += kWarps) {
         int dest[kPer], item[kPer];
         bool none[kPer], longer[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             item[k] = vv[k];
-            none[k] = kW ? (rr[k].y & ~1) == (rr[k].x & ~1) : degree_of(rr[k]) == 0;
-            longer[k] = kW ? (rr[k].x & 1) != 0 : degree_of(rr[k]) > kWin;
+            none[k] = kW ? ((rr[k].y ^ rr[k].x) & 0x7fffffff) == 0 : degree_of(rr[k]) == 0;
+            longer[k] = kW ? rr[k].x < 0 : degree_of(rr[k]) > kWin;
         }
-        if (tile + 1 < ntiles) fetch(tile + 1);
+        if (tile + kWarps < ntiles) fetch(tile + kWarps);
         unsigned long long act = 0, blue_n = 0;
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
             const int v = item[k];
             dest[k] = kDrop;
+            bool queue = false;
             if (v >= 0) {
                 const bool blue = colour_blue<kPolicy>(p, v, base_of(p, v), 0.0f, 0, seed);
                 // (every completed round leaves them zero: a cut list's last piece clears them)
-                if (longer[k] && p.zero_parts) {
+                if (p.zero_parts && longer[k]) {
                     p.part_key[v] = 0ull;
                     p.part_cnt[v] = 0;
                 }
                 ++act;
                 blue_n += blue;
-                int slot;
                 if (!kStats && p.sym && none[k] && (kPolicy || blue)) {
                     // no neighbours: unmatchable as soon as it is blue (learned
                     // colouring: at once, whatever its colour)
-                    p.col[v] = kDead;
                     p.match[v] = 2;
                     if (p.last) p.last[v] = 0;
                     if (!kPolicy) iso_last = max(iso_last, 0);
                     trace_left<kPolicy>(p, 0, v);
-                } else if (!kStats && !kPolicy && p.sym && none[k] && (slot = atomicAdd(&sm.iso_n, 1)) < kIsoHalf) {
-                    // red in round 0: queued, resolved with the block's others
-                    p.col[v] = kDead;
-                    sm.iso.half[0][slot] = v;
+                } else if (!kStats && !kPolicy && p.sym && none[k]) {
+                    queue = true;
                 } else {
-                    p.best[v] = 0ull;
-                    p.col[v] = blue ? kBlue : kRed;
+                    m.best_[v] = 0ull;
                     dest[k] = blue ? kToBlue : kToRed;
                 }
+            }
+            if (!kStats && !kPolicy && p.sym) {
+                const unsigned mq = __ballot_sync(kFull, queue);
+                if (queue) sm.iso.item[warp][iso_n + __popc(mq & ((1u << lane) - 1u))] = make_int2(v, 1);
+                iso_n += __popc(mq);
+            }
+            // the colours of 32 consecutive vertices: two words, written whole
+            if (k < per) {
+                const unsigned bits = dest[k] == kToRed ? (unsigned)kRed << (2 * (lane & 15)) : 0u;
+                const unsigned w0 = __reduce_or_sync(kFull, lane < 16 ? bits : 0u);
+                const unsigned w1 = __reduce_or_sync(kFull, lane < 16 ? 0u : bits);
+                if (v >= 0 && (lane & 15) == 0) m.col_[(unsigned)v >> 4] = lane < 16 ? w0 : w1;
             }
         }
         if (kStats) {
@@ -766,22 +779,23 @@ __device__ __forceinline__ void init_phase(const Params &p, Smem &sm, int *list,
             stat_add(p, 0, MM_ST_BLUE, blue_n);
             stat_add(p, 0, MM_ST_RED, act - blue_n);
         }
-        compact_tile(sm, list, p.region, (unsigned)tile, dest, item, cb, cr);
-        if (!kPolicy && !kStats && p.sym) {
-            __syncthreads();  // the tile's appends are complete
-            // (every thread reads the same count: appends resume after the next barrier)
-            const bool flush = sm.iso_n > kIsoHalf - kTileItems || (tile + 1 == ntiles && sm.iso_n > 0);
-            __syncthreads();
-            if (flush) resolve_isolated(p, sm, iso_last);
+        compact_tile<kSolo>(sm.count[0], list, p.region, dest, item);
+        if (!kStats && !kPolicy && p.sym) {
+            __syncwarp();
+            resolve_isolated(p, sm, iso_n, iso_last);
         }
     }
-    if (!kPolicy && !kStats) {
+    if (!kPolicy && !kStats && p.sym) {
+        // the ones left on the stack stay in the rounds: red, as in round 0
+        int dest[kPer] = {kDrop, kDrop, kDrop, kDrop}, item[kPer] = {-1, -1, -1, -1};
+        if (lane < iso_n) {
+            item[0] = sm.iso.item[warp][lane].x;
+            dest[0] = kToRed;
+            m.best_[item[0]] = 0ull;
+        }
+        compact_tile<kSolo>(sm.count[0], list, p.region, dest, item);
         iso_last = __reduce_max_sync(kFull, iso_last);
-        if ((threadIdx.x & 31) == 0 && iso_last >= 0) atomicMax(&p.ctl->iso_last, iso_last + 1);
-    }
-    if (threadIdx.x == 0) {  // for the first window scan (read after the barrier)
-        sm.wnext = 3 * kThreads;
-        sm.stage_n = sm.big_n = sm.big_next = sm.shared_n = 0;
+        if (lane == 0 && iso_last >= 0) atomicMax(&p.ctl->iso_last, iso_last + 1);
     }
 }
 
@@ -815,8 +829,8 @@ __device__ __forceinline__ void init_phase(const Params &p, Smem &sm, int *list,
 // 128 entries cut R-MAT rounds further than 32 did; 512 cut no more and cost
 // time.  A retired vertex's worklist item is marked with its id complemented,
 // so the commit phase sees the retirement in the item it loads anyway.
-template <bool kPolicy>
-__device__ __forceinline__ void retire_red(const Params &p, int t, int *list, int cr)
+template <bool kPolicy, bool kSolo>
+__device__ __forceinline__ void retire_red(const Params &p, const Mem<kSolo> &m, int t, int *list, int cr)
 {
     for (int i = kThreads - 1 - (int)threadIdx.x; i < cr; i += kThreads) {
         int *slot = list + (p.region - 1 - i);
@@ -830,10 +844,9 @@ __device__ __forceinline__ void retire_red(const Params &p, int t, int *list, in
             for (int u = 0; u < 16; ++u) nb[u] = j0 + u < r.y ? __ldg(p.nbrs + j0 + u) : -1;
 #pragma unroll
             for (int u = 0; u < 16; ++u)
-                if (nb[u] >= 0 && p.col[nb[u]] != kMatched) gone = false;
+                if (nb[u] >= 0 && m.col(nb[u]) != kMatched) gone = false;
         }
         if (gone) {
-            p.col[v] = kDead;
             p.match[v] = 2;
             if (p.last) p.last[v] = (uint8_t)t;
             *slot = ~v;
@@ -843,37 +856,37 @@ __device__ __forceinline__ void retire_red(const Params &p, int t, int *list, in
 }
 
 // Append blue vertex v (list r) to the round's shared fallback list: one
-// 64-bit atomic hands out the item and its offset in the concatenated entries.
-__device__ __forceinline__ void stage_shared(const Params &p, Smem &sm, int v, long long slot, int2 r)
+// 64-bit atomic hands out the item and its pieces.
+__device__ __forceinline__ void stage_shared(const Params &p, Smem &sm, int v, const ItemReq &rq, int2 r)
 {
-    const int deg = degree_of(r);
-    const unsigned long long old = atomicAdd(&p.ctl->staged_pack, (1ull << 32) | (unsigned long long)(unsigned)deg);
-    const int idx = (int)(old >> 32), off = (int)(old & 0xffffffffull);
-    p.staged[idx] = make_int4(v, r.x, r.y, off);
-    for (int s = (off + kSegEntries - 1) / kSegEntries; s * kSegEntries < off + deg; ++s) p.seg_first[s] = idx;
-    p.prop[slot] = kReqShared;  // it proposes through req[v]
-    atomicAdd(&sm.shared_n, 1);
+    const int pieces = (degree_of(r) + kPiece - 1) / kPiece;
+    const unsigned long long old = atomicAdd(&p.ctl->staged_pack, (1ull << 32) | (unsigned long long)(unsigned)pieces);
+    const int idx = (int)(old >> 32), first = (int)(old & 0xffffffffull);
+    p.staged[idx] = make_int4(v, r.x, r.y, first);
+    for (int s = 0; s < pieces; ++s) p.piece_item[first + s] = idx;
+    rq.put(kReqShared, 0u);  // it proposes through req[v]
+    sm.flag = 1;
 }
 
-// Window entries q and q + 1 of a blue vertex (window from `off`, length wl):
-// neighbours and second words (weight, position | flag, or position).
+// Group g of a blue vertex's window: four neighbours and their second words
+// (weight, position | flag, or position); -1 for entries outside the window.
 template <bool kW>
-__device__ __forceinline__ void window_pair(const Params &p, int off, int wl, int q, int &n0, int &j0, int &n1, int &j1)
+__device__ __forceinline__ void window_group(const Params &p, int g, int lo, int hi, int *nb, int *jv)
 {
-    n0 = n1 = -1;
-    j0 = j1 = 0;
-    if (q >= wl) return;
     if (kW) {
-        const int4 x = __ldg(reinterpret_cast<const int4 *>(p.pwin + off + q));
-        n0 = x.x;
-        j0 = x.y;
-        n1 = x.z;
-        j1 = x.w;
+        const int2 *a = p.pwin + 4ll * g;
+        asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(nb[0]), "=r"(jv[0]), "=r"(nb[1]), "=r"(jv[1]), "=r"(nb[2]), "=r"(jv[2]), "=r"(nb[3]),
+                       "=r"(jv[3])
+                     : "l"(a));
     } else {
-        j0 = off + q;
-        j1 = j0 + 1;
-        n0 = __ldg(p.nbrs + j0);
-        if (q + 1 < wl) n1 = __ldg(p.nbrs + j1);
+        const int4 x = __ldg(reinterpret_cast<const int4 *>(p.nbrs) + g);
+        const int v[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            jv[k] = 4 * g + k;
+            nb[k] = jv[k] >= lo && jv[k] < hi ? v[k] : -1;
+        }
     }
 }
 
@@ -882,30 +895,33 @@ __device__ __forceinline__ void window_pair(const Params &p, int off, int wl, in
 // weight; elsewhere for weighted types the position, bit 31 set for a weight
 // that can never be picked; random types: the position.
 template <bool kW>
-__device__ __forceinline__ bool window_choice(const Params &p, uint8_t c, int j)
+__device__ __forceinline__ bool window_choice(const Params &p, unsigned c, int j)
 {
     return c == kRed && (!kW || (p.sym ? __int_as_float(j) > -1.0f : j >= 0));
 }
 
-// A window's place: first slot, length (even for the weighted types, whose odd
-// windows end with a filler) and whether the list is longer.  raw is the pair
-// of window offsets (weighted) or the range.
+// A window's place: its groups [g, gend), for the random types the entries
+// [lo, hi) of the list (groups are aligned, so the first and last may be
+// partial), and whether the list is longer.  raw is the pair of window offsets
+// (weighted) or the range.
 template <bool kW>
 __device__ __forceinline__ int2 window_raw(const Params &p, int v)
 {
     return kW ? make_int2(__ldg(p.pwin_off + v), __ldg(p.pwin_off + v + 1)) : __ldg(p.ranges + v);
 }
 template <bool kW>
-__device__ __forceinline__ void window_place(int2 raw, int &off, int &wl, bool &longer)
+__device__ __forceinline__ void window_place(int2 raw, int &g, int &gend, int &lo, int &hi, bool &longer)
 {
     if (kW) {
-        off = raw.x & ~1;
-        wl = (raw.y & ~1) - off;
-        longer = (raw.x & 1) != 0;
+        g = raw.x & 0x7fffffff;
+        gend = raw.y & 0x7fffffff;
+        longer = raw.x < 0;
     } else {
         const int deg = degree_of(raw);
-        off = raw.x;
-        wl = win_len(deg);
+        lo = raw.x;
+        hi = lo + win_len(deg);
+        g = lo >> 2;
+        gend = deg > 0 ? (hi + 3) >> 2 : g;
         longer = deg > kWin;
     }
 }
@@ -913,8 +929,8 @@ __device__ __forceinline__ void window_place(int2 raw, int &off, int &wl, bool &
 // Full scan of a list by the lanes of one or more warps: entries b + first,
 // b + first + step, ... in rows of 32 * kRows per warp; the lanes' best keys.
 // Random types stop at the first row with a red entry.
-template <bool kW>
-__device__ __forceinline__ unsigned long long scan_rows(const Params &p, int b, int e, int first, int step)
+template <bool kW, bool kSolo>
+__device__ __forceinline__ unsigned long long scan_rows(const Params &p, const Mem<kSolo> &m, int b, int e, int first, int step)
 {
     const int lane = threadIdx.x & 31;
     float bw = -1.0f;
@@ -929,9 +945,9 @@ __device__ __forceinline__ unsigned long long scan_rows(const Params &p, int b, 
             nb[r] = j < e ? __ldg(p.nbrs + j) : -1;
             wv[r] = kW && j < e ? __ldg(p.w + j) : 0.0f;
         }
-        uint8_t c[kRows];
+        unsigned c[kRows];
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) c[r] = nb[r] >= 0 ? ld_col(p.col + nb[r]) : (uint8_t)kMatched;
+        for (int r = 0; r < kRows; ++r) c[r] = nb[r] >= 0 ? m.col(nb[r]) : (unsigned)kMatched;
 #pragma unroll
         for (int r = 0; r < kRows; ++r) fold_entry<kW>(c[r], wv[r], j0 + r * 32 + lane, bw, bj, alive);
         if (!kW && __any_sync(kFull, bw > -1.0f)) break;
@@ -966,8 +982,8 @@ __device__ __forceinline__ void count_fallback(const Params &p, int t, int deg)
 constexpr int kWarpList = 512;
 constexpr int kBlockList = 32768;
 
-template <bool kW, bool kStats>
-__device__ __noinline__ void scan_fallback(const Params &p, Smem &sm, int t, long long rbase)
+template <bool kW, bool kStats, bool kSolo>
+__device__ __noinline__ void scan_fallback(const Params &p, const Mem<kSolo> m, Smem &sm, int t, long long rbase)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ns = min(sm.stage_n, kStageCap);
@@ -976,14 +992,14 @@ __device__ __noinline__ void scan_fallback(const Params &p, Smem &sm, int t, lon
         const int2 r = __ldg(p.ranges + it.x);
         const int deg = degree_of(r);
         if (deg > kBlockList) {
-            if (lane == 0) stage_shared(p, sm, it.x, rbase + it.y, r);
+            if (lane == 0) stage_shared(p, sm, it.x, ItemReq{p, sm, rbase, it.y}, r);
         } else if (deg > kWarpList) {
             if (lane == 0) sm.fb.big[atomicAdd(&sm.big_n, 1)] = (unsigned short)i;
         } else {
-            const unsigned long long key = warp_max_u64(scan_rows<kW>(p, r.x, r.y, 0, 32 * kRows));
+            const unsigned long long key = warp_max_u64(scan_rows<kW>(p, m, r.x, r.y, 0, 32 * kRows));
             if (lane == 0) {
                 count_fallback<kStats>(p, t, deg);
-                propose_key<kW, kStats>(p, ItemReq{p, rbase + it.y}, it.x, r.x, deg, key, t);
+                propose_key<kW, kStats>(p, m, ItemReq{p, sm, rbase, it.y}, it.x, r.x, deg, key, t);
             }
         }
     }
@@ -993,14 +1009,14 @@ __device__ __noinline__ void scan_fallback(const Params &p, Smem &sm, int t, lon
         const int2 it = sm.fb.item[sm.fb.big[i]];
         const int2 r = __ldg(p.ranges + it.x);
         const int deg = degree_of(r);
-        const unsigned long long mine = warp_max_u64(scan_rows<kW>(p, r.x, r.y, warp * 32 * kRows, kThreads * kRows));
+        const unsigned long long mine = warp_max_u64(scan_rows<kW>(p, m, r.x, r.y, warp * 32 * kRows, kThreads * kRows));
         if (lane == 0) sm.red_key[warp] = mine;
         __syncthreads();
         if (threadIdx.x == 0) {
             unsigned long long key = 0ull;
             for (int w = 0; w < kWarps; ++w) key = sm.red_key[w] > key ? sm.red_key[w] : key;
             count_fallback<kStats>(p, t, deg);
-            propose_key<kW, kStats>(p, ItemReq{p, rbase + it.y}, it.x, r.x, deg, key, t);
+            propose_key<kW, kStats>(p, m, ItemReq{p, sm, rbase, it.y}, it.x, r.x, deg, key, t);
         }
         __syncthreads();  // the keys are reused
     }
@@ -1008,18 +1024,20 @@ __device__ __noinline__ void scan_fallback(const Params &p, Smem &sm, int t, lon
 
 // Phase A1 over the block's cb blue items.  The first items go to the threads
 // in order, the rest to the warps from a counter in shared memory.  A lane
-// holds one vertex at a time and reads its window eight entries a step (four
-// 16-byte loads, then the eight colours); as soon as a lane's vertex is
+// holds one vertex at a time and reads its window eight entries a step (two
+// 32-byte loads, then the colours of two entries and, where these do not
+// decide, of the other six); as soon as a lane's vertex is
 // decided it takes the next one, whose window offsets it has prefetched, loads
 // the offsets of the one after that, whose id it has prefetched, and prefetches
 // another id.  So every lane keeps an independent chain of loads in flight and
 // no lane waits for the slowest vertex of its warp or block.
-template <bool kW, bool kStats, bool kPolicy>
-__device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, int *list, long long rbase, int cb, int cr)
+template <bool kW, bool kStats, bool kPolicy, bool kSolo>
+__device__ __forceinline__ void scan_window(const Params &p, const Mem<kSolo> &m, Smem &sm, int t, int *list, long long rbase, int cb, int cr)
 {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     bool dry = 3 * kThreads >= cb;  // warp-uniform: the block's items are handed out
+    const bool few = cb <= 2 * kThreads;
     // Items for the lanes in `mask`: one shared atomic per warp.  Returns this
     // lane's item, or -1.
     auto grab = [&](unsigned mask) -> int {
@@ -1036,37 +1054,49 @@ __device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, in
     ci = ci < cb ? ci : -1;
     ni = ni < cb ? ni : -1;
     mi = mi < cb ? mi : -1;
-    int cv = ci >= 0 ? __ldcs(list + ci) : -1, nv = ni >= 0 ? __ldcs(list + ni) : -1, mv = mi >= 0 ? __ldcs(list + mi) : -1;
+    int cv = ci >= 0 ? m.item(list + ci) : -1, nv = ni >= 0 ? m.item(list + ni) : -1, mv = mi >= 0 ? m.item(list + mi) : -1;
     int2 nraw = make_int2(0, 0);
-    int off = 0, wl = 0;
+    int g = 0, gend = 0, lo = 0, hi = 0;
     bool longer = false;
-    if (cv >= 0) window_place<kW>(window_raw<kW>(p, cv), off, wl, longer);
+    if (cv >= 0) window_place<kW>(window_raw<kW>(p, cv), g, gend, lo, hi, longer);
     if (nv >= 0) nraw = window_raw<kW>(p, nv);
     bool has = cv >= 0, alive = false;
-    int q = 0;
+    bool narrow = kW && t == 0;
+    int seen = 0;
     while (__any_sync(kFull, has)) {
         if (has) {
             // eight entries a step (one dependent round trip for each 8: the scan
-            // is bound by the latency of its load chains); the first step of
-            // round 0, where most vertices stop at their first or second entry,
-            // reads four
-            const int width = q == 0 && t == 0 ? 4 : 8;
+            // is bound by the latency of its load chains); the first step of a
+            // weighted type's round 0, where most vertices stop at their first or
+            // second entry, reads four (a list of a random type starts anywhere in
+            // its first group)
             int nb[8], jv[8];
 #pragma unroll
-            for (int h = 0; h < 4; ++h) {
-                nb[2 * h] = nb[2 * h + 1] = -1;
-                jv[2 * h] = jv[2 * h + 1] = 0;
-                if (2 * h < width) window_pair<kW>(p, off, wl, q + 2 * h, nb[2 * h], jv[2 * h], nb[2 * h + 1], jv[2 * h + 1]);
+            for (int x = 0; x < 8; ++x) {
+                nb[x] = -1;
+                jv[x] = 0;
             }
-            uint8_t c[8];
+            if (g < gend) window_group<kW>(p, g, lo, hi, nb, jv);
+            if (!narrow && g + 1 < gend) window_group<kW>(p, g + 1, lo, hi, nb + 4, jv + 4);
+            g += narrow ? 1 : 2;
+            narrow = false;
+            // a full block reads the first two colours, and the others only for a
+            // vertex that they leave undecided (the phase is then bound by the
+            // sectors it requests: RGG 2^20's round 0 took 26.1 us for 29.7); a
+            // block with few items reads all at once, a round trip less
+            unsigned c[8];
 #pragma unroll
-            for (int x = 0; x < 8; ++x) c[x] = nb[x] >= 0 ? ld_col(p.col + nb[x]) : (uint8_t)kMatched;
+            for (int x = 0; x < 8; ++x) c[x] = (x < 2 || few) && nb[x] >= 0 ? m.col(nb[x]) : (unsigned)kMatched;
+            if (!few && !window_choice<kW>(p, c[0], jv[0]) && !window_choice<kW>(p, c[1], jv[1])) {
+#pragma unroll
+                for (int x = 2; x < 8; ++x) c[x] = nb[x] >= 0 ? m.col(nb[x]) : (unsigned)kMatched;
+            }
             bool found = false;
-            int cj = -1, ct = 0, seen = q;
+            int cj = -1, ct = 0;
 #pragma unroll
             for (int x = 0; x < 8; ++x) {
                 if (nb[x] < 0 || found) continue;
-                seen = q + x + 1;
+                if (kStats) ++seen;
                 if (window_choice<kW>(p, c[x], jv[x])) {
                     found = true;
                     cj = jv[x];
@@ -1075,9 +1105,8 @@ __device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, in
                     alive |= c[x] != kMatched;
                 }
             }
-            q += width;
-            if (found || q >= wl) {
-                const ItemReq rq{p, rbase + ci};
+            if (found || g >= gend) {
+                const ItemReq rq{p, sm, rbase, ci};
                 if (kStats) {
                     atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_WINDOW_ENTRIES], (unsigned long long)seen);
                     if (found || !longer) {
@@ -1088,8 +1117,8 @@ __device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, in
                     }
                 }
                 if (found) {
-                    if (kW && p.sym) propose_weight(p, rq, cv, __int_as_float(cj), ct);
-                    else propose_to<kW>(p, rq, cv, kW && !p.contiguous ? __ldg(p.ranges + cv).x : off, cj & 0x7fffffff, ct);
+                    if (kW && p.sym) propose_weight(m, rq, cv, __int_as_float(cj), ct);
+                    else propose_to<kW>(p, m, rq, cv, kW ? (p.contiguous ? 0 : __ldg(p.ranges + cv).x) : lo, cj & 0x7fffffff, ct);
                 } else if (!longer) {
                     no_proposal(p, rq, cv, alive, t);
                 } else {
@@ -1097,7 +1126,7 @@ __device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, in
                     // finds the block's buffer full goes to the shared list at once
                     const int slot = atomicAdd(&sm.stage_n, 1);
                     if (slot < kStageCap) sm.fb.item[slot] = make_int2(cv, ci);
-                    else stage_shared(p, sm, cv, rbase + ci, __ldg(p.ranges + cv));
+                    else stage_shared(p, sm, cv, rq, __ldg(p.ranges + cv));
                 }
                 has = false;
             }
@@ -1109,10 +1138,11 @@ __device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, in
             if (take) {
                 cv = nv;
                 ci = ni;
-                window_place<kW>(nraw, off, wl, longer);
+                window_place<kW>(nraw, g, gend, lo, hi, longer);
                 has = true;
                 alive = false;
-                q = 0;
+                narrow = kW && t == 0;
+                seen = 0;
                 nv = mv;
                 ni = mi;
                 mv = mi = -1;
@@ -1122,238 +1152,69 @@ __device__ __forceinline__ void scan_window(const Params &p, Smem &sm, int t, in
                 const int i = grab(need);
                 if (i >= 0) {
                     mi = i;
-                    mv = __ldcs(list + i);
+                    mv = m.item(list + i);
                 }
             }
         }
     }
-    if (kPolicy && p.sym && t >= kRetireFrom) retire_red<kPolicy>(p, t, list, cr);
+    if (kPolicy && p.sym && t >= kRetireFrom) retire_red<kPolicy>(p, m, t, list, cr);
+    if (threadIdx.x < 2) sm.count[(t & 1) ^ 1][threadIdx.x] = 0;  // for the commit phase (read after the barrier)
     __syncthreads();
-    if (sm.stage_n > 0) scan_fallback<kW, kStats>(p, sm, t, rbase);
+    if (sm.stage_n > 0) scan_fallback<kW, kStats>(p, m, sm, t, rbase);
 }
 
-// ---- phase A2: fallback lists, entry-balanced segments ----
+// ---- phase A2: shared fallback lists ----
 //
-// The round's fallback lists are concatenated (each item's .w is its offset)
-// and cut into kSegEntries-entry segments; seg_first[s] is the first item
-// overlapping segment s.  Items are numbered in offset order: one 64-bit
-// atomic hands out both.  A warp takes a segment: lane l describes the l-th
-// list piece in it (at most 9), then the warp walks the segment in rows of
-// 32 consecutive entries.  Every piece but the segment's first and last is a
-// whole list of more than 32 entries, so a row holds at most one piece
-// boundary and the piece being scanned is the same for the whole warp: each
-// lane keeps a running best (weight, position, alive) for it, and at the
-// boundary the warp max-reduces the lanes' keys with shuffles and the lane
-// describing the piece finishes it.  A list inside one segment proposes at
-// once; a cut list max-combines its piece into part_key and the piece that
-// arrives last proposes.
-//
-// Loads are pipelined over iterations of kRows rows: the neighbour ids and
-// weights of iteration i+2 stream into shared memory (cp.async, kStages
-// buffers) and the colour gathers of iteration i+1 are in flight while
-// iteration i is folded.
-template <bool kW, bool kStats>
-__device__ __forceinline__ void finish_piece(const Params &p, int4 it, int pieces, unsigned long long key, int t)
-{
-    if (pieces == 1) {
-        propose_key<kW, kStats>(p, VertexReq{p, it.x}, it.x, it.y, degree_of(it), key, t);
-        return;
-    }
-    const int v = it.x;
-    if (key) atomicMax(&p.part_key[v], key);
-    // acq_rel: this piece's max is visible before its arrival counts, and the
-    // last arrival sees every other piece's max
-    int done;
-    asm volatile("atom.add.acq_rel.gpu.s32 %0, [%1], 1;" : "=r"(done) : "l"(p.part_cnt + v) : "memory");
-    if (done == pieces - 1) {
-        const unsigned long long all = atomicExch(&p.part_key[v], 0ull);
-        atomicExch(&p.part_cnt[v], 0);
-        propose_key<kW, kStats>(p, VertexReq{p, v}, v, it.y, degree_of(it), all, t);
-    }
-}
-
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait1() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
-__device__ __forceinline__ void cp_async4_s(unsigned saddr, const void *gmem)
-{
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(saddr), "l"(gmem) : "memory");
-}
-
-// Finish piece k of the segment table: lane k holds its item.
-template <bool kW, bool kStats>
-__device__ __forceinline__ void finish_table_piece(const Params &p, int k, int lane, int4 it, int pieces, int lo, int hi,
-                                                   unsigned long long key, int t)
-{
-    if (lane == k) {
-        if (kStats) {
-            atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_STAGED_DEG], (unsigned long long)(hi - lo));
-            atomicAdd(&p.stats[(size_t)t * MM_STATS_COLS + MM_ST_STAGED_ITEMS], 1ull);
-        }
-        finish_piece<kW, kStats>(p, it, pieces, key, t);
-    }
-}
-
-template <bool kW, bool kStats>
-__device__ void scan_long(const Params &p, Smem &sm, int t, int gwarp, int nwarps)
+// A warp scans a piece of kPiece entries.  A list of several pieces
+// max-combines them in part_key; the piece that arrives last proposes.
+template <bool kW, bool kStats, bool kSolo>
+__device__ __noinline__ void scan_shared(const Params &p, const Mem<kSolo> m, int t)
 {
     const unsigned long long pack = __ldcg(&p.ctl->staged_pack);
-    const int nitems = (int)(pack >> 32);
-    const int nentries = (int)(pack & 0xffffffffull);
-    const int nseg = (nentries + kSegEntries - 1) / kSegEntries;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int *pend = sm.ls.pend[warp];
-    int *delta = sm.ls.delta[warp];
-    LongStage &stg = sm.ls.stage[warp];
-    // shared addresses of this lane's slots in stage 0 (stage k: + k * kStageBytes)
-    constexpr unsigned kStageBytes = kRows * 32 * 4;
-    const unsigned nb_slot = (unsigned)__cvta_generic_to_shared(&stg.nb[0][lane]);
-    const unsigned w_slot = (unsigned)__cvta_generic_to_shared(&stg.w[0][lane]);
-    const int4 *list = p.staged;
-    const int *seg_first = p.seg_first;
-    // the piece table of segment s + nwarps is loaded while segment s is
-    // scanned: seg_first two segments ahead, the items one segment ahead
-    int sf_a = gwarp < nseg ? __ldcg(seg_first + gwarp) + lane : nitems;
-    int sf_b = gwarp + nwarps < nseg ? __ldcg(seg_first + gwarp + nwarps) + lane : nitems;
-    int4 x_a = sf_a < nitems ? __ldcg(list + sf_a) : make_int4(-1, 0, 0, -1);
-    for (int s = gwarp; s < nseg; s += nwarps) {
-        const int s_lo = s * kSegEntries;
-        const int seg_len = min(kSegEntries, nentries - s_lo);
-        const int idx = sf_a;
-        const int4 x = x_a;
-        x_a = sf_b < nitems ? __ldcg(list + sf_b) : make_int4(-1, 0, 0, -1);
-        sf_a = sf_b;
-        sf_b = s + 2 * nwarps < nseg ? __ldcg(seg_first + s + 2 * nwarps) + lane : nitems;
-        int4 it = make_int4(-1, 0, 0, 0);
-        int pieces = 1, lo = 0, hi = 0;
-        if (idx < nitems) {
-            const int deg = degree_of(x);
-            if (x.w < s_lo + seg_len && x.w + deg > s_lo) {
-                it = x;
-                lo = max(x.w, s_lo) - x.w;
-                hi = min(x.w + deg, s_lo + seg_len) - x.w;
-                pieces = (x.w + deg - 1) / kSegEntries - x.w / kSegEntries + 1;
-            }
+    const int npieces = (int)(pack & 0xffffffffull);
+    const int lane = threadIdx.x & 31;
+    for (int s = (int)(blockIdx.x * kWarps + (threadIdx.x >> 5)); s < npieces; s += (int)(gridDim.x * kWarps)) {
+        const int4 it = __ldcg(p.staged + __ldcg(p.piece_item + s));
+        const int deg = degree_of(it), pieces = (deg + kPiece - 1) / kPiece;
+        const int b = it.y + (s - it.w) * kPiece, e = min(it.z, b + kPiece), v = it.x;
+        const unsigned long long key = warp_max_u64(scan_rows<kW>(p, m, b, e, 0, 32 * kRows));
+        if (lane != 0) continue;
+        count_fallback<kStats>(p, t, e - b);
+        if (pieces == 1) {
+            propose_key<kW, kStats>(p, m, VertexReq{p, v}, v, it.y, deg, key, t);
+            continue;
         }
-        pend[lane] = it.x >= 0 ? it.w + hi - s_lo : 0x7fffffff;
-        if (lane == 0) pend[32] = 0x7fffffff;
-        delta[lane] = it.y - it.w + s_lo;
-        if (lane == 0) delta[32] = 0;
-        __syncwarp();
-        const int nit = (seg_len + 32 * kRows - 1) / (32 * kRows);
-        // Load side: piece kl holds the first entry of the row being staged;
-        // its end and the position offsets of kl and kl + 1 stay in registers.
-        int kl = 0, endl = pend[0], dl0 = delta[0], dl1 = delta[1];
-        int stage_in = 0;  // stage that iteration i + 2 is staged into
-        auto issue = [&](int i) {
-            if (i < nit) {
-                const unsigned so = (unsigned)stage_in * kStageBytes;
-#pragma unroll
-                for (int r = 0; r < kRows; ++r) {
-                    const int rb = i * 32 * kRows + r * 32;
-                    if (rb < seg_len) {
-                        while (endl <= rb) {
-                            ++kl;
-                            endl = pend[kl];
-                            dl0 = dl1;
-                            dl1 = delta[kl + 1];
-                        }
-                        const int e = rb + lane;
-                        if (e < seg_len) {
-                            const int pos = e + (e >= endl ? dl1 : dl0);
-                            cp_async4_s(nb_slot + so + r * 128, p.nbrs + pos);
-                            if (kW) cp_async4_s(w_slot + so + r * 128, p.w + pos);
-                        }
-                    }
-                }
-            }
-            cp_async_commit();
-            stage_in = stage_in == kStages - 1 ? 0 : stage_in + 1;
-        };
-        // colours of iteration i (staged in stage st), one byte per row
-        auto gather = [&](int i, int st) -> unsigned {
-            unsigned c = 0x03030303u;  // kMatched in every row
-            if (i < nit) {
-#pragma unroll
-                for (int r = 0; r < kRows; ++r) {
-                    const int e = i * 32 * kRows + r * 32 + lane;
-                    if (e < seg_len) {
-                        const unsigned x = ld_col(p.col + stg.nb[st][r * 32 + lane]);
-                        c = (c & ~(0xffu << (8 * r))) | (x << (8 * r));
-                    }
-                }
-            }
-            return c;
-        };
-        issue(0);
-        issue(1);
-        cp_async_wait1();
-        unsigned cc = gather(0, 0);
-        // Fold side: piece kp, its end and the offsets of kp and kp + 1.
-        int kp = 0, endp = pend[0], dp0 = delta[0], dp1 = delta[1];
-        int st = 0;  // stage of iteration i
-        float bw = -1.0f;
-        int bj = 0;
-        bool alive = false;
-        for (int i = 0; i < nit; ++i) {
-            issue(i + 2);
-            cp_async_wait1();
-            const int st1 = st == kStages - 1 ? 0 : st + 1;
-            const unsigned cn = gather(i + 1, st1);
-#pragma unroll
-            for (int r = 0; r < kRows; ++r) {
-                const int rb = i * 32 * kRows + r * 32;
-                if (rb >= seg_len) break;
-                const int e = rb + lane;
-                const bool in = e < seg_len;
-                const uint8_t c = (uint8_t)(cc >> (8 * r));
-                const float wv = kW ? stg.w[st][r * 32 + lane] : 0.0f;
-                if (endp < min(rb + 32, seg_len)) {
-                    // piece kp ends inside this row: finish it, then start kp + 1
-                    const bool second = e >= endp;
-                    if (in && !second) fold_entry<kW>(c, wv, e + dp0, bw, bj, alive);
-                    const unsigned long long key = warp_max_u64(strip_key<kW>(bw, bj, alive));
-                    finish_table_piece<kW, kStats>(p, kp, lane, it, pieces, lo, hi, key, t);
-                    bw = -1.0f;
-                    alive = false;
-                    ++kp;
-                    endp = pend[kp];
-                    dp0 = dp1;
-                    dp1 = delta[kp + 1];
-                    if (in && second) fold_entry<kW>(c, wv, e + dp0, bw, bj, alive);
-                } else if (in) {
-                    fold_entry<kW>(c, wv, e + dp0, bw, bj, alive);
-                }
-            }
-            cc = cn;
-            st = st1;
+        if (key) atomicMax(&p.part_key[v], key);
+        // acq_rel: this piece's max is visible before its arrival counts, and the
+        // last arrival sees every other piece's max
+        int done;
+        asm volatile("atom.add.acq_rel.gpu.s32 %0, [%1], 1;" : "=r"(done) : "l"(p.part_cnt + v) : "memory");
+        if (done == pieces - 1) {
+            const unsigned long long all = atomicExch(&p.part_key[v], 0ull);
+            atomicExch(&p.part_cnt[v], 0);
+            propose_key<kW, kStats>(p, m, VertexReq{p, v}, v, it.y, deg, all, t);
         }
-        {
-            const unsigned long long key = warp_max_u64(strip_key<kW>(bw, bj, alive));
-            finish_table_piece<kW, kStats>(p, kp, lane, it, pieces, lo, hi, key, t);
-        }
-        __syncwarp();  // the tables and stages are refilled by the next segment
     }
 }
 
 // Phase B: commit proposals, recolour survivors with the next seed, compact
-// the block's lists of round t+1 (ncb blue, ncr red).  A colour byte is
-// written only when it changes.
-template <bool kW, bool kStats, bool kPolicy>
-__device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, bool has_next, const int *list, int *next,
-                                             long long rbase, int cb, int cr, int &ncb, int &ncr)
+// the block's lists of round t+1.  Colours are
+// written only where they change.
+template <bool kW, bool kStats, bool kPolicy, bool kSolo>
+__device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &m, Smem &sm, int t, bool has_next, const int *list, int *next,
+                                             long long rbase, int cb, int cr)
 {
     const uint32_t next_seed = has_next ? p.seeds[t + 1] : 0u;
     const int total = cb + cr;
-    const int per = tile_per(total), first = tile_first(per), tsize = per * kThreads;
-    ncb = ncr = 0;
-    for (int base = 0, tile = 0; base < total; base += tsize, ++tile) {
+    const int per = tile_per(total), tsize = 32 * per;
+    for (int base = (int)(threadIdx.x >> 5) * tsize; base < total; base += kWarps * tsize) {
         // items, and with a blue item its request, loaded together
         int vv[kPer], tg[kPer];
         uint32_t low[kPer];
         bool blue[kPer], gone[kPer];
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const int i = base + first + k * 32;
+            const int i = base + k * 32 + (int)(threadIdx.x & 31);
             const bool in = k < per && i < total;
             blue[k] = in && i < cb;
             gone[k] = false;
@@ -1361,11 +1222,11 @@ __device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, b
             tg[k] = kReqNone;
             low[k] = 0u;
             if (blue[k]) {
-                vv[k] = __ldcs(list + i);
-                tg[k] = __ldcs(p.prop + rbase + i);
+                vv[k] = m.item(list + i);
+                tg[k] = i < kPropCap ? sm.req.target[i] : __ldcs(p.prop + rbase + i);
                 if (!p.sym) low[k] = __ldcs(p.prop_key + rbase + i);
             } else if (in) {
-                vv[k] = __ldcs(list + (p.region - 1 - (i - cb)));
+                vv[k] = m.item(list + (p.region - 1 - (i - cb)));
                 // learned colouring: a red item retired in phase A carries its id complemented
                 if (kPolicy && vv[k] < 0) {
                     gone[k] = true;
@@ -1387,9 +1248,9 @@ __device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, b
                 } else if (p.sym) {
                     low[k] = ~(uint32_t)vv[k];
                 }
-                if (tg[k] >= 0 && low[k] != 0u) key[k] = __ldcg(p.best + tg[k]);
+                if (tg[k] >= 0 && low[k] != 0u) key[k] = m.best(tg[k]);
             } else if (vv[k] >= 0) {
-                key[k] = __ldcg(p.best + vv[k]);
+                key[k] = m.best(vv[k]);
             }
         }
         int dest[kPer];
@@ -1431,7 +1292,7 @@ __device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, b
             if (partner >= 0) {
                 trace_left<kPolicy>(p, t, v);
                 p.match[v] = 4 + min(v, partner) - base_of(p, v);
-                p.col[v] = kMatched;
+                m.flip(v, kMatched ^ (blue[k] ? kBlue : kRed));
                 if (p.last) p.last[v] = (uint8_t)t;
                 ++matched;
                 continue;
@@ -1450,7 +1311,7 @@ __device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, b
             const bool nb = colour_blue<kPolicy>(p, v, base_of(p, v), role, t + 1, next_seed);
             ++act;
             nblue += nb;
-            if (nb != blue[k]) p.col[v] = nb ? kBlue : kRed;
+            if (nb != blue[k]) m.flip(v, kBlue ^ kRed);
             dest[k] = nb ? kToBlue : kToRed;
         }
         if (kStats) {
@@ -1463,11 +1324,11 @@ __device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, b
                 stat_add(p, t + 1, MM_ST_RED, act - nblue);
             }
         }
-        compact_tile(sm, next, p.region, (unsigned)tile, dest, vv, ncb, ncr);
+        compact_tile<kSolo>(sm.count[(t & 1) ^ 1], next, p.region, dest, vv);
     }
     if (threadIdx.x == 0) {  // for the next window scan (read after the barrier)
         sm.wnext = 3 * kThreads;
-        sm.stage_n = sm.big_n = sm.big_next = sm.shared_n = 0;
+        sm.stage_n = sm.big_n = sm.flag = 0;
     }
 }
 
@@ -1499,8 +1360,8 @@ __device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, b
 //          component that a lane cannot hold (records incomplete, more than
 //          kFinTMembers members) is searched and played by the warp, lane l
 //          holding member l (up to kFinMembers members, kFinEntries entries).
-// A larger component, a list longer than kFinMaxDeg or an unmatchable
-// neighbour calls the attempt off (ctl->fin_abort), and round t runs as
+// A larger component or a list longer than kFinMaxDeg calls the attempt off,
+// and round t runs as
 // usual; values already written are the ones the rounds write again.  The
 // instrumented kernel checks first and resolves in a third pass, so that its
 // counters never include a called-off attempt.
@@ -1509,14 +1370,22 @@ __device__ __forceinline__ void commit_phase(const Params &p, Smem &sm, int t, b
 // (at most the cap).
 constexpr int kFinShort = 32;      // lists a thread scans on its own; longer ones its warp scans
 constexpr int kFinMaxDeg = 2048;   // longest list the finish phase accepts
-constexpr int kFinDiv = 12;        // default: first attempt once the active set is at most 1/kFinDiv of round 0's
+// Default: first attempt once the active set is at most 1/kFinDiv of round 0's.
+// A round costs 7-8 us once the set is small; an attempt a round too early
+// meets components that lanes cannot hold (RGG 2^20 at 1/13: 188 us a call,
+// at 1/27: 176), a round too late costs that round.  Sparse graphs fall apart
+// sooner (512 x 512 grid at 1/14: 74 us, at 1/28: 78).
+constexpr int kFinDiv = 24;
+constexpr int kFinDivSparse = 12;
+constexpr int kFinSparse = 6;      // entries a vertex on average, at most
 enum : int { kFinSingle = 1, kFinMember = 2, kFinRootCand = 3 };
 enum : int { kFinNotRoot = 0, kFinRoot = 1, kFinTooBig = 2 };
 
 // Item i of the block's lists (cb blue, then the red ones).
+template <bool kSolo>
 __device__ __forceinline__ int item_at(const Params &p, const int *list, int cb, int i)
 {
-    return __ldcs(list + (i < cb ? i : p.region - 1 - (i - cb)));
+    return Mem<kSolo>::item(list + (i < cb ? i : p.region - 1 - (i - cb)));
 }
 
 // Preference key of an entry naming u with weight w, as the finish phase
@@ -1530,19 +1399,19 @@ __device__ __forceinline__ unsigned long long fin_key(int u, float w)
 }
 
 // Own-list scan of vertex v, entries [b, e): active neighbours (blue or red),
-// whether one has a smaller id, whether a neighbour is unmatchable, and the
-// positions and ids of the first kFinRec active neighbours.
+// whether one has a smaller id, and the positions and ids of the first kFinRec
+// of them.
 constexpr int kFinRec = 4;  // active neighbours a record holds
 __device__ __forceinline__ void fin_scan_thread(const Params &p, int v, int b, int e, int &nint, bool &lower,
-                                                bool &bad, int (&jr)[kFinRec], int (&ur)[kFinRec])
+                                                int (&jr)[kFinRec], int (&ur)[kFinRec])
 {
     for (int j0 = b; j0 < e; j0 += 8) {
         int u[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) u[k] = j0 + k < e ? __ldg(p.nbrs + j0 + k) : -1;
-        uint8_t c[8];
+        unsigned c[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) c[k] = u[k] >= 0 ? p.col[u[k]] : (uint8_t)kMatched;
+        for (int k = 0; k < 8; ++k) c[k] = u[k] >= 0 ? colour_bits(p.col[(unsigned)u[k] >> 4], u[k]) : (unsigned)kMatched;
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             if (c[k] <= kRed) {
@@ -1556,7 +1425,6 @@ __device__ __forceinline__ void fin_scan_thread(const Params &p, int v, int b, i
                 ++nint;
                 lower |= u[k] < v;
             }
-            bad |= c[k] == kDead;
         }
     }
 }
@@ -1565,23 +1433,22 @@ __device__ __forceinline__ void fin_scan_thread(const Params &p, int v, int b, i
 // kFinShort; every lane gets the results (the first kFinRec active
 // neighbours in list order too).
 __device__ __forceinline__ void fin_scan_warp(const Params &p, int v, int b, int e, int &nint, bool &lower,
-                                              bool &bad, int (&jr)[kFinRec], int (&ur)[kFinRec])
+                                              int (&jr)[kFinRec], int (&ur)[kFinRec])
 {
     const int lane = threadIdx.x & 31;
     int cnt = 0;
-    bool lo = false, bd = false;
+    bool lo = false;
     for (int r0 = b; r0 < e; r0 += 32 * 4) {
         int u[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) u[k] = r0 + 32 * k + lane < e ? __ldg(p.nbrs + r0 + 32 * k + lane) : -1;
-        uint8_t c[4];
+        unsigned c[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) c[k] = u[k] >= 0 ? p.col[u[k]] : (uint8_t)kMatched;
+        for (int k = 0; k < 4; ++k) c[k] = u[k] >= 0 ? colour_bits(p.col[(unsigned)u[k] >> 4], u[k]) : (unsigned)kMatched;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const bool in = c[k] <= kRed;
             lo |= in && u[k] < v;
-            bd |= c[k] == kDead;
             unsigned m = __ballot_sync(kFull, in);
             while (m && cnt < kFinRec) {
                 const int sb = __ffs(m) - 1;
@@ -1601,7 +1468,6 @@ __device__ __forceinline__ void fin_scan_warp(const Params &p, int v, int b, int
     }
     nint = cnt;
     lower = __any_sync(kFull, lo);
-    bad = __any_sync(kFull, bd);
 }
 
 // Component search for root candidate v by its warp.  Members are numbered in
@@ -1625,22 +1491,19 @@ __device__ __forceinline__ int fin_search(const Params &p, FinWarp &fw, int v, i
         if (e - b > kFinMaxDeg) return kFinTooBig;
         if (lane == 0) {
             fw.eoff[f] = ne;
-            fw.mbeg[f] = b;
-            fw.mdeg[f] = e - b;
         }
         seen += (unsigned long long)(e - b);
         for (int j0 = b; j0 < e; j0 += 32) {
             const int j = j0 + lane;
             int u = -1;
             float wj = 0.0f;
-            uint8_t c = kMatched;
+            unsigned c = kMatched;
             if (j < e) {
                 u = __ldg(p.nbrs + j);
                 if (kW) wj = __ldg(p.w + j);  // with the id: no dependent load once the colour is known
-                c = p.col[u];
+                c = colour_bits(p.col[(unsigned)u >> 4], u);
             }
             const bool in = c <= kRed;
-            if (__any_sync(kFull, c == kDead)) return kFinTooBig;
             if (__any_sync(kFull, in && u < v)) return kFinNotRoot;
             unsigned m = __ballot_sync(kFull, in);
             unsigned long long pref = 0;
@@ -1711,9 +1574,12 @@ __device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, int t0, in
     if (own) {
         eb = fw.eoff[lane];
         ee = fw.eoff[lane + 1];
-        deg = fw.mdeg[lane];
-        beg = fw.mbeg[lane];
         fw.best[lane] = 0ull;
+        if (kStats) {
+            const int2 r = __ldg(p.ranges + g);
+            deg = degree_of(r);
+            beg = r.x;
+        }
     }
     // learned colouring: whether a red member may retire (its list is short enough)
     const bool may_retire = p.fin_retire && own && degree_of(__ldg(p.ranges + g)) <= kRetireMaxDeg;
@@ -1823,8 +1689,6 @@ enum : int { kFinOverflow = 3 };
 struct FinComp {
     unsigned long long pref[kFinTEntries];
     int mem[kFinTMembers];
-    int mbeg[kFinTMembers];
-    int mdeg[kFinTMembers];
     uint8_t tgt[kFinTEntries];
     uint8_t eoff[kFinTMembers + 1];
     int k;
@@ -1843,9 +1707,8 @@ __device__ __forceinline__ int fin_meta_count(int meta) { return (meta >> 8) & 0
 // As fin_search, by one thread for root candidate v (record i), following the
 // records instead of the lists: each member costs two loads from L2 (its
 // record's index, its record).  kFinOverflow when a member's record is
-// incomplete or the component does not fit FinComp.  The lists' bounds are
-// read only for the instrumented kernel's counters.
-template <bool kW, bool kStats>
+// incomplete or the component does not fit FinComp.
+template <bool kW>
 __device__ __forceinline__ int fin_search_thread(const Params &p, int v, int i, FinComp &cp)
 {
     int ix[kFinTMembers];
@@ -1858,11 +1721,6 @@ __device__ __forceinline__ int fin_search_thread(const Params &p, int v, int i, 
         const int cnt = fin_meta_count(r0.x);
         if (cnt > kFinRec) return kFinOverflow;
         cp.eoff[f] = (uint8_t)ne;
-        if (kStats) {
-            const int2 r = __ldg(p.ranges + cp.mem[f]);
-            cp.mbeg[f] = r.x;
-            cp.mdeg[f] = r.y > r.x ? r.y - r.x : 0;
-        }
         const int uu[kFinRec] = {r0.z, r0.w, r1.x, r1.y};
         const int ww[kFinRec] = {r1.z, r1.w, r2.x, r2.y};
 #pragma unroll
@@ -1944,8 +1802,8 @@ __device__ __forceinline__ void fin_share(int cnt, int &lo, int &hi)
 // (a thread each, its warp for lists longer than kFinShort), classify it,
 // record its first active neighbours (and in req[v].x the record's index),
 // and, with kSingles, resolve the singletons at once.  Returns whether the
-// attempt has to be called off: a list longer than kFinMaxDeg, an unmatchable
-// neighbour, or more items than the block has records for.
+// attempt has to be called off: a list longer than kFinMaxDeg, or more items
+// than the block has records for.
 template <bool kW, bool kStats, bool kSingles>
 __device__ __forceinline__ bool finish_scan(const Params &p, int t, const int *list, int cb, int cr)
 {
@@ -1957,12 +1815,12 @@ __device__ __forceinline__ bool finish_scan(const Params &p, int t, const int *l
     fin_share(cnt_all, lo_i, hi_i);
     for (int base = lo_i; base < hi_i; base += 32) {
         const int i = base + lane;
-        const int v = i < hi_i ? item_at(p, list, cb, i) : -1;
+        const int v = i < hi_i ? item_at<false>(p, list, cb, i) : -1;
         const int2 r = v >= 0 ? __ldg(p.ranges + v) : make_int2(0, 0);
         const int deg = degree_of(r);
         int nint = 0, jr[kFinRec] = {0, 0, 0, 0}, ur[kFinRec] = {0, 0, 0, 0};
         bool lower = false, bad = false;
-        if (v >= 0 && deg <= kFinShort) fin_scan_thread(p, v, r.x, r.x + deg, nint, lower, bad, jr, ur);
+        if (v >= 0 && deg <= kFinShort) fin_scan_thread(p, v, r.x, r.x + deg, nint, lower, jr, ur);
         unsigned longs = __ballot_sync(kFull, v >= 0 && deg > kFinShort);
         while (longs) {
             const int s = __ffs(longs) - 1;
@@ -1974,12 +1832,11 @@ __device__ __forceinline__ bool finish_scan(const Params &p, int t, const int *l
                 continue;
             }
             int n2, j2[kFinRec], u2[kFinRec];
-            bool l2, b2;
-            fin_scan_warp(p, vs, bs, bs + ds, n2, l2, b2, j2, u2);
+            bool l2;
+            fin_scan_warp(p, vs, bs, bs + ds, n2, l2, j2, u2);
             if (lane == s) {
                 nint = n2;
                 lower = l2;
-                bad = b2;
 #pragma unroll
                 for (int q = 0; q < kFinRec; ++q) {
                     jr[q] = j2[q];
@@ -2050,7 +1907,7 @@ __device__ __forceinline__ bool finish_roots(const Params &p, Smem &sm, int t, i
         const int v = c == kFinRootCand ? r0.y : -1;
         int rres = kFinNotRoot;
         FinComp cp;
-        if (c == kFinRootCand) rres = fin_search_thread<kW, kStats>(p, v, at, cp);
+        if (c == kFinRootCand) rres = fin_search_thread<kW>(p, v, at, cp);
         // the lanes' components, packed into the warp and played together, a lane
         // per member (a lane playing its component alone would colour its
         // members one after another)
@@ -2076,8 +1933,6 @@ __device__ __forceinline__ bool finish_roots(const Params &p, Smem &sm, int t, i
                 for (int l = 0; l < km; ++l) {
                     fw.mem[mo + l] = cp.mem[l];
                     fw.eoff[mo + l] = eo + cp.eoff[l];
-                    fw.mdeg[mo + l] = cp.mdeg[l];
-                    fw.mbeg[mo + l] = cp.mbeg[l];
                 }
                 for (int e = 0; e < nem; ++e) {
                     fw.pref[eo + e] = cp.pref[e];
@@ -2115,10 +1970,11 @@ __device__ __forceinline__ bool finish_roots(const Params &p, Smem &sm, int t, i
     return abort;
 }
 
-// One barrier of k_match, with the block's summand and the sum over the blocks.
-__device__ __forceinline__ bool barrier_sum(const Params &p, Smem &sm, unsigned &turn, unsigned add, unsigned *sum, int mark)
+// One barrier of k_match, with the block's summand (two words of shared memory)
+// and the sum over the blocks.
+__device__ __forceinline__ bool barrier_sum(const Params &p, Smem &sm, unsigned &turn, const int *part, unsigned *sum, int mark)
 {
-    return grid_sync(sm, p.ctl, turn, add, sum, p.result, p.tstamp, mark, p.spin_limit, p.skip_mark);
+    return grid_sync(sm, p.ctl, turn, part, sum, p.result, p.tstamp, mark, p.spin_limit, p.skip_mark);
 }
 
 // The finish phase of round t.  Returns -1 if a barrier wait gave up, else
@@ -2129,20 +1985,27 @@ template <bool kW, bool kStats>
 __device__ __forceinline__ int finish_phase(const Params &p, Smem &sm, unsigned &turn, int t, const int *list, int cb, int cr)
 {
     unsigned off;
+    auto call_off = [&](bool abort) {  // the block's summand: sm.flag + sm.zero
+        if (abort) sm.flag = 1;
+    };
     // counters must not count a called-off attempt: the instrumented kernel
     // checks, then resolves; the plain one is speculative (a called-off attempt
     // leaves only values that the rounds write again)
-    bool abort = finish_scan<kW, kStats, !kStats>(p, t, list, cb, cr);
-    if (!barrier_sum(p, sm, turn, (unsigned)__syncthreads_or(abort), &off, 3 * t + 1)) return -1;
+    call_off(finish_scan<kW, kStats, !kStats>(p, t, list, cb, cr));
+    if (!barrier_sum(p, sm, turn, &sm.flag, &off, 3 * t + 1)) return -1;
     if (kStats && !off) {
-        abort = finish_roots<kW, kStats, false, false>(p, sm, t, cb, cr);
-        if (!barrier_sum(p, sm, turn, (unsigned)__syncthreads_or(abort), &off, -1)) return -1;
+        call_off(finish_roots<kW, kStats, false, false>(p, sm, t, cb, cr));
+        if (!barrier_sum(p, sm, turn, &sm.flag, &off, -1)) return -1;
     }
     if (!off) {
-        abort = finish_roots<kW, kStats, true, kStats>(p, sm, t, cb, cr);
-        if (!barrier_sum(p, sm, turn, (unsigned)__syncthreads_or(abort), &off, 3 * t + 2)) return -1;
+        call_off(finish_roots<kW, kStats, true, kStats>(p, sm, t, cb, cr));
+        if (!barrier_sum(p, sm, turn, &sm.flag, &off, 3 * t + 2)) return -1;
     }
-    if (off) return 0;
+    if (off) {
+        if (threadIdx.x == 0) sm.flag = 0;
+        __syncthreads();  // the working areas change hands
+        return 0;
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         const int last = max(__ldcg(&p.ctl->fin_last), __ldcg(&p.ctl->iso_last) - 1);
         p.result->rounds = p.maximal ? min(last + 2, p.cap) : p.cap;
@@ -2159,11 +2022,13 @@ __device__ __forceinline__ int finish_phase(const Params &p, Smem &sm, unsigned 
 // and leave the loop at the same round.  Vertices that could still be matched
 // at the end keep their last colour as their match value (the reference
 // leaves match[v] = 0 / 1 for them).
-template <bool kW, bool kStats, bool kPolicy>
-__global__ void __launch_bounds__(kThreads, 2) k_match(const __grid_constant__ Params p)
+template <bool kW, bool kStats, bool kPolicy, bool kSolo>
+__global__ void __launch_bounds__(kThreads, kSolo ? 1 : 2) k_match(const __grid_constant__ Params p)
 {
     extern __shared__ __align__(16) unsigned char dsmem[];
     Smem &sm = *reinterpret_cast<Smem *>(dsmem);
+    SoloMem &solo = *reinterpret_cast<SoloMem *>(dsmem + kSmemBytes);
+    const Mem<kSolo> m = kSolo ? Mem<kSolo>{solo.col, solo.best} : Mem<kSolo>{p.col, p.best};
     const long long rbase = (long long)blockIdx.x * p.region;
     const bool first = blockIdx.x == 0 && threadIdx.x == 0;
     // the next call's control block (no block of this call reads it)
@@ -2171,39 +2036,37 @@ __global__ void __launch_bounds__(kThreads, 2) k_match(const __grid_constant__ P
         for (int i = threadIdx.x; i < (int)(sizeof(Ctl) / 8); i += kThreads)
             reinterpret_cast<unsigned long long *>(p.ctl_next)[i] = 0ull;
     unsigned turn = 0, act = 0, shared = 0;
-    int cb, cr, t = 0;
-    init_phase<kW, kStats, kPolicy>(p, sm, p.lists[0] + rbase, cb, cr);
-    if (!barrier_sum(p, sm, turn, (unsigned)(cb + cr), &act, 0)) return;
+    int t = 0;
+    init_phase<kW, kStats, kPolicy>(p, m, sm, kSolo ? solo.lists[0] : p.lists[0] + rbase);
+    if (!barrier_sum(p, sm, turn, sm.count[0], &act, 0)) return;
     const unsigned active0 = act;  // active vertices at round 0
     unsigned fin_next = active0;   // finish phase: attempt once the active set is this small
     for (;; ++t) {
-        int *list = p.lists[t & 1] + rbase, *next = p.lists[(t & 1) ^ 1] + rbase;
+        int *list = kSolo ? solo.lists[t & 1] : p.lists[t & 1] + rbase;
+        int *next = kSolo ? solo.lists[(t & 1) ^ 1] : p.lists[(t & 1) ^ 1] + rbase;
+        const int cb = sm.count[t & 1][0], cr = sm.count[t & 1][1];
         // the finish phase (the symmetric path of a constant colouring only); in
         // one block the rounds cost less than it does
-        if ((!kPolicy || p.fin_retire) && p.sym && t > 0 && gridDim.x > 1 && p.fin_div > 0 && act > 0 && act <= fin_next &&
+        if (!kSolo && (!kPolicy || p.fin_retire) && p.sym && t > 0 && gridDim.x > 1 && p.fin_div > 0 && act > 0 && act <= fin_next &&
             (unsigned long long)act * (unsigned)p.fin_div <= active0) {
             const int done = finish_phase<kW, kStats>(p, sm, turn, t, list, cb, cr);
             if (done < 0) return;
             if (done) break;
             fin_next = act / 2;  // called off: again when the set has halved
-            __syncthreads();     // the working areas change hands
         }
-        scan_window<kW, kStats, kPolicy>(p, sm, t, list, rbase, cb, cr);
-        if (!barrier_sum(p, sm, turn, sm.shared_n > 0 ? 1u : 0u, &shared, 3 * t + 1)) return;
+        scan_window<kW, kStats, kPolicy>(p, m, sm, t, list, rbase, cb, cr);
+        if (!barrier_sum(p, sm, turn, &sm.flag, &shared, 3 * t + 1)) return;
         if (shared) {
-            scan_long<kW, kStats>(p, sm, t, (int)(blockIdx.x * kWarps + (threadIdx.x >> 5)), (int)(gridDim.x * kWarps));
-            if (!barrier_sum(p, sm, turn, 0u, &shared, -1)) return;
+            scan_shared<kW, kStats>(p, m, t);
+            if (!barrier_sum(p, sm, turn, &sm.flag, &shared, -1)) return;
             if (first) p.ctl->staged_pack = 0ull;  // empty again for the next round
         }
         if (p.tstamp && first) p.tstamp[3 * t + 2] = global_ns();
         bool has_next = t + 1 < p.cap;
         const bool seeds_short = has_next && t + 1 >= p.nseeds;
         if (seeds_short) has_next = false;
-        int ncb, ncr;
-        commit_phase<kW, kStats, kPolicy>(p, sm, t, has_next, list, next, rbase, cb, cr, ncb, ncr);
-        cb = ncb;
-        cr = ncr;
-        if (!barrier_sum(p, sm, turn, (unsigned)(cb + cr), &act, 3 * t + 3)) return;
+        commit_phase<kW, kStats, kPolicy>(p, m, sm, t, has_next, list, next, rbase, cb, cr);
+        if (!barrier_sum(p, sm, turn, sm.count[(t & 1) ^ 1], &act, 3 * t + 3)) return;
         if (has_next && act > 0) continue;
         // the loop ends; survivors of the last round keep its colours
         if (first) {
@@ -2214,14 +2077,14 @@ __global__ void __launch_bounds__(kThreads, 2) k_match(const __grid_constant__ P
             p.result->rounds = rounds;
             if (seeds_short) p.result->status = 1;
         }
-        for (int i = threadIdx.x; i < cb + cr; i += kThreads) {
-            const int v = item_at(p, next, cb, i);
-            p.match[v] = i < cb ? kBlue : kRed;
+        const int eb = sm.count[(t & 1) ^ 1][0], er = sm.count[(t & 1) ^ 1][1];
+        for (int i = threadIdx.x; i < eb + er; i += kThreads) {
+            const int v = item_at<kSolo>(p, next, eb, i);
+            p.match[v] = i < eb ? kBlue : kRed;
             if (p.last) p.last[v] = (uint8_t)t;
         }
         break;
     }
-    release_lines(p.col, p.n);
 }
 
 // ---------------------------------------------------------------------------
@@ -2376,18 +2239,27 @@ __device__ __forceinline__ void warp_sort_desc(unsigned long long &k, int &nb, i
         for (int stride = size >> 1; stride > 0; stride >>= 1) cas_step(k, nb, j, lane, stride, (lane & size) == 0);
 }
 
-// Window offsets as the kernels read them: the first slot (even), and in bit 0
-// whether the list is longer than its window.
+// Window offsets as the kernels read them: the first group of four entries,
+// and in bit 31 whether the list is longer than its window.
 __global__ void k_win_offsets(const int2 *ranges, const long long *off, int n, int *pwin_off)
 {
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
-        pwin_off[v] = (int)off[v] | (v < n && degree_of(ranges[v]) > kWin ? 1 : 0);
+        pwin_off[v] = (int)((unsigned)off[v] | (v < n && degree_of(ranges[v]) > kWin ? 0x80000000u : 0u));
 }
 
-__global__ void k_win_sizes(const int2 *ranges, int n, long long *slots)
+// Groups of each vertex's window; *even receives the sum of the windows'
+// lengths rounded up to even numbers.
+__global__ void k_win_sizes(const int2 *ranges, int n, long long *groups, unsigned long long *even)
 {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x)
-        slots[v] = (win_len(degree_of(ranges[v])) + 1) & ~1;
+    unsigned long long sum = 0;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const int wl = win_len(degree_of(ranges[v]));
+        groups[v] = (wl + 3) >> 2;
+        sum += (wl + 1) & ~1;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(kFull, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(even, sum);
 }
 
 constexpr int kWinRows = 8;       // rows of 32 entries tested against the window threshold per step
@@ -2449,7 +2321,7 @@ __device__ __forceinline__ void win_store(int2 *pwin, long long off, int deg, in
 {
     const int wl = win_len(deg);
     if (lane < wl) pwin[off + lane] = make_int2(nb, k >= (1ull << 32) ? j : (int)((unsigned)j | 0x80000000u));
-    if (lane == wl && (wl & 1)) pwin[off + lane] = make_int2(-1, (int)0x80000000u);  // an odd window's filler
+    else if (lane < ((wl + 3) & ~3)) pwin[off + lane] = make_int2(-1, (int)0x80000000u);  // fillers
 }
 
 // Windows of lists of at most kWinChunk entries, a warp per list (vertices
@@ -2472,7 +2344,7 @@ __global__ void __launch_bounds__(256) k_win_build(const int2 *ranges, const int
         unsigned long long k;
         int nb, j;
         win_top32(nbrs, w, r.x, r.y, lane, k, nb, j);
-        win_store(pwin, pwin_off[v] & ~1, deg, lane, k, nb, j);
+        win_store(pwin, 4ll * (pwin_off[v] & 0x7fffffff), deg, lane, k, nb, j);
     }
 }
 
@@ -2539,7 +2411,7 @@ __global__ void __launch_bounds__(256) k_win_chunk_merge(const int2 *ranges, con
             for (int stride = 16; stride > 0; stride >>= 1) cas_step(k, nb, j, lane, stride, true);
         }
         const int v = big[i];
-        win_store(pwin, pwin_off[v] & ~1, degree_of(ranges[v]), lane, k, nb, j);
+        win_store(pwin, 4ll * (pwin_off[v] & 0x7fffffff), degree_of(ranges[v]), lane, k, nb, j);
     }
 }
 
@@ -2723,12 +2595,9 @@ __global__ void k_batch_rounds(const uint8_t *last, const int *goff, int ngraphs
 
 constexpr int kStampCount = 3 * kMaxRounds + 1;
 constexpr size_t kResultBytes = 256;
-// Graphs of at most this many vertices are matched by one block: its rounds
-// need no grid barrier, and its reads stay in its L1.
-constexpr int kSoloVertices = 4096;
 
 struct PushState {
-    uint8_t *col = nullptr;
+    uint32_t *col = nullptr;
     int2 *req = nullptr;
     unsigned long long *best = nullptr;
     unsigned long long *part_key = nullptr;
@@ -2740,7 +2609,7 @@ struct PushState {
     int4 *rec = nullptr;              // finish phase: records, 3 int4 each, once a type on the symmetric path needs them
     size_t rec_cap = 0;               // records that rec holds
     int4 *staged = nullptr;
-    int *seg_first = nullptr;
+    int *piece_item = nullptr;
     Ctl *ctl = nullptr;               // two control blocks, used by alternate calls
     int ctl_turn = 0;
     Result *result = nullptr;         // pinned: written by the kernel
@@ -2769,7 +2638,7 @@ void free_state(PushState *s)
     dev_free(s->prop_key, 0);
     dev_free(s->rec, 0);
     dev_free(s->staged, 0);
-    dev_free(s->seg_first, 0);
+    dev_free(s->piece_item, 0);
     dev_free(s->ctl, 0);
     pinned_put(s->result, kResultBytes);
     dev_free(s->stats, 0);
@@ -2778,15 +2647,17 @@ void free_state(PushState *s)
     delete s;
 }
 
-template <bool kW, bool kStats, bool kPolicy>
+constexpr size_t smem_bytes(bool solo) { return kSmemBytes + (solo ? sizeof(SoloMem) : 0); }
+
+template <bool kW, bool kStats, bool kPolicy, bool kSolo>
 int coresident_blocks(int sms)
 {
     int occ = 0;
-    if (cudaFuncSetAttribute(k_match<kW, kStats, kPolicy>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(Smem)) != cudaSuccess)
+    if (cudaFuncSetAttribute(k_match<kW, kStats, kPolicy, kSolo>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem_bytes(kSolo)) != cudaSuccess)
         return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_match<kW, kStats, kPolicy>, kThreads, sizeof(Smem)) !=
-        cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_match<kW, kStats, kPolicy, kSolo>, kThreads,
+                                                      smem_bytes(kSolo)) != cudaSuccess)
         return 0;
     return occ * sms;
 }
@@ -2803,13 +2674,13 @@ mm_status alloc_state(mm_graph *g, PushState **out)
     const size_t n = (size_t)(g->n > 0 ? g->n : 1);
     // list capacities: every vertex is in at most one list per parity; only
     // lists longer than the window can fall back
-    const size_t nseg_cap = (size_t)(g->long_entries / kSegEntries) + 2;
+    const size_t npiece_cap = (size_t)(g->long_entries / kPiece + g->long_count) + 1;
     const size_t nstaged = (size_t)(g->long_count > 0 ? g->long_count : 1);
     // whatever the grid, its blocks' regions fit: (n / kChunk / blocks + 1) chunks each
     s->list_cap = n + (size_t)kChunk * (kMaxBlocks + 1);
     // pooled on the legacy stream, then synchronised so that any stream may use them
     cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->col, n, 0);
+    if (e == cudaSuccess) e = dev_alloc((void **)&s->col, (n + 15) / 16 * sizeof(uint32_t), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->req, n * sizeof(int2), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->best, n * sizeof(unsigned long long), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->part_key, n * sizeof(unsigned long long), 0);
@@ -2817,7 +2688,7 @@ mm_status alloc_state(mm_graph *g, PushState **out)
     if (e == cudaSuccess) e = dev_alloc((void **)&s->list_mem, 2 * s->list_cap * sizeof(int), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->prop, s->list_cap * sizeof(int), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->staged, nstaged * sizeof(int4), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->seg_first, nseg_cap * sizeof(int), 0);
+    if (e == cudaSuccess) e = dev_alloc((void **)&s->piece_item, npiece_cap * sizeof(int), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&s->ctl, 2 * sizeof(Ctl), 0);
     if (e == cudaSuccess) e = pinned_get((void **)&s->result, kResultBytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(s->ctl, 0, 2 * sizeof(Ctl), 0);
@@ -2836,12 +2707,13 @@ mm_status alloc_state(mm_graph *g, PushState **out)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     s->sms = sms;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    s->grid[0][0] = coresident_blocks<false, false, false>(sms);
-    s->grid[0][1] = coresident_blocks<false, true, false>(sms);
-    s->grid[0][2] = coresident_blocks<false, false, true>(sms);
-    s->grid[1][0] = coresident_blocks<true, false, false>(sms);
-    s->grid[1][1] = coresident_blocks<true, true, false>(sms);
-    s->grid[1][2] = coresident_blocks<true, false, true>(sms);
+    s->grid[0][0] = coresident_blocks<false, false, false, false>(sms);
+    s->grid[0][1] = coresident_blocks<false, true, false, false>(sms);
+    s->grid[0][2] = coresident_blocks<false, false, true, false>(sms);
+    s->grid[1][0] = coresident_blocks<true, false, false, false>(sms);
+    s->grid[1][1] = coresident_blocks<true, true, false, false>(sms);
+    s->grid[1][2] = coresident_blocks<true, false, true, false>(sms);
+    const bool solo = coresident_blocks<false, false, false, true>(sms) > 0 && coresident_blocks<true, false, false, true>(sms) > 0;
     cudaError_t le = cudaGetLastError();
     if (le != cudaSuccess) {
         free_state(s);
@@ -2859,7 +2731,7 @@ mm_status alloc_state(mm_graph *g, PushState **out)
         set_error("push: more co-resident blocks than the lists are sized for");
         return MM_ERR_UNSUPPORTED;
     }
-    if (!coop || under) {
+    if (!coop || under || !solo) {
         free_state(s);
         set_error("push: the device cannot run the cooperative round kernel");
         return MM_ERR_UNSUPPORTED;
@@ -2919,7 +2791,7 @@ mm_status launch_match(const Call &c)
     p.lists[1] = s->list_mem + s->list_cap;
     p.prop = s->prop;
     p.staged = s->staged;
-    p.seg_first = s->seg_first;
+    p.piece_item = s->piece_item;
     p.vbase = g->ngraphs > 0 ? g->d_vbase : nullptr;
     p.last = g->ngraphs > 0 ? g->d_last : nullptr;
     p.wfeat = s->wfeat;
@@ -2935,7 +2807,8 @@ mm_status launch_match(const Call &c)
     p.stats = kStats ? s->stats : nullptr;
     p.tstamp = c.timing ? s->tstamp : nullptr;
     p.zero_parts = s->zero_next ? 1 : 0;
-    p.fin_div = g->opt_fin_div < 0 ? 0 : (g->opt_fin_div == 0 ? kFinDiv : max(g->opt_fin_div, 2));
+    const bool sparse = g->sum_degree <= (long long)kFinSparse * g->n;
+    p.fin_div = g->opt_fin_div < 0 ? 0 : (g->opt_fin_div == 0 ? (sparse && !kPolicy ? kFinDivSparse : kFinDiv) : max(g->opt_fin_div, 2));
     p.spin_limit = debug_spin_limit();
     p.skip_mark = debug_skip_mark();
     if (kPolicy) {
@@ -2947,11 +2820,6 @@ mm_status launch_match(const Call &c)
         p.trace_rounds = pol->trace_rounds;
         // the finish phase knows the policy's threshold, not its features
         p.fin_retire = pol->constant && !pol->trace ? 1 : 0;
-        // Retirement shrinks the active set from round kRetireFrom on, so the
-        // default threshold comes a round or two earlier than on the plain
-        // path, while components are still too large for the finish phase: the
-        // default divisor is doubled here.
-        if (g->opt_fin_div == 0) p.fin_div = 2 * kFinDiv;
     }
     // blocks: all that fit at once, or the tuned number per SM (never more), and
     // no more than give every thread a vertex
@@ -2961,6 +2829,7 @@ mm_status launch_match(const Call &c)
     grid = g->n <= kSoloVertices ? 1 : min(grid, (g->n + kThreads - 1) / kThreads);
     const int chunks = (int)(((long long)g->n + kChunk - 1) / kChunk);
     p.region = (chunks + grid - 1) / grid * kChunk;
+    p.turn_magic = grid > 1 ? (uint32_t)((1ull << 32) / (unsigned)grid + 1) : 0u;
     if (!p.sym) {
         if (!s->prop_key)
             MM_CUDA_TRY(dev_alloc((void **)&s->prop_key, sizeof(uint32_t) * s->list_cap, c.stream), "request keys");
@@ -2980,8 +2849,13 @@ mm_status launch_match(const Call &c)
         p.rec = s->rec;
     }
     void *args[] = {&p};
-    MM_CUDA_TRY(cudaLaunchCooperativeKernel((void *)k_match<kW, kStats, kPolicy>, dim3(grid), dim3(kThreads), args,
-                                            sizeof(Smem), c.stream),
+    // one block, in its shared memory (the instrumented and policy kernels keep
+    // global memory: they are not for speed, or for larger graphs)
+    constexpr bool kMaySolo = !kStats && !kPolicy;
+    const bool solo = kMaySolo && grid == 1 && g->n <= kSoloVertices;
+    const void *kernel = solo ? (const void *)k_match<kW, kStats, kPolicy, kMaySolo>
+                              : (const void *)k_match<kW, kStats, kPolicy, false>;
+    MM_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3(grid), dim3(kThreads), args, smem_bytes(solo), c.stream),
                 "round kernel launch");
     return MM_OK;
 }
@@ -3229,29 +3103,31 @@ mm_status build_revkey(mm_graph *g, int weighted, cudaStream_t stream)
 mm_status windows_begin(mm_graph *g, cudaStream_t stream)
 {
     const int n = g->n;
-    long long *slots = nullptr, *off = nullptr;
+    long long *groups = nullptr, *off = nullptr;  // groups[n + 1]: the even sum
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
-    MM_CUDA_TRY(dev_alloc((void **)&slots, sizeof(long long) * ((size_t)n + 1), stream), "window sizes");
+    MM_CUDA_TRY(dev_alloc((void **)&groups, sizeof(long long) * ((size_t)n + 2), stream), "window sizes");
     cudaError_t e = dev_alloc((void **)&off, sizeof(long long) * ((size_t)n + 1), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(slots + n, 0, sizeof(long long), stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(groups + n, 0, 2 * sizeof(long long), stream);
     if (e == cudaSuccess) {
-        k_win_sizes<<<grid_for(n, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, n, slots);
+        k_win_sizes<<<grid_for(n, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, n, groups,
+                                                                  reinterpret_cast<unsigned long long *>(groups + n + 1));
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, slots, off, n + 1, stream);
+    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, groups, off, n + 1, stream);
     if (e == cudaSuccess) e = dev_alloc(&tmp, tmp_bytes, stream);
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, slots, off, n + 1, stream);
-    long long total = 0;
+    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, groups, off, n + 1, stream);
+    long long total = 0, even = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&total, off + n, sizeof total, cudaMemcpyDeviceToHost, stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&even, groups + n + 1, sizeof even, cudaMemcpyDeviceToHost, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     dev_free(tmp, stream);
-    dev_free(slots, stream);
+    dev_free(groups, stream);
     if (e != cudaSuccess) {
         dev_free(off, stream);
         return cuda_fail(e, "window offsets");
     }
-    if (total >= (1ll << 31)) {
+    if (even >= (1ll << 31)) {
         dev_free(off, stream);
         set_error("push: more than 2^31 - 1 preference-window slots are not supported");
         return MM_ERR_UNSUPPORTED;
@@ -3264,7 +3140,7 @@ mm_status windows_begin(mm_graph *g, cudaStream_t stream)
         k_win_offsets<<<grid_for(n + 1ll, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, off, n, packed);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = dev_alloc((void **)&win, sizeof(int2) * (size_t)(total > 0 ? total : 1), stream);
+    if (e == cudaSuccess) e = dev_alloc((void **)&win, 4 * sizeof(int2) * (size_t)(total > 0 ? total : 1), stream);
     if (e == cudaSuccess) e = dev_alloc((void **)&big, sizeof(int) * ((size_t)n + 1), stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(big + n, 0, sizeof(int), stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
@@ -3357,7 +3233,7 @@ __global__ void k_win_weights(const int2 *ranges, const float *w, const int *pwi
 {
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int wl = win_len(degree_of(ranges[v]));
-        const int o = pwin_off[v] & ~1;
+        const long long o = 4ll * (pwin_off[v] & 0x7fffffff);
         for (int e = 0; e < wl; ++e) {
             int2 x = pwin[o + e];
             x.y = __float_as_int(__ldg(w + (x.y & 0x7fffffff)));

@@ -233,7 +233,8 @@ template <bool kSolo>
 struct Mem {
     uint32_t *col_;
     unsigned long long *best_;
-    __device__ __forceinline__ unsigned col(int u) const { return colour_bits(col_[(unsigned)u >> 4], u); }
+    __device__ __forceinline__ uint32_t word(int u) const { return col_[(unsigned)u >> 4]; }
+    __device__ __forceinline__ unsigned col(int u) const { return colour_bits(word(u), u); }
     __device__ __forceinline__ void flip(int v, unsigned delta) const
     {
         atomicXor(col_ + ((unsigned)v >> 4), delta << (2u * ((unsigned)v & 15u)));
@@ -604,27 +605,26 @@ __device__ __forceinline__ bool colour_blue(const Params &p, int v, int base, fl
 
 // ---- worklist compaction for the set-up and commit passes ----
 //
-// A warp handles tiles of up to 128 consecutive items (lane l items l, l + 32,
-// l + 64, l + 96) and takes its places in the block's lists with one shared
+// A warp handles tiles of 32 W consecutive items (lane l items l, l + 32, ..;
+// W = 4 where the block has enough for all its warps, so that four items'
+// loads and hashes overlap, else 1) and takes its places in the block's lists with one shared
 // atomic a tile and colour, so no warp waits for another: with block-wide
 // prefix sums, three block barriers a tile left the set-up of R-MAT 2^22 at
 // half the instruction rate its pipes allow.
 enum : int { kDrop = -1, kToBlue = 0, kToRed = 1 };
 
-// Items a lane handles in a tile: fewer when the block has few, so that all
-// warps share them.
-__device__ __forceinline__ int tile_per(int total) { return min(kPer, max(1, (total + kThreads - 1) / kThreads)); }
+constexpr int kWideItems = 2 * kThreads;  // items from which a block takes tiles of W = 4
 
-template <bool kSolo>
-__device__ __forceinline__ void compact_tile(int *count, int *list, int region, const int (&dest)[kPer],
-                                             const int (&item)[kPer])
+template <bool kSolo, int W>
+__device__ __forceinline__ void compact_tile(int *count, int *list, int region, const int (&dest)[W],
+                                             const int (&item)[W])
 {
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    unsigned mb[kPer], mr[kPer];
+    unsigned mb[W], mr[W];
     int nb = 0, nr = 0;
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
+    for (int k = 0; k < W; ++k) {
         mb[k] = __ballot_sync(kFull, dest[k] == kToBlue);
         mr[k] = __ballot_sync(kFull, dest[k] == kToRed);
         nb += __popc(mb[k]);
@@ -634,7 +634,7 @@ __device__ __forceinline__ void compact_tile(int *count, int *list, int region, 
     if (lane < 2) at = atomicAdd(count + lane, lane == 0 ? nb : nr);
     int *blue = list + __shfl_sync(kFull, at, 0), *red = list + (region - 1 - __shfl_sync(kFull, at, 1));
 #pragma unroll
-    for (int k = 0; k < kPer; ++k) {
+    for (int k = 0; k < W; ++k) {
         if (dest[k] == kToBlue) Mem<kSolo>::put(blue + __popc(mb[k] & below), item[k]);
         if (dest[k] == kToRed) Mem<kSolo>::put(red - __popc(mr[k] & below), item[k]);
         blue += __popc(mb[k]);
@@ -691,29 +691,22 @@ __device__ __forceinline__ void resolve_isolated(const Params &p, Smem &sm, int 
 // rounds, whose per-round counters count them as the reference does.  A list
 // is known to be empty, or longer than its window, from its window's offsets
 // (weighted types) or from its range.
-template <bool kW, bool kStats, bool kPolicy, bool kSolo>
-__device__ __forceinline__ void init_phase(const Params &p, const Mem<kSolo> &m, Smem &sm, int *list)
+template <bool kW, bool kStats, bool kPolicy, bool kSolo, int W>
+__device__ __forceinline__ void init_tiles(const Params &p, const Mem<kSolo> &m, Smem &sm, int *list, int &iso_n,
+                                           int &iso_last)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t seed = p.seeds[0];
-    if (threadIdx.x == 0) {
-        sm.count[0][0] = sm.count[0][1] = sm.count[1][0] = sm.count[1][1] = 0;
-        sm.wnext = 3 * kThreads;
-        sm.stage_n = sm.big_n = sm.flag = sm.zero = 0;
-    }
-    for (int i = threadIdx.x; i < 256; i += kThreads) sm.iso.seeds[i] = p.seeds[i];
-    __syncthreads();
-    int iso_n = 0, iso_last = -1;
-    const int per = tile_per(p.region), tsize = 32 * per;
+    constexpr int tsize = 32 * W;
     const int ntiles = (p.region + tsize - 1) / tsize;
     // each tile's ranges are loaded while the tile before it is coloured and compacted
-    int vv[kPer];
-    int2 rr[kPer];
+    int vv[W];
+    int2 rr[W];
     auto fetch = [&](int tile) {
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
+        for (int k = 0; k < W; ++k) {
             const int s = tile * tsize + k * 32 + lane;
-            vv[k] = k < per && s < p.region ? own_vertex(p, s) : -1;
+            vv[k] = s < p.region ? own_vertex(p, s) : -1;
             rr[k] = make_int2(0, 0);
             if (vv[k] >= 0) {
                 if (kW) rr[k] = make_int2(__ldg(p.pwin_off + vv[k]), __ldg(p.pwin_off + vv[k] + 1));
@@ -723,23 +716,28 @@ __device__ __forceinline__ void init_phase(const Params &p, const Mem<kSolo> &m,
     };
     fetch(warp);
     for (int tile = warp; tile < ntiles; tile += kWarps) {
-        int dest[kPer], item[kPer];
-        bool none[kPer], longer[kPer];
+        int dest[W], item[W], base_v[W];
+        bool none[W], longer[W], blue_k[W];
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
+        for (int k = 0; k < W; ++k) {
             item[k] = vv[k];
+            base_v[k] = p.vbase && vv[k] >= 0 ? __ldg(p.vbase + vv[k]) : 0;
             none[k] = kW ? ((rr[k].y ^ rr[k].x) & 0x7fffffff) == 0 : degree_of(rr[k]) == 0;
             longer[k] = kW ? rr[k].x < 0 : degree_of(rr[k]) > kWin;
         }
         if (tile + kWarps < ntiles) fetch(tile + kWarps);
+        // straight-line hashes, the four items' instructions interleaved
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+            blue_k[k] = kPolicy ? false : colour_of((uint32_t)(item[k] - base_v[k]), seed, p.barrier) == kBlue;
         unsigned long long act = 0, blue_n = 0;
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
+        for (int k = 0; k < W; ++k) {
             const int v = item[k];
             dest[k] = kDrop;
             bool queue = false;
             if (v >= 0) {
-                const bool blue = colour_blue<kPolicy>(p, v, base_of(p, v), 0.0f, 0, seed);
+                const bool blue = kPolicy ? colour_blue<kPolicy>(p, v, base_v[k], 0.0f, 0, seed) : blue_k[k];
                 // (every completed round leaves them zero: a cut list's last piece clears them)
                 if (p.zero_parts && longer[k]) {
                     p.part_key[v] = 0ull;
@@ -767,7 +765,7 @@ __device__ __forceinline__ void init_phase(const Params &p, const Mem<kSolo> &m,
                 iso_n += __popc(mq);
             }
             // the colours of 32 consecutive vertices: two words, written whole
-            if (k < per) {
+            {
                 const unsigned bits = dest[k] == kToRed ? (unsigned)kRed << (2 * (lane & 15)) : 0u;
                 const unsigned w0 = __reduce_or_sync(kFull, lane < 16 ? bits : 0u);
                 const unsigned w1 = __reduce_or_sync(kFull, lane < 16 ? 0u : bits);
@@ -785,9 +783,25 @@ __device__ __forceinline__ void init_phase(const Params &p, const Mem<kSolo> &m,
             resolve_isolated(p, sm, iso_n, iso_last);
         }
     }
+}
+
+template <bool kW, bool kStats, bool kPolicy, bool kSolo>
+__device__ __forceinline__ void init_phase(const Params &p, const Mem<kSolo> &m, Smem &sm, int *list)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) {
+        sm.count[0][0] = sm.count[0][1] = sm.count[1][0] = sm.count[1][1] = 0;
+        sm.wnext = 3 * kThreads;
+        sm.stage_n = sm.big_n = sm.flag = sm.zero = 0;
+    }
+    for (int i = threadIdx.x; i < 256; i += kThreads) sm.iso.seeds[i] = p.seeds[i];
+    __syncthreads();
+    int iso_n = 0, iso_last = -1;
+    if (p.region > kWideItems) init_tiles<kW, kStats, kPolicy, kSolo, kPer>(p, m, sm, list, iso_n, iso_last);
+    else init_tiles<kW, kStats, kPolicy, kSolo, 1>(p, m, sm, list, iso_n, iso_last);
     if (!kPolicy && !kStats && p.sym) {
         // the ones left on the stack stay in the rounds: red, as in round 0
-        int dest[kPer] = {kDrop, kDrop, kDrop, kDrop}, item[kPer] = {-1, -1, -1, -1};
+        int dest[1] = {kDrop}, item[1] = {-1};
         if (lane < iso_n) {
             item[0] = sm.iso.item[warp][lane].x;
             dest[0] = kToRed;
@@ -947,9 +961,9 @@ __device__ __forceinline__ unsigned long long scan_rows(const Params &p, const M
         }
         unsigned c[kRows];
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) c[r] = nb[r] >= 0 ? m.col(nb[r]) : (unsigned)kMatched;
+        for (int r = 0; r < kRows; ++r) c[r] = nb[r] >= 0 ? m.word(nb[r]) : 0xffffffffu;
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) fold_entry<kW>(c[r], wv[r], j0 + r * 32 + lane, bw, bj, alive);
+        for (int r = 0; r < kRows; ++r) fold_entry<kW>(colour_bits(c[r], nb[r]), wv[r], j0 + r * 32 + lane, bw, bj, alive);
         if (!kW && __any_sync(kFull, bw > -1.0f)) break;
     }
     return strip_key<kW>(bw, bj, alive);
@@ -1025,8 +1039,7 @@ __device__ __noinline__ void scan_fallback(const Params &p, const Mem<kSolo> m, 
 // Phase A1 over the block's cb blue items.  The first items go to the threads
 // in order, the rest to the warps from a counter in shared memory.  A lane
 // holds one vertex at a time and reads its window eight entries a step (two
-// 32-byte loads, then the colours of two entries and, where these do not
-// decide, of the other six); as soon as a lane's vertex is
+// 32-byte loads, then the eight colours); as soon as a lane's vertex is
 // decided it takes the next one, whose window offsets it has prefetched, loads
 // the offsets of the one after that, whose id it has prefetched, and prefetches
 // another id.  So every lane keeps an independent chain of loads in flight and
@@ -1037,7 +1050,6 @@ __device__ __forceinline__ void scan_window(const Params &p, const Mem<kSolo> &m
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
     bool dry = 3 * kThreads >= cb;  // warp-uniform: the block's items are handed out
-    const bool few = cb <= 2 * kThreads;
     // Items for the lanes in `mask`: one shared atomic per warp.  Returns this
     // lane's item, or -1.
     auto grab = [&](unsigned mask) -> int {
@@ -1062,7 +1074,7 @@ __device__ __forceinline__ void scan_window(const Params &p, const Mem<kSolo> &m
     if (nv >= 0) nraw = window_raw<kW>(p, nv);
     bool has = cv >= 0, alive = false;
     bool narrow = kW && t == 0;
-    int seen = 0;
+    int seen = 0, last = 0;  // instrumented: entries read, the choice's place in its step
     while (__any_sync(kFull, has)) {
         if (has) {
             // eight entries a step (one dependent round trip for each 8: the scan
@@ -1080,30 +1092,29 @@ __device__ __forceinline__ void scan_window(const Params &p, const Mem<kSolo> &m
             if (!narrow && g + 1 < gend) window_group<kW>(p, g + 1, lo, hi, nb + 4, jv + 4);
             g += narrow ? 1 : 2;
             narrow = false;
-            // a full block reads the first two colours, and the others only for a
-            // vertex that they leave undecided (the phase is then bound by the
-            // sectors it requests: RGG 2^20's round 0 took 26.1 us for 29.7); a
-            // block with few items reads all at once, a round trip less
+            // the colours' words first, all in flight together, then the choice
+            // from the last entry down (straight-line code: with a branch an
+            // entry the loads went out one after another, RGG 2^20's round 1 20.6
+            // us for 17.4)
             unsigned c[8];
 #pragma unroll
-            for (int x = 0; x < 8; ++x) c[x] = (x < 2 || few) && nb[x] >= 0 ? m.col(nb[x]) : (unsigned)kMatched;
-            if (!few && !window_choice<kW>(p, c[0], jv[0]) && !window_choice<kW>(p, c[1], jv[1])) {
-#pragma unroll
-                for (int x = 2; x < 8; ++x) c[x] = nb[x] >= 0 ? m.col(nb[x]) : (unsigned)kMatched;
-            }
+            for (int x = 0; x < 8; ++x) c[x] = nb[x] >= 0 ? m.word(nb[x]) : 0xffffffffu;
             bool found = false;
             int cj = -1, ct = 0;
 #pragma unroll
-            for (int x = 0; x < 8; ++x) {
-                if (nb[x] < 0 || found) continue;
-                if (kStats) ++seen;
-                if (window_choice<kW>(p, c[x], jv[x])) {
+            for (int x = 7; x >= 0; --x) {
+                const unsigned b = colour_bits(c[x], nb[x]);
+                alive |= b != kMatched;
+                if (window_choice<kW>(p, b, jv[x])) {
                     found = true;
                     cj = jv[x];
                     ct = nb[x];
-                } else {
-                    alive |= c[x] != kMatched;
+                    if (kStats) last = x;
                 }
+            }
+            if (kStats) {
+#pragma unroll
+                for (int x = 0; x < 8; ++x) seen += nb[x] >= 0 && (!found || x <= last);
             }
             if (found || g >= gend) {
                 const ItemReq rq{p, sm, rbase, ci};
@@ -1200,74 +1211,71 @@ __device__ __noinline__ void scan_shared(const Params &p, const Mem<kSolo> m, in
 // Phase B: commit proposals, recolour survivors with the next seed, compact
 // the block's lists of round t+1.  Colours are
 // written only where they change.
-template <bool kW, bool kStats, bool kPolicy, bool kSolo>
-__device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &m, Smem &sm, int t, bool has_next, const int *list, int *next,
+template <bool kW, bool kStats, bool kPolicy, bool kSolo, int W>
+__device__ __forceinline__ void commit_tiles(const Params &p, const Mem<kSolo> &m, Smem &sm, int t, bool has_next, const int *list, int *next,
                                              long long rbase, int cb, int cr)
 {
     const uint32_t next_seed = has_next ? p.seeds[t + 1] : 0u;
     const int total = cb + cr;
-    const int per = tile_per(total), tsize = 32 * per;
+    constexpr int tsize = 32 * W;
     for (int base = (int)(threadIdx.x >> 5) * tsize; base < total; base += kWarps * tsize) {
-        // items, and with a blue item its request, loaded together
-        int vv[kPer], tg[kPer];
-        uint32_t low[kPer];
-        bool blue[kPer], gone[kPer];
+        // The loads of the tile's items go out together, pass by pass: item and
+        // request, then the best proposal (blue: its target's, red: its own).
+        int vv[W], tg[W], base_v[W];
+        uint32_t low[W];
+        bool blue[W], gone[W];
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
+        for (int k = 0; k < W; ++k) {
             const int i = base + k * 32 + (int)(threadIdx.x & 31);
-            const bool in = k < per && i < total;
+            const bool in = i < total;
             blue[k] = in && i < cb;
-            gone[k] = false;
-            vv[k] = -1;
+            vv[k] = in ? m.item(list + (i < cb ? i : p.region - 1 - (i - cb))) : -1;
             tg[k] = kReqNone;
             low[k] = 0u;
             if (blue[k]) {
-                vv[k] = m.item(list + i);
                 tg[k] = i < kPropCap ? sm.req.target[i] : __ldcs(p.prop + rbase + i);
                 if (!p.sym) low[k] = __ldcs(p.prop_key + rbase + i);
-            } else if (in) {
-                vv[k] = m.item(list + (p.region - 1 - (i - cb)));
-                // learned colouring: a red item retired in phase A carries its id complemented
-                if (kPolicy && vv[k] < 0) {
-                    gone[k] = true;
-                    vv[k] = ~vv[k];
-                }
             }
+            // learned colouring: a red item retired in phase A carries its id complemented
+            gone[k] = kPolicy && in && vv[k] < 0;
+            if (gone[k]) vv[k] = ~vv[k];
         }
-        // proposal state: blue -> its request (a shared fallback list's is in req), red -> the
-        // best proposal it received
-        unsigned long long key[kPer];
+        unsigned long long key[W];
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
-            key[k] = 0ull;
-            if (blue[k]) {
-                if (tg[k] == kReqShared) {
-                    const int2 q = __ldcg(p.req + vv[k]);
-                    tg[k] = q.x;
-                    low[k] = (uint32_t)q.y;
-                } else if (p.sym) {
-                    low[k] = ~(uint32_t)vv[k];
-                }
-                if (tg[k] >= 0 && low[k] != 0u) key[k] = m.best(tg[k]);
-            } else if (vv[k] >= 0) {
-                key[k] = m.best(vv[k]);
+        for (int k = 0; k < W; ++k) {
+            if (blue[k] && tg[k] == kReqShared) {  // a shared fallback list's request is in req
+                const int2 q = __ldcg(p.req + vv[k]);
+                tg[k] = q.x;
+                low[k] = (uint32_t)q.y;
             }
+            if (p.sym) low[k] = ~(uint32_t)vv[k];
+            // blue: a request whose key is not 0
+            const int at = blue[k] ? (low[k] != 0u ? tg[k] : -1) : vv[k];
+            key[k] = at >= 0 ? m.best(at) : 0ull;
+            base_v[k] = p.vbase && vv[k] >= 0 ? __ldg(p.vbase + vv[k]) : 0;
         }
-        int dest[kPer];
+        int partner[W];
+        bool nb[W];
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+            partner[k] = -1;
+            if (key[k]) {
+                const uint32_t kl = (uint32_t)key[k];
+                // the low half of a red vertex's key names the proposer: its id on
+                // the symmetric path, else the position of the red's entry for it
+                if (blue[k]) partner[k] = kl == low[k] ? tg[k] : -1;
+                else partner[k] = p.sym ? (int)~kl : __ldg(p.nbrs + (int)~kl);
+            }
+            // the next colour, straight-line for all items (the matched ones' is not used)
+            nb[k] = kPolicy ? false : colour_of((uint32_t)(vv[k] - base_v[k]), next_seed, p.barrier) == kBlue;
+        }
+        int dest[W];
         unsigned long long matched = 0, seen = 0, rdeg = 0, act = 0, nblue = 0;
 #pragma unroll
-        for (int k = 0; k < kPer; ++k) {
+        for (int k = 0; k < W; ++k) {
             dest[k] = kDrop;
             const int v = vv[k];
             if (v < 0) continue;
-            int partner = -1;
-            if (blue[k]) {
-                if (tg[k] >= 0 && low[k] != 0u && (uint32_t)key[k] == low[k]) partner = tg[k];
-            } else if (key[k]) {
-                // the low half of the key names the proposer: its id on the
-                // symmetric path, else the position of the red's entry for it
-                partner = p.sym ? (int)~(uint32_t)key[k] : __ldg(p.nbrs + (int)~(uint32_t)key[k]);
-            }
             if (kStats && !blue[k]) {
                 const int2 r = __ldg(p.ranges + v);
                 const int deg = degree_of(r);
@@ -1289,30 +1297,29 @@ __device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &
                 }
                 seen += at >= 0 ? (unsigned long long)(at - r.x + 1) : (unsigned long long)deg;
             }
-            if (partner >= 0) {
+            unsigned delta = 0u;
+            if (partner[k] >= 0) {
                 trace_left<kPolicy>(p, t, v);
-                p.match[v] = 4 + min(v, partner) - base_of(p, v);
-                m.flip(v, kMatched ^ (blue[k] ? kBlue : kRed));
+                p.match[v] = 4 + min(v, partner[k]) - base_v[k];
                 if (p.last) p.last[v] = (uint8_t)t;
+                delta = blue[k] ? kMatched ^ kBlue : kMatched ^ kRed;
                 ++matched;
-                continue;
-            }
-            // unmatchable (marked in phase A; learned colouring: red ones too)
-            if ((blue[k] && tg[k] == kReqDead) || gone[k]) {
+            } else if ((blue[k] && tg[k] == kReqDead) || gone[k]) {
+                // unmatchable (marked in phase A; learned colouring: red ones too)
                 trace_left<kPolicy>(p, t, v);
-                continue;
-            }
-            // survivor
-            if (!has_next) {
+            } else if (!has_next) {
                 dest[k] = blue[k] ? kToBlue : kToRed;
-                continue;
+            } else {
+                if (kPolicy) {
+                    const float role = blue[k] ? (tg[k] >= 0 && low[k] != 0u ? 1.0f : 0.5f) : 0.0f;
+                    nb[k] = colour_blue<kPolicy>(p, v, base_v[k], role, t + 1, next_seed);
+                }
+                ++act;
+                nblue += nb[k];
+                delta = nb[k] != blue[k] ? kBlue ^ kRed : 0u;
+                dest[k] = nb[k] ? kToBlue : kToRed;
             }
-            const float role = blue[k] ? (tg[k] >= 0 && low[k] != 0u ? 1.0f : 0.5f) : 0.0f;
-            const bool nb = colour_blue<kPolicy>(p, v, base_of(p, v), role, t + 1, next_seed);
-            ++act;
-            nblue += nb;
-            if (nb != blue[k]) m.flip(v, kBlue ^ kRed);
-            dest[k] = nb ? kToBlue : kToRed;
+            if (delta) m.flip(v, delta);
         }
         if (kStats) {
             stat_add(p, t, MM_ST_MATCHED, matched);
@@ -1326,6 +1333,14 @@ __device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &
         }
         compact_tile<kSolo>(sm.count[(t & 1) ^ 1], next, p.region, dest, vv);
     }
+}
+
+template <bool kW, bool kStats, bool kPolicy, bool kSolo>
+__device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &m, Smem &sm, int t, bool has_next,
+                                             const int *list, int *next, long long rbase, int cb, int cr)
+{
+    if (cb + cr > kWideItems) commit_tiles<kW, kStats, kPolicy, kSolo, kPer>(p, m, sm, t, has_next, list, next, rbase, cb, cr);
+    else commit_tiles<kW, kStats, kPolicy, kSolo, 1>(p, m, sm, t, has_next, list, next, rbase, cb, cr);
     if (threadIdx.x == 0) {  // for the next window scan (read after the barrier)
         sm.wnext = 3 * kThreads;
         sm.stage_n = sm.big_n = sm.flag = 0;

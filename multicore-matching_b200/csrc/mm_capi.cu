@@ -173,32 +173,14 @@ namespace {
 //   sorted       every list is strictly increasing (no duplicate entries);
 //   symmetric    the multiset of entries (v, u) equals that of (u, v), and
 //                with weights, of (v, u, w) and (u, v, w).
-// Symmetry is tested with two pairs of 64-bit sums of a hash of the ordered
-// entry (splitmix64's finalizer): a transposed multiset has equal sums, a
-// different one has equal sums only by a 64-bit coincidence.
+// (add_skew in mm_common.cuh).
 struct GraphCheck {
-    unsigned long long fwd_s, rev_s;  // structure: sum F(v, u), sum F(u, v)
-    unsigned long long fwd_w, rev_w;  // with weight bits
+    unsigned long long skew_s, skew_w;  // 0: symmetric in structure, with weights
     int bad;        // 1: a range outside [0, nnz); 2: an id outside [0, n)
     int noncontig;  // ranges do not tile [0, nnz) in vertex order
     int unsorted;   // some list is not strictly increasing
     int pad;
 };
-
-__device__ __forceinline__ unsigned long long mix64(unsigned long long z)
-{
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    return z ^ (z >> 31);
-}
-__device__ __forceinline__ unsigned long long hash_s(unsigned a, unsigned b)
-{
-    return mix64((((unsigned long long)a << 32) | b) + 0x9E3779B97F4A7C15ull);
-}
-__device__ __forceinline__ unsigned long long hash_w(unsigned a, unsigned b, unsigned wbits)
-{
-    return mix64((((unsigned long long)a << 32) | b) ^ mix64((unsigned long long)wbits + 0xD1B54A32D192ED03ull));
-}
 
 __global__ void k_check_ranges(const int2 *ranges, int n, long long nnz, GraphCheck *c)
 {
@@ -236,7 +218,7 @@ __global__ void __launch_bounds__(256) k_check_entries(const int2 *ranges, const
 {
     __shared__ int start[kChk + 1];
     __shared__ int s_v0, s_cnt;
-    unsigned long long fs = 0, rs = 0, fw = 0, rw = 0;
+    unsigned long long ss = 0, sw = 0;
     int bad = 0, uns = 0;
     const long long chunks = (j1 - j0 + kChk - 1) / kChk;
     for (long long ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
@@ -273,31 +255,14 @@ __global__ void __launch_bounds__(256) k_check_entries(const int2 *ranges, const
             }
             // compared with the entry before (earlier chunks have arrived; later ones may not have)
             if (j > (long long)ranges[v].x && nbrs[j - 1] >= u) uns = 1;
-            fs += hash_s((unsigned)v, (unsigned)u);
-            rs += hash_s((unsigned)u, (unsigned)v);
-            if (kWeights) {
-                const unsigned wb = __float_as_uint(w[j]);
-                fw += hash_w((unsigned)v, (unsigned)u, wb);
-                rw += hash_w((unsigned)u, (unsigned)v, wb);
-            }
+            add_skew((unsigned)v, (unsigned)u, kWeights ? __float_as_uint(w[j]) : 0u, kWeights, ss, sw);
         }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        fs += __shfl_down_sync(0xffffffffu, fs, o);
-        rs += __shfl_down_sync(0xffffffffu, rs, o);
-        fw += __shfl_down_sync(0xffffffffu, fw, o);
-        rw += __shfl_down_sync(0xffffffffu, rw, o);
-    }
+    block_add(&c->skew_s, ss);
+    if (kWeights) block_add(&c->skew_w, sw);
     bad = __any_sync(0xffffffffu, bad);
     uns = __any_sync(0xffffffffu, uns);
     if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&c->fwd_s, fs);
-        atomicAdd(&c->rev_s, rs);
-        if (kWeights) {
-            atomicAdd(&c->fwd_w, fw);
-            atomicAdd(&c->rev_w, rw);
-        }
         if (bad) atomicOr(&c->bad, 2);
         if (uns) atomicOr(&c->unsorted, 1);
     }
@@ -446,9 +411,9 @@ mm_status upload_and_check(mm_graph *g, const int *ranges, const int *nbrs, cons
         return MM_ERR_GRAPH;
     }
     g->has_weights = have_w;
-    g->sym_struct = contiguous && !c.unsorted && c.fwd_s == c.rev_s;
+    g->sym_struct = contiguous && !c.unsorted && c.skew_s == 0;
     // unit weights are symmetric whenever the structure is
-    g->sym_weights = g->sym_struct && (!have_w || c.fwd_w == c.rev_w);
+    g->sym_weights = g->sym_struct && (!have_w || c.skew_w == 0);
     return MM_OK;
 }
 
@@ -479,9 +444,7 @@ mm_status create_common(int n, const int *ranges, long long nnz, const int *nbrs
     cudaGetDevice(&g->device);
     g->n = n;
     g->nnz = nnz;
-    // Neighbour and weight arrays are padded to a multiple of 4 entries plus 4 so
-    // that 16-byte vector loads starting at any in-range, 4-aligned slot stay inside.
-    const size_t nv = (size_t)(n > 0 ? n : 1), ne = ((size_t)nnz + 3) / 4 * 4 + 4;
+    const size_t nv = (size_t)(n > 0 ? n : 1), ne = padded_entries(nnz);
     const cudaMemcpyKind kind = from_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     cudaError_t e = dev_alloc((void **)&g->d_ranges, nv * sizeof(int2), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&g->d_nbrs, ne * sizeof(int), 0);
@@ -502,6 +465,31 @@ mm_status create_common(int n, const int *ranges, long long nnz, const int *nbrs
     *out = g;
     return MM_OK;
 }
+
+}  // namespace
+
+mm_status adopt_arrays(int device, int n, long long nnz, int2 *ranges, int *nbrs, float *w, bool sym_struct, bool sym_w,
+                       mm_graph **out)
+{
+    mm_graph *g = new (std::nothrow) mm_graph();
+    if (!g) {
+        set_error("mm_graph_create: host allocation failed");
+        return MM_ERR_NOMEM;
+    }
+    g->device = device;
+    g->n = n;
+    g->nnz = nnz;
+    g->d_ranges = ranges;
+    g->d_nbrs = nbrs;
+    g->d_w = w;
+    g->has_weights = true;
+    g->sym_struct = sym_struct;
+    g->sym_weights = sym_struct && sym_w;
+    *out = g;
+    return MM_OK;
+}
+
+namespace {
 
 struct DeviceGuard {
     int prev = -1;

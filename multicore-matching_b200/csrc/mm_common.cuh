@@ -154,6 +154,62 @@ constexpr long long kSpinLimitDefault = 1ll << 22;
 long long debug_spin_limit();
 int debug_skip_mark();
 
+// Entries that neighbour and weight arrays are allocated for: a multiple of 4
+// plus 4, so that 16-byte vector loads starting at any in-range, 4-aligned slot
+// stay inside.
+inline size_t padded_entries(long long nnz) { return ((size_t)nnz + 3) / 4 * 4 + 4; }
+
+// A graph from device arrays of the pool, which it takes over: valid lists that
+// tile [0, nnz) in vertex order, strictly increasing, arrays padded with zeros.
+mm_status adopt_arrays(int device, int n, long long nnz, int2 *ranges, int *nbrs, float *w, bool sym_struct, bool sym_w,
+                       mm_graph **out);
+
+// Symmetry of a graph's entries: the multiset of entries (v, u) equals that of
+// (u, v), and with weights, of (v, u, w) and (u, v, w).  Each entry below the
+// diagonal adds a 64-bit hash of its ordered pair (and weight), each above takes
+// it away; a symmetric multiset leaves 0, another one only by a 64-bit
+// coincidence.  (splitmix64's finalizer; one hash a pair and one more for its
+// weight, where sums of both orders took five.)
+__device__ __forceinline__ unsigned long long mix64(unsigned long long z)
+{
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    return z ^ (z >> 31);
+}
+__device__ __forceinline__ void add_skew(unsigned v, unsigned u, unsigned wbits, bool weights, unsigned long long &skew_s,
+                                         unsigned long long &skew_w)
+{
+    if (v == u) return;
+    const unsigned lo = v < u ? v : u, hi = v < u ? u : v;
+    const unsigned long long h = mix64((((unsigned long long)lo << 32) | hi) + 0x9E3779B97F4A7C15ull);
+    skew_s += v < u ? h : 0ull - h;
+    if (weights) {
+        const unsigned long long x = mix64(h ^ ((unsigned long long)wbits * 0xD1B54A32D192ED03ull + 0x2545F4914F6CDD1Dull));
+        skew_w += v < u ? x : 0ull - x;
+    }
+}
+
+// Add the block's sum of v to *dst with one atomic (called by all threads of a
+// block of at most 1024, any number of times): atomics of all warps on one
+// word took longer than the passes that made them (k_pairs over 2^20 vertices:
+// 45 us with two a warp).
+__device__ __forceinline__ void block_add(unsigned long long *dst, unsigned long long v)
+{
+    __shared__ unsigned long long part[32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __syncthreads();  // part[] may still be read
+    if (lane == 0) part[warp] = v;
+    __syncthreads();
+    if (warp == 0) {
+        v = lane < (int)(blockDim.x + 31) / 32 ? part[lane] : 0ull;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0 && v) atomicAdd(dst, v);
+    }
+}
+
 // Ensure g->scratch holds at least `bytes`; returns MM_OK or an error.
 mm_status ensure_scratch(mm_graph *g, size_t bytes);
 

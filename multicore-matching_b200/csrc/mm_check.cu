@@ -7,6 +7,15 @@
 //   mm_matching_check   GraphMatching::testMatching (src/matchcpu.cu:127-246)
 // Both read the graph's device CSR and a device match array, and report
 // through their outputs; nothing is printed.
+//
+// A matching whose every value is held by exactly two vertices, one of them
+// the vertex that the value names, needs neither a sort nor a gather of match
+// values: k_pairs finds each vertex's partner (and whether the matching is of
+// that kind), and one pass over the lists looks for the partner's id, a group
+// of lanes per vertex.  That is every matching the matchers write; on RGG 2^20
+// weight and check together take 371 us by the general kernels (a thread a
+// vertex and its list, a radix sort of the values, three synchronisations).
+// Anything else takes the general kernels, which follow the reference's walk.
 #include <cuda_runtime.h>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_reduce.cuh>
@@ -21,12 +30,231 @@ namespace {
 
 __device__ __forceinline__ bool is_matched(int m) { return m >= 4; }  // matchcpu.h:41
 
+// ---- matchings made of clean pairs ----
+
+// Scratch of the pair passes, cleared before them.
+struct PairState {
+    unsigned long long nmin;       // vertices that their own value names
+    unsigned long long nother;     // vertices whose value names another
+    unsigned long long counts[5];  // as mm_matching_check's
+    unsigned long long size;       // as mm_matching_weight's
+    unsigned long long size_general;  // the same by the general kernel
+    double weight;
+    int broken;                    // a value that names no vertex, one that does not hold it, or one of two that do
+    int nlong;                     // lists left to the block scans
+};
+
+// other[a]: 1 + the partner of the vertex a that a value names (0: none).  The matching is
+// clean iff nothing is broken, nmin == nother and every other vertex is the
+// only one to claim its named vertex (which holds the value too).
+__global__ void k_pairs(const int *match, int n, int *other, PairState *st)
+{
+    int nmin = 0, nother = 0, broken = 0;
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
+        const int m = match[v];
+        if (!is_matched(m)) continue;
+        const long long a = (long long)m - 4;
+        if (a == v) {
+            ++nmin;
+        } else if (a >= n || match[a] != m) {
+            broken = 1;
+        } else {
+            other[a] = v + 1;  // the last of several stays; the others find that out (k_pair_lists)
+            ++nother;
+        }
+    }
+    block_add(&st->nmin, (unsigned long long)nmin);
+    block_add(&st->nother, (unsigned long long)nother);
+    if (__any_sync(0xffffffffu, broken) && (threadIdx.x & 31) == 0) atomicOr(&st->broken, 1);
+}
+
+__device__ __forceinline__ bool clean(const PairState *st) { return !st->broken && st->nmin == st->nother; }
+
+// Whether an entry naming u is what a pass looks for at vertex v:
+//   partner >= 0  the partner (kSelf: or the vertex itself, whose match value
+//                 is the same)
+//   partner < 0   (unmatched, the check only) an unmatched neighbour
+template <bool kSelf>
+__device__ __forceinline__ bool entry_hit(const int *match, int v, int partner, int u)
+{
+    if (partner >= 0) return u == partner || (kSelf && u == v);
+    return u != v && !is_matched(match[u]);
+}
+
+// What one vertex adds: kWeight the matched entry's weight and 1, else the
+// check's counts (cnt: invalid, matchable, unmatched).  A pair is invalid if
+// either list misses the other vertex: the first of the two to say so (bad[],
+// at the vertex that the value names) counts it.
+template <bool kWeight>
+__device__ __forceinline__ void pair_result(const float *w, int v, int partner, int at, double *contrib,
+                                            unsigned (&cnt)[3], int *bad)
+{
+    if (kWeight) {
+        contrib[v] = at >= 0 ? (double)w[at] : 0.0;
+        cnt[0] += at >= 0;
+    } else if (partner >= 0) {
+        if (at < 0 && atomicExch(bad + min(v, partner), 1) == 0) ++cnt[0];
+    } else {
+        ++cnt[2];
+        cnt[1] += at >= 0;
+    }
+}
+
+template <bool kWeight>
+__device__ __forceinline__ void add_counts(const unsigned (&cnt)[3], PairState *st)
+{
+    if (kWeight) {
+        if (cnt[0]) atomicAdd(&st->size, (unsigned long long)cnt[0]);
+    } else {
+        for (int k = 0; k < 3; ++k)
+            if (cnt[k]) atomicAdd(&st->counts[2 + k], (unsigned long long)cnt[k]);
+    }
+}
+
+// One pass over all vertices, a group of G lanes each, 4 G entries a step: the
+// pass waits on the chain vertex -> list -> entries, so what counts is how many
+// lists a warp has in flight (RGG 2^20: 8 with G = 4).  Longer lists than
+// kPairList are queued for a block each.
+constexpr int kPairList = 1024;
+
+template <int G, bool kWeight>
+__global__ void __launch_bounds__(256) k_pair_lists(const int2 *ranges, const int *nbrs, const float *w, const int *match,
+                                                    int n, const int *other, int *bad, int *queue, double *contrib,
+                                                    PairState *st)
+{
+    if (!clean(st)) return;
+    constexpr int kPerWarp = 32 / G;
+    const int lane = threadIdx.x & 31, l = lane & (G - 1), shift = lane & ~(G - 1);
+    const unsigned gmask = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long stride = ((long long)gridDim.x * blockDim.x >> 5) * kPerWarp;
+    unsigned cnt[3] = {0u, 0u, 0u};
+    bool broken = false;
+    // the next vertex's match value, range and partner are loaded while this one's list is read
+    int vn = -1, mn = 0, on = -1;
+    int2 rn = make_int2(0, 0);
+    auto fetch = [&](long long base) {
+        const long long v0 = base + lane / G;
+        vn = base < n && v0 < n ? (int)v0 : -1;
+        if (vn >= 0) {
+            mn = match[vn];
+            rn = ranges[vn];
+            on = other[vn];
+        }
+    };
+    fetch(warp * kPerWarp);
+    for (long long base = warp * kPerWarp; base < n; base += stride) {  // warp-uniform
+        const int v = vn, mv = v >= 0 ? mn : 0, ov = on;
+        const int2 r = v >= 0 ? rn : make_int2(0, 0);
+        fetch(base + stride);
+        const bool matched = is_matched(mv);
+        const int a = mv - 4, partner = !matched ? -1 : (a == v ? ov - 1 : a);
+        if (matched && a != v && l == 0) broken |= other[a] != v + 1;
+        bool want = v >= 0 && (!kWeight || matched);
+        if (kWeight && v >= 0 && !matched && l == 0) contrib[v] = 0.0;
+        if (want && r.y > r.x && r.y - r.x > kPairList) {
+            if (l == 0) queue[atomicAdd(&st->nlong, 1)] = v;
+            want = false;
+        }
+        int at = -1;
+        bool go = want && r.x < r.y;
+        for (int j = r.x; __any_sync(0xffffffffu, go); j += 4 * G) {
+            int u[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) u[k] = go && j + k * G + l < r.y ? __ldg(nbrs + j + k * G + l) : -1;
+            bool hit[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) hit[k] = u[k] >= 0 && entry_hit<kWeight>(match, v, partner, u[k]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const unsigned bits = (__ballot_sync(0xffffffffu, hit[k]) >> shift) & gmask;
+                if (go && bits) {
+                    at = j + k * G + __ffs(bits) - 1;
+                    go = false;
+                }
+            }
+            go = go && j + 4 * G < r.y;
+        }
+        if (want && l == 0) pair_result<kWeight>(w, v, partner, at, contrib, cnt, bad);
+    }
+    if (__any_sync(0xffffffffu, broken) && lane == 0) atomicOr(&st->broken, 1);
+    if (kWeight) {
+        block_add(&st->size, cnt[0]);
+    } else {
+        for (int k = 0; k < 3; ++k) block_add(&st->counts[2 + k], cnt[k]);
+    }
+}
+
+// The queued long lists, a block each (the lowest hit of a step is the first).
+template <bool kWeight>
+__global__ void __launch_bounds__(256) k_pair_long(const int2 *ranges, const int *nbrs, const float *w, const int *match,
+                                                   const int *other, int *bad, const int *queue, double *contrib,
+                                                   PairState *st)
+{
+    if (!clean(st)) return;
+    __shared__ int s_at;
+    const int nlong = st->nlong;
+    for (int i = blockIdx.x; i < nlong; i += gridDim.x) {
+        const int v = queue[i], mv = match[v];
+        const int a = mv - 4, partner = !is_matched(mv) ? -1 : (a == v ? other[v] - 1 : a);
+        const int2 r = ranges[v];
+        if (threadIdx.x == 0) s_at = 0x7fffffff;
+        __syncthreads();
+        for (int j = r.x; j < r.y; j += 4 * 256) {
+            int first = 0x7fffffff;
+#pragma unroll
+            for (int k = 3; k >= 0; --k) {
+                const int q = j + k * 256 + (int)threadIdx.x;
+                if (q < r.y && entry_hit<kWeight>(match, v, partner, __ldg(nbrs + q))) first = q;
+            }
+            if (first != 0x7fffffff) atomicMin(&s_at, first);
+            __syncthreads();
+            const bool done = s_at != 0x7fffffff;
+            __syncthreads();
+            if (done) break;
+        }
+        if (threadIdx.x == 0) {
+            unsigned cnt[3] = {0u, 0u, 0u};
+            pair_result<kWeight>(w, v, partner, s_at == 0x7fffffff ? -1 : s_at, contrib, cnt, bad);
+            add_counts<kWeight>(cnt, st);
+        }
+        __syncthreads();
+    }
+}
+
+// Host side: the pair passes of one call.  st is followed by other[n], bad[n]
+// (the check only) and queue[n]; all but the queue is cleared at once.
+size_t pair_bytes(int n) { return 128 + sizeof(int) * 3 * (size_t)n; }
+static_assert(sizeof(PairState) <= 128, "the arrays follow it");
+
+template <bool kWeight>
+cudaError_t launch_pairs(const mm_graph *g, const int *d_match, double *contrib, PairState *st, cudaStream_t s)
+{
+    const int n = g->n;
+    int *other = reinterpret_cast<int *>(reinterpret_cast<char *>(st) + 128), *bad = other + n, *queue = bad + n;
+    const cudaError_t e = cudaMemsetAsync(st, 0, 128 + sizeof(int) * (kWeight ? 1 : 2) * (size_t)n, s);
+    if (e != cudaSuccess) return e;
+    k_pairs<<<grid_for(n, 256, 148 * 8), 256, 0, s>>>(d_match, n, other, st);
+    const long long per = n > 0 ? g->nnz / n : 0;
+    auto run = [&](auto kernel, int lanes) {
+        kernel<<<grid_for((long long)n * lanes, 256, 148 * 8), 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, n, other,
+                                                                           bad, queue, contrib, st);
+    };
+    if (per <= 20) run(k_pair_lists<4, kWeight>, 4);
+    else if (per <= 80) run(k_pair_lists<8, kWeight>, 8);
+    else run(k_pair_lists<32, kWeight>, 32);
+    if (g->nnz > kPairList && !(g->scanned && g->max_degree <= kPairList))
+        k_pair_long<kWeight><<<148 * 4, 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, other, bad, queue, contrib, st);
+    return cudaGetLastError();
+}
+
 // getWeight: a matched vertex i adds the weight of the first entry of its list
 // whose neighbour carries the same match value, and counts 1.  contrib[i]
 // holds that weight (0 otherwise); size is counted alongside.
 __global__ void k_weight(const int2 *ranges, const int *nbrs, const float *w, const int *match, int n,
-                         double *contrib, unsigned long long *size)
+                         double *contrib, PairState *st)
 {
+    if (clean(st)) return;
     unsigned long long cnt = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int m = match[i];
@@ -44,7 +272,7 @@ __global__ void k_weight(const int2 *ranges, const int *nbrs, const float *w, co
         contrib[i] = x;
     }
     for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(size, cnt);
+    if ((threadIdx.x & 31) == 0 && cnt) atomicAdd(&st->size_general, cnt);
 }
 
 // Sort keys for testMatching's order: unmatched vertices first, then by match
@@ -208,34 +436,30 @@ MM_API mm_status mm_matching_weight(mm_graph *g, const int *d_match, double *wei
     DeviceScope scope(g->device);
     cudaStream_t st = (cudaStream_t)stream;
     const int n = g->n;
-    double *contrib = nullptr, *sum = nullptr;
-    unsigned long long *cnt = nullptr;
+    double *contrib = nullptr;
+    PairState *ps = nullptr;
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
     cudaError_t e = dev_alloc((void **)&contrib, sizeof(double) * (size_t)n, st);
-    if (e == cudaSuccess) e = dev_alloc((void **)&sum, sizeof(double), st);
-    if (e == cudaSuccess) e = dev_alloc((void **)&cnt, sizeof(unsigned long long), st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), st);
+    if (e == cudaSuccess) e = dev_alloc((void **)&ps, pair_bytes(n), st);
+    if (e == cudaSuccess) e = launch_pairs<true>(g, d_match, contrib, ps, st);
     if (e == cudaSuccess) {
-        k_weight<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, n, contrib, cnt);
+        k_weight<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, n, contrib, ps);
         e = cudaGetLastError();
     }
     // a fixed reduction tree: the same sum on every run
-    if (e == cudaSuccess) e = cub::DeviceReduce::Sum(nullptr, tmp_bytes, contrib, sum, n, st);
+    if (e == cudaSuccess) e = cub::DeviceReduce::Sum(nullptr, tmp_bytes, contrib, &ps->weight, n, st);
     if (e == cudaSuccess) e = dev_alloc(&tmp, tmp_bytes, st);
-    if (e == cudaSuccess) e = cub::DeviceReduce::Sum(tmp, tmp_bytes, contrib, sum, n, st);
-    double total = 0.0;
-    unsigned long long count = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&total, sum, sizeof total, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&count, cnt, sizeof count, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cub::DeviceReduce::Sum(tmp, tmp_bytes, contrib, &ps->weight, n, st);
+    PairState h = {};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, ps, sizeof h, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     dev_free(tmp, st);
     dev_free(contrib, st);
-    dev_free(sum, st);
-    dev_free(cnt, st);
+    dev_free(ps, st);
     if (e != cudaSuccess) return cuda_fail(e, "mm_matching_weight");
-    *weight = total / 2.0;  // every matched edge is counted from both ends
-    *size = (long long)count;
+    *weight = h.weight / 2.0;  // every matched edge is counted from both ends
+    *size = (long long)(!h.broken && h.nmin == h.nother ? h.size : h.size_general);
     return MM_OK;
 }
 
@@ -251,12 +475,29 @@ MM_API mm_status mm_matching_check(mm_graph *g, const int *d_match, long long *c
     DeviceScope scope(g->device);
     cudaStream_t st = (cudaStream_t)stream;
     const int n = g->n;
+    cudaError_t e = cudaSuccess;
+    {
+        PairState *ps = nullptr;
+        e = dev_alloc((void **)&ps, pair_bytes(n), st);
+        if (e == cudaSuccess) e = launch_pairs<false>(g, d_match, nullptr, ps, st);
+        PairState h = {};
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&h, ps, sizeof h, cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        dev_free(ps, st);
+        if (e != cudaSuccess) return cuda_fail(e, "mm_matching_check");
+        if (!h.broken && h.nmin == h.nother) {
+            for (int k = 2; k < 5; ++k) counts[k] = (long long)h.counts[k];
+            *valid = counts[2] == 0 ? 1 : 0;
+            return MM_OK;
+        }
+    }
+    // the reference's walk
     unsigned *k0 = nullptr, *k1 = nullptr;
     int *v0 = nullptr, *v1 = nullptr;
     unsigned long long *c = nullptr;
     void *tmp = nullptr;
     size_t tmp_bytes = 0;
-    cudaError_t e = dev_alloc((void **)&k0, sizeof(unsigned) * (size_t)n, st);
+    e = dev_alloc((void **)&k0, sizeof(unsigned) * (size_t)n, st);
     if (e == cudaSuccess) e = dev_alloc((void **)&k1, sizeof(unsigned) * (size_t)n, st);
     if (e == cudaSuccess) e = dev_alloc((void **)&v0, sizeof(int) * (size_t)n, st);
     if (e == cudaSuccess) e = dev_alloc((void **)&v1, sizeof(int) * (size_t)n, st);

@@ -309,6 +309,7 @@ void free_graph(mm_graph *g)
     dev_free(g->d_goff, 0);
     dev_free(g->d_vbase, 0);
     dev_free(g->d_last, 0);
+    dev_free(g->d_glast, 0);
     cudaStreamSynchronize(0);
     if (prev >= 0) cudaSetDevice(prev);
     delete g;
@@ -785,13 +786,14 @@ MM_API mm_status mm_graph_set_batch(mm_graph *g, int ngraphs, const int *offsets
             return MM_ERR_ARG;
         }
     DeviceGuard guard(g->device);
-    int *goff = nullptr, *vbase = nullptr, *vend = nullptr, *bad = nullptr;
+    int *goff = nullptr, *vbase = nullptr, *vend = nullptr, *bad = nullptr, *glast = nullptr;
     uint8_t *last = nullptr;
     const size_t nv = (size_t)(g->n > 0 ? g->n : 1);
     cudaError_t e = dev_alloc((void **)&goff, sizeof(int) * ((size_t)ngraphs + 1), 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&vbase, sizeof(int) * nv, 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&vend, sizeof(int) * nv, 0);  // for the check only
     if (e == cudaSuccess) e = dev_alloc((void **)&last, nv, 0);
+    if (e == cudaSuccess) e = dev_alloc((void **)&glast, sizeof(int) * (size_t)ngraphs, 0);
     if (e == cudaSuccess) e = dev_alloc((void **)&bad, sizeof(int), 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(bad, 0, sizeof(int), 0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(goff, offsets, sizeof(int) * ((size_t)ngraphs + 1), cudaMemcpyHostToDevice, 0);
@@ -810,6 +812,7 @@ MM_API mm_status mm_graph_set_batch(mm_graph *g, int ngraphs, const int *offsets
         dev_free(goff, 0);
         dev_free(vbase, 0);
         dev_free(last, 0);
+        dev_free(glast, 0);
         cudaStreamSynchronize(0);
         if (e != cudaSuccess) return cuda_fail(e, "mm_graph_set_batch");
         set_error("mm_graph_set_batch: an edge joins two graphs of the batch");
@@ -818,6 +821,8 @@ MM_API mm_status mm_graph_set_batch(mm_graph *g, int ngraphs, const int *offsets
     dev_free(g->d_goff, 0);
     dev_free(g->d_vbase, 0);
     dev_free(g->d_last, 0);
+    dev_free(g->d_glast, 0);
+    g->d_glast = glast;
     g->d_goff = goff;
     g->d_vbase = vbase;
     g->d_last = last;

@@ -124,6 +124,7 @@ struct mm_graph {
     int *d_goff = nullptr;
     int *d_vbase = nullptr;
     uint8_t *d_last = nullptr;
+    int *d_glast = nullptr;  // last active round of each graph
 };
 
 namespace mm {

@@ -132,6 +132,8 @@ void pinned_put(void *p, size_t bytes)
     g_pinned_free.push_back(PinnedBlock{p, (bytes + 4095) / 4096 * 4096});
 }
 
+static void lanes_release_cached(int device);
+
 mm_status release_cached(int device)
 {
     cudaMemPool_t pool = nullptr;
@@ -144,6 +146,7 @@ mm_status release_cached(int device)
     cudaGetDevice(&prev);
     MM_CUDA_TRY(cudaSetDevice(device), "set device");
     cudaError_t e = cudaDeviceSynchronize();
+    lanes_release_cached(device);
     if (e == cudaSuccess) e = cudaMemPoolTrimTo(pool, 0);
     if (prev >= 0) cudaSetDevice(prev);
     if (e != cudaSuccess) return cuda_fail(e, "release cached memory");
@@ -175,27 +178,11 @@ namespace {
 //                with weights, of (v, u, w) and (u, v, w).
 // (add_skew in mm_common.cuh).
 struct GraphCheck {
+    RangeInfo r;
     unsigned long long skew_s, skew_w;  // 0: symmetric in structure, with weights
-    int bad;        // 1: a range outside [0, nnz); 2: an id outside [0, n)
-    int noncontig;  // ranges do not tile [0, nnz) in vertex order
+    int bad;        // 2: an id outside [0, n)
     int unsorted;   // some list is not strictly increasing
-    int pad;
 };
-
-__global__ void k_check_ranges(const int2 *ranges, int n, long long nnz, GraphCheck *c)
-{
-    int bad = 0, nc = 0;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const int2 r = ranges[v];
-        if (r.y > r.x && (r.x < 0 || (long long)r.y > nnz)) bad = 1;
-        if (r.y < r.x) nc = 1;
-        if (v == 0 && r.x != 0) nc = 1;
-        if (v + 1 < n && ranges[v + 1].x != r.y) nc = 1;
-        if (v == n - 1 && (long long)r.y != nnz) nc = 1;
-    }
-    if (__any_sync(0xffffffffu, bad) && (threadIdx.x & 31) == 0) atomicOr(&c->bad, 1);
-    if (__any_sync(0xffffffffu, nc) && (threadIdx.x & 31) == 0) atomicOr(&c->noncontig, 1);
-}
 
 // Contiguous CSR: slots [j0, j1) in chunks of kChk, a block per chunk; the
 // owner of each slot comes from a table of the chunk's list starts.
@@ -216,6 +203,7 @@ template <bool kWeights>
 __global__ void __launch_bounds__(256) k_check_entries(const int2 *ranges, const int *nbrs, const float *w, int n,
                                                        long long j0, long long j1, GraphCheck *c)
 {
+    if (c->r.noncontig || c->r.bad) return;  // (the small upload launches both checks)
     __shared__ int start[kChk + 1];
     __shared__ int s_v0, s_cnt;
     unsigned long long ss = 0, sw = 0;
@@ -271,6 +259,7 @@ __global__ void __launch_bounds__(256) k_check_entries(const int2 *ranges, const
 // Any CSR: bounds of every id, a warp per list.
 __global__ void k_validate(const int2 *ranges, const int *nbrs, int n, long long nnz, GraphCheck *c)
 {
+    if (!c->r.noncontig || c->r.bad) return;
     const int lane = threadIdx.x & 31;
     const long long warp0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -315,59 +304,178 @@ void free_graph(mm_graph *g)
     delete g;
 }
 
-// Graph upload and validation.  The ranges go first and are checked; for a
-// contiguous CSR the neighbour ids and weights then follow in chunks on a copy
-// stream while a second stream checks each chunk that has arrived, so the
-// checks hide under the transfer.
-constexpr long long kUploadChunk = 1ll << 24;  // entries per chunk
+// Graph upload and validation.
+//
+// A large graph from host memory: the ranges go first, the entries follow in
+// chunks on the same copy stream, two chunks ahead of the second stream, which
+// checks the ranges and then each chunk as it arrives and builds its preference
+// windows.  So the copies run back to back, and what is left to do when the
+// last one ends is the last chunk (1/24 of the entries; with chunks of 2^24
+// entries an R-MAT 2^20 graph's was half of it).  A small one, or one that is on
+// the device already: copies and checks in order on the legacy stream, one
+// synchronisation; its windows are built when a weighted type asks for them.
+constexpr long long kSmallUpload = 1ll << 19;  // entries
+constexpr int kUploadChunks = 24;
+constexpr int kAhead = 2;
 
-mm_status upload_and_check(mm_graph *g, const int *ranges, const int *nbrs, const float *w,
-                           cudaMemcpyKind kind)
+// Two streams and the chunks' events, kept for the next upload (at most
+// kLanesKept of them; mm_release_cached_memory gives them back).
+struct Lanes {
+    int device = -1;
+    cudaStream_t copy = nullptr, check = nullptr;
+    cudaEvent_t ev[kUploadChunks + 1] = {};
+};
+constexpr size_t kLanesKept = 4;
+std::mutex g_lanes_mu;
+std::vector<Lanes *> g_lanes;
+
+void lanes_free(Lanes *l)
+{
+    for (cudaEvent_t ev : l->ev)
+        if (ev) cudaEventDestroy(ev);
+    if (l->copy) cudaStreamDestroy(l->copy);
+    if (l->check) cudaStreamDestroy(l->check);
+    delete l;
+}
+
+cudaError_t lanes_get(int device, Lanes **out)
+{
+    {
+        std::lock_guard<std::mutex> lock(g_lanes_mu);
+        for (size_t i = 0; i < g_lanes.size(); ++i)
+            if (g_lanes[i]->device == device) {
+                *out = g_lanes[i];
+                g_lanes.erase(g_lanes.begin() + (long)i);
+                return cudaSuccess;
+            }
+    }
+    Lanes *l = new (std::nothrow) Lanes();
+    if (!l) return cudaErrorMemoryAllocation;
+    l->device = device;
+    cudaError_t e = cudaStreamCreateWithFlags(&l->copy, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&l->check, cudaStreamNonBlocking);
+    for (cudaEvent_t &ev : l->ev)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    if (e != cudaSuccess) {
+        lanes_free(l);
+        return e;
+    }
+    *out = l;
+    return cudaSuccess;
+}
+
+// (both streams are idle)
+void lanes_put(Lanes *l)
+{
+    {
+        std::lock_guard<std::mutex> lock(g_lanes_mu);
+        if (g_lanes.size() < kLanesKept) {
+            g_lanes.push_back(l);
+            return;
+        }
+    }
+    lanes_free(l);
+}
+
+void lanes_release(int device)
+{
+    std::vector<Lanes *> mine;
+    {
+        std::lock_guard<std::mutex> lock(g_lanes_mu);
+        for (size_t i = 0; i < g_lanes.size();)
+            if (g_lanes[i]->device == device) {
+                mine.push_back(g_lanes[i]);
+                g_lanes.erase(g_lanes.begin() + (long)i);
+            } else {
+                ++i;
+            }
+    }
+    for (Lanes *l : mine) lanes_free(l);
+}
+
+cudaError_t check_entries(const mm_graph *g, bool have_w, long long j0, long long j1, GraphCheck *c, cudaStream_t s)
+{
+    const int grid = grid_for(j1 - j0, kChk, 148 * 8);
+    if (have_w) k_check_entries<true><<<grid, 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, g->n, j0, j1, c);
+    else k_check_entries<false><<<grid, 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, g->n, j0, j1, c);
+    return cudaGetLastError();
+}
+
+cudaError_t check_any(const mm_graph *g, GraphCheck *c, cudaStream_t s)
+{
+    k_validate<<<grid_for((long long)g->n * 32, 256, 148 * 16), 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->n, g->nnz, c);
+    return cudaGetLastError();
+}
+
+cudaError_t fill_unit(mm_graph *g, cudaStream_t s)
+{
+    const size_t m = (size_t)(g->nnz > 0 ? g->nnz : 1);
+    k_fill_one<<<grid_for((long long)m, 256, 148 * 8), 256, 0, s>>>(g->d_w, (long long)m);
+    return cudaGetLastError();
+}
+
+cudaError_t upload_small(mm_graph *g, const int *ranges, const int *nbrs, const float *w, cudaMemcpyKind kind,
+                         GraphCheck *d_c, GraphCheck *c)
 {
     const int n = g->n;
     const long long nnz = g->nnz;
-    GraphCheck *d_c = nullptr;
-    MM_CUDA_TRY(dev_alloc((void **)&d_c, sizeof(GraphCheck), 0), "validation state");
-    cudaError_t e = cudaMemsetAsync(d_c, 0, sizeof(GraphCheck), 0);
-    if (e == cudaSuccess && n > 0) e = cudaMemcpyAsync(g->d_ranges, ranges, (size_t)n * sizeof(int2), kind, 0);
-    if (e == cudaSuccess && n > 0) {
-        k_check_ranges<<<grid_for(n, 256, 148 * 8), 256>>>(g->d_ranges, n, nnz, d_c);
-        e = cudaGetLastError();
-    }
-    GraphCheck c = {};
-    if (e == cudaSuccess) e = cudaMemcpy(&c, d_c, sizeof c, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess && (c.bad & 1)) {
-        dev_free(d_c, 0);
-        set_error("mm_graph_create: a neighbour range lies outside [0, nnz)");
-        return MM_ERR_GRAPH;
-    }
-    const bool contiguous = n > 0 && !c.noncontig;
-    const bool have_w = w != nullptr;
-    // Weighted graphs from host memory also get their preference windows here:
-    // a chunk's check is followed by the windows of the vertices whose lists
-    // end in it (host ranges say which), so they too hide under the transfer.
-    bool windows = e == cudaSuccess && contiguous && nnz > 0 && have_w && kind == cudaMemcpyHostToDevice;
-    if (windows && windows_begin(g, 0) != MM_OK) windows = false;
-    if (e == cudaSuccess && contiguous && nnz > 0) {
-        cudaStream_t cs = nullptr, ks = nullptr;
-        cudaEvent_t ev = nullptr;
-        e = cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ks, cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+    cudaError_t e = cudaSuccess;
+    if (n > 0) e = cudaMemcpyAsync(g->d_ranges, ranges, (size_t)n * sizeof(int2), kind, 0);
+    if (e == cudaSuccess && nnz > 0) e = cudaMemcpyAsync(g->d_nbrs, nbrs, (size_t)nnz * sizeof(int), kind, 0);
+    if (e == cudaSuccess && nnz > 0 && w) e = cudaMemcpyAsync(g->d_w, w, (size_t)nnz * sizeof(float), kind, 0);
+    if (e == cudaSuccess && n > 0) e = scan_ranges(g->d_ranges, n, nnz, &d_c->r, nullptr, 0);
+    if (e == cudaSuccess && n > 0 && nnz > 0) e = check_entries(g, w != nullptr, 0, nnz, d_c, 0);
+    if (e == cudaSuccess && n > 0) e = check_any(g, d_c, 0);
+    if (e == cudaSuccess && !w) e = fill_unit(g, 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c, d_c, sizeof *c, cudaMemcpyDeviceToHost, 0);
+    const cudaError_t s = cudaStreamSynchronize(0);
+    return e == cudaSuccess ? s : e;
+}
+
+cudaError_t upload_large(mm_graph *g, const int *ranges, const int *nbrs, const float *w, GraphCheck *d_c, GraphCheck *c)
+{
+    const int n = g->n;
+    const long long nnz = g->nnz;
+    const cudaMemcpyKind kind = cudaMemcpyHostToDevice;
+    Lanes *l = nullptr;
+    cudaError_t e = lanes_get(g->device, &l);
+    if (e != cudaSuccess) return e;
+    const cudaStream_t cs = l->copy, ks = l->check;
+    // (the pool's allocations and the clears on the legacy stream are done: create_common)
+    const long long chunk = ((nnz + kUploadChunks - 1) / kUploadChunks + 65535) / 65536 * 65536;
+    const int nchunks = (int)((nnz + chunk - 1) / chunk);
+    auto copy_chunk = [&](int k) {
+        const long long j0 = k * chunk, j1 = j0 + chunk < nnz ? j0 + chunk : nnz;
+        cudaError_t x = cudaMemcpyAsync(g->d_nbrs + j0, nbrs + j0, (size_t)(j1 - j0) * sizeof(int), kind, cs);
+        if (x == cudaSuccess && w) x = cudaMemcpyAsync(g->d_w + j0, w + j0, (size_t)(j1 - j0) * sizeof(float), kind, cs);
+        if (x == cudaSuccess) x = cudaEventRecord(l->ev[k + 1], cs);
+        return x;
+    };
+    if (n > 0) e = cudaMemcpyAsync(g->d_ranges, ranges, (size_t)n * sizeof(int2), kind, cs);
+    if (e == cudaSuccess) e = cudaEventRecord(l->ev[0], cs);
+    int copied = 0;
+    for (; e == cudaSuccess && copied < nchunks && copied < kAhead; ++copied) e = copy_chunk(copied);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(ks, l->ev[0], 0);
+    if (e == cudaSuccess && n > 0) e = scan_ranges(g->d_ranges, n, nnz, &d_c->r, nullptr, ks);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(c, d_c, sizeof *c, cudaMemcpyDeviceToHost, ks);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ks);
+    if (e == cudaSuccess && !c->r.bad) {
+        apply_ranges(g, c->r);
+        const bool contiguous = n > 0 && g->contiguous;
+        // Weighted graphs get their preference windows here: a chunk's check is
+        // followed by the windows of the vertices whose lists end in it (host
+        // ranges say which).
+        bool windows = contiguous && w && windows_begin(g, ks) == MM_OK;
         int va = 0;  // first vertex whose window is not built yet
-        for (long long j0 = 0; e == cudaSuccess && j0 < nnz; j0 += kUploadChunk) {
-            const long long j1 = j0 + kUploadChunk < nnz ? j0 + kUploadChunk : nnz;
-            const size_t cnt = (size_t)(j1 - j0);
-            e = cudaMemcpyAsync(g->d_nbrs + j0, nbrs + j0, cnt * sizeof(int), kind, cs);
-            if (e == cudaSuccess && have_w) e = cudaMemcpyAsync(g->d_w + j0, w + j0, cnt * sizeof(float), kind, cs);
-            if (e == cudaSuccess) e = cudaEventRecord(ev, cs);
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(ks, ev, 0);
-            if (e == cudaSuccess) {
-                const int grid = grid_for((long long)cnt, kChk, 148 * 8);
-                if (have_w) k_check_entries<true><<<grid, 256, 0, ks>>>(g->d_ranges, g->d_nbrs, g->d_w, n, j0, j1, d_c);
-                else k_check_entries<false><<<grid, 256, 0, ks>>>(g->d_ranges, g->d_nbrs, g->d_w, n, j0, j1, d_c);
-                e = cudaGetLastError();
+        for (int k = 0; e == cudaSuccess && k < nchunks; ++k) {
+            if (copied < nchunks) {
+                e = copy_chunk(copied);
+                ++copied;
             }
+            if (!contiguous || e != cudaSuccess) continue;
+            const long long j0 = k * chunk, j1 = j0 + chunk < nnz ? j0 + chunk : nnz;
+            e = cudaStreamWaitEvent(ks, l->ev[k + 1], 0);
+            if (e == cudaSuccess) e = check_entries(g, w != nullptr, j0, j1, d_c, ks);
             if (e == cudaSuccess && windows) {
                 // vertices whose lists end at or before j1 (ends rise with v)
                 int lo = va, hi = n;
@@ -382,39 +490,51 @@ mm_status upload_and_check(mm_graph *g, const int *ranges, const int *nbrs, cons
             }
         }
         if (e == cudaSuccess && windows && windows_end(g, ks) != MM_OK) windows = false;
-        // both streams are drained on every path: buffers may be freed next
-        const cudaError_t eks = ks ? cudaStreamSynchronize(ks) : cudaSuccess;
-        const cudaError_t ecs = cs ? cudaStreamSynchronize(cs) : cudaSuccess;
-        if (e == cudaSuccess) e = eks != cudaSuccess ? eks : ecs;
-        if (ev) cudaEventDestroy(ev);
-        if (cs) cudaStreamDestroy(cs);
-        if (ks) cudaStreamDestroy(ks);
-    } else if (e == cudaSuccess) {
-        if (nnz > 0) e = cudaMemcpy(g->d_nbrs, nbrs, (size_t)nnz * sizeof(int), kind);
-        if (e == cudaSuccess && nnz > 0 && have_w) e = cudaMemcpy(g->d_w, w, (size_t)nnz * sizeof(float), kind);
-        if (e == cudaSuccess && n > 0) {
-            k_validate<<<grid_for((long long)n * 32, 256, 148 * 16), 256>>>(g->d_ranges, g->d_nbrs, n, nnz, d_c);
-            e = cudaGetLastError();
+        if (e == cudaSuccess && !contiguous && n > 0) {
+            e = cudaStreamWaitEvent(ks, l->ev[nchunks], 0);
+            if (e == cudaSuccess) e = check_any(g, d_c, ks);
+        }
+        if (e == cudaSuccess && !w) {
+            e = cudaStreamWaitEvent(ks, l->ev[nchunks], 0);
+            if (e == cudaSuccess) e = fill_unit(g, ks);
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(c, d_c, sizeof *c, cudaMemcpyDeviceToHost, ks);
+        if (!windows) {
+            cudaStreamSynchronize(ks);
+            windows_discard(g);  // built later, on demand, if the upload could not
         }
     }
-    if (e == cudaSuccess && !have_w) {
-        const size_t m = (size_t)(nnz > 0 ? nnz : 1);
-        k_fill_one<<<grid_for((long long)m, 256, 148 * 8), 256>>>(g->d_w, (long long)m);
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cudaMemcpy(&c, d_c, sizeof c, cudaMemcpyDeviceToHost);
-    dev_free(d_c, 0);
-    if (!windows) windows_discard(g);  // built later, on demand, if the upload could not
+    // both streams are drained on every path: buffers may be freed next
+    const cudaError_t eks = cudaStreamSynchronize(ks), ecs = cudaStreamSynchronize(cs);
+    if (e == cudaSuccess) e = eks != cudaSuccess ? eks : ecs;
+    lanes_put(l);
+    return e;
+}
+
+mm_status upload_and_check(mm_graph *g, const int *ranges, const int *nbrs, const float *w, cudaMemcpyKind kind,
+                           GraphCheck *d_c)
+{
+    GraphCheck c = {};
+    const cudaError_t e = kind == cudaMemcpyHostToDevice && g->nnz > kSmallUpload
+                              ? upload_large(g, ranges, nbrs, w, d_c, &c)
+                              : upload_small(g, ranges, nbrs, w, kind, d_c, &c);
     cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(e, "graph upload and validation");
+    if (c.r.bad) {
+        set_error("mm_graph_create: a neighbour range lies outside [0, nnz)");
+        return MM_ERR_GRAPH;
+    }
     if (c.bad & 2) {
         set_error("mm_graph_create: a neighbour id lies outside [0, n)");
         return MM_ERR_GRAPH;
     }
-    g->has_weights = have_w;
+    apply_ranges(g, c.r);
+    const bool contiguous = g->n > 0 && g->contiguous;
+    g->scanned = contiguous;
+    g->has_weights = w != nullptr;
     g->sym_struct = contiguous && !c.unsorted && c.skew_s == 0;
     // unit weights are symmetric whenever the structure is
-    g->sym_weights = g->sym_struct && (!have_w || c.skew_w == 0);
+    g->sym_weights = g->sym_struct && (!w || c.skew_w == 0);
     return MM_OK;
 }
 
@@ -452,11 +572,15 @@ mm_status create_common(int n, const int *ranges, long long nnz, const int *nbrs
     if (e == cudaSuccess) e = dev_alloc((void **)&g->d_w, ne * sizeof(float), 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(g->d_nbrs + nnz, 0, (ne - (size_t)nnz) * sizeof(int), 0);
     if (e == cudaSuccess) e = cudaMemsetAsync(g->d_w + nnz, 0, (ne - (size_t)nnz) * sizeof(float), 0);
+    GraphCheck *d_c = nullptr;
+    if (e == cudaSuccess) e = dev_alloc((void **)&d_c, sizeof(GraphCheck), 0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(d_c, 0, sizeof(GraphCheck), 0);
     // the non-blocking upload streams do not wait for the legacy stream: settle the pool first
-    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+    if (e == cudaSuccess && kind == cudaMemcpyHostToDevice && nnz > kSmallUpload) e = cudaStreamSynchronize(0);
     mm_status s = MM_OK;
     if (e != cudaSuccess) s = cuda_fail(e, "graph allocation");
-    if (s == MM_OK) s = upload_and_check(g, ranges, nbrs, w, kind);
+    if (s == MM_OK) s = upload_and_check(g, ranges, nbrs, w, kind, d_c);
+    dev_free(d_c, 0);
     if (s != MM_OK) {
         free_graph(g);
         if (prev >= 0) cudaSetDevice(prev);
@@ -468,6 +592,8 @@ mm_status create_common(int n, const int *ranges, long long nnz, const int *nbrs
 }
 
 }  // namespace
+
+static void lanes_release_cached(int device) { lanes_release(device); }
 
 mm_status adopt_arrays(int device, int n, long long nnz, int2 *ranges, int *nbrs, float *w, bool sym_struct, bool sym_w,
                        mm_graph **out)
@@ -636,7 +762,10 @@ MM_API mm_status mm_graph_prepare(mm_graph *g, int type)
         return MM_ERR_ARG;
     }
     DeviceGuard guard(g->device);
-    return push_prepare(g, is_weighted(type) ? 1 : 0, 0);
+    const mm_status s = push_prepare(g, is_weighted(type) ? 1 : 0, 0);
+    // a matching may come on a stream that does not wait for the legacy one
+    if (s == MM_OK) MM_CUDA_TRY(cudaStreamSynchronize(0), "mm_graph_prepare");
+    return s;
 }
 
 MM_API void mm_graph_destroy(mm_graph *g) { free_graph(g); }
@@ -705,8 +834,7 @@ MM_API mm_status mm_match(mm_graph *g, int type, uint32_t barrier, const uint32_
     DeviceGuard guard(g->device);
     cudaStream_t st = (cudaStream_t)stream;
     if (!g->d_out) {
-        MM_CUDA_TRY(dev_alloc((void **)&g->d_out, (size_t)(g->n > 0 ? g->n : 1) * sizeof(int), 0), "match buffer");
-        MM_CUDA_TRY(cudaStreamSynchronize(0), "match buffer");
+        MM_CUDA_TRY(dev_alloc((void **)&g->d_out, (size_t)(g->n > 0 ? g->n : 1) * sizeof(int), st), "match buffer");
     }
     s = push_match(g, type, barrier, seeds, nseeds, g->d_out, rounds_out, nullptr, 0, st);
     if (s == MM_OK && g->n > 0) {

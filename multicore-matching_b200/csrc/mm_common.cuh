@@ -94,6 +94,8 @@ struct mm_graph {
     long long short_count = 0;     // vertices with at most 32 neighbour entries
     long long long_count = 0;      // vertices with more
     long long long_entries = 0;    // entries in those longer lists
+    long long win_groups = 0;      // groups of 4 entries of all preference windows
+    long long win_even = 0;        // windows' lengths rounded up to even numbers, in all
 
     // device buffer for host-output calls (mm_match)
     int *d_out = nullptr;
@@ -210,6 +212,21 @@ __device__ __forceinline__ void block_add(unsigned long long *dst, unsigned long
         if (lane == 0 && v) atomicAdd(dst, v);
     }
 }
+
+// What one pass over the ranges tells (zero before it).
+struct RangeInfo {
+    unsigned long long sum_deg;
+    unsigned long long max_deg;
+    unsigned long long short_count;   // lists of at most 32 entries
+    unsigned long long long_count;    // longer lists
+    unsigned long long long_entries;  // entries in longer lists
+    unsigned long long win_groups;    // preference windows: groups of 4 entries
+    unsigned long long win_even;      // preference windows: lengths rounded up to even numbers
+    int noncontig;                    // ranges do not tile [0, nnz) in vertex order
+    int bad;                          // a range outside [0, nnz)
+};
+cudaError_t scan_ranges(const int2 *ranges, int n, long long nnz, RangeInfo *d_info, long long *deg_out, cudaStream_t stream);
+void apply_ranges(mm_graph *g, const RangeInfo &info);
 
 // Ensure g->scratch holds at least `bytes`; returns MM_OK or an error.
 mm_status ensure_scratch(mm_graph *g, size_t bytes);

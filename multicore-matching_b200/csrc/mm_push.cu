@@ -66,6 +66,7 @@
 #include <cstddef>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 
 #include "mm_common.cuh"
@@ -2105,55 +2106,50 @@ __global__ void __launch_bounds__(kThreads, kSolo ? 1 : 2) k_match(const __grid_
 // ---------------------------------------------------------------------------
 // Preparation: degree classes and reverse proposal keys.
 
-struct PrepInfo {
-    unsigned long long sum_deg;
-    unsigned long long max_deg;
-    unsigned long long short_count;   // lists of at most kWin entries
-    unsigned long long long_count;    // longer lists
-    unsigned long long long_entries;  // entries in longer lists
-    int noncontig;
-    int pad;
-};
-
-__global__ void k_scan_ranges(const int2 *ranges, int n, long long nnz, PrepInfo *info, long long *deg_out)
+// (block sums: an atomic a warp and word had all warps queue on seven words)
+__global__ void __launch_bounds__(256) k_scan_ranges(const int2 *ranges, int n, long long nnz, RangeInfo *info, long long *deg_out)
 {
-    unsigned long long sum = 0, mx = 0, nshort = 0, nlong = 0, elong = 0;
-    int nc = 0;
+    unsigned long long sum = 0, nshort = 0, nlong = 0, elong = 0, groups = 0, even = 0;
+    int mx = 0, nc = 0, bad = 0;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int2 r = ranges[v];
-        const int d = degree_of(r);
-        sum += d;
-        mx = d > (long long)mx ? d : mx;
+        const int d = degree_of(r), wl = win_len(d);
+        if (d > 0 && (r.x < 0 || (long long)r.y > nnz)) bad = 1;
+        sum += (unsigned long long)d;
+        mx = max(mx, d);
         if (d > kWin) {
             nlong += 1;
-            elong += d;
+            elong += (unsigned long long)d;
         } else {
             nshort += 1;
         }
+        groups += (wl + 3) >> 2;
+        even += (wl + 1) & ~1;
         if (deg_out) deg_out[v] = d;
         if (r.y < r.x) nc = 1;
         if (v == 0 && r.x != 0) nc = 1;
         if (v + 1 < n && ranges[v + 1].x != r.y) nc = 1;
         if (v == n - 1 && (long long)r.y != nnz) nc = 1;
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        sum += __shfl_down_sync(kFull, sum, o);
-        const unsigned long long m2 = __shfl_down_sync(kFull, mx, o);
-        mx = m2 > mx ? m2 : mx;
-        nshort += __shfl_down_sync(kFull, nshort, o);
-        nlong += __shfl_down_sync(kFull, nlong, o);
-        elong += __shfl_down_sync(kFull, elong, o);
-        nc |= __shfl_down_sync(kFull, nc, o);
-    }
+    block_add(&info->sum_deg, sum);
+    block_add(&info->short_count, nshort);
+    block_add(&info->long_count, nlong);
+    block_add(&info->long_entries, elong);
+    block_add(&info->win_groups, groups);
+    block_add(&info->win_even, even);
+    __shared__ int s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    mx = __reduce_max_sync(kFull, mx);
+    nc = __any_sync(kFull, nc);
+    bad = __any_sync(kFull, bad);
     if ((threadIdx.x & 31) == 0) {
-        if (sum) atomicAdd(&info->sum_deg, sum);
-        if (mx) atomicMax(&info->max_deg, mx);
-        if (nshort) atomicAdd(&info->short_count, nshort);
-        if (nlong) atomicAdd(&info->long_count, nlong);
-        if (elong) atomicAdd(&info->long_entries, elong);
+        atomicMax(&s_max, mx);
         if (nc) atomicOr(&info->noncontig, 1);
+        if (bad) atomicOr(&info->bad, 1);
     }
+    __syncthreads();
+    if (threadIdx.x == 0 && s_max) atomicMax(&info->max_deg, (unsigned long long)s_max);
 }
 
 // One item per (owner, slot): key = (min << B | max) << 1 | (owner == max).
@@ -2262,19 +2258,11 @@ __global__ void k_win_offsets(const int2 *ranges, const long long *off, int n, i
         pwin_off[v] = (int)((unsigned)off[v] | (v < n && degree_of(ranges[v]) > kWin ? 0x80000000u : 0u));
 }
 
-// Groups of each vertex's window; *even receives the sum of the windows'
-// lengths rounded up to even numbers.
-__global__ void k_win_sizes(const int2 *ranges, int n, long long *groups, unsigned long long *even)
+// Groups of each vertex's window.
+__global__ void k_win_sizes(const int2 *ranges, int n, long long *groups)
 {
-    unsigned long long sum = 0;
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const int wl = win_len(degree_of(ranges[v]));
-        groups[v] = (wl + 3) >> 2;
-        sum += (wl + 1) & ~1;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(kFull, sum, o);
-    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(even, sum);
+    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v <= n; v += gridDim.x * blockDim.x)
+        groups[v] = v < n ? (win_len(degree_of(ranges[v])) + 3) >> 2 : 0;
 }
 
 constexpr int kWinRows = 8;       // rows of 32 entries tested against the window threshold per step
@@ -2647,6 +2635,8 @@ constexpr int kStampCount = 3 * kMaxRounds + 1;
 constexpr size_t kResultBytes = 256;
 
 struct PushState {
+    // one allocation: the arrays from col to ctl
+    void *arena = nullptr;
     uint32_t *col = nullptr;
     int2 *req = nullptr;
     unsigned long long *best = nullptr;
@@ -2655,18 +2645,16 @@ struct PushState {
     int *list_mem = nullptr;          // the two parities' lists, list_cap items each
     size_t list_cap = 0;
     int *prop = nullptr;              // list_cap requests
-    uint32_t *prop_key = nullptr;     // list_cap key halves, once a type off the symmetric path needs them
-    int4 *rec = nullptr;              // finish phase: records, 3 int4 each, once a type on the symmetric path needs them
-    size_t rec_cap = 0;               // records that rec holds
     int4 *staged = nullptr;
     int *piece_item = nullptr;
     Ctl *ctl = nullptr;               // two control blocks, used by alternate calls
     int ctl_turn = 0;
+    uint32_t *prop_key = nullptr;     // list_cap key halves, once a type off the symmetric path needs them
+    int4 *rec = nullptr;              // finish phase: records, 3 int4 each, once a type on the symmetric path needs them
+    size_t rec_cap = 0;               // records that rec holds
     Result *result = nullptr;         // pinned: written by the kernel
     unsigned long long *stats = nullptr;
     unsigned long long *tstamp = nullptr;
-    int grid[2][3] = {{0, 0, 0}, {0, 0, 0}};  // co-resident blocks of k_match by weighting and mode
-    int sms = 0;                              // multiprocessors of the device
     // The last call on this state ended with every grid barrier complete (the
     // next call's control block is clear) and every fallback list combined
     // (part_key and part_cnt all zero); false after a call that gave up or failed.
@@ -2678,18 +2666,9 @@ struct PushState {
 void free_state(PushState *s)
 {
     // callers have synchronised the device (graph destroy or a failed set-up)
-    dev_free(s->col, 0);
-    dev_free(s->req, 0);
-    dev_free(s->best, 0);
-    dev_free(s->part_key, 0);
-    dev_free(s->part_cnt, 0);
-    dev_free(s->list_mem, 0);
-    dev_free(s->prop, 0);
+    dev_free(s->arena, 0);
     dev_free(s->prop_key, 0);
     dev_free(s->rec, 0);
-    dev_free(s->staged, 0);
-    dev_free(s->piece_item, 0);
-    dev_free(s->ctl, 0);
     pinned_put(s->result, kResultBytes);
     dev_free(s->stats, 0);
     dev_free(s->tstamp, 0);
@@ -2714,7 +2693,63 @@ int coresident_blocks(int sms)
 
 constexpr int kMaxBlocks = 1024;
 
-mm_status alloc_state(mm_graph *g, PushState **out)
+// What the device allows, found out once (the kernels' shared memory limits are
+// set on the way).
+struct DeviceLimits {
+    bool known = false;
+    int coop = 0;
+    int sms = 0;
+    int grid[2][3] = {{0, 0, 0}, {0, 0, 0}};  // co-resident blocks of k_match by weighting and mode
+    int solo = 0;                             // the one-block kernels fit
+};
+std::mutex g_limits_mu;
+DeviceLimits g_limits[256];
+
+mm_status device_limits(int dev, DeviceLimits *out)
+{
+    if (dev < 0 || dev >= 256) {
+        set_error("push: device ordinal out of range");
+        return MM_ERR_UNSUPPORTED;
+    }
+    std::lock_guard<std::mutex> lock(g_limits_mu);
+    DeviceLimits &d = g_limits[dev];
+    if (!d.known) {
+        DeviceLimits x;
+        cudaDeviceGetAttribute(&x.sms, cudaDevAttrMultiProcessorCount, dev);
+        cudaDeviceGetAttribute(&x.coop, cudaDevAttrCooperativeLaunch, dev);
+        x.grid[0][0] = coresident_blocks<false, false, false, false>(x.sms);
+        x.grid[0][1] = coresident_blocks<false, true, false, false>(x.sms);
+        x.grid[0][2] = coresident_blocks<false, false, true, false>(x.sms);
+        x.grid[1][0] = coresident_blocks<true, false, false, false>(x.sms);
+        x.grid[1][1] = coresident_blocks<true, true, false, false>(x.sms);
+        x.grid[1][2] = coresident_blocks<true, false, true, false>(x.sms);
+        x.solo = coresident_blocks<false, false, false, true>(x.sms) > 0 && coresident_blocks<true, false, false, true>(x.sms) > 0;
+        const cudaError_t le = cudaGetLastError();
+        if (le != cudaSuccess) return cuda_fail(le, "push: kernel attributes");
+        x.known = true;
+        d = x;
+    }
+    bool over = false, under = !d.coop || !d.solo;
+    for (int a = 0; a < 2; ++a)
+        for (int b = 0; b < 3; ++b) {
+            over |= d.grid[a][b] > kMaxBlocks;
+            under |= d.grid[a][b] < 1;
+        }
+    if (over) {
+        set_error("push: more co-resident blocks than the lists are sized for");
+        return MM_ERR_UNSUPPORTED;
+    }
+    if (under) {
+        set_error("push: the device cannot run the cooperative round kernel");
+        return MM_ERR_UNSUPPORTED;
+    }
+    *out = d;
+    return MM_OK;
+}
+
+// The state's arrays, allocated and cleared on the call's stream (each call
+// ends with its stream synchronised, so the next may come on another).
+mm_status alloc_state(mm_graph *g, cudaStream_t stream, PushState **out)
 {
     PushState *s = new (std::nothrow) PushState();
     if (!s) {
@@ -2726,25 +2761,26 @@ mm_status alloc_state(mm_graph *g, PushState **out)
     // lists longer than the window can fall back
     const size_t npiece_cap = (size_t)(g->long_entries / kPiece + g->long_count) + 1;
     const size_t nstaged = (size_t)(g->long_count > 0 ? g->long_count : 1);
+    const size_t nparts = g->long_count > 0 ? n : 1;
     // whatever the grid, its blocks' regions fit: (n / kChunk / blocks + 1) chunks each
-    s->list_cap = n + (size_t)kChunk * (kMaxBlocks + 1);
-    // pooled on the legacy stream, then synchronised so that any stream may use them
-    cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->col, (n + 15) / 16 * sizeof(uint32_t), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->req, n * sizeof(int2), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->best, n * sizeof(unsigned long long), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->part_key, n * sizeof(unsigned long long), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->part_cnt, n * sizeof(int), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->list_mem, 2 * s->list_cap * sizeof(int), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->prop, s->list_cap * sizeof(int), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->staged, nstaged * sizeof(int4), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->piece_item, npiece_cap * sizeof(int), 0);
-    if (e == cudaSuccess) e = dev_alloc((void **)&s->ctl, 2 * sizeof(Ctl), 0);
+    const int most = (int)((n + kThreads - 1) / kThreads);
+    s->list_cap = n + (size_t)kChunk * ((size_t)(most < kMaxBlocks ? most : kMaxBlocks) + 1);
+    size_t at = 0;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at += (bytes + 255) / 256 * 256;
+        return o;
+    };
+    // the cleared ones first
+    const size_t o_ctl = take(2 * sizeof(Ctl)), o_pk = take(nparts * sizeof(unsigned long long)),
+                 o_pc = take(nparts * sizeof(int)), cleared = at;
+    const size_t o_col = take((n + 15) / 16 * sizeof(uint32_t)), o_req = take(n * sizeof(int2)),
+                 o_best = take(n * sizeof(unsigned long long)), o_lists = take(2 * s->list_cap * sizeof(int)),
+                 o_prop = take(s->list_cap * sizeof(int)), o_staged = take(nstaged * sizeof(int4)),
+                 o_piece = take(npiece_cap * sizeof(int));
+    cudaError_t e = dev_alloc(&s->arena, at, stream);
     if (e == cudaSuccess) e = pinned_get((void **)&s->result, kResultBytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->ctl, 0, 2 * sizeof(Ctl), 0);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->part_key, 0, n * sizeof(unsigned long long), 0);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->part_cnt, 0, n * sizeof(int), 0);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->arena, 0, cleared, stream);
     if (e != cudaSuccess) {
         cudaDeviceSynchronize();
         free_state(s);
@@ -2752,40 +2788,17 @@ mm_status alloc_state(mm_graph *g, PushState **out)
         set_error(std::string("push: device allocation failed: ") + cudaGetErrorString(e));
         return MM_ERR_NOMEM;
     }
-    int sms = 0, dev = 0, coop = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    s->sms = sms;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev);
-    s->grid[0][0] = coresident_blocks<false, false, false, false>(sms);
-    s->grid[0][1] = coresident_blocks<false, true, false, false>(sms);
-    s->grid[0][2] = coresident_blocks<false, false, true, false>(sms);
-    s->grid[1][0] = coresident_blocks<true, false, false, false>(sms);
-    s->grid[1][1] = coresident_blocks<true, true, false, false>(sms);
-    s->grid[1][2] = coresident_blocks<true, false, true, false>(sms);
-    const bool solo = coresident_blocks<false, false, false, true>(sms) > 0 && coresident_blocks<true, false, false, true>(sms) > 0;
-    cudaError_t le = cudaGetLastError();
-    if (le != cudaSuccess) {
-        free_state(s);
-        return cuda_fail(le, "push: kernel attributes");
-    }
-    bool over = false, under = false;
-    for (int a = 0; a < 2; ++a) {
-        for (int b = 0; b < 3; ++b) {
-            over |= s->grid[a][b] > kMaxBlocks;
-            under |= s->grid[a][b] < 1;
-        }
-    }
-    if (over) {
-        free_state(s);
-        set_error("push: more co-resident blocks than the lists are sized for");
-        return MM_ERR_UNSUPPORTED;
-    }
-    if (!coop || under || !solo) {
-        free_state(s);
-        set_error("push: the device cannot run the cooperative round kernel");
-        return MM_ERR_UNSUPPORTED;
-    }
+    char *base = (char *)s->arena;
+    s->ctl = (Ctl *)(base + o_ctl);
+    s->part_key = (unsigned long long *)(base + o_pk);
+    s->part_cnt = (int *)(base + o_pc);
+    s->col = (uint32_t *)(base + o_col);
+    s->req = (int2 *)(base + o_req);
+    s->best = (unsigned long long *)(base + o_best);
+    s->list_mem = (int *)(base + o_lists);
+    s->prop = (int *)(base + o_prop);
+    s->staged = (int4 *)(base + o_staged);
+    s->piece_item = (int *)(base + o_piece);
     s->at_rest = true;
     *out = s;
     return MM_OK;
@@ -2820,6 +2833,9 @@ mm_status launch_match(const Call &c)
     mm_graph *g = c.g;
     PushState *s = c.s;
     const PolicyArgs *pol = c.pol;
+    DeviceLimits dev;
+    const mm_status lim = device_limits(g->device, &dev);
+    if (lim != MM_OK) return lim;
     Params p;
     std::memset(&p, 0, sizeof p);
     p.n = g->n;
@@ -2875,7 +2891,7 @@ mm_status launch_match(const Call &c)
     // no more than give every thread a vertex
     const int mode = kPolicy ? 2 : (kStats ? 1 : 0);
     const int bps = g->opt_blocks_per_sm;
-    int grid = bps > 0 ? min(s->grid[kW][mode], bps * s->sms) : s->grid[kW][mode];
+    int grid = bps > 0 ? min(dev.grid[kW][mode], bps * dev.sms) : dev.grid[kW][mode];
     grid = g->n <= kSoloVertices ? 1 : min(grid, (g->n + kThreads - 1) / kThreads);
     const int chunks = (int)(((long long)g->n + kChunk - 1) / kChunk);
     p.region = (chunks + grid - 1) / grid * kChunk;
@@ -2918,7 +2934,7 @@ mm_status begin_call(Call &c)
     if (st != MM_OK) return st;
     PushState *s = (PushState *)g->push_exec;
     if (!s) {
-        st = alloc_state(g, &s);
+        st = alloc_state(g, c.stream, &s);
         if (st != MM_OK) return st;
         g->push_exec = s;
     }
@@ -2932,6 +2948,13 @@ mm_status begin_call(Call &c)
     s->result->rounds = -1;
     s->result->status = 0;
     return MM_OK;
+}
+
+// A call that could not be launched leaves nothing in flight on its stream.
+mm_status call_failed(const Call &c, mm_status st)
+{
+    cudaStreamSynchronize(c.stream);
+    return st;
 }
 
 mm_status end_call(Call &c, int *rounds_out, long long *stats, int stats_rounds, unsigned long long *stamps)
@@ -2990,42 +3013,29 @@ mm_status run_rounds(Call &c)
 
 namespace {
 
-// Degrees, classes, contiguity, slot offsets (once per graph).
+// Degrees, classes, contiguity, slot offsets (once per graph; for lists that
+// tile the arrays the upload's pass over the ranges has done it).
 mm_status scan_graph(mm_graph *g, cudaStream_t stream)
 {
     const int n = g->n;
-    if (n == 0 || g->scanned) return MM_OK;
-    {
-        PrepInfo *d_info = nullptr;
+    if (n == 0) return MM_OK;
+    if (!g->scanned) {
+        RangeInfo *d_info = nullptr;
         long long *d_deg = nullptr;
-        MM_CUDA_TRY(dev_alloc((void **)&d_info, sizeof(PrepInfo), stream), "prep info");
-        MM_CUDA_TRY(cudaMemsetAsync(d_info, 0, sizeof(PrepInfo), stream), "prep info clear");
-        cudaError_t e = dev_alloc((void **)&d_deg, sizeof(long long) * (size_t)n, stream);
-        if (e != cudaSuccess) {
-            dev_free(d_info, stream);
-            return cuda_fail(e, "prep degrees");
-        }
-        k_scan_ranges<<<grid_for(n, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, n, g->nnz, d_info, d_deg);
-        PrepInfo info;
-        e = cudaMemcpyAsync(&info, d_info, sizeof info, cudaMemcpyDeviceToHost, stream);
+        MM_CUDA_TRY(dev_alloc((void **)&d_info, sizeof(RangeInfo), stream), "prep info");
+        cudaError_t e = cudaMemsetAsync(d_info, 0, sizeof(RangeInfo), stream);
+        if (e == cudaSuccess) e = dev_alloc((void **)&d_deg, sizeof(long long) * (size_t)n, stream);
+        if (e == cudaSuccess) e = scan_ranges(g->d_ranges, n, g->nnz, d_info, d_deg, stream);
+        RangeInfo info = {};
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&info, d_info, sizeof info, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
         dev_free(d_info, stream);
         if (e != cudaSuccess) {
             dev_free(d_deg, stream);
             return cuda_fail(e, "prep scan");
         }
-        g->sum_degree = (long long)info.sum_deg;
-        g->max_degree = (long long)info.max_deg;
-        g->short_count = (long long)info.short_count;
-        g->long_count = (long long)info.long_count;
-        g->long_entries = (long long)info.long_entries;
-        g->contiguous = info.noncontig == 0;
-        if (g->sum_degree >= (1ll << 31) - 1) {
-            dev_free(d_deg, stream);
-            set_error("push: more than 2^31 - 2 adjacency slots are not supported");
-            return MM_ERR_UNSUPPORTED;
-        }
-        if (!g->contiguous) {
+        apply_ranges(g, info);
+        if (!g->contiguous && g->sum_degree < (1ll << 31) - 1) {
             e = dev_alloc((void **)&g->d_slot_off, sizeof(long long) * (size_t)n, stream);
             void *tmp = nullptr;
             size_t tmp_bytes = 0;
@@ -3036,11 +3046,17 @@ mm_status scan_graph(mm_graph *g, cudaStream_t stream)
             dev_free(tmp, stream);
             if (e != cudaSuccess) {
                 dev_free(d_deg, stream);
+                dev_free(g->d_slot_off, stream);
+                g->d_slot_off = nullptr;
                 return cuda_fail(e, "slot offsets");
             }
         }
         dev_free(d_deg, stream);
         g->scanned = true;
+    }
+    if (g->sum_degree >= (1ll << 31) - 1) {
+        set_error("push: more than 2^31 - 2 adjacency slots are not supported");
+        return MM_ERR_UNSUPPORTED;
     }
     return MM_OK;
 }
@@ -3144,6 +3160,24 @@ mm_status build_revkey(mm_graph *g, int weighted, cudaStream_t stream)
 
 }  // namespace
 
+cudaError_t scan_ranges(const int2 *ranges, int n, long long nnz, RangeInfo *d_info, long long *deg_out, cudaStream_t stream)
+{
+    k_scan_ranges<<<grid_for(n, 256, 148 * 8), 256, 0, stream>>>(ranges, n, nnz, d_info, deg_out);
+    return cudaGetLastError();
+}
+
+void apply_ranges(mm_graph *g, const RangeInfo &info)
+{
+    g->sum_degree = (long long)info.sum_deg;
+    g->max_degree = (long long)info.max_deg;
+    g->short_count = (long long)info.short_count;
+    g->long_count = (long long)info.long_count;
+    g->long_entries = (long long)info.long_entries;
+    g->win_groups = (long long)info.win_groups;
+    g->win_even = (long long)info.win_even;
+    g->contiguous = info.noncontig == 0;
+}
+
 // Preference windows of the weighted types, built once per graph in three
 // steps so that the upload can build the windows of the lists that have
 // arrived while later chunks are still in transfer: windows_begin sizes and
@@ -3153,48 +3187,36 @@ mm_status build_revkey(mm_graph *g, int weighted, cudaStream_t stream)
 mm_status windows_begin(mm_graph *g, cudaStream_t stream)
 {
     const int n = g->n;
-    long long *groups = nullptr, *off = nullptr;  // groups[n + 1]: the even sum
-    void *tmp = nullptr;
-    size_t tmp_bytes = 0;
-    MM_CUDA_TRY(dev_alloc((void **)&groups, sizeof(long long) * ((size_t)n + 2), stream), "window sizes");
-    cudaError_t e = dev_alloc((void **)&off, sizeof(long long) * ((size_t)n + 1), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(groups + n, 0, 2 * sizeof(long long), stream);
-    if (e == cudaSuccess) {
-        k_win_sizes<<<grid_for(n, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, n, groups,
-                                                                  reinterpret_cast<unsigned long long *>(groups + n + 1));
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, groups, off, n + 1, stream);
-    if (e == cudaSuccess) e = dev_alloc(&tmp, tmp_bytes, stream);
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, groups, off, n + 1, stream);
-    long long total = 0, even = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&total, off + n, sizeof total, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&even, groups + n + 1, sizeof even, cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    dev_free(tmp, stream);
-    dev_free(groups, stream);
-    if (e != cudaSuccess) {
-        dev_free(off, stream);
-        return cuda_fail(e, "window offsets");
-    }
-    if (even >= (1ll << 31)) {
-        dev_free(off, stream);
+    if (g->win_even >= (1ll << 31)) {
         set_error("push: more than 2^31 - 1 preference-window slots are not supported");
         return MM_ERR_UNSUPPORTED;
     }
+    long long *groups = nullptr, *off = nullptr;
     int2 *win = nullptr;
     int *big = nullptr;  // [n + 1]: queued long lists, then their count
     int *packed = nullptr;
-    e = dev_alloc((void **)&packed, sizeof(int) * ((size_t)n + 1), stream);
+    void *tmp = nullptr;
+    size_t tmp_bytes = 0;
+    const size_t nv = (size_t)n + 1;
+    cudaError_t e = dev_alloc((void **)&groups, 2 * sizeof(long long) * nv, stream);
+    off = groups + nv;
+    if (e == cudaSuccess) e = dev_alloc((void **)&packed, sizeof(int) * nv, stream);
+    if (e == cudaSuccess)
+        e = dev_alloc((void **)&win, 4 * sizeof(int2) * (size_t)(g->win_groups > 0 ? g->win_groups : 1), stream);
+    if (e == cudaSuccess) e = dev_alloc((void **)&big, sizeof(int) * nv, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(big + n, 0, sizeof(int), stream);
+    if (e == cudaSuccess) {
+        k_win_sizes<<<grid_for(n + 1ll, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, n, groups);
+        e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, groups, off, n + 1, stream);
+    }
+    if (e == cudaSuccess) e = dev_alloc(&tmp, tmp_bytes, stream);
+    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, groups, off, n + 1, stream);
     if (e == cudaSuccess) {
         k_win_offsets<<<grid_for(n + 1ll, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, off, n, packed);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = dev_alloc((void **)&win, 4 * sizeof(int2) * (size_t)(total > 0 ? total : 1), stream);
-    if (e == cudaSuccess) e = dev_alloc((void **)&big, sizeof(int) * ((size_t)n + 1), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(big + n, 0, sizeof(int), stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    dev_free(off, stream);
+    dev_free(tmp, stream);
+    dev_free(groups, stream);
     if (e != cudaSuccess) {
         dev_free(win, stream);
         dev_free(big, stream);
@@ -3223,8 +3245,11 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream)
     int2 *win = g->win_build;
     const int *off = g->d_pwin_off;
     int nbig = 0;
-    cudaError_t e = cudaMemcpyAsync(&nbig, big + n, sizeof(int), cudaMemcpyDeviceToHost, stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    cudaError_t e = cudaSuccess;
+    if (g->max_degree > kWinChunk) {  // else nothing was queued
+        e = cudaMemcpyAsync(&nbig, big + n, sizeof(int), cudaMemcpyDeviceToHost, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    }
     if (e == cudaSuccess && nbig > 0) {
         long long *coff = nullptr, *ccnt = nullptr;
         WinCand *cand = nullptr;
@@ -3260,7 +3285,6 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream)
         dev_free(ccnt, stream);
         dev_free(coff, stream);
     }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     dev_free(big, stream);
     g->win_big = nullptr;
     if (e != cudaSuccess) {
@@ -3279,15 +3303,19 @@ namespace {
 // weight, so a proposal needs no dependent load of it (the proposal key is the
 // weight and the proposer's id).  An entry flagged as never chosen keeps a
 // weight that fails the same test (<= -1 or NaN).
-__global__ void k_win_weights(const int2 *ranges, const float *w, const int *pwin_off, int2 *pwin, int n)
+// Eight lanes a window: a list's weights lie together (a thread a window took
+// R-MAT 2^20 0.13 ms).
+__global__ void __launch_bounds__(256) k_win_weights(const float *w, const int *pwin_off, int2 *pwin, int n)
 {
-    for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const int wl = win_len(degree_of(ranges[v]));
-        const long long o = 4ll * (pwin_off[v] & 0x7fffffff);
-        for (int e = 0; e < wl; ++e) {
-            int2 x = pwin[o + e];
+    const int l = threadIdx.x & 7;
+    const long long stride = (long long)gridDim.x * blockDim.x / 8;
+    for (long long v = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 8; v < n; v += stride) {
+        const int g0 = pwin_off[v] & 0x7fffffff, g1 = pwin_off[v + 1] & 0x7fffffff;
+        for (long long e = 4ll * g0 + l; e < 4ll * g1; e += 8) {
+            int2 x = pwin[e];
+            if (x.x < 0) continue;  // a filler
             x.y = __float_as_int(__ldg(w + (x.y & 0x7fffffff)));
-            pwin[o + e] = x;
+            pwin[e] = x;
         }
     }
 }
@@ -3326,8 +3354,7 @@ mm_status push_prepare(mm_graph *g, int weighted, cudaStream_t stream)
     if (st == MM_OK && !sym) st = build_revkey(g, weighted, stream);
     if (st == MM_OK && weighted && g->n > 0 && !g->d_pwin) st = build_windows(g, stream);
     if (st == MM_OK && weighted && g->d_pwin && g->sym_weights && !g->pwin_weights) {
-        k_win_weights<<<grid_for(g->n, 256, 148 * 16), 256, 0, stream>>>(g->d_ranges, g->d_w, g->d_pwin_off, g->d_pwin,
-                                                                        g->n);
+        k_win_weights<<<grid_for(g->n * 8ll, 256, 148 * 8), 256, 0, stream>>>(g->d_w, g->d_pwin_off, g->d_pwin, g->n);
         MM_CUDA_TRY(cudaGetLastError(), "window weights");
         g->pwin_weights = true;
     }
@@ -3350,7 +3377,7 @@ mm_status push_match(mm_graph *g, int type, uint32_t barrier, const uint32_t *se
     Call c{g, nullptr, type, barrier, seeds, nseeds, d_match, stats != nullptr, false, nullptr, stream};
     mm_status st = begin_call(c);
     if (st == MM_OK) st = run_rounds(c);
-    if (st != MM_OK) return st;
+    if (st != MM_OK) return call_failed(c, st);
     return end_call(c, rounds_out, stats, stats_rounds, nullptr);
 }
 
@@ -3396,7 +3423,7 @@ mm_status push_match_policy(mm_graph *g, int type, uint32_t barrier, const uint3
     pol.trace_rounds = trace ? trace_rounds : 0;
     c.pol = &pol;
     st = run_rounds(c);
-    if (st != MM_OK) return st;
+    if (st != MM_OK) return call_failed(c, st);
     return end_call(c, rounds_out, nullptr, 0, nullptr);
 }
 
@@ -3410,7 +3437,7 @@ mm_status push_profile(mm_graph *g, int type, uint32_t barrier, const uint32_t *
     Call c{g, nullptr, type, barrier, seeds, nseeds, d_match, false, true, nullptr, stream};
     mm_status st = begin_call(c);
     if (st == MM_OK) st = run_rounds(c);
-    if (st != MM_OK) return st;
+    if (st != MM_OK) return call_failed(c, st);
     unsigned long long stamps[kStampCount];
     st = end_call(c, rounds_out, nullptr, 0, stamps);
     if (st != MM_OK) return st;

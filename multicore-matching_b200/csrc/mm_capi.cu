@@ -532,7 +532,8 @@ mm_status upload_and_check(mm_graph *g, const int *ranges, const int *nbrs, cons
     const bool contiguous = g->n > 0 && g->contiguous;
     g->scanned = contiguous;
     g->has_weights = w != nullptr;
-    g->sym_struct = contiguous && !c.unsorted && c.skew_s == 0;
+    g->sym_pairs = contiguous && c.skew_s == 0;
+    g->sym_struct = g->sym_pairs && !c.unsorted;
     // unit weights are symmetric whenever the structure is
     g->sym_weights = g->sym_struct && (!w || c.skew_w == 0);
     return MM_OK;
@@ -610,6 +611,7 @@ mm_status adopt_arrays(int device, int n, long long nnz, int2 *ranges, int *nbrs
     g->d_nbrs = nbrs;
     g->d_w = w;
     g->has_weights = true;
+    g->sym_pairs = sym_struct;
     g->sym_struct = sym_struct;
     g->sym_weights = sym_struct && sym_w;
     *out = g;

@@ -83,6 +83,7 @@ struct mm_graph {
     // the entries (v, u) are those (u, v) transposed -- with the weights too for
     // sym_weights.  Then a red vertex's order of preference over its proposers is
     // (weight, smaller proposer id) and the push path needs no reverse index.
+    bool sym_pairs = false;   // the ranges tile [0, nnz) and every entry has a reverse entry, in any order
     bool sym_struct = false;
     bool sym_weights = false;
     int2 *d_ranges = nullptr;

@@ -132,8 +132,10 @@ struct Params {
     int *part_cnt;                  // per cut fallback list: finished pieces
     int4 *staged;                   // shared fallback items {v, begin, end, first piece}
     int *piece_item;                // per piece of the shared fallback lists: its item
-    int4 *rec;                      // finish phase: records (3 int4 an item), rec_region of them for a block
+    int fin;                        // the finish phase applies: lists symmetric in structure
+    int4 *rec;                      // finish phase: records, rec_region of them for a block
     int rec_region;
+    int rec_stride;                 // int4 a record: 3 on the symmetric path, else 4
     int *match;                     // output array of this call
     uint32_t barrier;
     int cap;                        // 20 or 255
@@ -1355,9 +1357,9 @@ __device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &
 // that point at another active vertex, and its connected components have at
 // most 7 members (grids, random geometric and Erdos-Renyi graphs reach the same
 // state by round 3).  A vertex's future depends only on the colours and choices
-// of the active vertices it can reach: matched neighbours never change, and on
-// the symmetric path no active vertex has an unmatchable neighbour (a vertex
-// became unmatchable because every neighbour was matched).  So each component
+// of the active vertices it can reach: matched neighbours never change, and
+// where every entry has a reverse entry no active vertex has an unmatchable
+// neighbour (a vertex became unmatchable because every neighbour was matched).  So each component
 // can play all its remaining rounds on its own, with the same seeds, and the
 // grid needs no further barrier.
 //
@@ -1404,14 +1406,14 @@ __device__ __forceinline__ int item_at(const Params &p, const int *list, int cb,
     return Mem<kSolo>::item(list + (i < cb ? i : p.region - 1 - (i - cb)));
 }
 
-// Preference key of an entry naming u with weight w, as the finish phase
-// compares them: on the symmetric path a list is strictly increasing, so the
-// smaller id is the earlier position.  1: a neighbour that is never chosen.
+// Preference key of an entry of weight w, as the finish phase compares them.
+// at: its position in the arrays; on the symmetric path the neighbour's id, as
+// a list is strictly increasing there, so the smaller id is the earlier
+// position.  1: a neighbour that is never chosen.
 template <bool kW>
-__device__ __forceinline__ unsigned long long fin_key(int u, float w)
+__device__ __forceinline__ unsigned long long fin_key(int at, float w)
 {
-    if (kW) return w > -1.0f ? (((unsigned long long)weight_order(w) << 32) | (uint32_t)~u) : 1ull;
-    return (unsigned long long)(uint32_t)~u;
+    return cand_key<kW>(at, w);
 }
 
 // Own-list scan of vertex v, entries [b, e): active neighbours (blue or red),
@@ -1523,7 +1525,7 @@ __device__ __forceinline__ int fin_search(const Params &p, FinWarp &fw, int v, i
             if (__any_sync(kFull, in && u < v)) return kFinNotRoot;
             unsigned m = __ballot_sync(kFull, in);
             unsigned long long pref = 0;
-            if (in) pref = fin_key<kW>(u, wj);
+            if (in) pref = fin_key<kW>(p.sym ? u : j, wj);
             while (m) {
                 const int s = __ffs(m) - 1;
                 m &= m - 1;
@@ -1557,13 +1559,14 @@ __device__ __forceinline__ int fin_search(const Params &p, FinWarp &fw, int v, i
 
 // Adjacency entries the reference's respond loop inspects for red vertex v
 // (entries [b, b + deg)) whose best proposal key is kb: in random mode it
-// stops at its first proposer in list order, here the proposer with the
-// smallest id (kb's low half complemented), found in the sorted list.
+// stops at its first proposer in list order: kb's low half complemented is its
+// position, or on the symmetric path its id, found in the sorted list.
 template <bool kW>
 __device__ __forceinline__ unsigned long long respond_seen(const Params &p, int b, int deg, unsigned long long kb)
 {
     if (kW || !kb) return (unsigned long long)deg;
     const int first = (int)~(uint32_t)kb;
+    if (!p.sym) return (unsigned long long)(first - b + 1);  // a position
     int lo = b, hi = b + deg;
     while (lo < hi) {
         const int mid = (int)(((long long)lo + hi) >> 1);
@@ -1638,10 +1641,15 @@ __device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, int t0, in
         }
         unsigned long long crk = 0ull;
         if (act && blue && best >= 2) {
-            // the target's entry for this vertex has the same weight (symmetric path)
-            crk = kW ? (((best >> 32) << 32) | (unsigned long long)(uint32_t)~(uint32_t)g)
-                     : (unsigned long long)(uint32_t)~(uint32_t)g;
-            atomicMax(&fw.best[choice], crk);
+            // the proposal's key: on the symmetric path the target's entry for this
+            // vertex has the same weight; else the reverse key of the chosen entry
+            // (0: the target never picks it)
+            if (p.sym)
+                crk = kW ? (((best >> 32) << 32) | (unsigned long long)(uint32_t)~(uint32_t)g)
+                         : (unsigned long long)(uint32_t)~(uint32_t)g;
+            else
+                crk = __ldg(p.revkey + (int)~(uint32_t)best);
+            if (crk) atomicMax(&fw.best[choice], crk);
         }
         __syncwarp();
         const int gp = __shfl_sync(kFull, g, choice);
@@ -1649,7 +1657,7 @@ __device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, int t0, in
         unsigned long long kb = 0ull;
         if (act) {
             if (blue) {
-                if (best >= 2 && (uint32_t)fw.best[choice] == (uint32_t)crk) {
+                if (crk && (uint32_t)fw.best[choice] == (uint32_t)crk) {
                     val = 4 + min(g, gp) - base;
                     matched = true;
                 } else if (best == 0) {
@@ -1659,7 +1667,8 @@ __device__ __forceinline__ int fin_play(const Params &p, FinWarp &fw, int t0, in
             } else {
                 kb = fw.best[lane];
                 if (kb) {
-                    val = 4 + min(g, (int)~(uint32_t)kb) - base;
+                    const int from = (int)~(uint32_t)kb;
+                    val = 4 + min(g, p.sym ? from : __ldg(p.nbrs + from)) - base;
                     matched = true;
                 }
             }
@@ -1710,13 +1719,13 @@ struct FinComp {
     int k;
 };
 
-// The finish phase's record of an item: three int4, rec[3i .. 3i + 2] with i
-// counted from the block's own part of the record array: {meta, v, id 0, id 1},
-// {id 2, id 3, weight 0, weight 1}, {weight 2, weight 3, 0, 0}, the ids and
-// weight orders (0: never chosen) of its first kFinRec entries that point at
-// an active vertex.  meta = class | count << 8, count = its active neighbours,
-// kFinRec + 1 if more than a record holds.  A singleton needs the first int4
-// only, a vertex of two active neighbours of a random type too.
+// The finish phase's record of an item: rec_stride int4, the i-th record's from
+// rec[rec_stride * i], i counted from the block's own part of the record
+// array: {meta, v, id 0, id 1}, {id 2, id 3, weight 0, weight 1}, {weight 2,
+// weight 3, 0, 0}, the ids and weight orders (0: never chosen) of its first
+// kFinRec entries that point at an active vertex; off the symmetric path also
+// {position 0, .., position 3}.  meta = class | count << 8, count = its active
+// neighbours, kFinRec + 1 if more than a record holds.
 __device__ __forceinline__ int fin_meta_class(int meta) { return meta & 0xff; }
 __device__ __forceinline__ int fin_meta_count(int meta) { return (meta >> 8) & 0xff; }
 
@@ -1732,13 +1741,15 @@ __device__ __forceinline__ int fin_search_thread(const Params &p, int v, int i, 
     cp.mem[0] = v;
     ix[0] = i;
     for (int f = 0; f < k; ++f) {
-        const int4 *rec = p.rec + 3ll * ix[f];
+        const int4 *rec = p.rec + (long long)p.rec_stride * ix[f];
         const int4 r0 = __ldcg(rec), r1 = __ldcg(rec + 1), r2 = __ldcg(rec + 2);
+        const int4 r3 = p.sym ? make_int4(r0.z, r0.w, r1.x, r1.y) : __ldcg(rec + 3);
         const int cnt = fin_meta_count(r0.x);
         if (cnt > kFinRec) return kFinOverflow;
         cp.eoff[f] = (uint8_t)ne;
         const int uu[kFinRec] = {r0.z, r0.w, r1.x, r1.y};
         const int ww[kFinRec] = {r1.z, r1.w, r2.x, r2.y};
+        const int aa[kFinRec] = {r3.x, r3.y, r3.z, r3.w};
 #pragma unroll
         for (int q = 0; q < kFinRec; ++q) {
             if (q >= cnt) break;
@@ -1755,8 +1766,8 @@ __device__ __forceinline__ int fin_search_thread(const Params &p, int v, int i, 
                 ++k;
             }
             if (ne == kFinTEntries) return kFinOverflow;
-            cp.pref[ne] = !kW ? (unsigned long long)(uint32_t)~u
-                              : (ww[q] ? (((unsigned long long)(uint32_t)ww[q] << 32) | (uint32_t)~u) : 1ull);
+            cp.pref[ne] = !kW ? (unsigned long long)(uint32_t)~aa[q]
+                              : (ww[q] ? (((unsigned long long)(uint32_t)ww[q] << 32) | (uint32_t)~aa[q]) : 1ull);
             cp.tgt[ne] = (uint8_t)slot;
             ++ne;
         }
@@ -1865,7 +1876,7 @@ __device__ __forceinline__ bool finish_scan(const Params &p, int t, const int *l
         if (v >= 0) {
             const int cnt = min(nint, kFinRec + 1);
             const int at = blockIdx.x * p.rec_region + i;
-            int4 *rec = p.rec + 3ll * at;
+            int4 *rec = p.rec + (long long)p.rec_stride * at;
             rec[0] = make_int4(c | (cnt << 8), v, ur[0], ur[1]);
             if (nint > 0) {
                 p.req[v].x = at;
@@ -1881,6 +1892,7 @@ __device__ __forceinline__ bool finish_scan(const Params &p, int t, const int *l
                     }
                     rec[1] = make_int4(ur[2], ur[3], o[0], o[1]);
                     rec[2] = make_int4(o[2], o[3], 0, 0);
+                    if (!p.sym) rec[3] = make_int4(jr[0], jr[1], jr[2], jr[3]);
                 }
             }
         }
@@ -1914,7 +1926,7 @@ __device__ __forceinline__ bool finish_roots(const Params &p, Smem &sm, int t, i
     for (int base = lo_i; base < hi_i; base += 32) {
         const int i = base + lane;
         const int at = blockIdx.x * p.rec_region + i;
-        const int4 r0 = i < hi_i ? __ldcg(p.rec + 3ll * at) : make_int4(0, -1, 0, 0);
+        const int4 r0 = i < hi_i ? __ldcg(p.rec + (long long)p.rec_stride * at) : make_int4(0, -1, 0, 0);
         const int c = fin_meta_class(r0.x);
         if (kSingles) {
             const bool single = c == kFinSingle;
@@ -2061,9 +2073,8 @@ __global__ void __launch_bounds__(kThreads, kSolo ? 1 : 2) k_match(const __grid_
         int *list = kSolo ? solo.lists[t & 1] : p.lists[t & 1] + rbase;
         int *next = kSolo ? solo.lists[(t & 1) ^ 1] : p.lists[(t & 1) ^ 1] + rbase;
         const int cb = sm.count[t & 1][0], cr = sm.count[t & 1][1];
-        // the finish phase (the symmetric path of a constant colouring only); in
-        // one block the rounds cost less than it does
-        if (!kSolo && (!kPolicy || p.fin_retire) && p.sym && t > 0 && gridDim.x > 1 && p.fin_div > 0 && act > 0 && act <= fin_next &&
+        // the finish phase; in one block the rounds cost less than it does
+        if (!kSolo && p.fin && t > 0 && act > 0 && act <= fin_next &&
             (unsigned long long)act * (unsigned)p.fin_div <= active0) {
             const int done = finish_phase<kW, kStats>(p, sm, turn, t, list, cb, cr);
             if (done < 0) return;
@@ -2650,8 +2661,8 @@ struct PushState {
     Ctl *ctl = nullptr;               // two control blocks, used by alternate calls
     int ctl_turn = 0;
     uint32_t *prop_key = nullptr;     // list_cap key halves, once a type off the symmetric path needs them
-    int4 *rec = nullptr;              // finish phase: records, 3 int4 each, once a type on the symmetric path needs them
-    size_t rec_cap = 0;               // records that rec holds
+    int4 *rec = nullptr;              // finish phase: records, once a call needs them
+    size_t rec_cap = 0;               // int4 that rec holds
     Result *result = nullptr;         // pinned: written by the kernel
     unsigned long long *stats = nullptr;
     unsigned long long *tstamp = nullptr;
@@ -2896,20 +2907,26 @@ mm_status launch_match(const Call &c)
     const int chunks = (int)(((long long)g->n + kChunk - 1) / kChunk);
     p.region = (chunks + grid - 1) / grid * kChunk;
     p.turn_magic = grid > 1 ? (uint32_t)((1ull << 32) / (unsigned)grid + 1) : 0u;
+    // the finish phase plays constant colourings of lists that are symmetric in
+    // structure, whatever their order and weights (the policy's retirement rule
+    // is the symmetric path's)
+    p.fin = p.fin_div > 0 && grid > 1 && (kPolicy ? p.fin_retire && p.sym : p.sym || g->sym_pairs);
+    p.rec_stride = p.sym ? 3 : 4;
     if (!p.sym) {
         if (!s->prop_key)
             MM_CUDA_TRY(dev_alloc((void **)&s->prop_key, sizeof(uint32_t) * s->list_cap, c.stream), "request keys");
         p.prop_key = s->prop_key;
-    } else if (p.fin_div > 0 && grid > 1) {
+    }
+    if (p.fin) {
         // records for twice a block's share of the largest set the finish phase
         // accepts (a block that holds more calls the attempt off)
         p.rec_region = min(p.region, 2 * (p.region / p.fin_div) + kChunk);
-        const size_t need = (size_t)p.rec_region * grid;
+        const size_t need = (size_t)p.rec_region * grid * p.rec_stride;
         if (need > s->rec_cap) {
             dev_free(s->rec, c.stream);
             s->rec = nullptr;
             s->rec_cap = 0;
-            MM_CUDA_TRY(dev_alloc((void **)&s->rec, 3 * sizeof(int4) * need, c.stream), "finish records");
+            MM_CUDA_TRY(dev_alloc((void **)&s->rec, sizeof(int4) * need, c.stream), "finish records");
             s->rec_cap = need;
         }
         p.rec = s->rec;

@@ -182,6 +182,7 @@ struct GraphCheck {
     unsigned long long skew_s, skew_w;  // 0: symmetric in structure, with weights
     int bad;        // 2: an id outside [0, n)
     int unsorted;   // some list is not strictly increasing
+    int selfs;      // some list names its own vertex
 };
 
 // Contiguous CSR: slots [j0, j1) in chunks of kChk, a block per chunk; the
@@ -207,7 +208,7 @@ __global__ void __launch_bounds__(256) k_check_entries(const int2 *ranges, const
     __shared__ int start[kChk + 1];
     __shared__ int s_v0, s_cnt;
     unsigned long long ss = 0, sw = 0;
-    int bad = 0, uns = 0;
+    int bad = 0, uns = 0, self = 0;
     const long long chunks = (j1 - j0 + kChk - 1) / kChk;
     for (long long ch = blockIdx.x; ch < chunks; ch += gridDim.x) {
         const long long c0 = j0 + ch * kChk, c1 = min(c0 + kChk, j1);
@@ -243,6 +244,7 @@ __global__ void __launch_bounds__(256) k_check_entries(const int2 *ranges, const
             }
             // compared with the entry before (earlier chunks have arrived; later ones may not have)
             if (j > (long long)ranges[v].x && nbrs[j - 1] >= u) uns = 1;
+            self |= u == v;
             add_skew((unsigned)v, (unsigned)u, kWeights ? __float_as_uint(w[j]) : 0u, kWeights, ss, sw);
         }
     }
@@ -250,9 +252,11 @@ __global__ void __launch_bounds__(256) k_check_entries(const int2 *ranges, const
     if (kWeights) block_add(&c->skew_w, sw);
     bad = __any_sync(0xffffffffu, bad);
     uns = __any_sync(0xffffffffu, uns);
+    self = __any_sync(0xffffffffu, self);
     if ((threadIdx.x & 31) == 0) {
         if (bad) atomicOr(&c->bad, 2);
         if (uns) atomicOr(&c->unsorted, 1);
+        if (self) atomicOr(&c->selfs, 1);
     }
 }
 
@@ -534,6 +538,7 @@ mm_status upload_and_check(mm_graph *g, const int *ranges, const int *nbrs, cons
     g->has_weights = w != nullptr;
     g->sym_pairs = contiguous && c.skew_s == 0;
     g->sym_struct = g->sym_pairs && !c.unsorted;
+    g->no_self = contiguous && !c.selfs;
     // unit weights are symmetric whenever the structure is
     g->sym_weights = g->sym_struct && (!w || c.skew_w == 0);
     return MM_OK;
@@ -612,6 +617,7 @@ mm_status adopt_arrays(int device, int n, long long nnz, int2 *ranges, int *nbrs
     g->d_w = w;
     g->has_weights = true;
     g->sym_pairs = sym_struct;
+    g->no_self = true;
     g->sym_struct = sym_struct;
     g->sym_weights = sym_struct && sym_w;
     *out = g;

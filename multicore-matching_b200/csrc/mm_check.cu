@@ -12,9 +12,10 @@
 // the vertex that the value names, needs neither a sort nor a gather of match
 // values: k_pairs finds each vertex's partner (and whether the matching is of
 // that kind), and one pass over the lists looks for the partner's id, a group
-// of lanes per vertex.  That is every matching the matchers write; on RGG 2^20
-// weight and check together take 371 us by the general kernels (a thread a
-// vertex and its list, a radix sort of the values, three synchronisations).
+// of lanes per list (of symmetric graphs, one list a pair).  That is every
+// matching the matchers write; on RGG 2^20 weight and check together take 147 us
+// so, 371 us by the general kernels (a thread a vertex and its list, a radix
+// sort of the values, three synchronisations).
 // Anything else takes the general kernels, which follow the reference's walk.
 #include <cuda_runtime.h>
 #include <cub/device/device_radix_sort.cuh>
@@ -81,19 +82,23 @@ __device__ __forceinline__ bool entry_hit(const int *match, int v, int partner, 
     return u != v && !is_matched(match[u]);
 }
 
-// What one vertex adds: kWeight the matched entry's weight and 1, else the
-// check's counts (cnt: invalid, matchable, unmatched).  A pair is invalid if
+// What one list adds: kWeight the matched entry's weight and 1, else the
+// check's counts (cnt: invalid, matchable, unmatched).  kHalf: a pair's lists
+// name each other or neither does, with the same weight, so the list of the
+// vertex that the value names speaks for both.  Otherwise a pair is invalid if
 // either list misses the other vertex: the first of the two to say so (bad[],
 // at the vertex that the value names) counts it.
-template <bool kWeight>
+template <bool kWeight, bool kHalf>
 __device__ __forceinline__ void pair_result(const float *w, int v, int partner, int at, double *contrib,
                                             unsigned (&cnt)[3], int *bad)
 {
     if (kWeight) {
-        contrib[v] = at >= 0 ? (double)w[at] : 0.0;
-        cnt[0] += at >= 0;
+        const double x = at >= 0 ? (double)w[at] : 0.0;
+        contrib[v] = x;
+        if (kHalf && partner >= 0) contrib[partner] = x;  // (< 0: named by no other's value, so not clean)
+        cnt[0] += at >= 0 ? (kHalf ? 2u : 1u) : 0u;
     } else if (partner >= 0) {
-        if (at < 0 && atomicExch(bad + min(v, partner), 1) == 0) ++cnt[0];
+        if (at < 0 && (kHalf || atomicExch(bad + min(v, partner), 1) == 0)) ++cnt[0];
     } else {
         ++cnt[2];
         cnt[1] += at >= 0;
@@ -111,71 +116,94 @@ __device__ __forceinline__ void add_counts(const unsigned (&cnt)[3], PairState *
     }
 }
 
-// One pass over all vertices, a group of G lanes each, 4 G entries a step: the
+// One pass over all vertices, 32 a warp at a time: a lane reads a vertex's
+// match value, range and partner, then the lists that have to be searched are
+// dealt to groups of G lanes, kSlots a group, 4 G entries of each a step.  The
 // pass waits on the chain vertex -> list -> entries, so what counts is how many
-// lists a warp has in flight (RGG 2^20: 8 with G = 4).  Longer lists than
-// kPairList are queued for a block each.
+// lists a warp has in flight, and on its instructions.  RGG 2^20: weight 30 us,
+// check 31 us with one list a pair and 16 of them in flight; 50 us each with a
+// group for every vertex, 8 in flight and a ballot for each entry of a step.
+// Longer lists than kPairList are queued for a block each.
 constexpr int kPairList = 1024;
+constexpr int kSlots = 2;
+constexpr int kPairBlocks = 6;  // a multiprocessor (at 60 registers, 4 of them, the check took 54 us)
 
-template <int G, bool kWeight>
-__global__ void __launch_bounds__(256) k_pair_lists(const int2 *ranges, const int *nbrs, const float *w, const int *match,
+template <int G, bool kWeight, bool kHalf>
+__global__ void __launch_bounds__(256, kPairBlocks) k_pair_lists(const int2 *ranges, const int *nbrs, const float *w, const int *match,
                                                     int n, const int *other, int *bad, int *queue, double *contrib,
                                                     PairState *st)
 {
     if (!clean(st)) return;
-    constexpr int kPerWarp = 32 / G;
-    const int lane = threadIdx.x & 31, l = lane & (G - 1), shift = lane & ~(G - 1);
-    const unsigned gmask = G == 32 ? 0xffffffffu : (1u << (G & 31)) - 1u;
+    __shared__ uint8_t s_from[8][32];
+    constexpr int kGroups = 32 / G;
+    const int lane = threadIdx.x & 31, l = lane & (G - 1);
+    uint8_t *from = s_from[threadIdx.x >> 5];
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long stride = ((long long)gridDim.x * blockDim.x >> 5) * kPerWarp;
+    const long long stride = ((long long)gridDim.x * blockDim.x >> 5) * 32;
     unsigned cnt[3] = {0u, 0u, 0u};
     bool broken = false;
-    // the next vertex's match value, range and partner are loaded while this one's list is read
-    int vn = -1, mn = 0, on = -1;
-    int2 rn = make_int2(0, 0);
-    auto fetch = [&](long long base) {
-        const long long v0 = base + lane / G;
-        vn = base < n && v0 < n ? (int)v0 : -1;
-        if (vn >= 0) {
-            mn = match[vn];
-            rn = ranges[vn];
-            on = other[vn];
-        }
-    };
-    fetch(warp * kPerWarp);
-    for (long long base = warp * kPerWarp; base < n; base += stride) {  // warp-uniform
-        const int v = vn, mv = v >= 0 ? mn : 0, ov = on;
-        const int2 r = v >= 0 ? rn : make_int2(0, 0);
-        fetch(base + stride);
+    for (long long base = warp * 32; base < n; base += stride) {  // warp-uniform
+        const bool in = base + lane < n;
+        const int v = in ? (int)base + lane : -1, mv = in ? match[v] : 0;
+        const int2 r = in ? ranges[v] : make_int2(0, 0);
         const bool matched = is_matched(mv);
-        const int a = mv - 4, partner = !matched ? -1 : (a == v ? ov - 1 : a);
-        if (matched && a != v && l == 0) broken |= other[a] != v + 1;
-        bool want = v >= 0 && (!kWeight || matched);
-        if (kWeight && v >= 0 && !matched && l == 0) contrib[v] = 0.0;
+        const int a = mv - 4, o = matched ? other[a] : 0;
+        const int partner = !matched ? -1 : (a == v ? o - 1 : a);
+        broken |= matched && a != v && o != v + 1;
+        if (kWeight && in && !matched) contrib[v] = 0.0;
+        bool want = in && (matched ? !kHalf || a == v : !kWeight);
         if (want && r.y > r.x && r.y - r.x > kPairList) {
-            if (l == 0) queue[atomicAdd(&st->nlong, 1)] = v;
+            queue[atomicAdd(&st->nlong, 1)] = v;
             want = false;
         }
-        int at = -1;
-        bool go = want && r.x < r.y;
-        for (int j = r.x; __any_sync(0xffffffffu, go); j += 4 * G) {
-            int u[4];
+        const unsigned wants = __ballot_sync(0xffffffffu, want);
+        const int nw = __popc(wants);
+        __syncwarp();
+        if (want) from[__popc(wants & ((1u << lane) - 1u))] = (uint8_t)lane;
+        __syncwarp();
+        for (int b = 0; b < nw; b += kSlots * kGroups) {
+            int vs[kSlots], ps[kSlots], js[kSlots], je[kSlots], at[kSlots];
+            bool mine[kSlots], go[kSlots], any = false;
 #pragma unroll
-            for (int k = 0; k < 4; ++k) u[k] = go && j + k * G + l < r.y ? __ldg(nbrs + j + k * G + l) : -1;
-            bool hit[4];
+            for (int q = 0; q < kSlots; ++q) {
+                const int slot = b + q * kGroups + lane / G;
+                mine[q] = slot < nw;
+                const int src = mine[q] ? from[slot] : 0;
+                vs[q] = __shfl_sync(0xffffffffu, v, src);
+                ps[q] = __shfl_sync(0xffffffffu, partner, src);
+                js[q] = __shfl_sync(0xffffffffu, r.x, src);
+                je[q] = __shfl_sync(0xffffffffu, r.y, src);
+                at[q] = -1;
+                go[q] = mine[q] && js[q] < je[q];
+                any |= go[q];
+            }
+            while (__any_sync(0xffffffffu, any)) {
+                int u[kSlots][4];
 #pragma unroll
-            for (int k = 0; k < 4; ++k) hit[k] = u[k] >= 0 && entry_hit<kWeight>(match, v, partner, u[k]);
+                for (int q = 0; q < kSlots; ++q)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const unsigned bits = (__ballot_sync(0xffffffffu, hit[k]) >> shift) & gmask;
-                if (go && bits) {
-                    at = j + k * G + __ffs(bits) - 1;
-                    go = false;
+                    for (int k = 0; k < 4; ++k)
+                        u[q][k] = go[q] && k * G + l < je[q] - js[q] ? __ldg(nbrs + js[q] + k * G + l) : -1;
+                any = false;
+#pragma unroll
+                for (int q = 0; q < kSlots; ++q) {
+                    // the group's first hit of the step, counted from js
+                    int first = 4 * G;
+#pragma unroll
+                    for (int k = 3; k >= 0; --k)
+                        if (u[q][k] >= 0 && entry_hit<kWeight>(match, vs[q], ps[q], u[q][k])) first = k * G + l;
+#pragma unroll
+                    for (int o = G / 2; o > 0; o >>= 1) first = min(first, __shfl_xor_sync(0xffffffffu, first, o));
+                    if (go[q] && first < 4 * G) at[q] = js[q] + first;
+                    go[q] = go[q] && first == 4 * G && je[q] - js[q] > 4 * G;
+                    js[q] += go[q] ? 4 * G : 0;
+                    any |= go[q];
                 }
             }
-            go = go && j + 4 * G < r.y;
+#pragma unroll
+            for (int q = 0; q < kSlots; ++q)
+                if (mine[q] && l == 0) pair_result<kWeight, kHalf>(w, vs[q], ps[q], at[q], contrib, cnt, bad);
         }
-        if (want && l == 0) pair_result<kWeight>(w, v, partner, at, contrib, cnt, bad);
     }
     if (__any_sync(0xffffffffu, broken) && lane == 0) atomicOr(&st->broken, 1);
     if (kWeight) {
@@ -186,7 +214,7 @@ __global__ void __launch_bounds__(256) k_pair_lists(const int2 *ranges, const in
 }
 
 // The queued long lists, a block each (the lowest hit of a step is the first).
-template <bool kWeight>
+template <bool kWeight, bool kHalf>
 __global__ void __launch_bounds__(256) k_pair_long(const int2 *ranges, const int *nbrs, const float *w, const int *match,
                                                    const int *other, int *bad, const int *queue, double *contrib,
                                                    PairState *st)
@@ -215,7 +243,7 @@ __global__ void __launch_bounds__(256) k_pair_long(const int2 *ranges, const int
         }
         if (threadIdx.x == 0) {
             unsigned cnt[3] = {0u, 0u, 0u};
-            pair_result<kWeight>(w, v, partner, s_at == 0x7fffffff ? -1 : s_at, contrib, cnt, bad);
+            pair_result<kWeight, kHalf>(w, v, partner, s_at == 0x7fffffff ? -1 : s_at, contrib, cnt, bad);
             add_counts<kWeight>(cnt, st);
         }
         __syncthreads();
@@ -227,24 +255,24 @@ __global__ void __launch_bounds__(256) k_pair_long(const int2 *ranges, const int
 size_t pair_bytes(int n) { return 128 + sizeof(int) * 3 * (size_t)n; }
 static_assert(sizeof(PairState) <= 128, "the arrays follow it");
 
-template <bool kWeight>
+template <bool kWeight, bool kHalf>
 cudaError_t launch_pairs(const mm_graph *g, const int *d_match, double *contrib, PairState *st, cudaStream_t s)
 {
     const int n = g->n;
     int *other = reinterpret_cast<int *>(reinterpret_cast<char *>(st) + 128), *bad = other + n, *queue = bad + n;
-    const cudaError_t e = cudaMemsetAsync(st, 0, 128 + sizeof(int) * (kWeight ? 1 : 2) * (size_t)n, s);
+    const cudaError_t e = cudaMemsetAsync(st, 0, 128 + sizeof(int) * (kWeight || kHalf ? 1 : 2) * (size_t)n, s);
     if (e != cudaSuccess) return e;
     k_pairs<<<grid_for(n, 256, 148 * 8), 256, 0, s>>>(d_match, n, other, st);
     const long long per = n > 0 ? g->nnz / n : 0;
-    auto run = [&](auto kernel, int lanes) {
-        kernel<<<grid_for((long long)n * lanes, 256, 148 * 8), 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, n, other,
-                                                                           bad, queue, contrib, st);
+    auto run = [&](auto kernel) {
+        kernel<<<grid_for(n, 256, 148 * kPairBlocks), 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, n, other, bad, queue,
+                                                                   contrib, st);
     };
-    if (per <= 20) run(k_pair_lists<4, kWeight>, 4);
-    else if (per <= 80) run(k_pair_lists<8, kWeight>, 8);
-    else run(k_pair_lists<32, kWeight>, 32);
+    if (per <= 20) run(k_pair_lists<4, kWeight, kHalf>);
+    else if (per <= 80) run(k_pair_lists<8, kWeight, kHalf>);
+    else run(k_pair_lists<32, kWeight, kHalf>);
     if (g->nnz > kPairList && !(g->scanned && g->max_degree <= kPairList))
-        k_pair_long<kWeight><<<148 * 4, 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, other, bad, queue, contrib, st);
+        k_pair_long<kWeight, kHalf><<<148 * 4, 256, 0, s>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, other, bad, queue, contrib, st);
     return cudaGetLastError();
 }
 
@@ -442,7 +470,7 @@ MM_API mm_status mm_matching_weight(mm_graph *g, const int *d_match, double *wei
     size_t tmp_bytes = 0;
     cudaError_t e = dev_alloc((void **)&contrib, sizeof(double) * (size_t)n, st);
     if (e == cudaSuccess) e = dev_alloc((void **)&ps, pair_bytes(n), st);
-    if (e == cudaSuccess) e = launch_pairs<true>(g, d_match, contrib, ps, st);
+    if (e == cudaSuccess) e = (g->sym_weights && g->no_self ? launch_pairs<true, true> : launch_pairs<true, false>)(g, d_match, contrib, ps, st);
     if (e == cudaSuccess) {
         k_weight<<<grid_for(n, 256, 148 * 8), 256, 0, st>>>(g->d_ranges, g->d_nbrs, g->d_w, d_match, n, contrib, ps);
         e = cudaGetLastError();
@@ -479,7 +507,7 @@ MM_API mm_status mm_matching_check(mm_graph *g, const int *d_match, long long *c
     {
         PairState *ps = nullptr;
         e = dev_alloc((void **)&ps, pair_bytes(n), st);
-        if (e == cudaSuccess) e = launch_pairs<false>(g, d_match, nullptr, ps, st);
+        if (e == cudaSuccess) e = (g->sym_struct ? launch_pairs<false, true> : launch_pairs<false, false>)(g, d_match, nullptr, ps, st);
         PairState h = {};
         if (e == cudaSuccess) e = cudaMemcpyAsync(&h, ps, sizeof h, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);

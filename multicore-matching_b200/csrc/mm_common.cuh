@@ -84,6 +84,7 @@ struct mm_graph {
     // sym_weights.  Then a red vertex's order of preference over its proposers is
     // (weight, smaller proposer id) and the push path needs no reverse index.
     bool sym_pairs = false;   // the ranges tile [0, nnz) and every entry has a reverse entry, in any order
+    bool no_self = false;     // the ranges tile [0, nnz) and no list names its own vertex
     bool sym_struct = false;
     bool sym_weights = false;
     int2 *d_ranges = nullptr;

@@ -69,15 +69,16 @@ __global__ void k_reps(const int *match, int n, int *flag, ContractState *st)
 }
 
 // cmap[v] = coarse id of v's representative; mem[c] = the members of c (-1:
-// none), cleared to -1 before.  A third vertex of one value is no matching.
-__global__ void k_members(const int *match, const int *cid, int n, int *cmap, int2 *mem, ContractState *st)
+// none), cleared to -1 before.  A second vertex without entries adds nothing and
+// needs no place; a third one with entries is no matching.
+__global__ void k_members(const int *match, const int2 *ranges, const int *cid, int n, int *cmap, int2 *mem, ContractState *st)
 {
     bool bad = false;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int r = rep_of(match, n, v, bad), c = cid[r];
         cmap[v] = c;
         if (r == v) mem[c].x = v;
-        else if (atomicExch(&mem[c].y, v) != -1) bad = true;
+        else if (degree_of(ranges[v]) > 0 && atomicExch(&mem[c].y, v) != -1) bad = true;
     }
     if (bad) atomicOr(&st->bad, 1);
 }
@@ -564,7 +565,7 @@ mm_status contract(mm_graph *g, const int *d_match, mm_graph **coarse, int *d_cm
         e = sc.sums(flag, cid, nv);
     }
     if (e == cudaSuccess) {
-        k_members<<<gv, 256, 0, st>>>(d_match, cid, n, cmap, mem, cs);
+        k_members<<<gv, 256, 0, st>>>(d_match, g->d_ranges, cid, n, cmap, mem, cs);
         k_lengths<<<gv, 256, 0, st>>>(g->d_ranges, mem, cid, n, len);
         e = sc.sums(len, off, nv);
     }

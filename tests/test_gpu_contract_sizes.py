@@ -84,3 +84,23 @@ def test_checks_of_clean_and_broken_matchings(mm, orc, degrees):
             wt, size = dg.weight(d.data_ptr())
             ow = orc.weight(g, m)
             assert size == ow[1] and wt == pytest.approx(ow[0], rel=1e-12, abs=1e-12), i
+
+
+def test_contract_takes_a_value_with_one_list_beside_its_vertex(mm):
+    """Vertex 4 holds its pair's value too, and has no entries: it joins the pair's
+    coarse vertex and adds nothing.  With entries of its own it is refused."""
+    import torch
+
+    ends = np.array([1, 3, 5, 6, 6])
+    g = SmallGraph(5, np.stack([np.r_[0, ends[:-1]], ends], 1), np.array([1, 0, 2, 1, 3, 2]),
+                   np.array([1, 1, 2, 2, 3, 3], np.float32))
+    cmap = torch.empty(5, dtype=torch.int32, device="cuda")
+    with mm.DeviceGraph(g, device=0) as dg:
+        m = torch.tensor([4, 4, 0, 0, 4], dtype=torch.int32).cuda()
+        with dg.contract(m.data_ptr(), cmap.data_ptr()) as cg:
+            r, nb, w = cg.to_host()
+            assert cmap.tolist() == [0, 0, 1, 2, 0]
+            assert r.tolist() == [[0, 1], [1, 3], [3, 4]] and nb.tolist() == [1, 0, 2, 1] and w.tolist() == [2, 2, 3, 3]
+        m = torch.tensor([4, 4, 4, 0, 0], dtype=torch.int32).cuda()
+        with pytest.raises(mm.MatchError):
+            dg.contract(m.data_ptr())

@@ -7,9 +7,8 @@ duplicates removed, FP32 weights in (0, 1], graph seed 1, colouring seeds from
 srand(12345) as the reference CLI draws them (bin/match.cpp:382), select
 barrier 0x88B81733 (bin/match.cpp:183).
 
-One step = one matching of the whole graph to maximality: the round kernel,
-the finish kernel and (only if the finish phase is called off) the resumed
-round kernel, three launches on one stream.
+One step = one matching of the whole graph to maximality: one cooperative
+launch that plays the rounds and, for the late ones, the finish phase.
 
   value     edges traversed / s with the graph resident in HBM (the reference's
             t1 -> t2 "match time", bin/match.cpp:436-437).  Edges traversed =
@@ -23,8 +22,9 @@ round kernel, three launches on one stream.
             sum_r [24 |A_r| + 8 E_r] (weighted; 4 E_r random), over the step's
             CUDA-event time, against the measured HBM copy bandwidth; traffic =
             DRAM bytes of one matching's launches from an ncu capture recorded
-            in profiles/dram_traffic_<workload>.json.  The design's own byte
-            count of the kernels it runs, and per-round phase times (barrier
+            in profiles/dram_traffic_<workload>.json.  A byte count by phase
+            (16-byte items and 1-byte colours: an upper figure for the kernel's
+            4-byte items and 2-bit colours), and per-round phase times (barrier
             timestamps), are reported beside it.
   cpu_baseline  the reference's own GraphMatchingTBBWeighted (same algorithm,
             src/matchtbb.cu:567-623) compiled from its sources into
@@ -629,8 +629,7 @@ def main():
                     "d2h_bytes_per_step": d2h, "ms_create": e2e_split[0], "ms_first_match": e2e_split[1],
                     "ms_destroy": e2e_split[2], **e2e_detail},
             "roofline": {"bound": "hbm",
-                         "kernel": "one matching: k_rounds then k_finish (a resumed k_rounds only if the finish "
-                                   "phase is called off)",
+                         "kernel": "one matching: k_match",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                          "traffic": traffic, "peak_kind": peak_kind,
                          "bytes_per_step": work["reference_bytes"],

@@ -520,6 +520,10 @@ def roofline_bytes(stats: np.ndarray, weighted: bool) -> dict:
     reference_bytes: the bytes the reference's round loop must move,
         sum_r [24 |A_r| + (4 + 4 w) E_r] with E_r the entries its request and
         respond loops inspect (gathers of match/requests assumed L2-resident).
+    The figures by phase count 16-byte items, 8-byte requests and 1-byte colours:
+    a fixed measure across kernel designs.  The kernel's items are 4 bytes, its
+    requests 4 to 8 in shared memory where they fit, its colours 2 bits, so it
+    moves less.
     window_bytes[r]: the window scan: 32 per blue vertex (worklist item 16,
         reverse key 8, request 8) and per window entry read 8 (weighted:
         neighbour + position) or 4 (random: neighbour).

@@ -22,7 +22,7 @@
 //   * Select (gaSelect, matchgpu.cu:220-258) of round t+1 is fused into the
 //     commit pass of round t: a survivor recolours itself with seed t+1.
 //   * Dead marking (requests == n+1) happens as soon as the blue scan finds no
-//     unmatched neighbour; readers of that colour byte see "unmatched, not red"
+//     unmatched neighbour; readers of its colour see "unmatched, not red"
 //     either way, so their outcome is unchanged.
 //
 // Work layout.  Every vertex belongs to one block for the whole matching: the
@@ -1368,7 +1368,7 @@ __device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &
 //   scan   every item scans its own list: no active neighbour (a singleton),
 //          an active neighbour with a smaller id (a member: another vertex
 //          speaks for its component), or else a root candidate.  It records
-//          its first two active neighbours with their preference keys.  A
+//          its first four active neighbours with their preference keys.  A
 //          singleton walks its own hash sequence at once: it leaves (match
 //          value 2) in the first round it is blue, or keeps red to the cap.
 //   roots  each root candidate's lane follows the records breadth first to

@@ -30,7 +30,9 @@ ROOT = PKG.parent
 TUNED = PKG / "tuned.json"
 FIN_DIVS = (-1, 4, 6, 8, 10, 12, 16, 24)
 BLOCKS = (1, 2)
-DEFAULT = (12, 2)  # the library's defaults (mm_graph_tune value 0)
+# The pair that a choice has to beat.  (The library's own default, mm_graph_tune
+# value 0, is 24 or on sparse graphs 12, with 2 blocks.)
+DEFAULT = (12, 2)
 
 
 def tune(mm, dg, type_, seeds, batch=False, fin_divs=FIN_DIVS, blocks=BLOCKS, repeats=5):
@@ -69,7 +71,7 @@ def tune(mm, dg, type_, seeds, batch=False, fin_divs=FIN_DIVS, blocks=BLOCKS, re
 
 def pick(rows, default=DEFAULT, margin=0.03):
     """The choice for a workload class from tune()'s rows: the fastest pair if it
-    beats the library's default by more than `margin` (a fraction of the
+    beats the default pair by more than `margin` (a fraction of the
     default's time), else the default.  Returns (choice row, default row, tuned?)."""
     dflt = next(r for r in rows if (r["finish_div"], r["blocks_per_sm"]) == tuple(default))
     best = min(rows, key=lambda x: x["ms"])
@@ -135,10 +137,10 @@ def main():
             cells = [f"{next(r['ms'] for r in rows if r['finish_div'] == d and r['blocks_per_sm'] == b):.3f}"
                      for b in BLOCKS]
             lines.append(f"| {d} | " + " | ".join(cells) + " |")
-        lines += ["", f"Default (d = {DEFAULT[0]}, {DEFAULT[1]} blocks per SM): {dflt['ms']:.3f} ms; fastest: "
+        lines += ["", f"Compared with d = {DEFAULT[0]}, {DEFAULT[1]} blocks per SM: {dflt['ms']:.3f} ms; fastest: "
                       f"d = {best['finish_div']}, {best['blocks_per_sm']} blocks per SM, {best['ms']:.3f} ms; "
                       f"chosen: d = {choice['finish_div']}, {choice['blocks_per_sm']} "
-                      f"({'tuned' if wins else 'default kept: the fastest is within 3%'}).", ""]
+                      f"({'tuned' if wins else 'kept: the fastest is within 3%'}).", ""]
         print(name, tuned[name], flush=True)
     TUNED.write_text(json.dumps(tuned, indent=1) + "\n")
     (ROOT / "profiles" / "tuning.md").write_text("\n".join(lines) + "\n")

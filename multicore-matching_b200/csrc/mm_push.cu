@@ -2124,8 +2124,11 @@ __global__ void __launch_bounds__(256) k_scan_ranges(const int2 *ranges, int n, 
     int mx = 0, nc = 0, bad = 0;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int2 r = ranges[v];
-        const int d = degree_of(r), wl = win_len(d);
-        if (d > 0 && (r.x < 0 || (long long)r.y > nnz)) bad = 1;
+        // the ends are compared before their difference is taken: (-1, 2^31 - 1)
+        // has none in 32 bits
+        const bool out = r.y > r.x && (r.x < 0 || (long long)r.y > nnz);
+        if (out) bad = 1;
+        const int d = out ? 0 : degree_of(r), wl = win_len(d);
         sum += (unsigned long long)d;
         mx = max(mx, d);
         if (d > kWin) {

@@ -271,7 +271,7 @@ __global__ void k_validate(const int2 *ranges, const int *nbrs, int n, long long
         const int2 r = ranges[v];
         if (r.y <= r.x || r.x < 0 || (long long)r.y > nnz) continue;
         int local = 0;
-        for (int j = r.x + lane; j < r.y; j += 32) {
+        for (unsigned j = r.x + lane; j < (unsigned)r.y; j += 32) {  // (unsigned: r.y may be 2^31 - 1)
             const int u = nbrs[j];
             local |= (u < 0 || u >= n);
         }

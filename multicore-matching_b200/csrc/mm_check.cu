@@ -228,12 +228,13 @@ __global__ void __launch_bounds__(256) k_pair_long(const int2 *ranges, const int
         const int2 r = ranges[v];
         if (threadIdx.x == 0) s_at = 0x7fffffff;
         __syncthreads();
-        for (int j = r.x; j < r.y; j += 4 * 256) {
+        // unsigned: a list may end at 2^31 - 1, and a step beyond it must not wrap
+        for (unsigned j = r.x; j < (unsigned)r.y; j += 4 * 256) {
             int first = 0x7fffffff;
 #pragma unroll
             for (int k = 3; k >= 0; --k) {
-                const int q = j + k * 256 + (int)threadIdx.x;
-                if (q < r.y && entry_hit<kWeight>(match, v, partner, __ldg(nbrs + q))) first = q;
+                const unsigned q = j + k * 256 + threadIdx.x;
+                if (q < (unsigned)r.y && entry_hit<kWeight>(match, v, partner, __ldg(nbrs + q))) first = (int)q;
             }
             if (first != 0x7fffffff) atomicMin(&s_at, first);
             __syncthreads();

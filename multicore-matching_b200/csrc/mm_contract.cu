@@ -108,7 +108,7 @@ struct Entries {
         da = degree_of(a);
         db = degree_of(b);
     }
-    __device__ __forceinline__ int pos(int i) const { return i < da ? a.x + i : b.x + (i - da); }
+    __device__ __forceinline__ int pos(long long i) const { return (int)(i < da ? a.x + i : b.x + (i - da)); }
     __device__ __forceinline__ long long total() const { return (long long)da + db; }
 };
 
@@ -410,7 +410,7 @@ __global__ void k_long_gather(const int2 *ranges, const int *nbrs, const float *
         const Entries e(ranges, mem[c]);
         const long long total = e.total(), o = loff[i];
         for (long long k = threadIdx.x; k < total; k += blockDim.x) {
-            const int j = e.pos((int)k), cu = cmap[__ldg(nbrs + j)];
+            const int j = e.pos(k), cu = cmap[__ldg(nbrs + j)];
             key[o + k] = cu == c ? INT_MAX : cu;
             val[o + k] = __ldg(w + j);
         }

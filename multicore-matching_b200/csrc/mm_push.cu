@@ -189,6 +189,12 @@ __device__ __forceinline__ int degree_of(int2 r) { return r.y > r.x ? r.y - r.x 
 __device__ __forceinline__ int degree_of(int4 it) { return it.z > it.y ? it.z - it.y : 0; }
 __device__ __forceinline__ int win_len(int deg) { return deg < kWin ? deg : kWin; }
 
+// A scan's position in the entry arrays.  A list may end at 2^31 - 1, where a
+// step of up to kThreads * kRows entries beyond its end would wrap a signed one
+// to a place before it.  (Only for scans of lists that have entries: the ends of
+// an empty range may be anything.)
+typedef unsigned Pos;
+
 template <class P>
 __device__ __forceinline__ void stat_add(const P &p, int round, int col, unsigned long long v)
 {
@@ -855,10 +861,10 @@ __device__ __forceinline__ void retire_red(const Params &p, const Mem<kSolo> &m,
         const int2 r = __ldg(p.ranges + v);
         if (degree_of(r) > kRetireMaxDeg) continue;
         bool gone = true;
-        for (int j0 = r.x; gone && j0 < r.y; j0 += 16) {
+        for (Pos j0 = r.x; gone && j0 < (Pos)r.y; j0 += 16) {  // (the symmetric path has no reversed ranges)
             int nb[16];
 #pragma unroll
-            for (int u = 0; u < 16; ++u) nb[u] = j0 + u < r.y ? __ldg(p.nbrs + j0 + u) : -1;
+            for (int u = 0; u < 16; ++u) nb[u] = j0 + u < (Pos)r.y ? __ldg(p.nbrs + (j0 + u)) : -1;
 #pragma unroll
             for (int u = 0; u < 16; ++u)
                 if (nb[u] >= 0 && m.col(nb[u]) != kMatched) gone = false;
@@ -901,7 +907,7 @@ __device__ __forceinline__ void window_group(const Params &p, int g, int lo, int
         const int v[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            jv[k] = 4 * g + k;
+            jv[k] = (int)(4u * (unsigned)g + k);
             nb[k] = jv[k] >= lo && jv[k] < hi ? v[k] : -1;
         }
     }
@@ -938,7 +944,7 @@ __device__ __forceinline__ void window_place(int2 raw, int &g, int &gend, int &l
         lo = raw.x;
         hi = lo + win_len(deg);
         g = lo >> 2;
-        gend = deg > 0 ? (hi + 3) >> 2 : g;
+        gend = deg > 0 ? (int)(((Pos)hi + 3u) >> 2) : g;
         longer = deg > kWin;
     }
 }
@@ -953,20 +959,20 @@ __device__ __forceinline__ unsigned long long scan_rows(const Params &p, const M
     float bw = -1.0f;
     int bj = 0;
     bool alive = false;
-    for (int j0 = b + first; j0 < e; j0 += step) {
+    for (Pos j0 = (Pos)b + first; j0 < (Pos)e; j0 += step) {
         int nb[kRows];
         float wv[kRows];
 #pragma unroll
         for (int r = 0; r < kRows; ++r) {
-            const int j = j0 + r * 32 + lane;
-            nb[r] = j < e ? __ldg(p.nbrs + j) : -1;
-            wv[r] = kW && j < e ? __ldg(p.w + j) : 0.0f;
+            const Pos j = j0 + r * 32 + lane;
+            nb[r] = j < (Pos)e ? __ldg(p.nbrs + j) : -1;
+            wv[r] = kW && j < (Pos)e ? __ldg(p.w + j) : 0.0f;
         }
         unsigned c[kRows];
 #pragma unroll
         for (int r = 0; r < kRows; ++r) c[r] = nb[r] >= 0 ? m.word(nb[r]) : 0xffffffffu;
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) fold_entry<kW>(colour_bits(c[r], nb[r]), wv[r], j0 + r * 32 + lane, bw, bj, alive);
+        for (int r = 0; r < kRows; ++r) fold_entry<kW>(colour_bits(c[r], nb[r]), wv[r], (int)(j0 + r * 32 + lane), bw, bj, alive);
         if (!kW && __any_sync(kFull, bw > -1.0f)) break;
     }
     return strip_key<kW>(bw, bj, alive);
@@ -1190,7 +1196,7 @@ __device__ __noinline__ void scan_shared(const Params &p, const Mem<kSolo> m, in
     for (int s = (int)(blockIdx.x * kWarps + (threadIdx.x >> 5)); s < npieces; s += (int)(gridDim.x * kWarps)) {
         const int4 it = __ldcg(p.staged + __ldcg(p.piece_item + s));
         const int deg = degree_of(it), pieces = (deg + kPiece - 1) / kPiece;
-        const int b = it.y + (s - it.w) * kPiece, e = min(it.z, b + kPiece), v = it.x;
+        const int b = it.y + (s - it.w) * kPiece, e = b + min(kPiece, it.z - b), v = it.x;
         const unsigned long long key = warp_max_u64(scan_rows<kW>(p, m, b, e, 0, 32 * kRows));
         if (lane != 0) continue;
         count_fallback<kStats>(p, t, e - b);
@@ -1423,10 +1429,10 @@ constexpr int kFinRec = 4;  // active neighbours a record holds
 __device__ __forceinline__ void fin_scan_thread(const Params &p, int v, int b, int e, int &nint, bool &lower,
                                                 int (&jr)[kFinRec], int (&ur)[kFinRec])
 {
-    for (int j0 = b; j0 < e; j0 += 8) {
+    for (Pos j0 = b; j0 < (Pos)e; j0 += 8) {
         int u[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) u[k] = j0 + k < e ? __ldg(p.nbrs + j0 + k) : -1;
+        for (int k = 0; k < 8; ++k) u[k] = j0 + k < (Pos)e ? __ldg(p.nbrs + (j0 + k)) : -1;
         unsigned c[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) c[k] = u[k] >= 0 ? colour_bits(p.col[(unsigned)u[k] >> 4], u[k]) : (unsigned)kMatched;
@@ -1436,7 +1442,7 @@ __device__ __forceinline__ void fin_scan_thread(const Params &p, int v, int b, i
 #pragma unroll
                 for (int q = 0; q < kFinRec; ++q) {
                     if (nint == q) {
-                        jr[q] = j0 + k;
+                        jr[q] = (int)(j0 + k);
                         ur[q] = u[k];
                     }
                 }
@@ -1456,10 +1462,10 @@ __device__ __forceinline__ void fin_scan_warp(const Params &p, int v, int b, int
     const int lane = threadIdx.x & 31;
     int cnt = 0;
     bool lo = false;
-    for (int r0 = b; r0 < e; r0 += 32 * 4) {
+    for (Pos r0 = b; r0 < (Pos)e; r0 += 32 * 4) {
         int u[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) u[k] = r0 + 32 * k + lane < e ? __ldg(p.nbrs + r0 + 32 * k + lane) : -1;
+        for (int k = 0; k < 4; ++k) u[k] = r0 + 32 * k + lane < (Pos)e ? __ldg(p.nbrs + (r0 + 32 * k + lane)) : -1;
         unsigned c[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) c[k] = u[k] >= 0 ? colour_bits(p.col[(unsigned)u[k] >> 4], u[k]) : (unsigned)kMatched;
@@ -1475,7 +1481,7 @@ __device__ __forceinline__ void fin_scan_warp(const Params &p, int v, int b, int
 #pragma unroll
                 for (int q = 0; q < kFinRec; ++q) {
                     if (cnt == q) {
-                        jr[q] = r0 + 32 * k + sb;
+                        jr[q] = (int)(r0 + 32 * k + sb);
                         ur[q] = us;
                     }
                 }
@@ -1511,12 +1517,12 @@ __device__ __forceinline__ int fin_search(const Params &p, FinWarp &fw, int v, i
             fw.eoff[f] = ne;
         }
         seen += (unsigned long long)(e - b);
-        for (int j0 = b; j0 < e; j0 += 32) {
-            const int j = j0 + lane;
+        for (Pos j0 = b; j0 < (Pos)e; j0 += 32) {
+            const Pos j = j0 + lane;
             int u = -1;
             float wj = 0.0f;
             unsigned c = kMatched;
-            if (j < e) {
+            if (j < (Pos)e) {
                 u = __ldg(p.nbrs + j);
                 if (kW) wj = __ldg(p.w + j);  // with the id: no dependent load once the colour is known
                 c = colour_bits(p.col[(unsigned)u >> 4], u);
@@ -1525,7 +1531,7 @@ __device__ __forceinline__ int fin_search(const Params &p, FinWarp &fw, int v, i
             if (__any_sync(kFull, in && u < v)) return kFinNotRoot;
             unsigned m = __ballot_sync(kFull, in);
             unsigned long long pref = 0;
-            if (in) pref = fin_key<kW>(p.sym ? u : j, wj);
+            if (in) pref = fin_key<kW>(p.sym ? u : (int)j, wj);
             while (m) {
                 const int s = __ffs(m) - 1;
                 m &= m - 1;
@@ -2176,10 +2182,10 @@ __global__ void k_pair_items(const int2 *ranges, const int *nbrs, int n, int bit
     for (long long v = warp0; v < n; v += nwarps) {
         const int2 r = ranges[v];
         const long long s0 = contiguous ? (long long)r.x : slot_off[v];
-        for (int j = r.x + lane; j < r.y; j += 32) {
-            const unsigned long long a = (unsigned long long)v, b = (unsigned long long)nbrs[j];
+        for (Pos i = lane; i < (Pos)degree_of(r); i += 32) {
+            const unsigned long long a = (unsigned long long)v, b = (unsigned long long)nbrs[r.x + i];
             const unsigned long long lo = a < b ? a : b, hi = a < b ? b : a;
-            const long long slot = s0 + (j - r.x);
+            const long long slot = s0 + i;
             keys[slot] = (((lo << bits) | hi) << 1) | (a > b ? 1ull : 0ull);
             vals[slot] = (int)slot;
         }
@@ -2284,24 +2290,24 @@ constexpr int kWinChunk = 4096;   // lists longer than this are split into chunk
 
 // Merge entries [from, to) of a list into its sorted best 32 (k, nb, j): a row
 // can change them only if one of its keys beats the 32nd.
-__device__ __forceinline__ void win_merge_range(const int *nbrs, const float *w, int from, int to, int lane,
+__device__ __forceinline__ void win_merge_range(const int *nbrs, const float *w, Pos from, Pos to, int lane,
                                                 unsigned long long &k, int &nb, int &j)
 {
-    for (int base = from; base < to; base += 32 * kWinRows) {
+    for (Pos base = from; base < to; base += 32 * kWinRows) {
         float wr[kWinRows];
 #pragma unroll
         for (int q = 0; q < kWinRows; ++q) {
-            const int jj = base + q * 32 + lane;
+            const Pos jj = base + q * 32 + lane;
             wr[q] = jj < to ? __ldg(w + jj) : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < kWinRows; ++q) {
-            const int jj = base + q * 32 + lane;
+            const Pos jj = base + q * 32 + lane;
             if (base + q * 32 >= to) break;
             const unsigned long long thr = __shfl_sync(kFull, k, 31);
-            unsigned long long k2 = jj < to ? pref_key(wr[q], jj) : 0ull;
+            unsigned long long k2 = jj < to ? pref_key(wr[q], (int)jj) : 0ull;
             if (!__any_sync(kFull, k2 > thr)) continue;
-            int nb2 = jj < to ? __ldg(nbrs + jj) : 0, j2 = jj;
+            int nb2 = jj < to ? __ldg(nbrs + jj) : 0, j2 = (int)jj;
             warp_sort_desc(k2, nb2, j2, lane);
             // the larger of T[l] and R[31 - l] is a bitonic sequence holding
             // the best 32 of both; sort it descending
@@ -2325,13 +2331,13 @@ __device__ __forceinline__ void win_top32(const int *nbrs, const float *w, int f
     k = 0ull;
     nb = 0;
     j = 0;
-    if (from + lane < to) {
+    if (lane < to - from) {
         j = from + lane;
         nb = __ldg(nbrs + j);
         k = pref_key(__ldg(w + j), j);
     }
     warp_sort_desc(k, nb, j, lane);
-    if (to - from > 32) win_merge_range(nbrs, w, from + 32, to, lane, k, nb, j);
+    if (to - from > 32) win_merge_range(nbrs, w, (Pos)from + 32, (Pos)to, lane, k, nb, j);
 }
 
 __device__ __forceinline__ void win_store(int2 *pwin, long long off, int deg, int lane, unsigned long long k, int nb, int j)
@@ -2390,7 +2396,7 @@ __global__ void __launch_bounds__(256) k_win_chunks(const int2 *ranges, const in
         }
         const int2 r = ranges[big[lo]];
         const int from = r.x + (int)(c - chunk_off[lo]) * kWinChunk;
-        const int to = min(from + kWinChunk, r.y);
+        const int to = from + min(kWinChunk, r.y - from);
         unsigned long long k;
         int nb, j;
         win_top32(nbrs, w, from, to, lane, k, nb, j);
@@ -2572,8 +2578,8 @@ __global__ void k_wfeat(const int2 *ranges, const float *w, int n, float2 *wfeat
         const int2 r = ranges[v];
         float mx = 0.0f, sum = 0.0f;
         int cnt = 0;
-        for (int j = r.x + lane; j < r.y; j += 32) {
-            const float x = __ldg(w + j);
+        for (Pos i = lane; i < (Pos)degree_of(r); i += 32) {
+            const float x = __ldg(w + r.x + i);
             if (x > -1.0f) {
                 mx = cnt ? fmaxf(mx, x) : x;
                 sum += x;

@@ -41,13 +41,14 @@ struct PairState {
     unsigned long long size;       // as mm_matching_weight's
     unsigned long long size_general;  // the same by the general kernel
     double weight;
-    int broken;                    // a value that names no vertex, one that does not hold it, or one of two that do
+    int broken;                    // a value that names no vertex, or one that does not hold it (k_pairs)
+    int clash;                     // a vertex that is not the only other one with its value (k_pair_lists)
     int nlong;                     // lists left to the block scans
 };
 
 // other[a]: 1 + the partner of the vertex a that a value names (0: none).  The matching is
 // clean iff nothing is broken, nmin == nother and every other vertex is the
-// only one to claim its named vertex (which holds the value too).
+// only one to claim its named vertex (which holds the value too; no clash).
 __global__ void k_pairs(const int *match, int n, int *other, PairState *st)
 {
     int nmin = 0, nother = 0, broken = 0;
@@ -69,7 +70,12 @@ __global__ void k_pairs(const int *match, int n, int *other, PairState *st)
     if (__any_sync(0xffffffffu, broken) && (threadIdx.x & 31) == 0) atomicOr(&st->broken, 1);
 }
 
-__device__ __forceinline__ bool clean(const PairState *st) { return !st->broken && st->nmin == st->nother; }
+// What k_pairs found.  The list pass looks at nothing else before it starts: a
+// word that its own blocks write would let warps of one block part ways ahead of
+// the block's barriers.
+__host__ __device__ __forceinline__ bool paired(const PairState *st) { return !st->broken && st->nmin == st->nother; }
+// The matching is clean (after the list pass).
+__host__ __device__ __forceinline__ bool clean(const PairState *st) { return paired(st) && !st->clash; }
 
 // Whether an entry naming u is what a pass looks for at vertex v:
 //   partner >= 0  the partner (kSelf: or the vertex itself, whose match value
@@ -133,7 +139,7 @@ __global__ void __launch_bounds__(256, kPairBlocks) k_pair_lists(const int2 *ran
                                                     int n, const int *other, int *bad, int *queue, double *contrib,
                                                     PairState *st)
 {
-    if (!clean(st)) return;
+    if (!paired(st)) return;
     __shared__ uint8_t s_from[8][32];
     constexpr int kGroups = 32 / G;
     const int lane = threadIdx.x & 31, l = lane & (G - 1);
@@ -141,7 +147,7 @@ __global__ void __launch_bounds__(256, kPairBlocks) k_pair_lists(const int2 *ran
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long stride = ((long long)gridDim.x * blockDim.x >> 5) * 32;
     unsigned cnt[3] = {0u, 0u, 0u};
-    bool broken = false;
+    bool clash = false;
     for (long long base = warp * 32; base < n; base += stride) {  // warp-uniform
         const bool in = base + lane < n;
         const int v = in ? (int)base + lane : -1, mv = in ? match[v] : 0;
@@ -149,7 +155,7 @@ __global__ void __launch_bounds__(256, kPairBlocks) k_pair_lists(const int2 *ran
         const bool matched = is_matched(mv);
         const int a = mv - 4, o = matched ? other[a] : 0;
         const int partner = !matched ? -1 : (a == v ? o - 1 : a);
-        broken |= matched && a != v && o != v + 1;
+        clash |= matched && a != v && o != v + 1;
         if (kWeight && in && !matched) contrib[v] = 0.0;
         bool want = in && (matched ? !kHalf || a == v : !kWeight);
         if (want && r.y > r.x && r.y - r.x > kPairList) {
@@ -205,7 +211,7 @@ __global__ void __launch_bounds__(256, kPairBlocks) k_pair_lists(const int2 *ran
                 if (mine[q] && l == 0) pair_result<kWeight, kHalf>(w, vs[q], ps[q], at[q], contrib, cnt, bad);
         }
     }
-    if (__any_sync(0xffffffffu, broken) && lane == 0) atomicOr(&st->broken, 1);
+    if (__any_sync(0xffffffffu, clash) && lane == 0) atomicOr(&st->clash, 1);
     if (kWeight) {
         block_add(&st->size, cnt[0]);
     } else {
@@ -488,7 +494,7 @@ MM_API mm_status mm_matching_weight(mm_graph *g, const int *d_match, double *wei
     dev_free(ps, st);
     if (e != cudaSuccess) return cuda_fail(e, "mm_matching_weight");
     *weight = h.weight / 2.0;  // every matched edge is counted from both ends
-    *size = (long long)(!h.broken && h.nmin == h.nother ? h.size : h.size_general);
+    *size = (long long)(clean(&h) ? h.size : h.size_general);
     return MM_OK;
 }
 
@@ -514,7 +520,7 @@ MM_API mm_status mm_matching_check(mm_graph *g, const int *d_match, long long *c
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
         dev_free(ps, st);
         if (e != cudaSuccess) return cuda_fail(e, "mm_matching_check");
-        if (!h.broken && h.nmin == h.nother) {
+        if (clean(&h)) {
             for (int k = 2; k < 5; ++k) counts[k] = (long long)h.counts[k];
             *valid = counts[2] == 0 ? 1 : 0;
             return MM_OK;

@@ -189,10 +189,11 @@ __device__ __forceinline__ int degree_of(int2 r) { return r.y > r.x ? r.y - r.x 
 __device__ __forceinline__ int degree_of(int4 it) { return it.z > it.y ? it.z - it.y : 0; }
 __device__ __forceinline__ int win_len(int deg) { return deg < kWin ? deg : kWin; }
 
-// A scan's position in the entry arrays.  A list may end at 2^31 - 1, where a
-// step of up to kThreads * kRows entries beyond its end would wrap a signed one
-// to a place before it.  (Only for scans of lists that have entries: the ends of
-// an empty range may be anything.)
+// Positions in scans.  A list may end at 2^31 - 1, where a step of up to kThreads
+// * kRows entries beyond its end would wrap a signed position to a place before
+// the list.  So a scan counts down what is left of its list, or a position that
+// may lie beyond the end is unsigned (Pos; not for empty ranges, whose ends may
+// be anything).
 typedef unsigned Pos;
 
 template <class P>
@@ -861,7 +862,7 @@ __device__ __forceinline__ void retire_red(const Params &p, const Mem<kSolo> &m,
         const int2 r = __ldg(p.ranges + v);
         if (degree_of(r) > kRetireMaxDeg) continue;
         bool gone = true;
-        for (Pos j0 = r.x; gone && j0 < (Pos)r.y; j0 += 16) {  // (the symmetric path has no reversed ranges)
+        for (Pos j0 = r.x; gone && j0 < (Pos)r.y; j0 += 16) {  // (no reversed ranges on the symmetric path)
             int nb[16];
 #pragma unroll
             for (int u = 0; u < 16; ++u) nb[u] = j0 + u < (Pos)r.y ? __ldg(p.nbrs + (j0 + u)) : -1;
@@ -959,20 +960,23 @@ __device__ __forceinline__ unsigned long long scan_rows(const Params &p, const M
     float bw = -1.0f;
     int bj = 0;
     bool alive = false;
-    for (Pos j0 = (Pos)b + first; j0 < (Pos)e; j0 += step) {
+    Pos j0 = (Pos)b + first + lane;
+    const int *a = p.nbrs + b + first + lane;
+    const float *wa = p.w + b + first + lane;
+    for (int left = e - b - first; left > 0; left -= step, a += step, wa += step, j0 += step) {
         int nb[kRows];
         float wv[kRows];
 #pragma unroll
         for (int r = 0; r < kRows; ++r) {
-            const Pos j = j0 + r * 32 + lane;
-            nb[r] = j < (Pos)e ? __ldg(p.nbrs + j) : -1;
-            wv[r] = kW && j < (Pos)e ? __ldg(p.w + j) : 0.0f;
+            const bool in = r * 32 + lane < left;
+            nb[r] = in ? __ldg(a + r * 32) : -1;
+            wv[r] = kW && in ? __ldg(wa + r * 32) : 0.0f;
         }
         unsigned c[kRows];
 #pragma unroll
         for (int r = 0; r < kRows; ++r) c[r] = nb[r] >= 0 ? m.word(nb[r]) : 0xffffffffu;
 #pragma unroll
-        for (int r = 0; r < kRows; ++r) fold_entry<kW>(colour_bits(c[r], nb[r]), wv[r], (int)(j0 + r * 32 + lane), bw, bj, alive);
+        for (int r = 0; r < kRows; ++r) fold_entry<kW>(colour_bits(c[r], nb[r]), wv[r], (int)(j0 + r * 32), bw, bj, alive);
         if (!kW && __any_sync(kFull, bw > -1.0f)) break;
     }
     return strip_key<kW>(bw, bj, alive);
@@ -1429,10 +1433,11 @@ constexpr int kFinRec = 4;  // active neighbours a record holds
 __device__ __forceinline__ void fin_scan_thread(const Params &p, int v, int b, int e, int &nint, bool &lower,
                                                 int (&jr)[kFinRec], int (&ur)[kFinRec])
 {
-    for (Pos j0 = b; j0 < (Pos)e; j0 += 8) {
+    // (with an unsigned position for the count the kernel spilled: R-MAT 2^23 821 us for 793)
+    for (int left = e - b; left > 0; left -= 8) {
         int u[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) u[k] = j0 + k < (Pos)e ? __ldg(p.nbrs + (j0 + k)) : -1;
+        for (int k = 0; k < 8; ++k) u[k] = k < left ? __ldg(p.nbrs + (e - left + k)) : -1;
         unsigned c[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) c[k] = u[k] >= 0 ? colour_bits(p.col[(unsigned)u[k] >> 4], u[k]) : (unsigned)kMatched;
@@ -1442,7 +1447,7 @@ __device__ __forceinline__ void fin_scan_thread(const Params &p, int v, int b, i
 #pragma unroll
                 for (int q = 0; q < kFinRec; ++q) {
                     if (nint == q) {
-                        jr[q] = (int)(j0 + k);
+                        jr[q] = e - left + k;
                         ur[q] = u[k];
                     }
                 }

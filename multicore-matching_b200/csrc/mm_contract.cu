@@ -543,7 +543,7 @@ mm_status contract(mm_graph *g, const int *d_match, mm_graph **coarse, int *d_cm
     cudaStream_t st = 0;
     Scratch sc(st);
     ContractState *cs = nullptr, h = {};
-    int *flag = nullptr, *cid = nullptr, *cmap = d_cmap, *cnt = nullptr, *q = nullptr;
+    int *flag = nullptr, *cid = nullptr, *cmap = nullptr, *cnt = nullptr, *q = nullptr;
     int2 *mem = nullptr;
     long long *len = nullptr, *off = nullptr, *roff = nullptr;
     const size_t nv = (size_t)n + 1;
@@ -556,7 +556,9 @@ mm_status contract(mm_graph *g, const int *d_match, mm_graph **coarse, int *d_cm
     if (e == cudaSuccess) e = sc.get(&roff, nv);
     if (e == cudaSuccess) e = sc.get(&cnt, nv);
     if (e == cudaSuccess) e = sc.get(&q, 3 * nv);
-    if (e == cudaSuccess && !cmap) e = sc.get(&cmap, nv);
+    // the caller's map is written last: it may be the match array itself, and a
+    // refused call leaves it as it is (4 bytes a vertex copied: 2 us at 2^20)
+    if (e == cudaSuccess) e = sc.get(&cmap, nv);
     if (e == cudaSuccess) e = cudaMemsetAsync(cs, 0, sizeof(ContractState), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(mem, 0xff, sizeof(int2) * nv, st);
     const int gv = grid_for(n + 1ll, 256, 148 * 64);  // a vertex a thread: the passes are chains of gathers
@@ -661,6 +663,8 @@ mm_status contract(mm_graph *g, const int *d_match, mm_graph **coarse, int *d_cm
         k_emit<<<grid_for(nc * 8ll, 256, 148 * 8), 256, 0, st>>>(tkey, tw, off, cnt, roff, nc, cranges, out_nbr, out_w, cs);
         e = cudaGetLastError();
     }
+    if (e == cudaSuccess && d_cmap && n > 0)
+        e = cudaMemcpyAsync(d_cmap, cmap, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = read_back(&h, cs, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "mm_graph_contract");

@@ -155,7 +155,7 @@ __device__ __forceinline__ void merge_group(const long long *off, int c, K key, 
     wt = __shfl_sync(kAll, wt, in ? (int)(key & 31) : lane);
     const K before = __shfl_up_sync(kAll, nb, 1);
     const bool head = in && (l == 0 || before != nb);
-    double sum = (double)wt;
+    double sum = 0.0 + (double)wt;  // as every way sums: from 0, so a -0 alone becomes 0
     for (int d = 1; d < S; ++d) {
         const K other = __shfl_down_sync(kAll, nb, d);  // (a dropped entry's differs from every id)
         const float x = __shfl_down_sync(kAll, wt, d);
@@ -232,7 +232,7 @@ __device__ __forceinline__ void sort_pairs(const int2 *ranges, const int *nbrs, 
     const K n0 = k0 >> 6, n1 = k1 >> 6;
     const K before0 = __shfl_up_sync(kAll, n0, 1), before1 = __shfl_up_sync(kAll, n1, 1), last0 = __shfl_sync(kAll, n0, 31);
     const bool h0 = in0 && (lane == 0 || before0 != n0), h1 = in1 && (lane == 0 ? last0 : before1) != n1;
-    double s0 = in0 ? (double)wt[(int)(k0 & 63)] : 0.0, s1 = in1 ? (double)wt[(int)(k1 & 63)] : 0.0;
+    double s0 = 0.0 + (in0 ? (double)wt[(int)(k0 & 63)] : 0.0), s1 = 0.0 + (in1 ? (double)wt[(int)(k1 & 63)] : 0.0);
     for (int d = 1; d < 64; ++d) {  // runs, in order
         const int q0 = lane + d, q1 = lane + 32 + d;
         const K a0 = __shfl_sync(kAll, k0, q0 & 31), a1 = __shfl_sync(kAll, k1, q0 & 31);

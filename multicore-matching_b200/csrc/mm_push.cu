@@ -3423,16 +3423,20 @@ mm_status push_match_policy(mm_graph *g, int type, uint32_t barrier, const uint3
     if (g->n == 0) return push_match(g, type, barrier, seeds, nseeds, d_match, rounds_out, nullptr, 0, stream);
     Call c{g, nullptr, type, barrier, seeds, nseeds, d_match, false, false, nullptr, stream};
     mm_status st = begin_call(c);
-    if (st != MM_OK) return st;
+    if (st != MM_OK) return call_failed(c, st);
     PushState *s = c.s;
     if (!s->wfeat) {
-        cudaError_t e = dev_alloc((void **)&s->wfeat, sizeof(float2) * (size_t)g->n, stream);
+        float2 *wfeat = nullptr;
+        cudaError_t e = dev_alloc((void **)&wfeat, sizeof(float2) * (size_t)g->n, stream);
         if (e == cudaSuccess) {
-            k_wfeat<<<grid_for((long long)g->n * 32, 256, 148 * 16), 256, 0, stream>>>(g->d_ranges, g->d_w, g->n,
-                                                                                    s->wfeat);
+            k_wfeat<<<grid_for((long long)g->n * 32, 256, 148 * 16), 256, 0, stream>>>(g->d_ranges, g->d_w, g->n, wfeat);
             e = cudaGetLastError();
         }
-        if (e != cudaSuccess) return cuda_fail(e, "policy state");
+        if (e != cudaSuccess) {  // the state's arrays may still be being cleared on this stream
+            dev_free(wfeat, stream);
+            return call_failed(c, cuda_fail(e, "policy state"));
+        }
+        s->wfeat = wfeat;
     }
     PolicyArgs pol;
     pol.mlp = mlp_host;

@@ -469,7 +469,7 @@ cudaError_t upload_large(mm_graph *g, const int *ranges, const int *nbrs, const 
         // Weighted graphs get their preference windows here: a chunk's check is
         // followed by the windows of the vertices whose lists end in it (host
         // ranges say which).
-        bool windows = contiguous && w && windows_begin(g, ks) == MM_OK;
+        bool windows = contiguous && w && windows_begin(g, ks, 0) == MM_OK;
         int va = 0;  // first vertex whose window is not built yet
         for (int k = 0; e == cudaSuccess && k < nchunks; ++k) {
             if (copied < nchunks) {
@@ -493,7 +493,7 @@ cudaError_t upload_large(mm_graph *g, const int *ranges, const int *nbrs, const 
                 va = vb;
             }
         }
-        if (e == cudaSuccess && windows && windows_end(g, ks) != MM_OK) windows = false;
+        if (e == cudaSuccess && windows && windows_end(g, ks, 0) != MM_OK) windows = false;
         if (e == cudaSuccess && !contiguous && n > 0) {
             e = cudaStreamWaitEvent(ks, l->ev[nchunks], 0);
             if (e == cudaSuccess) e = check_any(g, d_c, ks);

@@ -3215,45 +3215,52 @@ void apply_ranges(mm_graph *g, const RangeInfo &info)
 // allocates them (it needs only the ranges), windows_range builds those of
 // vertices [va, vb) and queues lists longer than kWinChunk, windows_end builds
 // the queued lists and publishes d_pwin.
-mm_status windows_begin(mm_graph *g, cudaStream_t stream)
+// Memory comes from and goes back to `mem`: the upload builds on a stream of its
+// own and passes the legacy one, as for every other array of a graph.  (Blocks
+// that came from two streams were found free or not as the moment had it, and
+// the pool then remapped what it had to make room, inside a later call: first
+// matchings of R-MAT 2^23 of 9 to 83 ms, for 8.9.)
+mm_status windows_begin(mm_graph *g, cudaStream_t stream, cudaStream_t mem)
 {
     const int n = g->n;
     if (g->win_even >= (1ll << 31)) {
         set_error("push: more than 2^31 - 1 preference-window slots are not supported");
         return MM_ERR_UNSUPPORTED;
     }
-    long long *groups = nullptr, *off = nullptr;
     int2 *win = nullptr;
     int *big = nullptr;  // [n + 1]: queued long lists, then their count
     int *packed = nullptr;
     void *tmp = nullptr;
-    size_t tmp_bytes = 0;
     const size_t nv = (size_t)n + 1;
-    cudaError_t e = dev_alloc((void **)&groups, 2 * sizeof(long long) * nv, stream);
-    off = groups + nv;
-    if (e == cudaSuccess) e = dev_alloc((void **)&packed, sizeof(int) * nv, stream);
+    size_t tmp_bytes = 0;
+    cudaError_t e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (long long *)nullptr, (long long *)nullptr, n + 1, stream);
+    // the groups of every window, their sums and the scan's own memory, at once
+    const size_t sums = 2 * sizeof(long long) * nv, all = (sums + 255) / 256 * 256 + tmp_bytes;
+    if (e == cudaSuccess) e = dev_alloc((void **)&packed, sizeof(int) * nv, mem);
     if (e == cudaSuccess)
-        e = dev_alloc((void **)&win, 4 * sizeof(int2) * (size_t)(g->win_groups > 0 ? g->win_groups : 1), stream);
-    if (e == cudaSuccess) e = dev_alloc((void **)&big, sizeof(int) * nv, stream);
+        e = dev_alloc((void **)&win, 4 * sizeof(int2) * (size_t)(g->win_groups > 0 ? g->win_groups : 1), mem);
+    if (e == cudaSuccess) e = dev_alloc((void **)&big, sizeof(int) * nv, mem);
+    if (e == cudaSuccess) e = dev_alloc(&tmp, all, mem);
+    if (e == cudaSuccess && mem != stream) e = cudaStreamSynchronize(mem);
+    long long *groups = (long long *)tmp, *off = groups + nv;
     if (e == cudaSuccess) e = cudaMemsetAsync(big + n, 0, sizeof(int), stream);
     if (e == cudaSuccess) {
         k_win_sizes<<<grid_for(n + 1ll, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, n, groups);
-        e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, groups, off, n + 1, stream);
+        e = cub::DeviceScan::ExclusiveSum((char *)tmp + (all - tmp_bytes), tmp_bytes, groups, off, n + 1, stream);
     }
-    if (e == cudaSuccess) e = dev_alloc(&tmp, tmp_bytes, stream);
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, groups, off, n + 1, stream);
     if (e == cudaSuccess) {
         k_win_offsets<<<grid_for(n + 1ll, 256, 148 * 8), 256, 0, stream>>>(g->d_ranges, off, n, packed);
         e = cudaGetLastError();
     }
-    dev_free(tmp, stream);
-    dev_free(groups, stream);
     if (e != cudaSuccess) {
-        dev_free(win, stream);
-        dev_free(big, stream);
-        dev_free(packed, stream);
+        if (mem != stream) cudaStreamSynchronize(stream);
+        dev_free(tmp, mem);
+        dev_free(win, mem);
+        dev_free(big, mem);
+        dev_free(packed, mem);
         return cuda_fail(e, "window buffers");
     }
+    g->win_tmp = tmp;  // freed by windows_end
     g->win_build = win;
     g->win_big = big;
     g->d_pwin_off = packed;
@@ -3269,7 +3276,7 @@ mm_status windows_range(mm_graph *g, int va, int vb, cudaStream_t stream)
     return MM_OK;
 }
 
-mm_status windows_end(mm_graph *g, cudaStream_t stream)
+mm_status windows_end(mm_graph *g, cudaStream_t stream, cudaStream_t mem)
 {
     const int n = g->n;
     int *big = g->win_big;
@@ -3281,26 +3288,28 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream)
         e = cudaMemcpyAsync(&nbig, big + n, sizeof(int), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     }
+    WinCand *cand = nullptr;
+    void *tmp = nullptr;
     if (e == cudaSuccess && nbig > 0) {
-        long long *coff = nullptr, *ccnt = nullptr;
-        WinCand *cand = nullptr;
-        void *tmp2 = nullptr;
-        size_t tmp2_bytes = 0;
+        const size_t nb = (size_t)nbig + 1;
+        size_t tmp_bytes = 0;
         long long nchunks = 0;
-        e = dev_alloc((void **)&coff, sizeof(long long) * ((size_t)nbig + 1), stream);
-        if (e == cudaSuccess) e = dev_alloc((void **)&ccnt, sizeof(long long) * ((size_t)nbig + 1), stream);
+        e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (long long *)nullptr, (long long *)nullptr, nbig + 1, stream);
+        const size_t all = (2 * sizeof(long long) * nb + 255) / 256 * 256 + tmp_bytes;
+        if (e == cudaSuccess) e = dev_alloc(&tmp, all, mem);
+        if (e == cudaSuccess && mem != stream) e = cudaStreamSynchronize(mem);
+        long long *ccnt = (long long *)tmp, *coff = ccnt + nb;
         if (e == cudaSuccess) e = cudaMemsetAsync(ccnt + nbig, 0, sizeof(long long), stream);
         if (e == cudaSuccess) {
             k_win_chunk_counts<<<grid_for(nbig, 256, 148 * 4), 256, 0, stream>>>(g->d_ranges, big, nbig, ccnt);
             e = cudaGetLastError();
         }
-        if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, tmp2_bytes, ccnt, coff, nbig + 1, stream);
-        if (e == cudaSuccess) e = dev_alloc(&tmp2, tmp2_bytes, stream);
-        if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(tmp2, tmp2_bytes, ccnt, coff, nbig + 1, stream);
+        if (e == cudaSuccess)
+            e = cub::DeviceScan::ExclusiveSum((char *)tmp + (all - tmp_bytes), tmp_bytes, ccnt, coff, nbig + 1, stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&nchunks, coff + nbig, sizeof nchunks, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        dev_free(tmp2, stream);
-        if (e == cudaSuccess) e = dev_alloc((void **)&cand, sizeof(WinCand) * 32 * (size_t)(nchunks > 0 ? nchunks : 1), stream);
+        if (e == cudaSuccess) e = dev_alloc((void **)&cand, sizeof(WinCand) * 32 * (size_t)(nchunks > 0 ? nchunks : 1), mem);
+        if (e == cudaSuccess && mem != stream) e = cudaStreamSynchronize(mem);
         if (e == cudaSuccess) {
             k_win_chunks<<<grid_for(nchunks * 32, 256, 148 * 16), 256, 0, stream>>>(g->d_ranges, g->d_nbrs, g->d_w, big,
                                                                                   nbig, coff, cand);
@@ -3311,12 +3320,16 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream)
                 g->d_ranges, big, nbig, coff, cand, off, win);
             e = cudaGetLastError();
         }
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        dev_free(cand, stream);
-        dev_free(ccnt, stream);
-        dev_free(coff, stream);
     }
-    dev_free(big, stream);
+    if (mem != stream) {
+        const cudaError_t x = cudaStreamSynchronize(stream);
+        if (e == cudaSuccess) e = x;
+    }
+    dev_free(cand, mem);
+    dev_free(tmp, mem);
+    dev_free(g->win_tmp, mem);
+    dev_free(big, mem);
+    g->win_tmp = nullptr;
     g->win_big = nullptr;
     if (e != cudaSuccess) {
         windows_discard(g);
@@ -3355,8 +3368,10 @@ __global__ void __launch_bounds__(256) k_win_weights(const float *w, const int *
 
 void windows_discard(mm_graph *g)
 {
+    dev_free(g->win_tmp, 0);
     dev_free(g->win_build, 0);
     dev_free(g->win_big, 0);
+    g->win_tmp = nullptr;
     if (!g->d_pwin) {
         dev_free(g->d_pwin_off, 0);
         g->d_pwin_off = nullptr;
@@ -3369,9 +3384,9 @@ namespace {
 
 mm_status build_windows(mm_graph *g, cudaStream_t stream)
 {
-    mm_status st = windows_begin(g, stream);
+    mm_status st = windows_begin(g, stream, stream);
     if (st == MM_OK) st = windows_range(g, 0, g->n, stream);
-    if (st == MM_OK) st = windows_end(g, stream);
+    if (st == MM_OK) st = windows_end(g, stream, stream);
     return st;
 }
 

@@ -174,9 +174,11 @@ mm_status mm_match_drawn(mm_graph *g, int type, uint32_t barrier, uint32_t (*dra
  *                          component) starts at the first round whose active set
  *                          is at most 1/value of round 0's; default 24 (12 on
  *                          graphs of at most 6 entries a vertex, except for
- *                          mm_match_policy), at least 2, -1 never
+ *                          mm_match_policy; the average degree on graphs with 384
+ *                          or more entries a vertex in lists longer than 32), at
+ *                          least 2, -1 never
  *   MM_TUNE_BLOCKS_PER_SM  blocks of 512 threads per multiprocessor, at most;
- *                          default all that fit (2)
+ *                          default all that fit (2) and the graph has work for
  */
 enum { MM_TUNE_FINISH_DIV = 1, MM_TUNE_BLOCKS_PER_SM = 2 };
 mm_status mm_graph_tune(mm_graph *g, int key, int value);

@@ -63,6 +63,8 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
+#include <algorithm>
+#include <climits>
 #include <cstddef>
 #include <cmath>
 #include <cstring>
@@ -109,6 +111,7 @@ struct Params {
     int contiguous;
     int sym;                        // proposal keys computed from the proposer's entry (no reverse index)
     int region;                     // list slots of a block
+    int share_from;                 // fallback lists of a block from which it leaves them to all blocks
     uint32_t turn_magic;            // floor(2^32 / blocks) + 1
     const int2 *ranges;
     const int *nbrs;
@@ -365,8 +368,9 @@ struct Smem {
 static_assert(sizeof(Smem) <= 31 * 1024, "two blocks a multiprocessor in the 64 KB configuration");
 constexpr size_t kSmemBytes = (sizeof(Smem) + 127) / 128 * 128;
 
-// Graphs of at most this many vertices are matched by one block: its rounds
-// need no grid barrier, and its working arrays follow in its shared memory.
+// Graphs of at most this many vertices are matched by one block (unless their
+// long lists are many, launch_match): its rounds need no grid barrier, and its
+// working arrays follow in its shared memory.
 constexpr int kSoloVertices = 4096;
 struct SoloMem {
     unsigned long long best[kSoloVertices];
@@ -879,16 +883,23 @@ __device__ __forceinline__ void retire_red(const Params &p, const Mem<kSolo> &m,
     }
 }
 
-// Append blue vertex v (list r) to the round's shared fallback list: one
-// 64-bit atomic hands out the item and its pieces.
-__device__ __forceinline__ void stage_shared(const Params &p, Smem &sm, int v, const ItemReq &rq, int2 r)
+// Blue vertex v (list r) as item idx of the round's shared fallback list, its
+// pieces from `first` on.
+__device__ __forceinline__ int pieces_of(int deg) { return (deg + kPiece - 1) / kPiece; }
+__device__ __forceinline__ void put_shared(const Params &p, int v, const ItemReq &rq, int2 r, int idx, int first, int pieces)
 {
-    const int pieces = (degree_of(r) + kPiece - 1) / kPiece;
-    const unsigned long long old = atomicAdd(&p.ctl->staged_pack, (1ull << 32) | (unsigned long long)(unsigned)pieces);
-    const int idx = (int)(old >> 32), first = (int)(old & 0xffffffffull);
     p.staged[idx] = make_int4(v, r.x, r.y, first);
     for (int s = 0; s < pieces; ++s) p.piece_item[first + s] = idx;
     rq.put(kReqShared, 0u);  // it proposes through req[v]
+}
+
+// Append blue vertex v to the shared list: one 64-bit atomic hands out the item
+// and its pieces.
+__device__ __forceinline__ void stage_shared(const Params &p, Smem &sm, int v, const ItemReq &rq, int2 r)
+{
+    const int pieces = pieces_of(degree_of(r));
+    const unsigned long long old = atomicAdd(&p.ctl->staged_pack, (1ull << 32) | (unsigned long long)(unsigned)pieces);
+    put_shared(p, v, rq, r, (int)(old >> 32), (int)(unsigned)old, pieces);
     sm.flag = 1;
 }
 
@@ -1009,11 +1020,40 @@ __device__ __forceinline__ void count_fallback(const Params &p, int t, int deg)
 constexpr int kWarpList = 512;
 constexpr int kBlockList = 32768;
 
+// All the block's fallback lists to the round's shared list, an atomic a warp.
+__device__ __forceinline__ void share_all(const Params &p, Smem &sm, int ns, long long rbase)
+{
+    const int lane = threadIdx.x & 31;
+    for (int i0 = (int)threadIdx.x - lane; i0 < ns; i0 += kThreads) {
+        const bool in = i0 + lane < ns;
+        const int2 it = in ? sm.fb.item[i0 + lane] : make_int2(0, 0);
+        const int2 r = in ? __ldg(p.ranges + it.x) : make_int2(0, 0);
+        const int pieces = in ? pieces_of(degree_of(r)) : 0;
+        int upto = pieces;  // inclusive sum in lane order
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(kFull, upto, o);
+            if (lane >= o) upto += y;
+        }
+        const int count = min(32, ns - i0), all = __shfl_sync(kFull, upto, 31);
+        unsigned long long old = 0;
+        if (lane == 0)
+            old = atomicAdd(&p.ctl->staged_pack, ((unsigned long long)count << 32) | (unsigned long long)(unsigned)all);
+        old = __shfl_sync(kFull, old, 0);
+        if (in) put_shared(p, it.x, ItemReq{p, sm, rbase, it.y}, r, (int)(old >> 32) + lane, (int)(unsigned)old + upto - pieces, pieces);
+    }
+    if (threadIdx.x == 0) sm.flag = 1;
+}
+
 template <bool kW, bool kStats, bool kSolo>
 __device__ __noinline__ void scan_fallback(const Params &p, const Mem<kSolo> m, Smem &sm, int t, long long rbase)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ns = min(sm.stage_n, kStageCap);
+    if (!kSolo && ns >= p.share_from) {
+        share_all(p, sm, ns, rbase);
+        return;
+    }
     for (int i = warp; i < ns; i += kWarps) {
         const int2 it = sm.fb.item[i];
         const int2 r = __ldg(p.ranges + it.x);
@@ -1199,7 +1239,7 @@ __device__ __noinline__ void scan_shared(const Params &p, const Mem<kSolo> m, in
     const int lane = threadIdx.x & 31;
     for (int s = (int)(blockIdx.x * kWarps + (threadIdx.x >> 5)); s < npieces; s += (int)(gridDim.x * kWarps)) {
         const int4 it = __ldcg(p.staged + __ldcg(p.piece_item + s));
-        const int deg = degree_of(it), pieces = (deg + kPiece - 1) / kPiece;
+        const int deg = degree_of(it), pieces = pieces_of(deg);
         const int b = it.y + (s - it.w) * kPiece, e = b + min(kPiece, it.z - b), v = it.x;
         const unsigned long long key = warp_max_u64(scan_rows<kW>(p, m, b, e, 0, 32 * kRows));
         if (lane != 0) continue;
@@ -2772,6 +2812,43 @@ mm_status device_limits(int dev, DeviceLimits *out)
     return MM_OK;
 }
 
+// Blocks that a graph can use: one for 512 vertices, and one a multiprocessor
+// where the lists longer than a window have the entries for it, as those lists
+// are what a whole round can come to.  (Random maximal matching, 8192 vertices of
+// degree 512: 16 blocks 2760 us, 128 blocks 1580, 256 blocks 2200: two blocks on a
+// multiprocessor, the one that waits at a barrier takes the other's L1.)
+constexpr long long kBlockEntries = 32768;
+int useful_blocks(const mm_graph *g, int sms)
+{
+    const long long by_vertices = ((long long)g->n + kThreads - 1) / kThreads;
+    const long long by_entries = std::min<long long>(sms, g->long_entries / kBlockEntries);
+    return (int)std::min<long long>(std::max({1ll, by_vertices, by_entries}), kMaxBlocks);
+}
+
+// One block matches a graph of at most kSoloVertices vertices while its long
+// lists are few: below these many entries the grid barriers cost more than one
+// multiprocessor's scans.  A random type's window is a list's first entries, which
+// are the same few vertices for many lists, so it scans many lists whole; a
+// weighted type's are the heaviest, and it scans few.  (One block against the
+// grid, random maximal: 1024 vertices of degree 64 132 us / 162, 128 255 / 333; 4096 of
+// degree 64 335 / 250, 512 6400 / 990.  Weighted: 4096 of degree 512 132 / 380, 4000 372 / 133.)
+constexpr long long kSoloEntries[2] = {1 << 17, 1 << 23};
+
+// Dense graphs: this many entries a vertex in long lists, on average.  Random
+// types: a block that finds more than kOwnEntries of them to scan whole in a
+// round leaves its lists to all blocks.  A round of such a graph is such scans,
+// vertex by vertex in list order from the same few ends, and the blocks' shares of it are
+// uneven.  (Random maximal, own scans / shared ones: 65536 vertices of degree 300 926
+// us / 1085, 512 4510 / 1850; 4096 of 512 1070 / 990, 4000 16060 / 5560.  Weighted types scan
+// too few lists to gain: 4096 of 4000 133 / 204.)
+// Finish phase: an active set of 1/d of the vertices falls apart once its vertices
+// have about one active neighbour each, so d is the average degree there; attempts
+// at 1/24 meet components that no warp can hold, and are called off one after
+// another (weighted maximal, 200 000 vertices of degree 512: 790 us / 206).
+constexpr long long kDenseEntries = 384;
+constexpr long long kOwnEntries = 4096;
+bool is_dense(const mm_graph *g) { return g->long_count > 0 && g->long_entries >= kDenseEntries * g->n; }
+
 // The state's arrays, allocated and cleared on the call's stream (each call
 // ends with its stream synchronised, so the next may come on another).
 mm_status alloc_state(mm_graph *g, cudaStream_t stream, PushState **out)
@@ -2788,8 +2865,13 @@ mm_status alloc_state(mm_graph *g, cudaStream_t stream, PushState **out)
     const size_t nstaged = (size_t)(g->long_count > 0 ? g->long_count : 1);
     const size_t nparts = g->long_count > 0 ? n : 1;
     // whatever the grid, its blocks' regions fit: (n / kChunk / blocks + 1) chunks each
-    const int most = (int)((n + kThreads - 1) / kThreads);
-    s->list_cap = n + (size_t)kChunk * ((size_t)(most < kMaxBlocks ? most : kMaxBlocks) + 1);
+    DeviceLimits dev;
+    const mm_status lim = device_limits(g->device, &dev);
+    if (lim != MM_OK) {
+        delete s;
+        return lim;
+    }
+    s->list_cap = n + (size_t)kChunk * ((size_t)useful_blocks(g, dev.sms) + 1);
     size_t at = 0;
     auto take = [&](size_t bytes) {
         const size_t o = at;
@@ -2899,7 +2981,8 @@ mm_status launch_match(const Call &c)
     p.tstamp = c.timing ? s->tstamp : nullptr;
     p.zero_parts = s->zero_next ? 1 : 0;
     const bool sparse = g->sum_degree <= (long long)kFinSparse * g->n;
-    p.fin_div = g->opt_fin_div < 0 ? 0 : (g->opt_fin_div == 0 ? (sparse && !kPolicy ? kFinDivSparse : kFinDiv) : max(g->opt_fin_div, 2));
+    const int fin_default = is_dense(g) ? (int)(g->sum_degree / g->n) : (sparse && !kPolicy ? kFinDivSparse : kFinDiv);
+    p.fin_div = g->opt_fin_div < 0 ? 0 : (g->opt_fin_div == 0 ? fin_default : max(g->opt_fin_div, 2));
     p.spin_limit = debug_spin_limit();
     p.skip_mark = debug_skip_mark();
     if (kPolicy) {
@@ -2913,11 +2996,14 @@ mm_status launch_match(const Call &c)
         p.fin_retire = pol->constant && !pol->trace ? 1 : 0;
     }
     // blocks: all that fit at once, or the tuned number per SM (never more), and
-    // no more than give every thread a vertex
+    // no more than the graph has work for
     const int mode = kPolicy ? 2 : (kStats ? 1 : 0);
     const int bps = g->opt_blocks_per_sm;
     int grid = bps > 0 ? min(dev.grid[kW][mode], bps * dev.sms) : dev.grid[kW][mode];
-    grid = g->n <= kSoloVertices ? 1 : min(grid, (g->n + kThreads - 1) / kThreads);
+    grid = g->n <= kSoloVertices && g->long_entries <= kSoloEntries[kW] ? 1 : min(grid, useful_blocks(g, dev.sms));
+    p.share_from = INT_MAX;
+    if (!kW && is_dense(g))
+        p.share_from = (int)(kOwnEntries / (g->long_entries / g->long_count)) + 1;
     const int chunks = (int)(((long long)g->n + kChunk - 1) / kChunk);
     p.region = (chunks + grid - 1) / grid * kChunk;
     p.turn_magic = grid > 1 ? (uint32_t)((1ull << 32) / (unsigned)grid + 1) : 0u;

@@ -451,12 +451,17 @@ __global__ void __launch_bounds__(256) k_long_merge(const long long *off, const 
 }
 
 // The coarse graph from the merged lists (8 lanes a list): ranges, entries,
-// and the symmetry sums of what they hold.
+// and the symmetry sums of what they hold; and the caller's copy of the coarse
+// map (null: none), which is written here, last, as it may be the match array
+// itself and a refused call leaves it as it is.
 __global__ void __launch_bounds__(256) k_emit(const int *tkey, const float *tw, const long long *off, const int *cnt,
                                               const long long *roff, int nc, int2 *ranges, int *out_nbr,
-                                              float *out_w, ContractState *st)
+                                              float *out_w, const int *cmap, int *map_out, int n, ContractState *st)
 {
     constexpr int G = 8;
+    if (map_out)
+        for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (long long)gridDim.x * blockDim.x)
+            map_out[v] = cmap[v];
     const int l = threadIdx.x & (G - 1);
     const long long stride = (long long)gridDim.x * blockDim.x / G;
     unsigned long long ss = 0, sw = 0;
@@ -556,8 +561,6 @@ mm_status contract(mm_graph *g, const int *d_match, mm_graph **coarse, int *d_cm
     if (e == cudaSuccess) e = sc.get(&roff, nv);
     if (e == cudaSuccess) e = sc.get(&cnt, nv);
     if (e == cudaSuccess) e = sc.get(&q, 3 * nv);
-    // the caller's map is written last: it may be the match array itself, and a
-    // refused call leaves it as it is (4 bytes a vertex copied: 2 us at 2^20)
     if (e == cudaSuccess) e = sc.get(&cmap, nv);
     if (e == cudaSuccess) e = cudaMemsetAsync(cs, 0, sizeof(ContractState), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(mem, 0xff, sizeof(int2) * nv, st);
@@ -660,11 +663,10 @@ mm_status contract(mm_graph *g, const int *d_match, mm_graph **coarse, int *d_cm
     if (e == cudaSuccess) e = cudaMemsetAsync(out_nbr + ne, 0, (pad - (size_t)ne) * sizeof(int), st);
     if (e == cudaSuccess) e = cudaMemsetAsync(out_w + ne, 0, (pad - (size_t)ne) * sizeof(float), st);
     if (e == cudaSuccess && nc > 0) {
-        k_emit<<<grid_for(nc * 8ll, 256, 148 * 8), 256, 0, st>>>(tkey, tw, off, cnt, roff, nc, cranges, out_nbr, out_w, cs);
+        k_emit<<<grid_for(nc * 8ll, 256, 148 * 8), 256, 0, st>>>(tkey, tw, off, cnt, roff, nc, cranges, out_nbr, out_w, cmap, d_cmap, n,
+                                                               cs);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess && d_cmap && n > 0)
-        e = cudaMemcpyAsync(d_cmap, cmap, sizeof(int) * (size_t)n, cudaMemcpyDeviceToDevice, st);
     if (e == cudaSuccess) e = read_back(&h, cs, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return cuda_fail(e, "mm_graph_contract");

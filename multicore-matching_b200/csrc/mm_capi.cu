@@ -510,6 +510,7 @@ cudaError_t upload_large(mm_graph *g, const int *ranges, const int *nbrs, const 
     }
     // both streams are drained on every path: buffers may be freed next
     const cudaError_t eks = cudaStreamSynchronize(ks), ecs = cudaStreamSynchronize(cs);
+    windows_settle(g, 0);
     if (e == cudaSuccess) e = eks != cudaSuccess ? eks : ecs;
     lanes_put(l);
     return e;

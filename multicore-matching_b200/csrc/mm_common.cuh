@@ -114,7 +114,8 @@ struct mm_graph {
     bool pwin_weights = false;        // d_pwin's second words hold weights (symmetric weighted path)
     int2 *win_build = nullptr;        // windows while being built (d_pwin once complete)
     int *win_big = nullptr;           // while being built: queued lists longer than a window chunk
-    void *win_tmp = nullptr;          // while being built: scratch of the window offsets
+    void *win_tmp[3] = {};            // while being built: scratch, the first of win_tmp_bytes
+    size_t win_tmp_bytes = 0;
 
     // push path: per-call state of the round kernel
     void *push_exec = nullptr;  // internal (mm::PushState *)
@@ -253,6 +254,7 @@ mm_status push_match_policy(mm_graph *g, int type, uint32_t barrier, const uint3
 mm_status windows_begin(mm_graph *g, cudaStream_t stream, cudaStream_t mem);
 mm_status windows_range(mm_graph *g, int va, int vb, cudaStream_t stream);
 mm_status windows_end(mm_graph *g, cudaStream_t stream, cudaStream_t mem);
+void windows_settle(mm_graph *g, cudaStream_t mem);
 void windows_discard(mm_graph *g);
 
 inline int max_rounds_of(int type)

@@ -3346,7 +3346,8 @@ mm_status windows_begin(mm_graph *g, cudaStream_t stream, cudaStream_t mem)
         dev_free(packed, mem);
         return cuda_fail(e, "window buffers");
     }
-    g->win_tmp = tmp;  // freed by windows_end
+    g->win_tmp[0] = tmp;
+    g->win_tmp_bytes = all;
     g->win_build = win;
     g->win_big = big;
     g->d_pwin_off = packed;
@@ -3374,16 +3375,31 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream, cudaStream_t mem)
         e = cudaMemcpyAsync(&nbig, big + n, sizeof(int), cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     }
-    WinCand *cand = nullptr;
-    void *tmp = nullptr;
+    // scratch: from what the offsets needed, which is free again, else allocated
+    // (after the last copy of an upload an allocation is waited for)
+    size_t at = 0;
+    int own = 1;
+    auto take = [&](void **out, size_t bytes) {
+        bytes = (bytes + 255) / 256 * 256;
+        if (at + bytes <= g->win_tmp_bytes) {
+            *out = (char *)g->win_tmp[0] + at;
+            at += bytes;
+            return cudaSuccess;
+        }
+        cudaError_t x = dev_alloc(out, bytes, mem);
+        if (x == cudaSuccess) g->win_tmp[own++] = *out;
+        if (x == cudaSuccess && mem != stream) x = cudaStreamSynchronize(mem);
+        return x;
+    };
     if (e == cudaSuccess && nbig > 0) {
         const size_t nb = (size_t)nbig + 1;
         size_t tmp_bytes = 0;
         long long nchunks = 0;
+        void *tmp = nullptr;
+        WinCand *cand = nullptr;
         e = cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, (long long *)nullptr, (long long *)nullptr, nbig + 1, stream);
         const size_t all = (2 * sizeof(long long) * nb + 255) / 256 * 256 + tmp_bytes;
-        if (e == cudaSuccess) e = dev_alloc(&tmp, all, mem);
-        if (e == cudaSuccess && mem != stream) e = cudaStreamSynchronize(mem);
+        if (e == cudaSuccess) e = take(&tmp, all);
         long long *ccnt = (long long *)tmp, *coff = ccnt + nb;
         if (e == cudaSuccess) e = cudaMemsetAsync(ccnt + nbig, 0, sizeof(long long), stream);
         if (e == cudaSuccess) {
@@ -3394,8 +3410,7 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream, cudaStream_t mem)
             e = cub::DeviceScan::ExclusiveSum((char *)tmp + (all - tmp_bytes), tmp_bytes, ccnt, coff, nbig + 1, stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(&nchunks, coff + nbig, sizeof nchunks, cudaMemcpyDeviceToHost, stream);
         if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        if (e == cudaSuccess) e = dev_alloc((void **)&cand, sizeof(WinCand) * 32 * (size_t)(nchunks > 0 ? nchunks : 1), mem);
-        if (e == cudaSuccess && mem != stream) e = cudaStreamSynchronize(mem);
+        if (e == cudaSuccess) e = take((void **)&cand, sizeof(WinCand) * 32 * (size_t)(nchunks > 0 ? nchunks : 1));
         if (e == cudaSuccess) {
             k_win_chunks<<<grid_for(nchunks * 32, 256, 148 * 16), 256, 0, stream>>>(g->d_ranges, g->d_nbrs, g->d_w, big,
                                                                                   nbig, coff, cand);
@@ -3407,20 +3422,12 @@ mm_status windows_end(mm_graph *g, cudaStream_t stream, cudaStream_t mem)
             e = cudaGetLastError();
         }
     }
-    if (mem != stream) {
-        const cudaError_t x = cudaStreamSynchronize(stream);
-        if (e == cudaSuccess) e = x;
-    }
-    dev_free(cand, mem);
-    dev_free(tmp, mem);
-    dev_free(g->win_tmp, mem);
-    dev_free(big, mem);
-    g->win_tmp = nullptr;
-    g->win_big = nullptr;
     if (e != cudaSuccess) {
+        if (mem != stream) cudaStreamSynchronize(stream);
         windows_discard(g);
         return cuda_fail(e, "preference windows");
     }
+    if (mem == stream) windows_settle(g, mem);
     g->d_pwin = win;
     g->pwin_weights = false;
     g->win_build = nullptr;
@@ -3452,18 +3459,27 @@ __global__ void __launch_bounds__(256) k_win_weights(const float *w, const int *
 
 }  // namespace
 
+// Free what a build needed besides the windows, on `mem` (after windows_end; on
+// another stream than the build's once that has been waited for).
+void windows_settle(mm_graph *g, cudaStream_t mem)
+{
+    for (void *&x : g->win_tmp) {
+        dev_free(x, mem);
+        x = nullptr;
+    }
+    dev_free(g->win_big, mem);
+    g->win_big = nullptr;
+}
+
 void windows_discard(mm_graph *g)
 {
-    dev_free(g->win_tmp, 0);
+    windows_settle(g, 0);
     dev_free(g->win_build, 0);
-    dev_free(g->win_big, 0);
-    g->win_tmp = nullptr;
     if (!g->d_pwin) {
         dev_free(g->d_pwin_off, 0);
         g->d_pwin_off = nullptr;
     }
     g->win_build = nullptr;
-    g->win_big = nullptr;
 }
 
 namespace {

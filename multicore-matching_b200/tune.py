@@ -1,15 +1,17 @@
 """Autotuner for the launch options of the matching kernels (mm_graph_tune).
 
 The kernels' shapes inside a launch (window length 32, window steps of 8
-entries, a lane per vertex refilled from 64-item chunks, 256-entry fallback
-segments, 512 threads) were fixed by measurement.  What varies with the workload is where the round
+entries, vertices dealt to the blocks in chunks of 64, 2048-entry pieces of the
+shared lists, 512 threads) were fixed by measurement.  What varies with the workload is where the round
 kernel hands over to the finish phase (the first round whose active set is at
 most 1/d of round 0's: too early and components are too large, so the attempt
 is called off and its scans are wasted; too late and the grid pays for more
-rounds) and how many blocks per SM the two kernels use.  This tuner times each
-(d, blocks per SM) pair on a workload with CUDA events (best of `repeats`),
+rounds) and how many blocks per SM the kernel uses.  This tuner times each
+(d, blocks per SM) pair on a workload with CUDA events (best of `repeats` in
+each of `sweeps` turns),
 checks that every candidate gives the same matching and round count (the
-options never change the result), and picks the fastest.
+options never change the result), and picks the fastest, if it is clearly
+faster than the library's own choice, the pair (0, 0).
 
     python multicore-matching_b200/tune.py [--classes rmat23,rgg20,grid512,er20,batch4096]
 
@@ -28,16 +30,20 @@ import numpy as np
 PKG = Path(__file__).resolve().parent
 ROOT = PKG.parent
 TUNED = PKG / "tuned.json"
-FIN_DIVS = (-1, 4, 6, 8, 10, 12, 16, 24)
-BLOCKS = (1, 2)
-# The pair that a choice has to beat.  (The library's own default, mm_graph_tune
-# value 0, is 24 or on sparse graphs 12, with 2 blocks.)
-DEFAULT = (12, 2)
+FIN_DIVS = (0, -1, 4, 6, 8, 10, 12, 16, 24, 32)
+BLOCKS = (0, 1, 2)
+# The pair that a choice has to beat: the library's own choices (mm_graph_tune
+# value 0), which go by the graph.
+DEFAULT = (0, 0)
+# What a table without that pair is compared with.
+EXPLICIT = (12, 2)
 
 
-def tune(mm, dg, type_, seeds, batch=False, fin_divs=FIN_DIVS, blocks=BLOCKS, repeats=5):
+def tune(mm, dg, type_, seeds, batch=False, fin_divs=FIN_DIVS, blocks=BLOCKS, repeats=5, sweeps=4):
     """Time every (finish divisor, blocks per SM) pair on one device graph.
-    Returns rows {finish_div, blocks_per_sm, ms, rounds, same} and the best row."""
+    The library's own choice goes as a pair; 0 of one option with a value of the
+    other is no candidate.  Returns rows {finish_div, blocks_per_sm, ms, rounds,
+    same} and the best row."""
     import torch
 
     out = torch.empty(max(dg.n, 1), dtype=torch.int32, device="cuda")
@@ -47,33 +53,37 @@ def tune(mm, dg, type_, seeds, batch=False, fin_divs=FIN_DIVS, blocks=BLOCKS, re
             return int(dg.match_batch(type_, seeds, out.data_ptr()).max())
         return dg.match_device(type_, seeds, out.data_ptr())
 
-    rows, ref = [], None
-    for d in fin_divs:
-        for b in blocks:
-            dg.tune(d, b)
+    pairs = [(d, b) for d in fin_divs for b in blocks if (d == 0) == (b == 0)]
+    rows = [{"finish_div": d, "blocks_per_sm": b, "ms": 1e30, "rounds": 0, "same": True} for d, b in pairs]
+    ref = None
+    # all pairs in turn, several times: a pair is not judged by the moment it was timed in
+    for _ in range(sweeps):
+        for row in rows:
+            dg.tune(row["finish_div"], row["blocks_per_sm"])
             run()  # warm-up
-            best = 1e30
             for _ in range(repeats):
                 e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
                 e0.record()
                 r = run()
                 e1.record()
                 torch.cuda.synchronize()
-                best = min(best, e0.elapsed_time(e1))
+                row["ms"] = min(row["ms"], e0.elapsed_time(e1))
             got = out.cpu().numpy()
             if ref is None:
                 ref = (got.copy(), r)
-            rows.append({"finish_div": d, "blocks_per_sm": b, "ms": best, "rounds": r,
-                         "same": bool(np.array_equal(got, ref[0]) and r == ref[1])})
+            row["rounds"] = r
+            row["same"] &= bool(np.array_equal(got, ref[0]) and r == ref[1])
     dg.tune(0, 0)
     return rows, min(rows, key=lambda x: x["ms"])
 
 
 def pick(rows, default=DEFAULT, margin=0.03):
     """The choice for a workload class from tune()'s rows: the fastest pair if it
-    beats the default pair by more than `margin` (a fraction of the
-    default's time), else the default.  Returns (choice row, default row, tuned?)."""
-    dflt = next(r for r in rows if (r["finish_div"], r["blocks_per_sm"]) == tuple(default))
+    beats the default pair (EXPLICIT in a table that lacks it) by more than
+    `margin` (a fraction of the default's time), else the default.  Returns
+    (choice row, default row, tuned?)."""
+    pairs = {(r["finish_div"], r["blocks_per_sm"]): r for r in rows}
+    dflt = pairs[tuple(default)] if tuple(default) in pairs else pairs[EXPLICIT]
     best = min(rows, key=lambda x: x["ms"])
     wins = best["ms"] < (1.0 - margin) * dflt["ms"]
     return (best if wins else dflt), dflt, wins
@@ -114,9 +124,10 @@ def main():
     lines = ["# Launch options tuned per workload class (one B200)", "",
              "Command: `python multicore-matching_b200/tune.py` (writes this file and "
              "`multicore-matching_b200/tuned.json`).", "",
-             "Device time of one matching (best of 5 CUDA-event timings), for each finish-phase divisor d "
+             "Device time of one matching (best of 20 CUDA-event timings, 5 in each of 4 turns over all pairs), for each finish-phase divisor d "
              "(the phase starts at the first round whose active set is at most 1/d of round 0's; -1: never) and "
-             "blocks per SM.  Every candidate gave the same matching and round count.", ""]
+             "blocks per SM; 0 and 0: the library's own choice, which the fastest has to beat by 3%.  "
+             "Every candidate gave the same matching and round count.", ""]
     for name in args.classes.split(","):
         make, type_ = workloads(mm)[name]
         g, off = make()
@@ -131,13 +142,13 @@ def main():
         tuned[name] = {"finish_div": choice["finish_div"], "blocks_per_sm": choice["blocks_per_sm"],
                        "ms": choice["ms"], "default_ms": dflt["ms"], "type": type_}
         lines += [f"## {name} (type {type_}, n = {g.n:,}, {g.nnz:,} entries)", "",
-                  "| d \\\\ blocks per SM | " + " | ".join(str(b) for b in BLOCKS) + " |",
+                  "| d \\ blocks per SM | " + " | ".join(str(b) for b in BLOCKS) + " |",
                   "|---|" + "---:|" * len(BLOCKS)]
         for d in FIN_DIVS:
-            cells = [f"{next(r['ms'] for r in rows if r['finish_div'] == d and r['blocks_per_sm'] == b):.3f}"
+            cells = [next((f"{r['ms']:.3f}" for r in rows if r["finish_div"] == d and r["blocks_per_sm"] == b), "")
                      for b in BLOCKS]
             lines.append(f"| {d} | " + " | ".join(cells) + " |")
-        lines += ["", f"Compared with d = {DEFAULT[0]}, {DEFAULT[1]} blocks per SM: {dflt['ms']:.3f} ms; fastest: "
+        lines += ["", f"The library's own choice: {dflt['ms']:.3f} ms; fastest: "
                       f"d = {best['finish_div']}, {best['blocks_per_sm']} blocks per SM, {best['ms']:.3f} ms; "
                       f"chosen: d = {choice['finish_div']}, {choice['blocks_per_sm']} "
                       f"({'tuned' if wins else 'kept: the fastest is within 3%'}).", ""]

@@ -22,16 +22,21 @@ launch that plays the rounds and, for the late ones, the finish phase.
             sum_r [24 |A_r| + 8 E_r] (weighted; 4 E_r random), over the step's
             CUDA-event time, against the measured HBM copy bandwidth; traffic =
             DRAM bytes of one matching's launches from an ncu capture recorded
-            in profiles/dram_traffic_<workload>.json.  A byte count by phase
-            (16-byte items and 1-byte colours: an upper figure for the kernel's
-            4-byte items and 2-bit colours), and per-round phase times (barrier
-            timestamps), are reported beside it.
+            in profiles/dram_traffic_<workload>.json.  Per-round phase times
+            (barrier timestamps) are reported beside it, and a nominal byte
+            count by phase (16-byte items, 1-byte colours: the same measure for
+            every kernel design; this kernel's items are 4 bytes and its colours
+            2 bits, so it is no rate of this kernel).
   cpu_baseline  the reference's own GraphMatchingTBBWeighted (same algorithm,
             src/matchtbb.cu:567-623) compiled from its sources into
             oracle/_ref, on all host cores, on the same graph and seeds; its
             match[] is also compared with the GPU result ("parity").  Beside it
             the same matcher on one thread, and the sequential matchers
             (types 4 and 5 for weighted workloads, type 0 for random ones).
+            Where that build is absent ("kind": "port") the repository's own
+            restatement of the rounds (oracle/mm_oracle.c) runs in its place:
+            then neither the time nor the comparison is with the reference,
+            and the line says so.
   forms     (N = 1) plain vs batched vs learned: the 4096-graph batch matched
             in one batched call and as 4096 separate calls, and the learned
             colouring's shipped policy on the 2^22 R-MAT and RGG multilevel
@@ -215,6 +220,21 @@ def dist_setup():
     return world, rank, local
 
 
+def runs_what(kind):
+    """What a "kind" of CPU baseline ran."""
+    return {"reference": "the reference's TBB matcher (src/matchtbb.cu), built from its sources",
+            "port": "the repository's own restatement of the rounds (oracle/mm_oracle.c): no build of the "
+                    "reference here"}[kind]
+
+
+def parity_line(cpu):
+    """The parity object: bit-exact against what ran, null against what did not."""
+    ref = cpu["kind"] == "reference"
+    return {"bit_exact_vs_reference": cpu["parity"] if ref else None,
+            "bit_exact_vs_restatement": None if ref else cpu["parity"],
+            "valid": cpu["valid"], "maximal": cpu["maximal"], "weight": cpu["gpu_weight"], "size": cpu["gpu_size"]}
+
+
 def run_reference(args, spec, workload):
     """--impl reference: the reference's own CPU matcher on this machine's cores."""
     world, rank, _ = dist_setup()
@@ -257,7 +277,8 @@ def run_reference(args, spec, workload):
             "scaling": "weak", "vs_baseline": None, "dtype": "f32+int32", "data": "synthetic",
             "config": {"workload": workload, "n": g.n, "nnz": g.nnz, "type": t, "barrier": BARRIER,
                        "srand": MATCH_SEED, "parallelism": "host cores", "l2": "n/a (CPU)"},
-            "cpu_baseline": {"value": value, "unit": "edges/s", "cores": cores, "kind": kind, "sample": sample,
+            "cpu_baseline": {"value": value, "unit": "edges/s", "cores": cores, "kind": kind, "runs": runs_what(kind),
+                             "sample": sample,
                              "matcher": f"GraphMatchingTBB{'Weighted' if ref_type == 11 else 'Random'}"
                                         f"{' (20-round cap)' if fixed else ''}"},
             "e2e": {"value": value, "unit": "edges/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
@@ -379,8 +400,7 @@ def compare_batch(mm, local, seeds):
     res["plain_calls"] = {"ms_device": ms_dev, "ms_wall": wall, "rounds_max": int(max(rs)), "rounds_sum": int(sum(rs)),
                           "calls": len(dgs), "same_result_as_batched": same}
     cpu = cpu_baseline(mm, u, t, got, "batch4096_weighted_maximal", batch)
-    res["parity_sample"] = {"graphs": len(batch["sample"]), "bit_exact_vs_reference": cpu["parity"],
-                            "valid": cpu["valid"], "maximal": cpu["maximal"]}
+    res["parity_sample"] = {"graphs": len(batch["sample"]), **parity_line(cpu)}
     return res
 
 
@@ -627,7 +647,8 @@ def main():
             "ms_to_maximal": ms, "edges_per_step": edges_all,
             "e2e": {"value": e2e_value, "unit": "edges/s", "ms_per_step": e2e, "h2d_bytes_per_step": h2d,
                     "d2h_bytes_per_step": d2h, "ms_create": e2e_split[0], "ms_first_match": e2e_split[1],
-                    "ms_destroy": e2e_split[2], **e2e_detail},
+                    "ms_destroy": e2e_split[2], "ms_steps": [round(x, 3) for x in e2e_ms],
+                    "ms_first_match_steps": [round(x[1], 3) for x in e2e_parts], **e2e_detail},
             "roofline": {"bound": "hbm",
                          "kernel": "one matching: k_match",
                          "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -637,11 +658,8 @@ def main():
                                           "round loop (A_r active vertices, E_r entries its request and respond "
                                           "loops inspect)",
                          "launches_per_step": launches,
-                         "design_bytes_per_step": kernel_bytes,
-                         "design_frac": kernel_bytes / (ms / 1e3) / 1e9 / peak,
-                         "phases": {k: {"ms": float(ms_k[:, c].sum()), "bytes": float(phase_bytes[k].sum()),
-                                        "gbs": float(phase_bytes[k].sum() / max(ms_k[:, c].sum(), 1e-9) / 1e6),
-                                        "frac": float(phase_bytes[k].sum() / max(ms_k[:, c].sum(), 1e-9) / 1e6 / peak)}
+                         "nominal_bytes_per_step": kernel_bytes,
+                         "phases": {k: {"ms": float(ms_k[:, c].sum()), "nominal_bytes": float(phase_bytes[k].sum())}
                                     for c, k in enumerate(("window", "fallback", "commit"))},
                          "per_round_work": {k: [int(x) for x in st[:nr, c]] for k, c in
                                             (("active", mm.ST_ACTIVE), ("blue", mm.ST_BLUE),
@@ -660,10 +678,9 @@ def main():
         if cpu is not None:
             line["cpu_baseline"] = {"value": cpu["value"], "unit": "edges/s", "cores": cpu["cores"],
                                     "kind": cpu["kind"], "sample": cpu["sample"], "ms": cpu["ms"],
-                                    "matcher": "GraphMatchingTBB (src/matchtbb.cu) on all host cores",
+                                    "matcher": runs_what(cpu["kind"]) + ", on all host cores",
                                     "tbb_1_thread": cpu["tbb_1_thread"], "sequential": cpu["sequential"]}
-            line["parity"] = {"bit_exact_vs_reference": cpu["parity"], "valid": cpu["valid"],
-                              "maximal": cpu["maximal"], "weight": cpu["gpu_weight"], "size": cpu["gpu_size"]}
+            line["parity"] = parity_line(cpu)
         if forms is not None:
             line["forms"] = forms
         print(json.dumps(line), flush=True)

@@ -34,11 +34,15 @@ _P, _I, _LL, _U = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_uin
 _cache: dict = {}
 
 
+class ReferenceNotBuilt(OSError):
+    """The reference's own build (oracle/_ref) is asked for and not there."""
+
+
 def _load(path: Path, sigs: dict) -> ctypes.CDLL:
     key = str(path)
     if key not in _cache:
         if not path.exists():
-            raise OSError(f"{path} is not built (make -C oracle)")
+            raise (ReferenceNotBuilt if path.parent.name == "_ref" else OSError)(f"{path} is not built (make -C oracle)")
         lib = ctypes.CDLL(key)
         for fn, (res, args) in sigs.items():
             f = getattr(lib, fn)

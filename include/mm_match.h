@@ -314,8 +314,9 @@ mm_status mm_matching_check(mm_graph *g, const int *d_match, long long counts[5]
  * entries map to carries their weights' sum, taken in double and rounded once
  * (unit weights when g has none).  *coarse is a new graph on the same device,
  * to be freed with mm_graph_destroy.  d_cmap (n ints on the device, or NULL)
- * receives each vertex's coarse id.  A match array whose value names no
- * partner that names it back gives MM_ERR_ARG.
+ * receives each vertex's coarse id; it may be d_match itself.  A match array
+ * whose value names no partner that names it back, or whose value a third
+ * vertex with entries holds too, gives MM_ERR_ARG, and d_cmap is left as it was.
  */
 mm_status mm_graph_contract(mm_graph *g, const int *d_match, mm_graph **coarse, int *d_cmap);
 

@@ -93,11 +93,10 @@ struct mm_graph {
     long long max_degree = 0;
     long long sum_degree = 0;
     bool scanned = false;          // degree classes below are valid
-    long long short_count = 0;     // vertices with at most 32 neighbour entries
-    long long long_count = 0;      // vertices with more
+    long long long_count = 0;      // vertices with more than 32 neighbour entries
     long long long_entries = 0;    // entries in those longer lists
     long long win_groups = 0;      // groups of 4 entries of all preference windows
-    long long win_even = 0;        // windows' lengths rounded up to even numbers, in all
+    long long win_even = 0;        // windows' lengths rounded up to even numbers, in all (limited, windows_begin)
 
     // device buffer for host-output calls (mm_match)
     int *d_out = nullptr;
@@ -221,9 +220,8 @@ __device__ __forceinline__ void block_add(unsigned long long *dst, unsigned long
 struct RangeInfo {
     unsigned long long sum_deg;
     unsigned long long max_deg;
-    unsigned long long short_count;   // lists of at most 32 entries
-    unsigned long long long_count;    // longer lists
-    unsigned long long long_entries;  // entries in longer lists
+    unsigned long long long_count;    // lists of more than 32 entries
+    unsigned long long long_entries;  // entries in those
     unsigned long long win_groups;    // preference windows: groups of 4 entries
     unsigned long long win_even;      // preference windows: lengths rounded up to even numbers
     int noncontig;                    // ranges do not tile [0, nnz) in vertex order

@@ -38,8 +38,9 @@
 //                  soon as its vertex is decided (scan_window).
 //   fallback       a list longer than its window with no red candidate in it
 //                  is scanned whole, by a warp or by the block that owns it;
-//                  the longest lists (hubs) go to a list of the round that all
-//                  blocks share, cut into 256-entry segments (scan_long).
+//                  the longest lists (hubs), and on dense graphs all of a block
+//                  that has many, go to a list of the round that all blocks
+//                  share, cut into 2048-entry pieces (scan_shared).
 //   finish phase   once the active set is small its components are tiny, and
 //                  the remaining rounds of each component are played on their
 //                  own, with two more grid barriers in all (finish_scan,
@@ -1016,7 +1017,8 @@ __device__ __forceinline__ void count_fallback(const Params &p, int t, int deg)
 // list of up to kWarpList entries, the whole block one of up to kBlockList
 // (a round trip of its 16 warps covers 2048 entries); a longer one (a hub,
 // which would keep one block busy while the others wait) goes to the shared
-// list, at the price of one more grid barrier in that round.
+// list, at the price of one more grid barrier in that round.  From p.share_from
+// lists on all of them go there (share_all; launch_match says when).
 constexpr int kWarpList = 512;
 constexpr int kBlockList = 32768;
 
@@ -1409,7 +1411,8 @@ __device__ __forceinline__ void commit_phase(const Params &p, const Mem<kSolo> &
 // state by round 3).  A vertex's future depends only on the colours and choices
 // of the active vertices it can reach: matched neighbours never change, and
 // where every entry has a reverse entry no active vertex has an unmatchable
-// neighbour (a vertex became unmatchable because every neighbour was matched).  So each component
+// neighbour (a vertex became unmatchable because every neighbour was matched;
+// the colours would not tell one).  So each component
 // can play all its remaining rounds on its own, with the same seeds, and the
 // grid needs no further barrier.
 //
@@ -2168,10 +2171,10 @@ __global__ void __launch_bounds__(kThreads, kSolo ? 1 : 2) k_match(const __grid_
 // ---------------------------------------------------------------------------
 // Preparation: degree classes and reverse proposal keys.
 
-// (block sums: an atomic a warp and word had all warps queue on seven words)
+// (block sums: an atomic a warp and word had all warps queue on six words)
 __global__ void __launch_bounds__(256) k_scan_ranges(const int2 *ranges, int n, long long nnz, RangeInfo *info, long long *deg_out)
 {
-    unsigned long long sum = 0, nshort = 0, nlong = 0, elong = 0, groups = 0, even = 0;
+    unsigned long long sum = 0, nlong = 0, elong = 0, groups = 0, even = 0;
     int mx = 0, nc = 0, bad = 0;
     for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const int2 r = ranges[v];
@@ -2185,8 +2188,6 @@ __global__ void __launch_bounds__(256) k_scan_ranges(const int2 *ranges, int n, 
         if (d > kWin) {
             nlong += 1;
             elong += (unsigned long long)d;
-        } else {
-            nshort += 1;
         }
         groups += (wl + 3) >> 2;
         even += (wl + 1) & ~1;
@@ -2197,7 +2198,6 @@ __global__ void __launch_bounds__(256) k_scan_ranges(const int2 *ranges, int n, 
         if (v == n - 1 && (long long)r.y != nnz) nc = 1;
     }
     block_add(&info->sum_deg, sum);
-    block_add(&info->short_count, nshort);
     block_add(&info->long_count, nlong);
     block_add(&info->long_entries, elong);
     block_add(&info->win_groups, groups);
@@ -2286,7 +2286,8 @@ __global__ void k_pair_groups(const unsigned long long *keys, const int *vals, l
 // which the reference's gwRequest would prefer them: candidates (weight > -1)
 // by weight, then earlier position; entries whose weight can never be picked
 // after them, flagged by bit 31 of the position.  A vertex's window starts at
-// pwin_off[v], an even slot (pairs are read as one 16-byte load).
+// group pwin_off[v] (bit 31 apart), four entries a group, read by one 32-byte
+// load; the last group is filled up.
 __device__ __forceinline__ unsigned long long pref_key(float w, int j)
 {
     return w > -1.0f ? (((unsigned long long)weight_order(w) << 32) | (uint32_t)~j) : (unsigned long long)(uint32_t)~j;
@@ -3287,7 +3288,6 @@ void apply_ranges(mm_graph *g, const RangeInfo &info)
 {
     g->sum_degree = (long long)info.sum_deg;
     g->max_degree = (long long)info.max_deg;
-    g->short_count = (long long)info.short_count;
     g->long_count = (long long)info.long_count;
     g->long_entries = (long long)info.long_entries;
     g->win_groups = (long long)info.win_groups;
@@ -3309,6 +3309,8 @@ void apply_ranges(mm_graph *g, const RangeInfo &info)
 mm_status windows_begin(mm_graph *g, cudaStream_t stream, cudaStream_t mem)
 {
     const int n = g->n;
+    // the limit is in entries, window by window rounded up to even; fewer than that
+    // many have group numbers of 30 bits, where pwin_off has 31
     if (g->win_even >= (1ll << 31)) {
         set_error("push: more than 2^31 - 1 preference-window slots are not supported");
         return MM_ERR_UNSUPPORTED;

@@ -2336,24 +2336,29 @@ constexpr int kWinChunk = 4096;   // lists longer than this are split into chunk
 
 // Merge entries [from, to) of a list into its sorted best 32 (k, nb, j): a row
 // can change them only if one of its keys beats the 32nd.
-__device__ __forceinline__ void win_merge_range(const int *nbrs, const float *w, Pos from, Pos to, int lane,
+__device__ __forceinline__ void win_merge_range(const int *nbrs, const float *w, int from, int to, int lane,
                                                 unsigned long long &k, int &nb, int &j)
 {
-    for (Pos base = from; base < to; base += 32 * kWinRows) {
+    // offsets within the range (at most kWinChunk entries): positions past its end
+    // may not fit an int, and unsigned ones took the last chunk of an upload 60 us longer
+    const int len = to - from;
+    nbrs += from;
+    w += from;
+    for (int base = 0; base < len; base += 32 * kWinRows) {
         float wr[kWinRows];
 #pragma unroll
         for (int q = 0; q < kWinRows; ++q) {
-            const Pos jj = base + q * 32 + lane;
-            wr[q] = jj < to ? __ldg(w + jj) : 0.0f;
+            const int i = base + q * 32 + lane;
+            wr[q] = i < len ? __ldg(w + i) : 0.0f;
         }
 #pragma unroll
         for (int q = 0; q < kWinRows; ++q) {
-            const Pos jj = base + q * 32 + lane;
-            if (base + q * 32 >= to) break;
+            const int i = base + q * 32 + lane;
+            if (base + q * 32 >= len) break;
             const unsigned long long thr = __shfl_sync(kFull, k, 31);
-            unsigned long long k2 = jj < to ? pref_key(wr[q], (int)jj) : 0ull;
+            unsigned long long k2 = i < len ? pref_key(wr[q], from + i) : 0ull;
             if (!__any_sync(kFull, k2 > thr)) continue;
-            int nb2 = jj < to ? __ldg(nbrs + jj) : 0, j2 = (int)jj;
+            int nb2 = i < len ? __ldg(nbrs + i) : 0, j2 = i < len ? from + i : 0;
             warp_sort_desc(k2, nb2, j2, lane);
             // the larger of T[l] and R[31 - l] is a bitonic sequence holding
             // the best 32 of both; sort it descending
@@ -2383,7 +2388,7 @@ __device__ __forceinline__ void win_top32(const int *nbrs, const float *w, int f
         k = pref_key(__ldg(w + j), j);
     }
     warp_sort_desc(k, nb, j, lane);
-    if (to - from > 32) win_merge_range(nbrs, w, (Pos)from + 32, (Pos)to, lane, k, nb, j);
+    if (to - from > 32) win_merge_range(nbrs, w, from + 32, to, lane, k, nb, j);
 }
 
 __device__ __forceinline__ void win_store(int2 *pwin, long long off, int deg, int lane, unsigned long long k, int nb, int j)

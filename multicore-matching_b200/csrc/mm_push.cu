@@ -2840,18 +2840,23 @@ int useful_blocks(const mm_graph *g, int sms)
 // degree 64 335 / 250, 512 6400 / 990.  Weighted: 4096 of degree 512 132 / 380, 4000 372 / 133.)
 constexpr long long kSoloEntries[2] = {1 << 17, 1 << 23};
 
-// Dense graphs: this many entries a vertex in long lists, on average.  Random
-// types: a block that finds more than kOwnEntries of them to scan whole in a
-// round leaves its lists to all blocks.  A round of such a graph is such scans,
-// vertex by vertex in list order from the same few ends, and the blocks' shares of it are
-// uneven.  (Random maximal, own scans / shared ones: 65536 vertices of degree 300 926
-// us / 1085, 512 4510 / 1850; 4096 of 512 1070 / 990, 4000 16060 / 5560.  Weighted types scan
-// too few lists to gain: 4096 of 4000 133 / 204.)
+// Dense graphs: this many entries a vertex in long lists, on average.
+//
+// Random types, where those lists come near the length from which the whole block
+// scans one (kSharedLength on average): a block that finds more than kOwnEntries
+// of them to scan whole in a round leaves its lists to all blocks.  A round of such
+// a graph is such scans, in list order from the same few ends, one after another
+// in a block and uneven over the blocks.  (Random, own scans / shared ones: 65536
+// vertices of degree 400, 20 rounds, 464 us / 546; of 512, maximal, 4510 / 1850; 4096 of 512
+// 1070 / 990, of 4000 16060 / 5560.  Weighted types scan too few lists to gain: 4096 of
+// 4000 133 / 204.)
+//
 // Finish phase: an active set of 1/d of the vertices falls apart once its vertices
 // have about one active neighbour each, so d is the average degree there; attempts
 // at 1/24 meet components that no warp can hold, and are called off one after
 // another (weighted maximal, 200 000 vertices of degree 512: 790 us / 206).
 constexpr long long kDenseEntries = 384;
+constexpr long long kSharedLength = 448;
 constexpr long long kOwnEntries = 4096;
 bool is_dense(const mm_graph *g) { return g->long_count > 0 && g->long_entries >= kDenseEntries * g->n; }
 
@@ -3008,7 +3013,7 @@ mm_status launch_match(const Call &c)
     int grid = bps > 0 ? min(dev.grid[kW][mode], bps * dev.sms) : dev.grid[kW][mode];
     grid = g->n <= kSoloVertices && g->long_entries <= kSoloEntries[kW] ? 1 : min(grid, useful_blocks(g, dev.sms));
     p.share_from = INT_MAX;
-    if (!kW && is_dense(g))
+    if (!kW && is_dense(g) && g->long_entries >= kSharedLength * g->long_count)
         p.share_from = (int)(kOwnEntries / (g->long_entries / g->long_count)) + 1;
     const int chunks = (int)(((long long)g->n + kChunk - 1) / kChunk);
     p.region = (chunks + grid - 1) / grid * kChunk;

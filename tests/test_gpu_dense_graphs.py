@@ -58,8 +58,10 @@ def compare(mm, orc, g, seed, types, blocks=0, scanned=0):
 
 
 # 2^17 entries in long lists (one block or several, random types) lie between 362 and
-# 363 vertices that all list each other; 384 entries a vertex (shared lists) at 385
-@pytest.mark.parametrize("n,deg", [(64, 63), (362, 361), (363, 362), (384, 383), (385, 384), (386, 385), (700, 699),
+# 363 vertices that all list each other; 384 entries a vertex (dense) at 385, lists of
+# 448 on average (left to all blocks) at 449
+@pytest.mark.parametrize("n,deg", [(64, 63), (362, 361), (363, 362), (384, 383), (385, 384), (386, 385), (448, 447),
+                                   (449, 448), (700, 699),
                                    (1023, 500), (2049, 64), (4095, 130), (4097, 130), (4096, 700), (9001, 450)])
 def test_dense(mm, orc, n, deg):
     compare(mm, orc, random_dense(n, deg, n), n, mm.TYPES)

@@ -1,4 +1,4 @@
-"""The checker's two layers are told apart when one is missing: the reference's own
+"""The oracle's two layers are told apart when one is missing: the reference's own
 build may be absent (its tests skip), the restatement may not."""
 from __future__ import annotations
 
